@@ -211,3 +211,65 @@ def tolerance(case):
         # result move; 2e-3 in the INT8 path where the mean that is taken off the keys moves by a bit of bf16
         return {"rel": 4e-3 if case["precision"] == "nvfp4" else 8e-3}
     return "exact"                                             # quantisers and the rotary embedding: bit for bit
+
+
+def _nvfp4(x):
+    """x [rows, columns] to NVFP4 and back, in 64 bits: one scale for the tensor, an e4m3 scale per block of 16, e2m1 values."""
+    rows, cols = x.shape
+    x = torch.nn.functional.pad(x.float(), (0, -cols % 16)).reshape(rows, -1, 16)
+    amax = x.abs().amax(dim=2, keepdim=True)
+    scale = amax.max() / 2688.0
+    block = ((1.0 / scale) * (amax * (1.0 / 6.0))).clamp(max=448.0).to(torch.float8_e4m3fn).float()
+    a = torch.where(block > 0, x * ((1.0 / scale) * (1.0 / block)), torch.zeros_like(x))
+    code = torch.zeros(a.shape, dtype=torch.int64, device=a.device)
+    for at, up in ((0.25, False), (0.75, True), (1.25, False), (1.75, True), (2.5, False), (3.5, True), (5.0, False)):
+        code += (a.abs() >= at) if up else (a.abs() > at)         # a tie goes to the value of even mantissa
+    value = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0], dtype=torch.float64, device=a.device)[code]
+    return (value * a.sign() * block.double() * scale.double()).reshape(rows, -1)[:, :cols], scale
+
+
+def exact(case, seed):
+    """What `run` gives for these inputs, in 64 bits; None in the place of packed bytes and their block scales."""
+    g = _generator(seed)
+    kind = case["kind"]
+    if kind == "linear":
+        m, n, k = case["m"], case["n"], case["k"]
+        if case["out"] == "nvfp4":
+            return None, None, prepare(case, seed)["out_scale"].double()
+        weight = torch.randn((n, k), generator=g, device="cuda", dtype=torch.bfloat16) * 0.02
+        x = _activations((m, k), g)
+        y = _nvfp4(x)[0] @ _nvfp4(weight)[0].T
+        if case["bias"]:
+            y += torch.randn((n,), generator=g, device="cuda", dtype=torch.bfloat16)
+        return y
+    if kind == "quantize":
+        x = _activations((case["rows"], case["cols"]), g)
+        if case["precision"] == "nvfp4":
+            return None, None, x.abs().max().double() / 2688.0
+        scale = x.abs().amax(dim=1).double() / (448.0 if case["precision"] == "fp8e4m3" else 127.0)
+        return None, torch.nn.functional.pad(scale, (0, -case["rows"] % 16))
+    if kind == "attention":
+        # four-bit probabilities are further than a tenth from the exact ones; the longest take too long in 64 bits
+        if case["precision"] == "nvfp4" or case["b"] * case["h"] * case["nq"] * case["nkv"] > 2e10:
+            return None
+        state = prepare(case, seed)
+        q, k, v = (state[name] if case["layout"] == "BHND" else state[name].transpose(1, 2) for name in ("q", "k", "v"))
+        out = torch.empty(q.shape, dtype=torch.float64, device="cuda")
+        step = max(1, 2 ** 28 // case["nkv"])
+        for b in range(case["b"]):
+            for h in range(case["h"]):
+                kt, vt = k[b, h].double().T, v[b, h].double()
+                for i in range(0, case["nq"], step):
+                    out[b, h, i:i + step] = torch.softmax(q[b, h, i:i + step].double() @ kt / math.sqrt(case["d"]), dim=1) @ vt
+        return out if case["layout"] == "BHND" else out.transpose(1, 2)
+    state = prepare(case, seed)
+    x, freqs = state["x"], state["freqs"]
+    f, h, w = case["f"], case["h"], case["w"]
+    c = case["d"] // 2
+    parts = freqs.split([c - 2 * (c // 3), c // 3, c // 3], dim=1)
+    turn = torch.cat([parts[0][:f].view(f, 1, 1, -1).expand(f, h, w, -1), parts[1][:h].view(1, h, 1, -1).expand(f, h, w, -1),
+                      parts[2][:w].view(1, 1, w, -1).expand(f, h, w, -1)], dim=-1).reshape(f * h * w, 1, c)
+    out = torch.empty(x.shape, dtype=torch.float64, device="cuda")
+    for b in range(case["b"]):
+        out[b] = torch.view_as_real(torch.view_as_complex(x[b].double().reshape(f * h * w, case["heads"], c, 2)) * turn).flatten(2)
+    return out
