@@ -1,7 +1,10 @@
 // Arithmetic helpers shared by the attention kernels (mha_nvfp4.cu, mha_int8_fp8.cu).
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include "sm100_ptx.cuh"
 
 namespace ac4k {
 
@@ -42,23 +45,57 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
       : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
-// 2^x for two x (<= 8) on the FMA and integer pipes, for the share of the exponentials that the ex2 pipe (16 per clock per
-// SM, the bottleneck of the attention kernels) is relieved of: x = n + f with n = round(x), |f| <= 1/2; 2^f from a quartic with
-// relative error < 2.8e-6 (near-minimax on [-1/2, 1/2]; a cubic's 7.5e-5 moved enough roundings of the 4-bit P to show
-// against the CPU restatement on short sequences); n is added to the exponent field.  x is clamped at -125, where
-// the result (2.4e-38) is far below anything that survives the 4-bit quantisation of P or moves the row sum.
-__device__ __forceinline__ float2 exp2_fma_pipe(float2 x) {
-  constexpr float kMagic = 12582912.0f;        // 1.5 * 2^23: x + kMagic holds round(x) in its low mantissa bits
-  x.x = fmaxf(x.x, -125.0f);
-  x.y = fmaxf(x.y, -125.0f);
-  const float2 fi = fadd2(x, make_float2(kMagic, kMagic));
-  const float2 n = fadd2(fi, make_float2(-kMagic, -kMagic));
-  const float2 f = ffma2(n, make_float2(-1.0f, -1.0f), x);
-  float2 q = ffma2(f, make_float2(0.00957010128f, 0.00957010128f), make_float2(0.0559178591f, 0.0559178591f));
-  q = ffma2(q, f, make_float2(0.240247443f, 0.240247443f));
-  q = ffma2(q, f, make_float2(0.693121791f, 0.693121791f));
-  q = ffma2(q, f, make_float2(0.999999285f, 0.999999285f));
-  return make_float2(__int_as_float(__float_as_int(q.x) + (__float_as_int(fi.x) << 23)),
-                     __int_as_float(__float_as_int(q.y) + (__float_as_int(fi.y) << 23)));
+// 128 columns of this warp's 16 rows of O in tensor memory (16x256b shape) times a[r], r = 0, 1 the thread's two rows
+__device__ __forceinline__ void mha_rescale(uint32_t t_o, const float (&a)[2]) {
+  uint32_t ro[64];
+  ptx::tmem_ld_16x256b_x16(t_o, ro);
+  ptx::tmem_ld_wait();
+  ptx::tmem_pin(ro);
+#pragma unroll
+  for (int i = 0; i < 64; i += 2) {
+    const float f = a[(i >> 1) & 1];
+    const float2 v = fmul2(make_float2(__uint_as_float(ro[i]), __uint_as_float(ro[i + 1])), make_float2(f, f));
+    ro[i] = __float_as_uint(v.x);
+    ro[i + 1] = __float_as_uint(v.y);
+  }
+  ptx::tmem_st_16x256b_x16(t_o, ro);
+  ptx::tmem_st_wait();
+}
+// Query tiles per CTA.  A pair of tiles shares the K and V tiles and fills each other's waits (a pair's key tile takes 1.4 times
+// a single one's), but a launch of few CTAs leaves SMs idle: one tile per CTA where that ends sooner, counted in waves.
+inline int mha_query_tiles(int64_t q_blocks, int64_t heads, int sms) {
+  const int64_t pairs = heads * ((q_blocks + 1) / 2), singles = heads * q_blocks;
+  const int64_t wave2 = 14 * ((pairs + sms - 1) / sms), wave1 = 10 * ((singles + sms - 1) / sms);
+  return q_blocks > 1 && wave1 >= wave2 ? 2 : 1;
+}
+// O may be stored four columns at a time: its rows are contiguous and start on 8-byte boundaries
+__device__ __forceinline__ bool mha_rows_vec4(const void *O, int64_t o_b, int64_t o_h, int64_t o_n, int64_t o_d, int Dv) {
+  return o_d == 1 && (Dv & 3) == 0 && ((o_b | o_h | o_n) & 3) == 0 && (reinterpret_cast<uintptr_t>(O) & 7) == 0;
+}
+// One row's 32 columns c0 .. c0 + 31 of O from the four threads that hold it in the 16x256b shape: o[2 i + e] is column
+// c0 + 8 i + 2 t4 + e.  Vector form: neighbouring threads swap words, so that the even one has four columns of the first
+// eight of every sixteen and the odd one of the second, and the four of them write whole 32-byte sectors.
+__device__ __forceinline__ void mha_store_row(__nv_bfloat16 *dst, const float (&o)[8], int c0, int t4, int Dv, int64_t o_d, bool vec,
+                                              bool live) {
+  if (vec) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 h2 = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t *>(&h2);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, (t4 & 1) ? w[i] : w[i + 1], 1);
+      const int col = c0 + 8 * i + ((t4 & 1) ? 6 + 2 * t4 : 2 * t4);
+      if (live && col < Dv) *reinterpret_cast<uint2 *>(dst + col) = (t4 & 1) ? make_uint2(got, w[i + 1]) : make_uint2(w[i], got);
+    }
+  } else if (live) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int col = c0 + 8 * (i >> 1) + 2 * t4 + (i & 1);
+      if (col < Dv) dst[(int64_t)col * o_d] = __float2bfloat16_rn(o[i]);
+    }
+  }
 }
 }  // namespace ac4k

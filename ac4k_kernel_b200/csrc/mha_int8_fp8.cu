@@ -9,12 +9,21 @@
 // One difference: the reference accumulates the P V of one key tile in fp16 (its MMA's accumulator) before adding it
 // to the fp32 O; tcgen05's kind::f8f6f4 accumulates in fp32 throughout.
 //
-// Structure as in mha_nvfp4.cu: one CTA per (batch, head, 256 query rows) with two groups of four softmax warps (one
-// 128-row query tile each), one 128-column score buffer in tensor memory used by the groups in turn, key tiles of 128,
-// S by four tcgen05.mma kind::i8 (M 128, N 128, K 32) into int32 columns, P V by four kind::f8f6f4 from the P tile the
-// group wrote to shared memory (128-byte-swizzled K-major, in the key order of the reference's V quantiser: every 16
-// keys viewed as [2, 4, 2] and transposed to [4, 2, 2]).  The exponentials bound the kernel (16 ex2 per clock per SM);
-// a quarter of the exponentials run as a polynomial on the FMA pipe.  Because of the 7.5 offset a row's maximum rarely moves after the first tiles, so O is rarely rescaled.
+// Structure as in mha_nvfp4.cu: one CTA per (batch, head, one or two query tiles of 128 rows) with a group of eight softmax
+// warps per query tile (16 rows each, four threads to a row: the 16x256b tensor-memory shape, so a row's maximum takes two
+// shuffles), one 128-column score buffer in tensor memory used by the groups in turn, key tiles of 128, S by four
+// tcgen05.mma kind::i8 (M 128, N 128, K 32) into int32 columns, P V by four kind::f8f6f4 with P as the A operand in tensor
+// memory: the four keys of every 16 that a thread holds are four neighbouring positions in the key order of the reference's V
+// quantiser (every 16 keys viewed as [2, 4, 2] and transposed to [4, 2, 2]), i.e. one 32-bit column, and one 16x128b store
+// writes a warp's tile.  Tensor memory: S 128 + O 2 x 128 + P 2 groups x 2 buffers x 32 = 512 columns.
+//
+// What bounds it: issue slots and dependency latencies of the softmax warps (ncu, before P moved to tensor memory and the
+// polynomial exponentials to the ex2 pipe: 63 % of the issue slots, ex2 pipe 46 %, ALU 47 %, tensor memory 48 %, tensor pipe 30 %).
+// [1, 16384, 16, 128], kernel alone: 1 667 us with four warps per group, a row per thread; 1 566 with eight; 1 475 with O rescaled
+// behind the exponentials instead of in front of them; 1 406 with an eighth of the exponentials as a polynomial on the FMA
+// pipe instead of a quarter; 1 344 with P in tensor memory; 1 332 with every exponential on the ex2 pipe (the polynomial
+// relieved that pipe when it was the bottleneck, and costs thirteen issue slots a pair).  A score buffer per group (tensor
+// memory had room before P moved in) gained nothing.  [1, 75600, 40, 128], the whole call: 83.7 -> 74.9 ms (1.56 PFLOP/s).
 //
 // Supported: head dimensions up to 128 for Q/K (rows padded to a multiple of 16 bytes by the quantiser) and up to 128
 // for V; Q and K quantised in blocks of 16, 32, 64 or 128 tokens (the reference's defaults: 64 and 128).
@@ -25,13 +34,17 @@ namespace ac4k {
 using namespace ptx;
 
 namespace mha8 {
-static constexpr int BQ = 128, BKV = 128, D = 128;
-static constexpr int kThreads = 320;              // producer, MMA issuer, 2 x 4 softmax warps
+static constexpr int BQ = 128, BKV = 128;
+static constexpr int kThreads = 640;              // producer, MMA issuer, two idle warps, 2 x 8 softmax warps
+static constexpr int kGroupWarps = 8, kFirstSoftmaxWarp = 4;
+// 96 registers per thread at launch (five warps per scheduler); the first four warps hand 64 x 32 each of theirs over
+static constexpr int kControlRegs = 32, kSoftmaxRegs = 112;
+static_assert(kThreads * 96 >= 128 * kControlRegs + 2 * 32 * kGroupWarps * kSoftmaxRegs, "registers of the block at launch");
 static constexpr int TILE_BYTES = 128 * 128;      // 128 rows of 128 bytes (Q, K, V^T and P tiles alike)
-static constexpr int KV_STAGES = 3;
+static constexpr int KV_STAGES = 4;
 static constexpr int STAGE_BYTES = 2 * TILE_BYTES;
-static constexpr int SMEM_BYTES = 2 * TILE_BYTES + 4 * TILE_BYTES + KV_STAGES * STAGE_BYTES + 1024 + 256;
-static constexpr int S_COL = 0, O_COL = 128 /* + 128 * group */;
+static constexpr int SMEM_BYTES = 2 * TILE_BYTES + KV_STAGES * STAGE_BYTES + 1024 + 256;
+static constexpr int S_COL = 0, O_COL = 128 /* + 128 * group */, P_COL = 384 /* + 64 * group + 32 * buffer */;
 static constexpr int TMEM_COLS = 512;
 static constexpr float kExpOffset = 7.5f;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory overflow");
@@ -43,6 +56,7 @@ struct Mha8Args {
   int64_t o_b, o_h, o_n, o_d;           // strides of O in elements
   int B, H, Nq, Nkv, Dv;
   int q_blocks, kv_tiles;               // ceil(Nq / 128), ceil(Nkv / 128)
+  int q_tiles;                          // 128-row query tiles of a CTA, 1 or 2
   int q_block, q_nblk, v_pad;           // tokens per Q scale, Q scales per head, align16(Dv)
   int k_shift, k_nblk;                  // log2 of the tokens per K scale (4 .. 7), K scales per head
   float sm_scale_log2;                  // sm_scale * log2(e)
@@ -65,11 +79,12 @@ __device__ __forceinline__ void mma_i8_if(uint32_t pred, uint32_t d_tmem, uint64
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(pred)
       : "memory");
 }
-__device__ __forceinline__ void mma_f8_if(uint32_t pred, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// A in tensor memory: lane = row, four consecutive elements of K in each 32-bit column
+__device__ __forceinline__ void mma_f8_ts_if(uint32_t pred, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
-      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(pred)
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p;\n}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(pred)
       : "memory");
 }
 // four fp32 -> four e4m3 bytes, a in the lowest
@@ -89,25 +104,27 @@ mha_int8_fp8_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sQ = smem_base;                     // [group]
-  const uint32_t sP = sQ + 2 * TILE_BYTES;           // [group][buffer]
-  const uint32_t sKV = sP + 4 * TILE_BYTES;          // per stage: K | V^T
+  const uint32_t sKV = sQ + 2 * TILE_BYTES;          // per stage: K | V^T
   const uint32_t bars = sKV + KV_STAGES * STAGE_BYTES;
   const uint32_t q_full = bars, kv_full = bars + 8, kv_empty = kv_full + 8 * KV_STAGES;
   const uint32_t s_full = kv_empty + 8 * KV_STAGES;  // [group]
   const uint32_t s_free = s_full + 16;
-  const uint32_t p_full = s_free + 8;                // [group]
-  const uint32_t o_done = p_full + 16;               // [group][P buffer]
+  // [group][P buffer].  (One barrier per group would do for the buffers, but not for the warps: nothing keeps a warp that is
+  // done with tile j from finishing tile j + 1 before the slowest one has finished tile j, and its second arrival would
+  // complete the phase of tile j without that warp's rows.)
+  const uint32_t p_full = s_free + 8;
+  const uint32_t o_done = p_full + 32;               // [group][P buffer]
   const uint32_t tmem_slot = o_done + 32;
   uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int qt = blockIdx.x * p.q_tiles, h = blockIdx.y, b = blockIdx.z;
   const int64_t bh = (int64_t)b * p.H + h;
-  const int q_row0 = (int)(bh * p.Nq) + qt * 2 * BQ; // row of Q in the [B*H*Nq, row bytes] matrix
+  const int q_row0 = (int)(bh * p.Nq) + qt * BQ; // row of Q in the [B*H*Nq, row bytes] matrix
   const int k_row0 = (int)(bh * p.Nkv);
   const int v_row0 = (int)(bh * p.Dv);               // V^T rows of this head; rows past Dv belong to the next head and are not stored
   const int n_tiles = p.kv_tiles;
-  const bool both = 2 * qt + 1 < p.q_blocks;         // group B has query rows
+  const bool both = p.q_tiles == 2 && qt + 1 < p.q_blocks;         // group B has query rows
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -117,11 +134,12 @@ mha_int8_fp8_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_
     }
     for (int g = 0; g < 2; ++g) {
       mbar_init(s_full + 8 * g, 1);
-      mbar_init(p_full + 8 * g, 4);     // the group's four warps have written P
+      mbar_init(p_full + 16 * g, kGroupWarps);     // the group's warps have written P
+      mbar_init(p_full + 16 * g + 8, kGroupWarps);
       mbar_init(o_done + 16 * g, 1);
       mbar_init(o_done + 16 * g + 8, 1);
     }
-    mbar_init(s_free, 4);               // the four warps of the group whose turn it is hold S in registers
+    mbar_init(s_free, kGroupWarps);     // the warps of the group whose turn it is hold S in registers
     fence_barrier_init();
     prefetch_tmap(&tma_q);
     prefetch_tmap(&tma_k);
@@ -138,7 +156,9 @@ mha_int8_fp8_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_
   grid_launch_dependents();
   grid_dependency_wait();
 
-  if (warp == 0) {
+  if (warp < kFirstSoftmaxWarp) {
+   reg_dec<kControlRegs>();
+   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     const uint32_t el = elect_one();
     const int ng = both ? 2 : 1;
@@ -155,7 +175,7 @@ mha_int8_fp8_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_
       tma_load_2d_if(el, st + TILE_BYTES, &tma_v, j * BKV, v_row0, fb);    // keys past the row's end read as 0
     }
     if (!ok && el) atomicExch(p.status, kStatusTimeoutProducer);
-  } else if (warp == 1) {
+   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     const uint32_t el = elect_one();
     constexpr uint32_t idesc_s = make_idesc_i8(128, 128);
@@ -175,11 +195,11 @@ mha_int8_fp8_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_
     // O_g (+)= P V: four K = 32 steps over the tile's keys
     auto issue_pv = [&](int g, int j) {
       const uint32_t st = sKV + (j % KV_STAGES) * STAGE_BYTES;
-      const uint64_t pdesc = make_smem_desc(sP + (2 * g + (j & 1)) * TILE_BYTES, 16, 1024, kSwizzle128B);
+      const uint32_t t_p = tmem_base + P_COL + 64 * g + 32 * (j & 1);       // 32 bytes of K: 8 columns
       const uint64_t vdesc = make_smem_desc(st + TILE_BYTES, 16, 1024, kSwizzle128B);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        mma_f8_if(el, tmem_base + O_COL + 128 * g, pdesc + 2 * i, vdesc + 2 * i, idesc_o, (j > 0 || i > 0) ? 1u : 0u);
+        mma_f8_ts_if(el, tmem_base + O_COL + 128 * g, t_p + 8 * i, vdesc + 2 * i, idesc_o, (j > 0 || i > 0) ? 1u : 0u);
       tc_commit_if(el, o_done + 16 * g + 8 * (j & 1));
     };
     // The score buffer is used in the order A(0), B(0), A(1), B(1), ... (A(0), A(1), ... without group B); use n of the
@@ -204,7 +224,7 @@ mha_int8_fp8_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_
       if (ok) ok = issue_s_when_free(0, 1);
     }
     for (int j = 0; j < n_tiles && ok; ++j) {
-      ok = warp_all(mbar_wait(p_full, j & 1, p.wait_ns));
+      ok = warp_all(mbar_wait(p_full + 8 * (j & 1), (j >> 1) & 1, p.wait_ns));
       if (!ok) break;
       tc_fence_after();
       issue_pv(0, j);
@@ -213,7 +233,7 @@ mha_int8_fp8_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_
           ok = issue_s_when_free(1, j + 1);
           if (!ok) break;
         }
-        ok = warp_all(mbar_wait(p_full + 8, j & 1, p.wait_ns));
+        ok = warp_all(mbar_wait(p_full + 16 + 8 * (j & 1), (j >> 1) & 1, p.wait_ns));
         if (!ok) break;
         tc_fence_after();
         issue_pv(1, j);
@@ -227,164 +247,152 @@ mha_int8_fp8_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_
       }
     }
     if (!ok && el) atomicExch(p.status, kStatusTimeoutMma);
-  } else if (warp < 6 || both) {
+   }
+  } else if (warp < kFirstSoftmaxWarp + kGroupWarps || both) {
+    reg_inc<kSoftmaxRegs>();
     // ------------------------------------------------------------------ softmax, correction, epilogue
-    const int g = (warp - 2) >> 2;            // group: query tile A or B
-    const int q = warp & 3;                   // tensor-memory lane quarter (warps 2-5 and 6-9 -> 2, 3, 0, 1)
-    const int row_l = q * 32 + lane;          // query row inside the tile = tensor-memory lane
-    const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+    const int g = (warp - kFirstSoftmaxWarp) / kGroupWarps;   // group: query tile A or B
+    const int q = warp & 3;                   // tensor-memory lane quarter of the warp
+    const int half = (warp >> 2) & 1;         // its 16 lanes of the quarter
+    const int t4 = lane & 3;
+    const int row_l = q * 32 + half * 16 + (lane >> 2);          // query rows of the thread inside the tile: row_l, row_l + 8
+    const uint32_t lane_addr = (uint32_t)(q * 32 + half * 16) << 16;
     const uint32_t t_s = tmem_base + lane_addr + S_COL, t_o = tmem_base + lane_addr + O_COL + 128 * g;
-    const int n_row = (2 * qt + g) * BQ + row_l;                 // query row in the head
+    const int n_row = (qt + g) * BQ + row_l;                 // first query row in the head
     // scores in units of log2: s = int32 * c_row * k_scale[tile]
-    const float c_row = p.sm_scale_log2 * __ldg(p.q_sf + bh * p.q_nblk + min(n_row / p.q_block, p.q_nblk - 1));
+    float c_row[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      c_row[r] = p.sm_scale_log2 * __ldg(p.q_sf + bh * p.q_nblk + min((n_row + 8 * r) / p.q_block, p.q_nblk - 1));
     const float *k_sf = p.k_sf + bh * p.k_nblk;
-    const uint32_t p_row0 = sP + 2 * g * TILE_BYTES + row_l * 128;
-    const uint32_t p_xor = (uint32_t)(row_l & 7) << 4;           // 128-byte swizzle: 16-byte chunk ^ (row % 8)
-    const uint32_t my_s_full = s_full + 8 * g, my_p_full = p_full + 8 * g, my_o_done = o_done + 16 * g;
-    float m = -INFINITY, l = 0.0f;
+    const uint32_t t_p = tmem_base + lane_addr + P_COL + 64 * g;
+    const uint32_t my_s_full = s_full + 8 * g, my_p_full = p_full + 16 * g, my_o_done = o_done + 16 * g;
+    float m[2] = {-INFINITY, -INFINITY};
+    float2 l[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};     // this thread's share of the row sums
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
+      // (the scales are asked for before the wait for S)
+      float kc[K128 ? 1 : 8];
+#pragma unroll
+      for (int bk = 0; bk < (K128 ? 1 : 8); ++bk)
+        kc[bk] = __ldg(k_sf + (K128 ? j : min((j * BKV + 16 * bk) >> p.k_shift, p.k_nblk - 1)));
       ok = warp_all(mbar_wait(my_s_full, j & 1, p.wait_ns));
       if (!ok) break;
       tc_fence_after();
-      uint32_t lo[64], hi[64];               // scores of keys 0-63 and 64-127 (int32)
-      tmem_ld_32x32b_x64(t_s, lo);
-      tmem_ld_32x32b_x64(t_s + 64, hi);
+      uint32_t s[64];                        // s[4 i + 2 r + e]: score of row r of the thread and key 8 i + 2 t4 + e
+      tmem_ld_16x256b_x16(t_s, s);
       tmem_ld_wait();
-      tmem_pin(lo);
-      tmem_pin(hi);
-#define AC4K_S(i) ((i) < 64 ? lo[(i) & 63] : hi[(i) & 63])
+      tmem_pin(s);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(s_free);
       // to fp32 in place (|S| <= 127 * 127 * 128 < 2^24: exact)
 #pragma unroll
-      for (int i = 0; i < 64; ++i) {
-        lo[i] = __float_as_uint(__int2float_rn((int)lo[i]));
-        hi[i] = __float_as_uint(__int2float_rn((int)hi[i]));
-      }
-      const int ncols = p.Nkv - j * BKV;                 // keys of this tile that exist (>= 128 except in the last tile)
+      for (int i = 0; i < 64; ++i) s[i] = __float_as_uint(__int2float_rn((int)s[i]));
+      const int ncols = p.Nkv - j * BKV - 2 * t4;        // keys of this tile that exist, counted from the thread's first
       if (ncols < BKV) {
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          if (i >= ncols) lo[i] = 0xff800000u;           // -inf: out of the maximum, probability 0
-          if (64 + i >= ncols) hi[i] = 0xff800000u;
-        }
+        for (int i = 0; i < 64; ++i)
+          if (8 * (i >> 2) + (i & 1) >= ncols) s[i] = 0xff800000u;     // -inf: out of the maximum, probability 0
       }
       // Scale of every 16 keys of the tile (K is quantised in blocks of 16 to 128 tokens: one to eight scales per tile).
       // c >= 0 (scales and sm_scale are; the host rejects a negative sm_scale); the floor keeps -inf * c = -inf.
-      float c16[8];
-      if (K128) {
-        const float c = fmaxf(c_row * __ldg(k_sf + j), 1.17549435e-38f);
+      auto cs = [&](int r, int bk) { return fmaxf(c_row[r] * kc[K128 ? 0 : bk], 1.17549435e-38f); };
+      float m_new[2];
 #pragma unroll
-        for (int bk = 0; bk < 8; ++bk) c16[bk] = c;
-      } else {
+      for (int r = 0; r < 2; ++r) {
+        float v = -INFINITY;
 #pragma unroll
-        for (int bk = 0; bk < 8; ++bk)
-          c16[bk] = fmaxf(c_row * __ldg(k_sf + min((j * BKV + 16 * bk) >> p.k_shift, p.k_nblk - 1)), 1.17549435e-38f);
-      }
-      float bs[8];
-#pragma unroll
-      for (int bk = 0; bk < 8; ++bk) {
-        float v[16];
-#pragma unroll
-        for (int n = 0; n < 16; ++n) v[n] = __uint_as_float(AC4K_S(16 * bk + n));
-        const float t0 = max3(v[0], v[1], v[2]), t1 = max3(v[3], v[4], v[5]), t2 = max3(v[6], v[7], v[8]);
-        const float t3 = max3(v[9], v[10], v[11]), t4 = max3(v[12], v[13], v[14]);
-        bs[bk] = fmaxf(max3(t0, t1, t2), max3(t3, t4, v[15]));
-        if (!K128) bs[bk] *= c16[bk];
-      }
-      float rowmax = fmaxf(max3(bs[0], bs[1], bs[2]), max3(bs[3], bs[4], max3(bs[5], bs[6], bs[7])));
-      if (K128) rowmax *= c16[0];
-      const float m_new = fmaxf(m, rowmax - kExpOffset);
-      if (j > 0 && __any_sync(0xffffffffu, m_new != m)) {
-        // a maximum of this warp's rows moved: O is rescaled, once the previous tile's P V is complete
-        ok = warp_all(mbar_wait(my_o_done + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, p.wait_ns));
-        if (!ok) break;
-        tc_fence_after();
-        const float a = ex2_approx(m - m_new);
-#pragma unroll 1
-        for (int cc = 0; cc < 8; ++cc) {
-          uint32_t ro[16];
-          tmem_ld_32x32b_x16(t_o + 16 * cc, ro);
-          tmem_ld_wait();
-          tmem_pin(ro);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) ro[i] = __float_as_uint(__uint_as_float(ro[i]) * a);
-          tmem_st_32x32b_x16(t_o + 16 * cc, ro);
+        for (int i = 0; i < 16; i += 2) {    // 16 keys: four of them in this thread
+          const float a = __uint_as_float(s[4 * i + 2 * r]), b2 = __uint_as_float(s[4 * i + 2 * r + 1]);
+          const float c = __uint_as_float(s[4 * i + 4 + 2 * r]), d = __uint_as_float(s[4 * i + 5 + 2 * r]);
+          if (K128) v = max3(max3(v, a, b2), c, d);
+          else v = fmaxf(v, fmaxf(max3(a, b2, c), d) * cs(r, i >> 1));
         }
-        tmem_st_wait();
-        l *= a;
+        if (K128) v *= cs(r, 0);
+        v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+        v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+        m_new[r] = fmaxf(m[r], v - kExpOffset);
       }
-      m = m_new;
+      const bool moved = j > 0 && __any_sync(0xffffffffu, m_new[0] != m[0] || m_new[1] != m[1]);     // warp-uniform
+      float a[2] = {1.0f, 1.0f};
+      if (moved) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          a[r] = ex2_approx(m[r] - m_new[r]);
+          l[r] = fmul2(l[r], make_float2(a[r], a[r]));
+        }
+      }
+      m[0] = m_new[0];
+      m[1] = m_new[1];
       // This tile's P buffer was last read by the P V of two tiles ago, which was issued before this tile's S: s_full
       // of this tile implies that it is complete (the tensor pipe completes MMAs and commits in issue order).
       // Probabilities, row sum, P to e4m3 in the key order of the reference's V quantiser: position n of every 16 keys
-      // holds key ((n / 2) % 2 * 4 + n / 4) * 2 + n % 2.
-      const uint32_t p_row = p_row0 + (j & 1) * TILE_BYTES;
-      float2 lsum[4];
-      const float2 negm2 = make_float2(-m, -m);
+      // holds key ((n / 2) % 2 * 4 + n / 4) * 2 + n % 2, so the four keys of a thread are positions 4 t4 .. 4 t4 + 3.
+      uint32_t pw[16];
 #pragma unroll
-      for (int gg = 0; gg < 4; ++gg) {          // 32 keys = two 16-byte chunks of P
-        float2 pr[16];
-        lsum[gg] = make_float2(0.0f, 0.0f);
+      for (int bk = 0; bk < 8; ++bk) {
 #pragma unroll
-        for (int n = 0; n < 32; n += 2) {
-          const int n16 = n & 15;
-          const int i = 32 * gg + (n & 16) + (((n16 >> 1) & 1) * 4 + (n16 >> 2)) * 2;     // keys held at positions n, n + 1
-          const float cc = c16[2 * gg + (n >> 4)];
-          const float2 e = ffma2(make_float2(__uint_as_float(AC4K_S(i)), __uint_as_float(AC4K_S(i + 1))), make_float2(cc, cc), negm2);
-          // every fourth pair on the FMA pipe, the others on the ex2 pipe
-          pr[n >> 1] = ((n >> 1) & 3) == 1 ? exp2_fma_pipe(e) : make_float2(ex2_approx(e.x), ex2_approx(e.y));
-          lsum[gg] = fadd2(lsum[gg], pr[n >> 1]);
-        }
-#pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-          const float2 *q8 = pr + 8 * ch;
-          st_shared_v4u(p_row + (((uint32_t)(2 * gg + ch) << 4) ^ p_xor), e4m3x4(q8[0].x, q8[0].y, q8[1].x, q8[1].y),
-                        e4m3x4(q8[2].x, q8[2].y, q8[3].x, q8[3].y), e4m3x4(q8[4].x, q8[4].y, q8[5].x, q8[5].y),
-                        e4m3x4(q8[6].x, q8[6].y, q8[7].x, q8[7].y));
+        for (int r = 0; r < 2; ++r) {
+          const float c = cs(r, bk);
+          const float2 cc = make_float2(c, c), negm2 = make_float2(-m[r], -m[r]);
+          const int i = 8 * bk + 2 * r;
+          const float2 e0 = ffma2(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), cc, negm2);
+          const float2 e1 = ffma2(make_float2(__uint_as_float(s[i + 4]), __uint_as_float(s[i + 5])), cc, negm2);
+          const float2 p0 = make_float2(ex2_approx(e0.x), ex2_approx(e0.y));
+          const float2 p1 = make_float2(ex2_approx(e1.x), ex2_approx(e1.y));
+          l[r] = fadd2(l[r], fadd2(p0, p1));
+          pw[2 * bk + r] = e4m3x4(p0.x, p0.y, p1.x, p1.y);
         }
       }
-#undef AC4K_S
-      l += (lsum[0].x + lsum[0].y) + (lsum[1].x + lsum[1].y) + ((lsum[2].x + lsum[2].y) + (lsum[3].x + lsum[3].y));
-      fence_proxy_async_smem();
+      tmem_st_16x128b_x8(t_p + 32 * (j & 1), pw);      // 16 bytes of 4 keys each per column: 32 columns
+      if (moved) {
+        // A maximum of this warp's rows moved: O is rescaled, once the previous tile's P V is complete.  Here, behind the
+        // exponentials, that has long happened and the scores' registers are free for O (in front of them the wait for
+        // P V and four loads and stores of 32 columns one after the other cost 13 % of the kernel at 16 384 keys).
+        ok = warp_all(mbar_wait(my_o_done + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, p.wait_ns));
+        if (!ok) break;
+        tc_fence_after();
+        mha_rescale(t_o, a);                   // (ends with the wait for this warp's stores)
+      } else {
+        tmem_st_wait();
+      }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(my_p_full);
+      if (lane == 0) mbar_arrive(my_p_full + 8 * (j & 1));
     }
     if (ok) ok = warp_all(mbar_wait(my_o_done + 8 * ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, p.wait_ns));
     if (!ok) {
       if (lane == 0) atomicExch(p.status, kStatusTimeoutEpilogue);
     } else {
       tc_fence_after();
-      const float inv_l = 1.0f / l;
+      float inv_l[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        float v = l[r].x + l[r].y;
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        inv_l[r] = 1.0f / v;
+      }
       const float *v_sf = p.v_sf + bh * p.v_pad;
-      __nv_bfloat16 *dst = static_cast<__nv_bfloat16 *>(p.O) + (int64_t)b * p.o_b + (int64_t)h * p.o_h + (int64_t)n_row * p.o_n;
+      __nv_bfloat16 *dst0 = static_cast<__nv_bfloat16 *>(p.O) + (int64_t)b * p.o_b + (int64_t)h * p.o_h + (int64_t)n_row * p.o_n;
+      const bool vec = mha_rows_vec4(p.O, p.o_b, p.o_h, p.o_n, p.o_d, p.Dv);
+#pragma unroll 1
+      for (int c0 = 0; c0 < p.Dv; c0 += 32) {
+        uint32_t ro[16];
+        tmem_ld_16x256b_x4(t_o + c0, ro);
+        tmem_ld_wait();
+        tmem_pin(ro);
+        const int col = c0 + 2 * t4;
+        float vs[8];                         // (rows of v_sf are padded to 16 channels; O's columns past Dv are not stored)
 #pragma unroll
-      for (int cc = 0; cc < 4; ++cc) {
-        uint32_t ro[32];
-        tmem_ld_32x32b_x32_sync(t_o + 32 * cc, ro);
-        if (n_row < p.Nq) {
-          float o[32];
+        for (int i = 0; i < 8; ++i) vs[i] = __ldg(v_sf + min(col + 8 * (i >> 1) + (i & 1), p.Dv - 1));
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = 32 * cc + i < p.Dv ? __uint_as_float(ro[i]) * (inv_l * __ldg(v_sf + 32 * cc + i)) : 0.0f;
-          if (p.o_d == 1 && p.Dv == D && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
+        for (int r = 0; r < 2; ++r) {
+          float o[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint32_t w[4];
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const __nv_bfloat162 h2 = __floats2bfloat162_rn(o[8 * i + 2 * k], o[8 * i + 2 * k + 1]);
-                w[k] = *reinterpret_cast<const uint32_t *>(&h2);
-              }
-              reinterpret_cast<uint4 *>(dst + 32 * cc)[i] = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (32 * cc + i < p.Dv) dst[(int64_t)(32 * cc + i) * p.o_d] = __float2bfloat16_rn(o[i]);
-          }
+          for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(ro[4 * (i >> 1) + 2 * r + (i & 1)]) * (inv_l[r] * vs[i]);
+          mha_store_row(dst0 + 8 * r * p.o_n, o, c0, t4, p.Dv, p.o_d, vec, n_row + 8 * r < p.Nq);
         }
       }
     }
@@ -444,6 +452,7 @@ extern "C" int ac4k_mha_int8_x_fp8_fwd(void *O, const int64_t o_stride[4], const
   a.k_shift = k_block == 16 ? 4 : (k_block == 32 ? 5 : (k_block == 64 ? 6 : 7));
   a.k_nblk = (int)ceil_div(Nkv, k_block);
   a.sm_scale_log2 = sm_scale * 1.4426950408889634f;
+  a.q_tiles = mha_query_tiles(a.q_blocks, H * B, di.sms);
   a.status = status;
   a.wait_ns = kWaitTimeoutNs;
   static PerDevice<int> attr_set;
@@ -456,7 +465,7 @@ extern "C" int ac4k_mha_int8_x_fp8_fwd(void *O, const int64_t o_stride[4], const
       }))
     return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((a.q_blocks + 1) / 2), (unsigned)H, (unsigned)B);
+  cfg.gridDim = dim3((unsigned)ceil_div(a.q_blocks, a.q_tiles), (unsigned)H, (unsigned)B);
   cfg.blockDim = dim3(mha8::kThreads);
   cfg.dynamicSmemBytes = mha8::SMEM_BYTES;
   cfg.stream = stream;

@@ -6,8 +6,8 @@
 // P = exp(S - max) re-quantised per 16 keys with the fixed global scale 1 / (6 * 448)
 // (mha_nvfp4.cu:246-319), O accumulated in fp32 and divided by the row sum at the end.
 //
-// One CTA per (batch, head, 256 query rows), one CTA per SM; the CTA holds two query tiles of 128 rows (groups A, B)
-// and walks the keys in tiles of 128:
+// One CTA per (batch, head, one or two query tiles of 128 rows), one CTA per SM; a group (A, B) of warps per query tile walks the
+// keys in tiles of 128:
 //   warp 0     TMA producer: both Q tiles once; per key tile K [128 keys x D], V^T [D x 128 keys] and their scale
 //              chunks, four stages, shared by the two groups
 //   warp 1     MMA issuer: S = Q K^T (tcgen05.mma kind::mxf4nvf4, M = 128 queries, N = 128 keys, K = D) into ONE
@@ -15,17 +15,20 @@
 //              registers at once, which frees the buffer for the other group's MMA); once a group has written P:
 //              O_g (+)= P V (M = 128, N = D, K = 128 keys).  Block scales go from shared to tensor memory with
 //              tcgen05.cp in front of the MMAs.
-//   warps 2-5  softmax of group A, warps 6-9 of group B: thread = query row.  One pass over the 128 scores in
-//              registers: running maximum, O rescaled in tensor memory when a maximum of the warp moved, ex2.approx,
-//              row sum, P quantised to e2m1 + e4m3 block scales (fixed global scale 1 / 2688) and written into shared
-//              memory in the layouts the tensor core reads (64-byte-swizzled K-major operand, 32 x 16-byte scale
-//              chunks); at the end O * gV / (2688 * row sum) is stored as bf16.
-// The softmax bounds this kernel: an SM retires 16 ex2 per clock, 1024 cycles for 128 x 128 scores against 330 for the
-// four-bit MMAs.  One warp per scheduler keeps the ex2 pipe ~65 % busy, two keep it full, but two groups that run in
-// step also sit together in the phases that do not use it (wait for S, copy it out, maxima, rescale, fences, barrier
-// traffic: ~800 cycles per key tile).  Sharing one score buffer keeps the groups a few hundred cycles apart (group B's S
-// is issued when group A has copied its own out); an explicit token that made a group wait until the other was half way
-// through its exponentials helped earlier versions of this kernel and costs 3 % in this one.
+//   warp 2     re-orders block scales that come in the reference's layout
+//   warps 4-11 softmax of group A, warps 12-19 of group B: a warp has 16 query rows, four threads to a row (the 16x256b
+//              tensor-memory shape: a row's maximum takes two shuffles, a block's one).  One pass over a thread's 2 x 32
+//              scores in registers: running maximum, ex2.approx, row sum, P quantised to e2m1 + e4m3 block scales (fixed
+//              global scale 1 / 2688) and written into shared memory in the layouts the tensor core reads
+//              (64-byte-swizzled K-major operand, 32 x 16-byte scale chunks), then O rescaled in tensor memory if a
+//              maximum of the warp moved; at the end O * gV / (2688 * row sum) is stored as bf16.
+// The softmax warps bound this kernel: their issue slots and dependency latencies, with the ex2 pipe (16 per clock and SM)
+// next.  [1, 16384, 16, 128], kernel alone: 1 688 us with four warps per group, a row per thread, and O rescaled before the
+// exponentials (a wait for the previous P V and a chain of small loads and stores); 1 728 with eight warps per group, 1 654 with
+// the rescale behind the exponentials (a quarter of the exponentials as a polynomial on the FMA pipe); 1 640 with an eighth of
+// them there, 1 579 with none: the polynomial costs thirteen issue slots a pair, and those bound the kernel now.
+// Sharing one score buffer keeps the groups a few hundred cycles apart (group B's S is issued when group A has copied its own
+// out), so that one group's waits, maxima and fences run under the other's exponentials.
 // Tensor memory: S 128 + O_A 128 + O_B 128 + scales 40 columns of 512.
 //
 // Supported: head dimensions up to 128 (padded to 64 or 128 by the quantiser); block scales in the tiled layout
@@ -40,7 +43,11 @@ using namespace ptx;
 
 namespace mha {
 static constexpr int BQ = 128, BKV = 128, D = 128;
-static constexpr int kThreads = 352;              // producer, MMA issuer, 2 x 4 softmax warps, scale re-order warp
+static constexpr int kThreads = 640;              // producer, MMA issuer, scale re-order warp, an idle one, 2 x 8 softmax warps
+static constexpr int kGroupWarps = 8, kFirstSoftmaxWarp = 4;
+// 96 registers per thread at launch (five warps per scheduler); the first four warps hand 32 x 64 each of theirs over
+static constexpr int kControlRegs = 32, kSoftmaxRegs = 112;
+static_assert(kThreads * 96 >= 128 * kControlRegs + 2 * 32 * kGroupWarps * kSoftmaxRegs, "registers of the block at launch");
 static constexpr int Q_BYTES = BQ * 64;           // 128 rows x 128 e2m1, 64-byte rows
 static constexpr int K_BYTES = BKV * 64;          // 128 keys x 128 e2m1
 static constexpr int V_BYTES = D * 64;            // 128 head-dimension rows x 128 keys
@@ -66,6 +73,7 @@ struct MhaArgs {
   int64_t o_b, o_h, o_n, o_d;           // strides of O in elements
   int B, H, Nq, Nkv, Dv;
   int q_blocks, kv_tiles;               // ceil(Nq / 128), ceil(Nkv / 128): 128-row blocks of Q and of the keys
+  int q_tiles;                          // 128-row query tiles of a CTA, 1 or 2
   int v_k64;                            // align64(Nkv) / 64: K = 64 steps of V^T that exist
   int nkq;                              // align64(Dqk) / 64: K = 64 steps of the head dimension (1 or 2)
   int q_pad, k_pad, v_pad;              // align16 of Nq, Nkv, Dv: scale rows per K step in the reference's layout
@@ -98,9 +106,6 @@ __device__ __forceinline__ uint32_t e4m3x2_round_trip(float a, float b, float &f
   fb = __high2float(hh);
   return pk;
 }
-__device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared::cta.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
 __device__ __forceinline__ void tmem_st_32x32b_x32_f(uint32_t taddr, const float (&v)[32]) {
   uint32_t u[32];
 #pragma unroll
@@ -128,19 +133,22 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
   const uint32_t q_full = bars, kv_full = bars + 8, kv_empty = kv_full + 8 * KV_STAGES;
   const uint32_t s_full = kv_empty + 8 * KV_STAGES;  // [group]
   const uint32_t s_free = s_full + 16;
-  const uint32_t p_full = s_free + 8;                // [group]
-  const uint32_t o_done = p_full + 16;               // [group][P buffer]
+  // [group][P buffer].  (One barrier per group would do for the buffers, but not for the warps: nothing keeps a warp that is
+  // done with tile j from finishing tile j + 1 before the slowest one has finished tile j, and its second arrival would
+  // complete the phase of tile j without that warp's rows.)
+  const uint32_t p_full = s_free + 8;
+  const uint32_t o_done = p_full + 32;               // [group][P buffer]
   const uint32_t tmem_slot = o_done + 32;
   uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int qt = blockIdx.x * p.q_tiles, h = blockIdx.y, b = blockIdx.z;
   const int64_t bh = (int64_t)b * p.H + h;
-  const int q_row0 = (int)(bh * p.Nq) + qt * 2 * BQ; // row of Q in the [B*H*Nq, 64-byte] matrix
+  const int q_row0 = (int)(bh * p.Nq) + qt * BQ; // row of Q in the [B*H*Nq, 64-byte] matrix
   const int k_row0 = (int)(bh * p.Nkv);
   const int v_row0 = (int)(bh * p.Dv);               // V^T rows of this head; rows past Dv belong to the next head and are not stored
   const int n_tiles = p.kv_tiles;
-  const bool both = 2 * qt + 1 < p.q_blocks;         // group B has query rows
+  const bool both = p.q_tiles == 2 && qt + 1 < p.q_blocks;         // group B has query rows
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, SF_TILED ? 1 : 2);
@@ -150,11 +158,12 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
     }
     for (int g = 0; g < 2; ++g) {
       mbar_init(s_full + 8 * g, 1);
-      mbar_init(p_full + 8 * g, 4);     // the group's four warps have written P and its scales
+      mbar_init(p_full + 16 * g, kGroupWarps);     // the group's warps have written P
+      mbar_init(p_full + 16 * g + 8, kGroupWarps);
       mbar_init(o_done + 16 * g, 1);
       mbar_init(o_done + 16 * g + 8, 1);
     }
-    mbar_init(s_free, 4);               // the four warps of the group whose turn it is hold S in registers
+    mbar_init(s_free, kGroupWarps);     // the warps of the group whose turn it is hold S in registers
     fence_barrier_init();
     prefetch_tmap(&tma_q);
     prefetch_tmap(&tma_k);
@@ -179,7 +188,9 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
   grid_launch_dependents();
   grid_dependency_wait();
 
-  if (warp == 0) {
+  if (warp < kFirstSoftmaxWarp) {
+   reg_dec<kControlRegs>();
+   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     const uint32_t el = elect_one();
     const int ng = both ? 2 : 1;
@@ -187,7 +198,7 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
     for (int g = 0; g < ng; ++g) {
       tma_load_2d_if(el, sQ + g * Q_BYTES, &tma_q, 0, q_row0 + g * BQ, q_full);
       if (SF_TILED)
-        bulk_load_1d_if(el, sSFQ + g * SF_BYTES, p.sfq + ((bh * p.q_blocks + 2 * qt + g) * p.nkq) * 512, p.nkq * 512, q_full);
+        bulk_load_1d_if(el, sSFQ + g * SF_BYTES, p.sfq + ((bh * p.q_blocks + qt + g) * p.nkq) * 512, p.nkq * 512, q_full);
     }
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
@@ -206,7 +217,7 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       }
     }
     if (!ok && el) atomicExch(p.status, kStatusTimeoutProducer);
-  } else if (warp == 1) {
+   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     const uint32_t el = elect_one();
     constexpr uint32_t idesc = make_idesc_mxf4nvf4(128, 128);
@@ -271,7 +282,7 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
     }
     for (int j = 0; j < n_tiles && ok; ++j) {
       if (el) AC4K_TRM(1, j, 0);
-      ok = warp_all(mbar_wait(p_full, j & 1, p.wait_ns));
+      ok = warp_all(mbar_wait(p_full + 8 * (j & 1), (j >> 1) & 1, p.wait_ns));
       if (!ok) break;
       tc_fence_after();
       issue_pv(0, j);
@@ -282,7 +293,7 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
           if (!ok) break;
         }
         if (el) AC4K_TRM(1, j, 2);
-        ok = warp_all(mbar_wait(p_full + 8, j & 1, p.wait_ns));
+        ok = warp_all(mbar_wait(p_full + 16 + 8 * (j & 1), (j >> 1) & 1, p.wait_ns));
         if (!ok) break;
         tc_fence_after();
         issue_pv(1, j);
@@ -298,7 +309,7 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       if (el) AC4K_TRM(1, j, 4);
     }
     if (!ok && el) atomicExch(p.status, kStatusTimeoutMma);
-  } else if (warp == 10) {
+   } else if (warp == 2) {
     // ------------------------------------------------------------------ scale re-order (reference layout only)
     if (!SF_TILED) {
       // chunk of K = 64 step k and rows [row0, row0 + 128) of a [K/64, pad, 4-byte] scale array: lane l takes the words
@@ -317,7 +328,7 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       const uint8_t *k_base = p.sfk + bh * p.nkq * (int64_t)p.k_pad * 4;
       const uint8_t *v_base = p.sfv + bh * (int64_t)p.v_k64 * p.v_pad * 4;
       for (int g = 0; g < (both ? 2 : 1); ++g)
-        for (int i = 0; i < p.nkq; ++i) put_chunk(sSFQ + g * SF_BYTES + i * 512, q_base, i, p.q_pad, (2 * qt + g) * BQ);
+        for (int i = 0; i < p.nkq; ++i) put_chunk(sSFQ + g * SF_BYTES + i * 512, q_base, i, p.q_pad, (qt + g) * BQ);
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(q_full);
@@ -336,23 +347,30 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       }
       if (!ok && lane == 0) atomicExch(p.status, kStatusTimeoutSf);
     }
-  } else if (warp < 6 || both) {
+   }
+  } else if (warp < kFirstSoftmaxWarp + kGroupWarps || both) {
+    reg_inc<kSoftmaxRegs>();
     // ------------------------------------------------------------------ softmax, correction, epilogue
-    const int g = (warp - 2) >> 2;            // group: query tile A or B
-    const int q = warp & 3;                   // tensor-memory lane quarter (warps 2-5 and 6-9 -> 2, 3, 0, 1)
-    const int row_l = q * 32 + lane;          // query row inside the tile = tensor-memory lane
-    const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+    const int g = (warp - kFirstSoftmaxWarp) / kGroupWarps;      // group: query tile A or B
+    const int q = warp & 3;                   // tensor-memory lane quarter of the warp
+    const int half = (warp >> 2) & 1;         // its 16 lanes of the quarter
+    const int t4 = lane & 3;
+    const int row_l = q * 32 + half * 16 + (lane >> 2);          // query rows of the thread inside the tile: row_l, row_l + 8
+    const uint32_t lane_addr = (uint32_t)(q * 32 + half * 16) << 16;
     const uint32_t t_s = tmem_base + lane_addr + S_COL, t_o = tmem_base + lane_addr + O_COL + 128 * g;
     // scores in units of log2: p = exp2(s * c1 - m)
     // (c1 >= 0: the host rejects a negative sm_scale; the floor keeps -inf * c1 = -inf for masked keys when a global
     // scale is 0)
     const float c1 = fmaxf(__ldg(p.q_gs) * __ldg(p.k_gs) * p.sm_scale * 1.4426950408889634f, 1.17549435e-38f);
-    const uint32_t p_row0 = sP + 2 * g * P_BYTES + row_l * 64;
-    const uint32_t p_xor = (uint32_t)((row_l >> 1) & 3) << 4;       // 64-byte swizzle: 16-byte chunk ^ ((row / 2) % 4)
-    const uint32_t sfp0 = sSFP + 2 * g * SF_BYTES + lane * 16 + q * 4;
-    const uint32_t my_s_full = s_full + 8 * g, my_p_full = p_full + 8 * g, my_o_done = o_done + 16 * g;
-    const bool tracer = (q == 0 && lane == 0);
-    float m = -INFINITY, l = 0.0f;
+    const uint32_t p_row0 = sP + 2 * g * P_BYTES + row_l * 64 + 4 * t4;
+    const uint32_t p_xor = (uint32_t)((row_l >> 1) & 3) << 4;       // 64-byte swizzle: 16-byte chunk ^ ((row / 2) % 4), the same for both rows
+    // the thread's scale bytes: those of its blocks (t4 / 2 of every 32 keys) for its first row (t4 even) or its second
+    const int sf_row = row_l + 8 * (t4 & 1);
+    const uint32_t sfp0 = sSFP + 2 * g * SF_BYTES + (sf_row & 31) * 16 + (sf_row >> 5) * 4 + (t4 >> 1);
+    const uint32_t my_s_full = s_full + 8 * g, my_p_full = p_full + 16 * g, my_o_done = o_done + 16 * g;
+    const bool tracer = (q == 0 && half == 0 && lane == 0);
+    float m[2] = {-INFINITY, -INFINITY};
+    float2 l[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};     // this thread's share of the row sums
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
       if (tracer) AC4K_TRM(2 * g, j, 0);
@@ -360,127 +378,102 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       if (!ok) break;
       tc_fence_after();
       if (tracer) AC4K_TRM(2 * g, j, 1);
-      uint32_t lo[64], hi[64];               // scores of keys 0-63 and 64-127
-      tmem_ld_32x32b_x64(t_s, lo);
-      tmem_ld_32x32b_x64(t_s + 64, hi);
+      uint32_t s[64];                        // s[4 i + 2 r + e]: score of row r of the thread and key 8 i + 2 t4 + e
+      tmem_ld_16x256b_x16(t_s, s);
       tmem_ld_wait();
-      tmem_pin(lo);
-      tmem_pin(hi);
-#define AC4K_S(i) ((i) < 64 ? lo[(i) & 63] : hi[(i) & 63])
+      tmem_pin(s);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(s_free);
       if (tracer) AC4K_TRM(2 * g, j, 2);
-      const int ncols = p.Nkv - j * BKV;                 // keys of this tile that exist (>= 128 except in the last tile)
+      const int ncols = p.Nkv - j * BKV - 2 * t4;        // keys of this tile that exist, counted from the thread's first
       if (ncols < BKV) {
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          if (i >= ncols) lo[i] = 0xff800000u;           // -inf: out of the maximum, probability 0
-          if (64 + i >= ncols) hi[i] = 0xff800000u;
-        }
+        for (int i = 0; i < 64; ++i)
+          if (8 * (i >> 2) + (i & 1) >= ncols) s[i] = 0xff800000u;     // -inf: out of the maximum, probability 0
       }
       // Maxima of the scores per block of 16 in the stored key order (the reference's V quantiser's "swizzle": every 32
-      // keys viewed as [4, 4, 2] and transposed to [4(b), 4(a), 2]; positions n, n + 1 hold keys key0(n), key0(n) + 1),
-      // and the row maximum from them.  ex2 is monotonic, so a block's largest probability is ex2 of its largest score:
-      // it is known before the block's probabilities are, and their conversion does not have to wait for all of them.
-      float bs[8];
+      // keys viewed as [4, 4, 2] and transposed to [4(b), 4(a), 2]): of every 32 keys a thread holds 8 a + 2 t4 + e, the
+      // positions 8 t4 .. 8 t4 + 7, so threads t4 = 0, 1 share the first block and 2, 3 the second.  ex2 is monotonic, so a
+      // block's largest probability is ex2 of its largest score: it is known before the block's probabilities are, and
+      // their conversion does not have to wait for all of them.
+      float bs[4][2], m_new[2];
 #pragma unroll
-      for (int bk = 0; bk < 8; ++bk) {
-        float v[16];
+      for (int r = 0; r < 2; ++r) {
 #pragma unroll
-        for (int n = 0; n < 16; n += 2) {
-          const int nn = 16 * (bk & 1) + n;
-          const int i = 32 * (bk >> 1) + (((nn >> 1) & 3) * 4 + (nn >> 3)) * 2;
-          v[n] = __uint_as_float(AC4K_S(i));
-          v[n + 1] = __uint_as_float(AC4K_S(i + 1));
+        for (int gg = 0; gg < 4; ++gg) {
+          float v[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(s[16 * gg + 4 * (i >> 1) + 2 * r + (i & 1)]);
+          const float x = max3(max3(v[0], v[1], v[2]), max3(v[3], v[4], v[5]), fmaxf(v[6], v[7]));
+          bs[gg][r] = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
         }
-        const float t0 = max3(v[0], v[1], v[2]), t1 = max3(v[3], v[4], v[5]), t2 = max3(v[6], v[7], v[8]);
-        const float t3 = max3(v[9], v[10], v[11]), t4 = max3(v[12], v[13], v[14]);
-        bs[bk] = fmaxf(max3(t0, t1, t2), max3(t3, t4, v[15]));
+        float v = max3(fmaxf(bs[0][r], bs[1][r]), bs[2][r], bs[3][r]);
+        v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+        m_new[r] = fmaxf(m[r], v * c1);
       }
-      const float m_new = fmaxf(m, fmaxf(max3(bs[0], bs[1], bs[2]), max3(bs[3], bs[4], max3(bs[5], bs[6], bs[7]))) * c1);
-      if (j > 0 && __any_sync(0xffffffffu, m_new != m)) {
-        // a maximum of this warp's rows moved: O is rescaled, once the previous tile's P V is complete
-        ok = warp_all(mbar_wait(my_o_done + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, p.wait_ns));
-        if (!ok) break;
-        tc_fence_after();
-        const float a = ex2_approx(m - m_new);
-#pragma unroll 1
-        for (int c = 0; c < 8; ++c) {
-          uint32_t ro[16];
-          tmem_ld_32x32b_x16(t_o + 16 * c, ro);
-          tmem_ld_wait();
-          tmem_pin(ro);
+      const bool moved = j > 0 && __any_sync(0xffffffffu, m_new[0] != m[0] || m_new[1] != m[1]);     // warp-uniform
+      float a[2] = {1.0f, 1.0f};
+      if (moved) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) ro[i] = __float_as_uint(__uint_as_float(ro[i]) * a);
-          tmem_st_32x32b_x16(t_o + 16 * c, ro);
+        for (int r = 0; r < 2; ++r) {
+          a[r] = ex2_approx(m[r] - m_new[r]);
+          l[r] = fmul2(l[r], make_float2(a[r], a[r]));
         }
-        tmem_st_wait();
-        l *= a;
       }
-      m = m_new;
+      m[0] = m_new[0];
+      m[1] = m_new[1];
       if (tracer) AC4K_TRM(2 * g, j, 3);
-      if (tracer) AC4K_TRM(2 * g, j, 4);
       // This tile's P buffer was last read by the P V of two tiles ago.  That MMA was issued before this tile's S, and
       // the tensor pipe completes MMAs (and the commits behind them) in issue order: s_full of this tile, seen above,
       // implies it is complete, so no wait is needed here.
-      // Probabilities, row sum, NVFP4 quantisation of P in eight blocks of 16 keys.  P is stored in the key order of the
-      // reference's V quantiser ("swizzle": every 32 keys viewed as [4, 4, 2] and transposed to [4(b), 4(a), 2]; positions
-      // n, n + 1 hold keys key0(n), key0(n) + 1), so that position n of P meets position n of V^T.
+      // Probabilities, row sum, NVFP4 quantisation of P in blocks of 16 keys.
       const uint32_t p_row = p_row0 + (j & 1) * P_BYTES;
-      float2 lsum[4];
-      const float2 c1_2 = make_float2(c1, c1), negm2 = make_float2(-m, -m);
-      uint32_t sfw[2] = {0u, 0u};
+      const float2 c1_2 = make_float2(c1, c1);
 #pragma unroll
       for (int gg = 0; gg < 4; ++gg) {
-        float2 pr[16];
-        lsum[gg] = make_float2(0.0f, 0.0f);
-#pragma unroll
-        for (int n = 0; n < 32; n += 2) {
-          const int i = 32 * gg + (((n >> 1) & 3) * 4 + (n >> 3)) * 2;     // keys held at positions n, n + 1
-          const float2 e = ffma2(make_float2(__uint_as_float(AC4K_S(i)), __uint_as_float(AC4K_S(i + 1))), c1_2, negm2);
-          // every fourth pair on the FMA pipe, the others on the ex2 pipe (every second pair measured 7 % slower)
-          pr[n >> 1] = ((n >> 1) & 3) == 1 ? exp2_fma_pipe(e) : make_float2(ex2_approx(e.x), ex2_approx(e.y));
-          lsum[gg] = fadd2(lsum[gg], pr[n >> 1]);
-        }
-        float bm[2];
-        bm[0] = ex2_approx(fmaf(bs[2 * gg], c1, -m));
-        bm[1] = ex2_approx(fmaf(bs[2 * gg + 1], c1, -m));
+        // block scales of both rows: e4m3 byte (row 0 low) and, from the table, what the probabilities are multiplied with
+        const float b0 = ex2_approx(fmaf(bs[gg][0], c1, -m[0])), b1 = ex2_approx(fmaf(bs[gg][1], c1, -m[1]));
         uint16_t sb2;
-        asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(sb2) : "f"(__fmul_rn(kPGlobal, __fmul_rn(bm[1], kOneSixth))),
-            "f"(__fmul_rn(kPGlobal, __fmul_rn(bm[0], kOneSixth))));
-        sfw[gg >> 1] |= (uint32_t)sb2 << (16 * (gg & 1));
-        float sc0, sc1;
+        asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(sb2) : "f"(__fmul_rn(kPGlobal, __fmul_rn(b1, kOneSixth))),
+            "f"(__fmul_rn(kPGlobal, __fmul_rn(b0, kOneSixth))));
+        float sc[2];
         // (the table is written once before the first barrier: these loads may be scheduled freely)
-        asm("ld.shared::cta.f32 %0, [%1];" : "=f"(sc0) : "r"(sLUT + ((uint32_t)sb2 & 0xffu) * 4));
-        asm("ld.shared::cta.f32 %0, [%1];" : "=f"(sc1) : "r"(sLUT + ((uint32_t)sb2 >> 8) * 4));
-        uint32_t codes[4];
+        asm("ld.shared::cta.f32 %0, [%1];" : "=f"(sc[0]) : "r"(sLUT + ((uint32_t)sb2 & 0xffu) * 4));
+        asm("ld.shared::cta.f32 %0, [%1];" : "=f"(sc[1]) : "r"(sLUT + ((uint32_t)sb2 >> 8) * 4));
+        st_shared_u8(sfp0 + (j & 1) * SF_BYTES + (gg >> 1) * 512 + 2 * (gg & 1), (uint32_t)sb2 >> (8 * (t4 & 1)));
 #pragma unroll
-        for (int hh = 0; hh < 4; ++hh) {
-          const float sc = hh < 2 ? sc0 : sc1;
-          const float2 sc2 = make_float2(sc, sc);
+        for (int r = 0; r < 2; ++r) {
+          const float2 negm2 = make_float2(-m[r], -m[r]), sc2 = make_float2(sc[r], sc[r]);
           float x[8];
+          float2 pr[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float2 y = fmul2(pr[4 * hh + i], sc2);
-            x[2 * i] = y.x;
-            x[2 * i + 1] = y.y;
+          for (int a = 0; a < 4; ++a) {
+            const int i = 16 * gg + 4 * a + 2 * r;
+            const float2 e = ffma2(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), c1_2, negm2);
+            pr[a] = make_float2(ex2_approx(e.x), ex2_approx(e.y));
+            const float2 y = fmul2(pr[a], sc2);
+            x[2 * a] = y.x;
+            x[2 * a + 1] = y.y;
           }
-          codes[hh] = f32x8_to_e2m1x8(x);
+          l[r] = fadd2(l[r], fadd2(fadd2(pr[0], pr[1]), fadd2(pr[2], pr[3])));
+          st_shared_u32(p_row + (((uint32_t)gg << 4) ^ p_xor) + 512 * r, f32x8_to_e2m1x8(x));
         }
-        st_shared_v4u(p_row + (((uint32_t)gg << 4) ^ p_xor), codes[0], codes[1], codes[2], codes[3]);
       }
-#undef AC4K_S
-      l += (lsum[0].x + lsum[0].y) + (lsum[1].x + lsum[1].y) + ((lsum[2].x + lsum[2].y) + (lsum[3].x + lsum[3].y));
       if (tracer) AC4K_TRM(2 * g, j, 5);
-      // scale chunks of the two K = 64 steps: 32 rows of 16 bytes, row `lane` holding the words of query rows lane,
-      // 32 + lane, 64 + lane, 96 + lane
-      st_shared_u32(sfp0 + (j & 1) * SF_BYTES, sfw[0]);
-      st_shared_u32(sfp0 + (j & 1) * SF_BYTES + 512, sfw[1]);
+      if (moved) {
+        // A maximum of this warp's rows moved: O is rescaled, once the previous tile's P V is complete.  Here, behind the
+        // exponentials, that has long happened and the scores' registers are free for O (in front of them the wait for
+        // P V and four loads and stores of 32 columns one after the other cost 13 % of the kernel at 16 384 keys).
+        ok = warp_all(mbar_wait(my_o_done + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, p.wait_ns));
+        if (!ok) break;
+        tc_fence_after();
+        mha_rescale(t_o, a);
+      }
       fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(my_p_full);
+      if (lane == 0) mbar_arrive(my_p_full + 8 * (j & 1));
       if (tracer) AC4K_TRM(2 * g, j, 6);
     }
     if (ok) ok = warp_all(mbar_wait(my_o_done + 8 * ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, p.wait_ns));
@@ -488,31 +481,29 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       if (lane == 0) atomicExch(p.status, kStatusTimeoutEpilogue);
     } else {
       tc_fence_after();
-      const int n = (2 * qt + g) * BQ + row_l;
-      const float out_scale = __ldg(p.v_gs) / (kPGlobal * l);
-      __nv_bfloat16 *dst = static_cast<__nv_bfloat16 *>(p.O) + (int64_t)b * p.o_b + (int64_t)h * p.o_h + (int64_t)n * p.o_n;
+      const int n_row = (qt + g) * BQ + row_l;
+      float out_scale[2];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t ro[32];
-        tmem_ld_32x32b_x32_sync(t_o + 32 * c, ro);
-        if (n < p.Nq) {
-          if (p.o_d == 1 && p.Dv == D && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
+      for (int r = 0; r < 2; ++r) {
+        float v = l[r].x + l[r].y;
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        out_scale[r] = __ldg(p.v_gs) / (kPGlobal * v);
+      }
+      __nv_bfloat16 *dst0 = static_cast<__nv_bfloat16 *>(p.O) + (int64_t)b * p.o_b + (int64_t)h * p.o_h + (int64_t)n_row * p.o_n;
+      const bool vec = mha_rows_vec4(p.O, p.o_b, p.o_h, p.o_n, p.o_d, p.Dv);
+#pragma unroll 1
+      for (int c0 = 0; c0 < p.Dv; c0 += 32) {
+        uint32_t ro[16];
+        tmem_ld_16x256b_x4(t_o + c0, ro);
+        tmem_ld_wait();
+        tmem_pin(ro);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint32_t w[4];
+        for (int r = 0; r < 2; ++r) {
+          float o[8];
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(ro[8 * i + 2 * k]) * out_scale,
-                                                                __uint_as_float(ro[8 * i + 2 * k + 1]) * out_scale);
-                w[k] = *reinterpret_cast<const uint32_t *>(&h2);
-              }
-              reinterpret_cast<uint4 *>(dst + 32 * c)[i] = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (32 * c + i < p.Dv) dst[(int64_t)(32 * c + i) * p.o_d] = __float2bfloat16_rn(__uint_as_float(ro[i]) * out_scale);
-          }
+          for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(ro[4 * (i >> 1) + 2 * r + (i & 1)]) * out_scale[r];
+          mha_store_row(dst0 + 8 * r * p.o_n, o, c0, t4, p.Dv, p.o_d, vec, n_row + 8 * r < p.Nq);
         }
       }
     }
@@ -576,6 +567,7 @@ extern "C" int ac4k_mha_nvfp4_fwd(void *O, const int64_t o_stride[4], const void
   a.k_pad = (int)align_up(Nkv, 16);
   a.v_pad = (int)align_up(Dv, 16);
   a.sm_scale = sm_scale;
+  a.q_tiles = mha_query_tiles(a.q_blocks, H * B, di.sms);
   a.status = status;
   a.wait_ns = kWaitTimeoutNs;
   a.trace = debug_trace_ptr();
@@ -590,7 +582,7 @@ extern "C" int ac4k_mha_nvfp4_fwd(void *O, const int64_t o_stride[4], const void
       }))
     return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((a.q_blocks + 1) / 2), (unsigned)H, (unsigned)B);
+  cfg.gridDim = dim3((unsigned)ceil_div(a.q_blocks, a.q_tiles), (unsigned)H, (unsigned)B);
   cfg.blockDim = dim3(mha::kThreads);
   cfg.dynamicSmemBytes = mha::SMEM_BYTES;
   cfg.stream = stream;
