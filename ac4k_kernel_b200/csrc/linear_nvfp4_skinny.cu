@@ -7,11 +7,12 @@
 //     activation rows (padded to NT = 16 / 32 / 64) the N side.  The accumulator is 128 lanes x NT columns,
 //     an activation box is NT x 128 bytes instead of 128 x 128, and a call with M = 1 costs what M = 16 costs.
 //   * One work item per CTA: a tile of 128 weight rows x one slice of K.  The `splits` (1, 2 or 4) slices of a
-//     tile are the CTAs of one cluster.  The 128 rows of the tile are four quarters of 32 (one per epilogue
-//     warp); quarter q is finished by CTA q % splits: the other slices copy their fp32 partial sums of that
-//     quarter into a small region of its shared memory (one bulk copy through distributed shared memory,
-//     completing on the owner's mbarrier), it adds them in slice order, applies alpha and bias and stores.
-//     No workspace, no second kernel, no waiting for a leader.
+//     tile are the CTAs of one cluster.  The 128 rows of the tile are four quarters of 32, one per epilogue
+//     warp; the activation rows are divided among the slices: for each of its quarters a slice receives the other
+//     slices' fp32 partial sums of its rows in a small region of its shared memory (one bulk copy each through
+//     distributed shared memory, completing on an mbarrier there), adds them in slice order, applies alpha and
+//     bias and stores.  All four warps of all slices work at the end (a slice finishing one quarter of the weight
+//     rows kept three of its warps idle while one added 64 activation rows).  No workspace, no second kernel.
 //   * A CTA needs 97 - 111 KB of shared memory and 128 tensor-memory columns, so two of them fit on an
 //     SM and the CTAs of the next call of the stream (programmatic dependent launch) become resident while this
 //     call still runs; before they wait for it they ask L2 for their whole share of the weights (a prefetch
@@ -38,10 +39,11 @@ struct Cfg {
   static constexpr int X_BYTES = NT * BKB;
   static constexpr int STAGES = NT == 64 ? 3 : 4;       // two CTAs of this kernel fit on an SM in every configuration
   static constexpr int STAGE_BYTES = W_BYTES + X_BYTES + 2 * SF_BYTES;
-  // partial sums received from the other slices: up to 3 units of [NT][32] fp32 (4 slices: this CTA's one
-  // quarter from 3 slices; 2 slices: its two quarters from 1 slice each)
+  // partial sums received from the other slices: 4 quarters x (slices - 1) units of [rows of this slice][32] fp32, the
+  // rows at most NT / slices: up to 3 NT x 128 bytes
   static constexpr int PART_UNIT = NT * 128;
   static constexpr int PART_BYTES = 3 * PART_UNIT;
+  static_assert(4 * PART_UNIT <= STAGES * W_BYTES, "the warps' own partial sums reuse the weight buffers");
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + PART_BYTES + 1024 /*alignment*/ + 256 /*barriers*/;
   static constexpr int MIN_CTAS = 2;                     // CTAs of this kernel that fit on an SM
   static_assert(MIN_CTAS * (SMEM_BYTES + 1024) <= 228 * 1024, "shared memory per SM");
@@ -72,48 +74,51 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[NT]) 
   tmem_pin(r);
 }
 
-// The owner of a quarter of the rows: add the K slices in slice order (whichever of them this CTA computed
-// itself: `own`; the others from the partial-sum units, which skip the owner's own slice), apply alpha and
-// bias, round and store row by row.  Eight activation rows at a time so that their shared-memory loads are
-// independent of one another.
-template <int NT, int SPLITS, int OUT_DT>
-__device__ __forceinline__ void finish_rows(const uint32_t (&own)[NT], uint32_t part0, int slice, const GemmArgs &p, int n,
-                                            typename OutT<OUT_DT>::type *dst) {
-  using T = typename OutT<OUT_DT>::type;
-  constexpr int UNIT = NT * 128;
+template <int OUT_DT>
+__device__ __forceinline__ void store_out(typename OutT<OUT_DT>::type *dst, float v) {
+  if (OUT_DT == AC4K_DT_BF16) *dst = (typename OutT<OUT_DT>::type)__float2bfloat16_rn(v);
+  else if (OUT_DT == AC4K_DT_FP16) *dst = (typename OutT<OUT_DT>::type)__float2half_rn(v);
+  else *dst = (typename OutT<OUT_DT>::type)v;
+}
+
+// One K slice: the accumulator is the sum.  alpha, bias, round, store row by row.
+template <int NT, int OUT_DT>
+__device__ __forceinline__ void finish_rows(const uint32_t (&own)[NT], const GemmArgs &p, int n, typename OutT<OUT_DT>::type *dst) {
   const float alpha = __fmul_rn(__ldg(p.a_gs), __ldg(p.b_gs));
   const float b = p.bias != nullptr ? load_bias(p.bias, p.bias_dt, n) : 0.0f;
 #pragma unroll
-  for (int m0 = 0; m0 < NT; m0 += 8) {
-    if (m0 >= p.M) break;
-    float x[SPLITS > 1 ? SPLITS - 1 : 1][8];
-    if (SPLITS > 1) {
+  for (int m = 0; m < NT; ++m) {
+    float v = __fmul_rn(__uint_as_float(own[m]), alpha);
+    if (p.bias != nullptr) v = __fadd_rn(v, b);
+    if (m < p.M) store_out<OUT_DT>(dst + (int64_t)m * p.N, v);
+  }
+}
+
+// Several K slices: this CTA adds `rows` activation rows (of 128 output columns, one per thread of the four warps) in
+// slice order, its own partial sums from `own0`, the others' from `part0` (unit of `rs` rows each, the own slice skipped), applies
+// alpha and bias, rounds and stores.  Eight rows at a time so that their shared-memory loads are independent.
+template <int SPLITS, int OUT_DT>
+__device__ __forceinline__ void finish_split(uint32_t own0, uint32_t part0, int slice, int rows, int rs, const GemmArgs &p, int n,
+                                             typename OutT<OUT_DT>::type *dst) {
+  const float alpha = __fmul_rn(__ldg(p.a_gs), __ldg(p.b_gs));
+  const float b = p.bias != nullptr ? load_bias(p.bias, p.bias_dt, n) : 0.0f;
+#pragma unroll 1
+  for (int i0 = 0; i0 < rows; i0 += 8) {
+    float x[SPLITS][8];
 #pragma unroll
-      for (int j = 0; j < SPLITS - 1; ++j)
+    for (int sl = 0; sl < SPLITS; ++sl) {
+      const uint32_t base = (sl == slice ? own0 : part0 + (uint32_t)((sl < slice ? sl : sl - 1) * rs) * 128u) + (uint32_t)i0 * 128u;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[j][i] = ld_shared_f32(part0 + j * UNIT + (m0 + i) * 128);
+      for (int i = 0; i < 8; ++i) x[sl][i] = i0 + i < rows ? ld_shared_f32(base + i * 128) : 0.0f;
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int m = m0 + i;
-      float v = 0.0f;
+      float v = x[0][i];
 #pragma unroll
-      for (int sl = 0; sl < SPLITS; ++sl) {
-        float t = __uint_as_float(own[m]);
-        if (SPLITS > 1) {
-          // slice sl sits in unit sl if it comes before the owner's own slice, else in unit sl - 1
-          const float before = x[sl < SPLITS - 1 ? sl : SPLITS - 2][i], after = x[sl > 0 ? sl - 1 : 0][i];
-          t = sl == slice ? t : (sl < slice ? before : after);
-        }
-        v = sl == 0 ? t : __fadd_rn(v, t);
-      }
+      for (int sl = 1; sl < SPLITS; ++sl) v = __fadd_rn(v, x[sl][i]);
       v = __fmul_rn(v, alpha);
       if (p.bias != nullptr) v = __fadd_rn(v, b);
-      if (m < p.M) {
-        if (OUT_DT == AC4K_DT_BF16) dst[(int64_t)m * p.N] = (T)__float2bfloat16_rn(v);
-        else if (OUT_DT == AC4K_DT_FP16) dst[(int64_t)m * p.N] = (T)__float2half_rn(v);
-        else dst[(int64_t)m * p.N] = (T)v;
-      }
+      if (i0 + i < rows) store_out<OUT_DT>(dst + (int64_t)(i0 + i) * p.N, v);
     }
   }
 }
@@ -136,8 +141,8 @@ linear_nvfp4_skinny_kernel(const __grid_constant__ CUtensorMap tma_x, const __gr
   const uint32_t bars = sPart + C::PART_BYTES;
   const uint32_t full_bar = bars, empty_bar = bars + 8 * STAGES;
   const uint32_t tfull_bar = bars + 16 * STAGES;
-  const uint32_t part_bar = tfull_bar + 8;      // [2] the other slices' partial sums of this CTA's first / second quarter have landed
-  const uint32_t tmem_slot = part_bar + 16;
+  const uint32_t part_bar = tfull_bar + 8;      // [quarter] the other slices' partial sums of this CTA's activation rows have landed
+  const uint32_t tmem_slot = part_bar + 32;
   uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
 
 #ifdef AC4K_TRACE_ENABLED
@@ -155,6 +160,9 @@ linear_nvfp4_skinny_kernel(const __grid_constant__ CUtensorMap tma_x, const __gr
   const int k_tiles_all = (p.KT + KS - 1) / KS;
   const int kt0 = slice * p.kt_per_split, kt1 = min(k_tiles_all, kt0 + p.kt_per_split);
   const int n0 = tn * 128;
+  // activation rows that slice s finishes: [s * rs, s * rs + rows_of(s))
+  const int rs = (p.M + p.splits - 1) / p.splits;
+  auto rows_of = [&](int s) { return max(0, min(rs, p.M - s * rs)); };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -162,11 +170,10 @@ linear_nvfp4_skinny_kernel(const __grid_constant__ CUtensorMap tma_x, const __gr
       mbar_init(empty_bar + 8 * s, 1);
     }
     mbar_init(tfull_bar, 1);
-    mbar_init(part_bar, 1);
-    mbar_init(part_bar + 8, 1);
-    if (p.splits > 1) {
-      // this CTA finishes 4 / splits quarters; each receives one copy of NT x 128 bytes from every other slice
-      for (int lq = 0; lq < 4 / p.splits; ++lq) mbar_arrive_expect_tx(part_bar + 8 * lq, (p.splits - 1) * C::PART_UNIT);
+    for (int q = 0; q < 4; ++q) mbar_init(part_bar + 8 * q, 1);
+    if (p.splits > 1 && rows_of(slice) > 0) {
+      // each quarter receives one copy of this CTA's rows x 128 bytes from every other slice
+      for (int q = 0; q < 4; ++q) mbar_arrive_expect_tx(part_bar + 8 * q, (uint32_t)((p.splits - 1) * rows_of(slice)) * 128u);
     }
     fence_barrier_init();
     prefetch_tmap(&tma_x);
@@ -316,34 +323,36 @@ linear_nvfp4_skinny_kernel(const __grid_constant__ CUtensorMap tma_x, const __gr
     if (warp == 2 && lane == 0) AC4K_TRS(5);
     uint32_t r[NT];
     tmem_ld_cols<NT>(tmem_base + ((uint32_t)(q * 32) << 16), r);
-    const int owner = q % p.splits;           // the slice (CTA of the cluster) that finishes this quarter of the rows
-    const int lq = q / p.splits;              // which of the owner's quarters it is
-    if (owner != slice) {
-      // This warp's partial sums go to the owner: unit [lq][source slice, skipping the owner's own][m][lane].
-      // They are laid out in this CTA's first weight buffer (free: all its MMAs are complete) and travel as one
-      // bulk copy; plain remote stores were measured at ~0.1 us per activation row.
-      const int unit = lq * (p.splits - 1) + (slice < owner ? slice : slice - 1);
+    if (p.splits == 1) {
+      if (n < p.N && tfull_ok) finish_rows<NT, OUT_DT>(r, p, n, static_cast<T *>(p.D) + n);
+    } else {
+      // This warp's partial sums are laid out [activation row][lane] in this CTA's weight buffers (free: all its MMAs are
+      // complete); the rows of every other slice travel there as one bulk copy, to unit [quarter][source slice, skipping
+      // the owner's own].  (Plain remote stores were measured at ~0.1 us per activation row.)
       const uint32_t scratch = sW + (uint32_t)(warp - 2) * C::PART_UNIT;
 #pragma unroll
-      for (int m = 0; m < NT; ++m) st_shared_f32(scratch + m * 128 + lane * 4, __uint_as_float(r[m]));
+      for (int m = 0; m < NT; ++m)
+        if (m < p.M) st_shared_f32(scratch + m * 128 + lane * 4, __uint_as_float(r[m]));
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0)
-        bulk_copy_to_cluster(map_to_cta(sPart + unit * C::PART_UNIT, owner), scratch, C::PART_UNIT,
-                             map_to_cta(part_bar + 8 * lq, owner));
-      if (warp == 2 && lane == 0) AC4K_TRS(6);
-    } else {
-      if (p.splits > 1) {
-        const bool got = mbar_wait(part_bar + 8 * lq, 0, p.wait_ns);
-        if (!got && lane == 0) atomicExch(p.status, kStatusTimeoutEpilogue);
+      if (lane < p.splits && lane != slice && rows_of(lane) > 0) {
+        const int o = lane;
+        const uint32_t unit = (uint32_t)(q * (p.splits - 1) + (slice < o ? slice : slice - 1)) * (uint32_t)rs * 128u;
+        bulk_copy_to_cluster(map_to_cta(sPart + unit, o), scratch + (uint32_t)(o * rs) * 128u, (uint32_t)rows_of(o) * 128u,
+                             map_to_cta(part_bar + 8 * q, o));
       }
       if (warp == 2 && lane == 0) AC4K_TRS(6);
-      if (n < p.N && tfull_ok) {
-        const uint32_t part0 = sPart + lq * (p.splits - 1) * C::PART_UNIT + lane * 4;
-        T *dst = static_cast<T *>(p.D) + n;
-        if (p.splits == 4) finish_rows<NT, 4, OUT_DT>(r, part0, slice, p, n, dst);
-        else if (p.splits == 2) finish_rows<NT, 2, OUT_DT>(r, part0, slice, p, n, dst);
-        else finish_rows<NT, 1, OUT_DT>(r, part0, slice, p, n, dst);
+      const int rows = rows_of(slice);
+      if (rows > 0) {
+        const bool got = mbar_wait(part_bar + 8 * q, 0, p.wait_ns);
+        if (!got && lane == 0) atomicExch(p.status, kStatusTimeoutEpilogue);
+        if (n < p.N && tfull_ok) {
+          const uint32_t own0 = scratch + (uint32_t)(slice * rs) * 128u + lane * 4;
+          const uint32_t part0 = sPart + (uint32_t)(q * (p.splits - 1) * rs) * 128u + lane * 4;
+          T *dst = static_cast<T *>(p.D) + (int64_t)(slice * rs) * p.N + n;
+          if (p.splits == 4) finish_split<4, OUT_DT>(own0, part0, slice, rows, rs, p, n, dst);
+          else finish_split<2, OUT_DT>(own0, part0, slice, rows, rs, p, n, dst);
+        }
       }
     }
   }
