@@ -25,8 +25,12 @@ SIGNATURES = {
     "ac4k_global_scale_bf16": (ctypes.c_int, [_vp, ctypes.c_int64, ctypes.c_float, _vp, _vp]),
     "ac4k_quantize_nvfp4": (ctypes.c_int, [_vp, _vp, _vp, _vp, _c_i64p, _c_i64p, ctypes.c_int,
                                            ctypes.c_int, _vp]),
+    "ac4k_quantize_nvfp4_dynamic": (ctypes.c_int, [_vp, _vp, _vp, _vp, _vp, ctypes.c_float, _c_i64p, _c_i64p, ctypes.c_int,
+                                                   ctypes.c_int, _vp]),
     "ac4k_quantize_fp8": (ctypes.c_int, [_vp, _vp, _vp, _vp, _c_i64p, _c_i64p, ctypes.c_int, _vp]),
     "ac4k_quantize_int8": (ctypes.c_int, [_vp, _vp, _vp, _vp, _c_i64p, _c_i64p, _vp]),
+    "ac4k_quantize_fp8_max": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_float, _c_i64p, _c_i64p, ctypes.c_int, _vp]),
+    "ac4k_quantize_int8_max": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int32, _c_i64p, _c_i64p, _vp]),
     "ac4k_linear_nvfp4": (ctypes.c_int, [_vp, ctypes.c_int, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                                          ctypes.c_int, ctypes.c_int64, ctypes.c_int64,
                                          ctypes.c_int64, ctypes.c_int, _vp]),

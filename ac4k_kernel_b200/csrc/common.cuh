@@ -67,6 +67,23 @@ unsigned int *device_status_ptr();
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Launch; OVERLAP: with the attribute above, for a kernel that waits before it touches memory.
+template <bool OVERLAP, typename... KArgs, typename... Args>
+int launch_kernel(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = OVERLAP ? 1 : 0;
+  AC4K_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+  return 0;
+}
+
 // ---- small integer helpers --------------------------------------------------------------
 __host__ __device__ constexpr int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 __host__ __device__ constexpr int64_t align_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }

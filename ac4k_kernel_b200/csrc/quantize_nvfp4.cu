@@ -8,7 +8,10 @@
 // Three kernels: a tiled one for rows that are contiguous along K (the linear path), a transposing one
 // for rows that are contiguous along the cross dimension (attention's V), and a strided one (any
 // cross/reduce strides, optional K permutation) for everything else.
+#include <algorithm>
+
 #include "common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace ac4k {
 
@@ -23,6 +26,45 @@ __device__ __forceinline__ uint32_t quantize8(const uint4 &v, float r) {
   f[6] = __fmul_rn(__uint_as_float(v.w << 16), r);
   f[7] = __fmul_rn(__uint_as_float(v.w & 0xFFFF0000u), r);
   return f32x8_to_e2m1x8(f);
+}
+
+// Where a quantiser kernel takes the tensor's global scale from: a scalar on the device, or the per-CTA maxima (bf16 bits)
+// that amax_partial_kernel left, which every CTA reduces for itself (the first one stores the scale for the caller).  The
+// second form needs no zeroed accumulator, i.e. no memset in front of the reduction.
+struct ScaleSource {
+  const float *g;
+  const uint32_t *partial;
+  int n_partial;
+  float max_scale;
+  float *g_out;
+  bool last_first;      // tiled kernel: take the row tiles from the last to the first
+};
+
+// max|x| (bf16 bits) -> global scale; 0 for a tensor of zeros
+__device__ __forceinline__ float global_scale_of(uint32_t amax_bits, float max_scale) {
+  return amax_bits ? __fdiv_rn(bf16_bits_to_f32(amax_bits), max_scale) : 0.0f;
+}
+__device__ __forceinline__ float alpha_of(float g) { return g == 0.0f ? 0.0f : __frcp_rn(g); }
+
+// maximum of one value per thread over the CTA, in every thread (s_m: one word per warp; ends with all threads past a barrier)
+__device__ __forceinline__ uint32_t cta_max(uint32_t m, uint32_t *s_m) {
+  m = __reduce_max_sync(0xFFFFFFFFu, m);
+  if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
+  __syncthreads();
+  const int nw = blockDim.x >> 5;
+  m = (int)(threadIdx.x & 31) < nw ? s_m[threadIdx.x & 31] : 0u;
+  return __reduce_max_sync(0xFFFFFFFFu, m);
+}
+
+// 1 / global scale, in every thread.  PARTIAL: called by all threads of the CTA, behind the dependency wait.
+template <bool PARTIAL>
+__device__ __forceinline__ float resolve_alpha(const ScaleSource &src, uint32_t *s_m) {
+  if (!PARTIAL) return load_alpha(src.g);
+  uint32_t m = 0;
+  for (int i = threadIdx.x; i < src.n_partial; i += blockDim.x) m = max(m, __ldcg(src.partial + i));
+  const float g = global_scale_of(cta_max(m, s_m), src.max_scale);
+  if ((blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) *src.g_out = g;
+  return alpha_of(g);
 }
 
 // ----------------------------------------------------------------------------------------
@@ -62,10 +104,10 @@ __device__ __forceinline__ Block16 load_block16(const uint16_t *p) {
 
 // TK: K elements of a CTA's tile, 256 or - for rows of at most 128 elements (attention's q and k: one head's
 // features), where half of a 256-wide tile's threads would have nothing to load - 128.
-template <int SF_LAYOUT, bool WIDE, int TK>
+template <int SF_LAYOUT, bool WIDE, int TK, bool PARTIAL>
 __global__ void __launch_bounds__(kThreads)
 nvfp4_quantize_tiled_kernel(uint8_t *__restrict__ out, uint32_t *__restrict__ sf,
-                            const uint16_t *__restrict__ in, const float *__restrict__ gscale,
+                            const uint16_t *__restrict__ in, const ScaleSource src,
                             int64_t M, int64_t K, int64_t d1, int64_t stride0, int64_t stride1,
                             int64_t row_stride) {
   constexpr int kTileK = TK, kTileKch = TK / 64;
@@ -73,13 +115,15 @@ nvfp4_quantize_tiled_kernel(uint8_t *__restrict__ out, uint32_t *__restrict__ sf
   constexpr int kPassRows = kThreads / kRowThreads;     // rows the CTA covers per pass
   __shared__ uint32_t s_sf[kTileKch * kTileRows];
   __shared__ float s_rcp[128];
+  __shared__ uint32_t s_m[kThreads / 32];
 
   const int64_t Kp = align_up(K, 64);
   const int64_t KT = Kp / 64;
   const int64_t M16 = align_up(M, 16);
   const int64_t MT = ceil_div(M, 128);
   const int64_t batch = blockIdx.z;
-  const int64_t r0 = (int64_t)blockIdx.y * kTileRows;
+  const int64_t by = src.last_first ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
+  const int64_t r0 = by * kTileRows;
   const int64_t k0 = (int64_t)blockIdx.x * kTileK;
   const int blk = threadIdx.x % kRowThreads, prow = threadIdx.x / kRowThreads;
 
@@ -90,8 +134,6 @@ nvfp4_quantize_tiled_kernel(uint8_t *__restrict__ out, uint32_t *__restrict__ sf
     s_rcp[threadIdx.x] = threadIdx.x ? __frcp_rn(v) : 0.0f;
   }
   __syncthreads();
-
-  const float alpha = load_alpha(gscale);
   const int64_t k = k0 + blk * 16;
   const bool k_live = k < Kp;   // block belongs to the (padded) output
   const bool k_data = k < K;    // block has input data (K % 16 == 0 on this path)
@@ -99,6 +141,10 @@ nvfp4_quantize_tiled_kernel(uint8_t *__restrict__ out, uint32_t *__restrict__ sf
   uint8_t *out_p = out + (batch * M + r0 + prow) * (Kp / 2) + k / 2;
   uint8_t *s_bytes = reinterpret_cast<uint8_t *>(s_sf);
   const int kch = blk >> 2, sub = blk & 3;
+
+  if (PARTIAL) grid_dependency_wait();
+  grid_launch_dependents();
+  const float alpha = resolve_alpha<PARTIAL>(src, s_m);
 
 #pragma unroll 1
   for (int p0 = 0; p0 < kTileRows / kPassRows; p0 += kBatch) {
@@ -150,7 +196,7 @@ nvfp4_quantize_tiled_kernel(uint8_t *__restrict__ out, uint32_t *__restrict__ sf
       const int64_t row = r0 + w;
       if (row < M16) sf[(batch * KT + k64) * M16 + row] = s_sf[t];
     } else {
-      sf[((batch * MT + blockIdx.y) * KT + k64) * 128 + w] = s_sf[t];
+      sf[((batch * MT + by) * KT + k64) * 128 + w] = s_sf[t];
     }
   }
 }
@@ -161,10 +207,10 @@ nvfp4_quantize_tiled_kernel(uint8_t *__restrict__ out, uint32_t *__restrict__ sf
 // 32 viewed as [4][4][2] and transposed in its first two modes).  Threads are laid out so
 // that neighbouring lanes walk the dimension with the smaller stride.
 // ----------------------------------------------------------------------------------------
-template <int SF_LAYOUT, bool PERMUTE, bool ROW_FASTEST>
+template <int SF_LAYOUT, bool PERMUTE, bool ROW_FASTEST, bool PARTIAL>
 __global__ void __launch_bounds__(256)
 nvfp4_quantize_strided_kernel(uint8_t *__restrict__ out, uint8_t *__restrict__ sf,
-                              const uint16_t *__restrict__ in, const float *__restrict__ gscale,
+                              const uint16_t *__restrict__ in, const ScaleSource src,
                               int64_t M, int64_t K, int64_t d1, int64_t stride0, int64_t stride1,
                               int64_t stride_m, int64_t stride_k) {
   const int64_t Kp = align_up(K, 64);
@@ -183,10 +229,13 @@ nvfp4_quantize_strided_kernel(uint8_t *__restrict__ out, uint8_t *__restrict__ s
     row = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5);
     blk = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
   }
+  __shared__ uint32_t s_m[8];
+  if (PARTIAL) grid_dependency_wait();
+  grid_launch_dependents();
+  const float alpha = resolve_alpha<PARTIAL>(src, s_m);
   if (row >= rows_sf || blk >= nblk) return;
 
   const uint16_t *in_b = in + (batch / d1) * stride0 + (batch % d1) * stride1;
-  const float alpha = load_alpha(gscale);
 
   uint32_t w[8];
   uint32_t amax = 0;
@@ -196,13 +245,13 @@ nvfp4_quantize_strided_kernel(uint8_t *__restrict__ out, uint8_t *__restrict__ s
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int64_t p = blk * 16 + j * 2 + h;   // position in the (permuted) output row
-      int64_t src = p;
+      int64_t k = p;
       if (PERMUTE) {
         const int64_t q = p & 31;
-        src = (p - q) + 8 * ((q & 7) >> 1) + 2 * (q >> 3) + (q & 1);
+        k = (p - q) + 8 * ((q & 7) >> 1) + 2 * (q >> 3) + (q & 1);
       }
       uint32_t e = 0;
-      if (row < M && src < K) e = __ldg(in_b + row * stride_m + src * stride_k);
+      if (row < M && k < K) e = __ldg(in_b + row * stride_m + k * stride_k);
       pair |= e << (16 * h);
       const uint32_t a = e & 0x7FFFu;
       amax = a > amax ? a : amax;
@@ -235,10 +284,10 @@ nvfp4_quantize_strided_kernel(uint8_t *__restrict__ out, uint8_t *__restrict__ s
 // 16 in registers, and codes and scale bytes go through shared memory so that each output row leaves
 // as 64 contiguous bytes and the scales as whole words.
 // ----------------------------------------------------------------------------------------
-template <int SF_LAYOUT, bool PERMUTE>
+template <int SF_LAYOUT, bool PERMUTE, bool PARTIAL>
 __global__ void __launch_bounds__(256)
 nvfp4_quantize_transposed_kernel(uint8_t *__restrict__ out, uint8_t *__restrict__ sf, const uint16_t *__restrict__ in,
-                                 const float *__restrict__ gscale, int64_t M, int64_t K, int64_t d1, int64_t stride0,
+                                 const ScaleSource src, int64_t M, int64_t K, int64_t d1, int64_t stride0,
                                  int64_t stride1, int64_t stride_k) {
   __shared__ uint4 s_codes[128][4 + 1];          // [row][32-element group of the tile], padded
   __shared__ uint32_t s_sf[2][128];              // [K = 64 step of the tile][row]: four scale bytes
@@ -248,7 +297,10 @@ nvfp4_quantize_transposed_kernel(uint8_t *__restrict__ out, uint8_t *__restrict_
   const int cx = threadIdx.x & 63, kg = threadIdx.x >> 6;
   const int64_t m = m0 + 2 * cx, kb = k0 + 32 * kg;           // this thread: rows m, m + 1; K-elements kb .. kb + 31
   const uint16_t *base = in + (batch / d1) * stride0 + (batch % d1) * stride1;
-  const float alpha = load_alpha(gscale);
+  __shared__ uint32_t s_m[8];
+  if (PARTIAL) grid_dependency_wait();
+  grid_launch_dependents();
+  const float alpha = resolve_alpha<PARTIAL>(src, s_m);
 
   uint32_t w[32];                                // w[j]: element kb + j of row m (low half) and of row m + 1 (high half)
 #pragma unroll
@@ -312,12 +364,97 @@ nvfp4_quantize_transposed_kernel(uint8_t *__restrict__ out, uint8_t *__restrict_
 }
 
 // ----------------------------------------------------------------------------------------
+// Flat kernel, for tensors whose 128-row tiles would leave most of the chip idle (decode and short prompts): the 16-element
+// blocks of the tensor, in memory order, one per thread, which keeps it in registers from the maximum to the codes.
+//   CLUSTER  one cluster of up to eight CTAs holds the whole tensor and combines its maxima through distributed shared
+//            memory: global scale, codes and block scales in one launch.
+//   else     the maxima come from amax_partial_kernel; the data are loaded in front of the dependency wait (they were
+//            complete before that kernel began).
+// Four neighbouring lanes hold the blocks of one K = 64 step and write its scale word together.
+// ----------------------------------------------------------------------------------------
+template <int SF_LAYOUT, bool CLUSTER, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+nvfp4_quantize_flat_kernel(uint8_t *__restrict__ out, uint32_t *__restrict__ sf, const uint16_t *__restrict__ in,
+                           const ScaleSource src, int M, int K, int nbatch, int d1, int64_t stride0, int64_t stride1,
+                           int64_t row_stride) {
+  __shared__ uint32_t s_m[THREADS / 32];
+  __shared__ uint32_t s_peer[8];
+  const int Kp = (K + 63) / 64 * 64, KT = Kp / 64, nblk = Kp / 16;
+  const int rows_sf = SF_LAYOUT == AC4K_SF_AC4K ? (M + 15) / 16 * 16 : (M + 127) / 128 * 128;
+  const int items = nbatch * M * nblk;
+  const int stride = gridDim.x * blockDim.x;
+  const int it = blockIdx.x * blockDim.x + threadIdx.x;         // this thread's block
+  auto sf_word = [&](int b, int row, int k64) -> int64_t {
+    if (SF_LAYOUT == AC4K_SF_AC4K) return ((int64_t)b * KT + k64) * rows_sf + row;
+    return (((int64_t)b * (rows_sf >> 7) + (row >> 7)) * KT + k64) * 128 + (row & 31) * 4 + ((row & 127) >> 5);
+  };
+  grid_launch_dependents();
+  if (CLUSTER) grid_dependency_wait();
+
+  Block16 v;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v.w[i] = 0;
+  const int row_all = it / nblk, blk = it - row_all * nblk;
+  const int b = row_all / M, row = row_all - b * M;
+  if (it < items && blk * 16 < K)
+    v = load_block16<false>(in + (int64_t)(b / d1) * stride0 + (int64_t)(b % d1) * stride1 + row * row_stride + blk * 16);
+  // scale words of the padding rows
+  if (!CLUSTER) grid_dependency_wait();
+  {
+    const int pad = rows_sf - M, words = nbatch * KT * pad;
+    for (int w = it; w < words; w += stride) {
+      const int bk = w / pad, r = w - bk * pad, bw = bk / KT;
+      sf[sf_word(bw, M + r, bk - bw * KT)] = 0u;
+    }
+  }
+  float alpha;
+  if (CLUSTER) {
+    const uint32_t *w = v.w;
+    // (the 0 takes NaNs out, as in thread_amax)
+    const uint32_t m2 = max_bf16x2(0u, max_bf16x2(max_bf16x2(max_bf16x2(abs_bf16x2(w[0]), abs_bf16x2(w[1])), max_bf16x2(abs_bf16x2(w[2]), abs_bf16x2(w[3]))),
+                                                  max_bf16x2(max_bf16x2(abs_bf16x2(w[4]), abs_bf16x2(w[5])), max_bf16x2(abs_bf16x2(w[6]), abs_bf16x2(w[7])))));
+    uint32_t m = cta_max(max(m2 & 0xFFFFu, m2 >> 16), s_m);
+    if (gridDim.x > 1) {
+      const uint32_t rank = ptx::cluster_ctarank();
+      if (threadIdx.x < gridDim.x) ptx::st_shared_cluster_u32(ptx::map_to_cta(ptx::smem_u32(s_peer + rank), threadIdx.x), m);
+      ptx::cluster_sync();
+      m = 0;
+      for (int i = 0; i < (int)gridDim.x; ++i) m = max(m, s_peer[i]);
+    }
+    const float g = global_scale_of(m, src.max_scale);
+    if (it == 0) *src.g_out = g;
+    alpha = alpha_of(g);
+  } else {
+    alpha = resolve_alpha<true>(src, s_m);
+  }
+  {
+    const uint32_t *w = v.w;
+    const float s = __fmul_rn(alpha, __fmul_rn(amax16_bf16(w), kOneSixth));
+    uint16_t pk;
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(pk) : "f"(0.0f), "f"(s));
+    const uint32_t sb = pk & 0x7Fu;
+    const __half_raw h = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)sb, __NV_E4M3);
+    const float r = __fmul_rn(alpha, sb ? __frcp_rn(__half2float(__half(h))) : 0.0f);
+    uint32_t word = sb << (8 * (threadIdx.x & 3));
+    word |= __shfl_xor_sync(0xFFFFFFFFu, word, 1);
+    word |= __shfl_xor_sync(0xFFFFFFFFu, word, 2);
+    if (it < items) {
+      uint2 codes;
+      codes.x = quantize8_x2(w[0], w[1], w[2], w[3], r);
+      codes.y = quantize8_x2(w[4], w[5], w[6], w[7], r);
+      *reinterpret_cast<uint2 *>(out + (int64_t)it * 8) = codes;
+      if ((blk & 3) == 0) sf[sf_word(b, row, blk >> 2)] = word;
+    }
+  }
+}
+
+// ----------------------------------------------------------------------------------------
 // Global scale: max|x| / max_scale.  Division is monotonic, so each CTA divides its own
 // maximum and combines with an integer atomicMax on the (non-negative) float bits, the
 // same scheme as the reference's Triton kernel (python/ac4k_kernel/ops/quant.py:21-46).
 // ----------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(512)
-global_scale_kernel(const uint16_t *__restrict__ x, int64_t n, float max_scale, float *g_out) {
+// this thread's share of max|x| (bf16 bits) of `n` contiguous values
+__device__ __forceinline__ uint32_t thread_amax(const uint16_t *__restrict__ x, int64_t n) {
   uint32_t m2 = 0;   // packed pair of running maxima (bf16 bits, sign cleared)
   uint32_t m1 = 0;   // scalar head/tail
   // head: elements before the first 16-byte boundary
@@ -353,21 +490,25 @@ global_scale_kernel(const uint16_t *__restrict__ x, int64_t n, float max_scale, 
     uint32_t e = x[tail0 + tid] & 0x7FFFu;
     m1 = e > m1 ? e : m1;
   }
-  uint32_t m = max(max(m2 & 0xFFFFu, m2 >> 16), m1);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+  return max(max(m2 & 0xFFFFu, m2 >> 16), m1);
+}
+
+__global__ void __launch_bounds__(512)
+global_scale_kernel(const uint16_t *__restrict__ x, int64_t n, float max_scale, float *g_out) {
   __shared__ uint32_t s_m[16];
-  if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    m = threadIdx.x < (blockDim.x >> 5) ? s_m[threadIdx.x] : 0;
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-    if (threadIdx.x == 0 && m != 0) {
-      const float g = __fdiv_rn(bf16_bits_to_f32(m), max_scale);
-      atomicMax(reinterpret_cast<int *>(g_out), __float_as_int(g));
-    }
-  }
+  const uint32_t m = cta_max(thread_amax(x, n), s_m);
+  if (threadIdx.x == 0 && m != 0) atomicMax(reinterpret_cast<int *>(g_out), __float_as_int(global_scale_of(m, max_scale)));
+}
+
+// The same reduction up to one value per CTA; the quantiser that follows finishes it (ScaleSource).
+__global__ void __launch_bounds__(512)
+amax_partial_kernel(const uint16_t *__restrict__ x, int64_t n, uint32_t *__restrict__ partial) {
+  __shared__ uint32_t s_m[16];
+  // in this order: a quantiser that is running has every CTA of this grid past its wait, so `x` is complete for it too
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const uint32_t m = cta_max(thread_amax(x, n), s_m);
+  if (threadIdx.x == 0) partial[blockIdx.x] = m;
 }
 
 }  // namespace ac4k
@@ -403,27 +544,36 @@ extern "C" int ac4k_global_scale_bf16(const void *x, int64_t numel, float max_sc
   return 0;
 }
 
-extern "C" int ac4k_quantize_nvfp4(void *out, void *sf, const void *in, const float *global_scale,
-                                   const int64_t shape[4], const int64_t stride[4], int swizzle,
-                                   int sf_layout, ac4k_stream_t stream_) {
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+static int check_quantize(const void *out, const void *sf, const void *in, const int64_t shape[4], const int64_t stride[4], int sf_layout) {
   if (int e = check_view(shape, stride)) return e;
-  if (!out || !sf || !global_scale) return fail(AC4K_ERR_NULL, "out/sf/global_scale is NULL");
+  if (!out || !sf) return fail(AC4K_ERR_NULL, "out/sf is NULL");
   if (sf_layout != AC4K_SF_AC4K && sf_layout != AC4K_SF_TILE128X4)
     return fail(AC4K_ERR_ENUM, "unknown sf_layout %d", sf_layout);
-  const int64_t d0 = shape[0], d1 = shape[1], M = shape[2], K = shape[3];
-  const int64_t nbatch = d0 * d1;
-  if (nbatch == 0 || M == 0 || K == 0) return 0;   // nothing to write (padding needs K > 0 rows)
+  const int64_t nbatch = shape[0] * shape[1];
+  if (nbatch == 0 || shape[2] == 0 || shape[3] == 0) return 0;   // nothing to write (padding needs K > 0 rows)
   if (!in) return fail(AC4K_ERR_NULL, "in is NULL");
   if (nbatch > 65535) return fail(AC4K_ERR_SHAPE, "outer dims product %lld exceeds 65535", (long long)nbatch);
   if ((reinterpret_cast<uintptr_t>(out) & 7) || (reinterpret_cast<uintptr_t>(sf) & 3))
     return fail(AC4K_ERR_ALIGN, "out must be 8-byte and sf 4-byte aligned");
+  return 0;
+}
+
+// rows contiguous along K in whole 16-byte pieces, no permutation: the tiled and flat kernels
+static bool rows_vectorised(const void *in, const int64_t shape[4], const int64_t stride[4], int swizzle) {
+  return !swizzle && stride[3] == 1 && (shape[3] % 16 == 0) && (stride[2] % 8 == 0) && (stride[0] % 8 == 0) && (stride[1] % 8 == 0) &&
+         ((reinterpret_cast<uintptr_t>(in) & 15) == 0);
+}
+
+template <bool PARTIAL>
+static int quantize_impl(void *out, void *sf, const void *in, const ScaleSource &src, const int64_t shape[4], const int64_t stride[4],
+                         int swizzle, int sf_layout, cudaStream_t stream) {
+  const int64_t d0 = shape[0], d1 = shape[1], M = shape[2], K = shape[3];
+  const int64_t nbatch = d0 * d1;
   const int64_t Kp = align_up(K, 64);
   const uint16_t *inp = static_cast<const uint16_t *>(in);
 
-  const bool vec_ok = !swizzle && stride[3] == 1 && (K % 16 == 0) && (stride[2] % 8 == 0) &&
-                      (stride[0] % 8 == 0) && (stride[1] % 8 == 0) &&
-                      ((reinterpret_cast<uintptr_t>(in) & 15) == 0);
+  const bool vec_ok = rows_vectorised(in, shape, stride, swizzle);
+  int rc = 0;
   if (vec_ok) {
     const bool wide = (stride[2] % 16 == 0) && (stride[0] % 16 == 0) && (stride[1] % 16 == 0) &&
                       ((reinterpret_cast<uintptr_t>(in) & 31) == 0);
@@ -431,9 +581,9 @@ extern "C" int ac4k_quantize_nvfp4(void *out, void *sf, const void *in, const fl
     dim3 grid((unsigned)ceil_div(Kp, (int64_t)tile_k), (unsigned)ceil_div(M, kTileRows), (unsigned)nbatch);
     if (ceil_div(M, kTileRows) > 65535) return fail(AC4K_ERR_SHAPE, "M too large");
 #define AC4K_LAUNCH_TILED(L, W, T)                                                                \
-  nvfp4_quantize_tiled_kernel<L, W, T><<<grid, kThreads, 0, stream>>>(                            \
-      static_cast<uint8_t *>(out), static_cast<uint32_t *>(sf), inp, global_scale, M, K, d1,      \
-      stride[0], stride[1], stride[2])
+  rc = launch_kernel<PARTIAL>(nvfp4_quantize_tiled_kernel<L, W, T, PARTIAL>, grid, kThreads, 0, stream, \
+                                 static_cast<uint8_t *>(out), static_cast<uint32_t *>(sf), inp, src, M, K, d1, \
+                                 stride[0], stride[1], stride[2])
 #define AC4K_LAUNCH_TILED_K(L, W)                                                                 \
   do { if (tile_k == 128) AC4K_LAUNCH_TILED(L, W, 128); else AC4K_LAUNCH_TILED(L, W, 256); } while (0)
     if (sf_layout == AC4K_SF_AC4K) {
@@ -443,8 +593,7 @@ extern "C" int ac4k_quantize_nvfp4(void *out, void *sf, const void *in, const fl
     }
 #undef AC4K_LAUNCH_TILED_K
 #undef AC4K_LAUNCH_TILED
-    AC4K_LAUNCH_CHECK("nvfp4_quantize_tiled_kernel");
-    return 0;
+    return rc;
   }
 
   const int64_t rows_sf = (sf_layout == AC4K_SF_AC4K) ? align_up(M, 16) : align_up(M, 128);
@@ -456,16 +605,15 @@ extern "C" int ac4k_quantize_nvfp4(void *out, void *sf, const void *in, const fl
   if (tr_ok) {
     dim3 g((unsigned)ceil_div(Kp, 128), (unsigned)ceil_div(M, 128), (unsigned)nbatch);
 #define AC4K_LAUNCH_TR(L, P)                                                                                        \
-  nvfp4_quantize_transposed_kernel<L, P><<<g, 256, 0, stream>>>(static_cast<uint8_t *>(out), static_cast<uint8_t *>(sf), inp, \
-                                                                global_scale, M, K, d1, stride[0], stride[1], stride[3])
+  rc = launch_kernel<PARTIAL>(nvfp4_quantize_transposed_kernel<L, P, PARTIAL>, g, 256, 0, stream, static_cast<uint8_t *>(out), \
+                                 static_cast<uint8_t *>(sf), inp, src, M, K, d1, stride[0], stride[1], stride[3])
     if (sf_layout == AC4K_SF_AC4K) {
       if (swizzle) AC4K_LAUNCH_TR(AC4K_SF_AC4K, true); else AC4K_LAUNCH_TR(AC4K_SF_AC4K, false);
     } else {
       if (swizzle) AC4K_LAUNCH_TR(AC4K_SF_TILE128X4, true); else AC4K_LAUNCH_TR(AC4K_SF_TILE128X4, false);
     }
 #undef AC4K_LAUNCH_TR
-    AC4K_LAUNCH_CHECK("nvfp4_quantize_transposed_kernel");
-    return 0;
+    return rc;
   }
   dim3 grid;
   if (row_fastest)
@@ -474,9 +622,9 @@ extern "C" int ac4k_quantize_nvfp4(void *out, void *sf, const void *in, const fl
     grid = dim3((unsigned)ceil_div(Kp / 16, 32), (unsigned)ceil_div(rows_sf, 8), (unsigned)nbatch);
   if (grid.y > 65535) return fail(AC4K_ERR_SHAPE, "M too large for the strided path");
 #define AC4K_LAUNCH_STRIDED(L, P, R)                                                             \
-  nvfp4_quantize_strided_kernel<L, P, R><<<grid, 256, 0, stream>>>(                              \
-      static_cast<uint8_t *>(out), static_cast<uint8_t *>(sf), inp, global_scale, M, K, d1,      \
-      stride[0], stride[1], stride[2], stride[3])
+  rc = launch_kernel<PARTIAL>(nvfp4_quantize_strided_kernel<L, P, R, PARTIAL>, grid, 256, 0, stream, \
+                                 static_cast<uint8_t *>(out), static_cast<uint8_t *>(sf), inp, src, M, K, d1, \
+                                 stride[0], stride[1], stride[2], stride[3])
   const int sel = (sf_layout == AC4K_SF_TILE128X4 ? 4 : 0) | (swizzle ? 2 : 0) | (row_fastest ? 1 : 0);
   switch (sel) {
     case 0: AC4K_LAUNCH_STRIDED(AC4K_SF_AC4K, false, false); break;
@@ -489,6 +637,112 @@ extern "C" int ac4k_quantize_nvfp4(void *out, void *sf, const void *in, const fl
     default: AC4K_LAUNCH_STRIDED(AC4K_SF_TILE128X4, true, true); break;
   }
 #undef AC4K_LAUNCH_STRIDED
-  AC4K_LAUNCH_CHECK("nvfp4_quantize_strided_kernel");
+  return rc;
+}
+
+extern "C" int ac4k_quantize_nvfp4(void *out, void *sf, const void *in, const float *global_scale,
+                                   const int64_t shape[4], const int64_t stride[4], int swizzle,
+                                   int sf_layout, ac4k_stream_t stream) {
+  if (!global_scale) return fail(AC4K_ERR_NULL, "global_scale is NULL");
+  if (int e = check_quantize(out, sf, in, shape, stride, sf_layout)) return e;
+  if (shape[0] * shape[1] == 0 || shape[2] == 0 || shape[3] == 0) return 0;
+  const ScaleSource src{global_scale, nullptr, 0, 0.0f, nullptr, false};
+  return quantize_impl<false>(out, sf, in, src, shape, stride, swizzle, sf_layout, static_cast<cudaStream_t>(stream));
+}
+
+// The flat kernel over one cluster: at most 8 CTAs of a block per thread (four blocks per thread were slower than two
+// launches over the whole chip: 9.6 against 6.5 us for 50 x 8192)
+static constexpr int kFlatThreads = 1024;
+static_assert(AC4K_QUANTIZE_ONE_LAUNCH_BLOCKS == 8 * kFlatThreads, "one block per thread of the largest cluster");
+
+template <int L>
+static int launch_flat(void *out, void *sf, const void *in, const ScaleSource &src, const int64_t shape[4], const int64_t stride[4],
+                       int64_t items, bool cluster, cudaStream_t stream) {
+  const int64_t nbatch = shape[0] * shape[1];
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  uint8_t *o = static_cast<uint8_t *>(out);
+  uint32_t *f = static_cast<uint32_t *>(sf);
+  const uint16_t *x = static_cast<const uint16_t *>(in);
+  if (cluster) {
+    // as many CTAs as give a thread one block (or four padding words), up to eight
+    const int64_t rows_sf = align_up(shape[2], L == AC4K_SF_AC4K ? 16 : 128);
+    const int64_t work = items + nbatch * (rows_sf - shape[2]) * ceil_div(shape[3], 64) / 4;
+    int ctas = 1;
+    while (ctas < 8 && (int64_t)ctas * kFlatThreads < work) ctas *= 2;
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3((unsigned)(ctas == 1 ? align_up(work, 128) : kFlatThreads));
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = ctas;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+    AC4K_CUDA_TRY(cudaLaunchKernelEx(&cfg, nvfp4_quantize_flat_kernel<L, true, kFlatThreads>, o, f, x, src, (int)shape[2],
+                                     (int)shape[3], (int)nbatch, (int)shape[1], stride[0], stride[1], stride[2]));
+    return 0;
+  }
+  cfg.gridDim = dim3((unsigned)ceil_div(items, 256));
+  cfg.blockDim = dim3(256);
+  AC4K_CUDA_TRY(cudaLaunchKernelEx(&cfg, nvfp4_quantize_flat_kernel<L, false, 256>, o, f, x, src, (int)shape[2], (int)shape[3],
+                                   (int)nbatch, (int)shape[1], stride[0], stride[1], stride[2]));
   return 0;
+}
+
+template <bool OVERLAP>
+static int launch_reduction(unsigned blocks, const uint16_t *x, int64_t n, uint32_t *partial, cudaStream_t stream) {
+  return launch_kernel<OVERLAP>(amax_partial_kernel, dim3(blocks), 512, 0, stream, x, n, partial);
+}
+
+extern "C" int ac4k_quantize_nvfp4_dynamic(void *out, void *sf, float *g_out, void *scratch, const void *in, float max_scale,
+                                           const int64_t shape[4], const int64_t stride[4], int swizzle, int sf_layout,
+                                           ac4k_stream_t stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (!g_out) return fail(AC4K_ERR_NULL, "g_out is NULL");
+  if (!(max_scale > 0.0f)) return fail(AC4K_ERR_SHAPE, "max_scale must be positive");
+  if (int e = check_quantize(out, sf, in, shape, stride, sf_layout)) return e;
+  const int64_t nbatch = shape[0] * shape[1], M = shape[2], K = shape[3];
+  const int64_t numel = nbatch * M * K;
+  if (numel == 0) return ac4k_global_scale_bf16(in, 0, max_scale, g_out, stream_);
+  if (reinterpret_cast<uintptr_t>(in) & 1) return fail(AC4K_ERR_ALIGN, "in must be 2-byte aligned");
+  DeviceInfo di;
+  if (int e = get_device_info(&di)) return e;
+  // Routes by size (measured on a B200; microseconds of the whole call on resident inputs stand beside the kernels):
+  //   whole tensor in the registers of one cluster            one launch
+  //   up to 2^24 elements                                      maxima per CTA, then a quantiser that reduces them: two launches,
+  //                                                            the second one set up under the first
+  //   larger                                                   zeroed accumulator + atomic maximum + quantiser: a few hundred
+  //                                                            words read by each of thousands of CTAs would cost more
+  const bool vec = rows_vectorised(in, shape, stride, swizzle);
+  const int64_t Kp = align_up(K, 64), items = nbatch * M * (Kp / 16);
+  ScaleSource src{nullptr, nullptr, 0, max_scale, g_out, false};
+  if (vec && items <= AC4K_QUANTIZE_ONE_LAUNCH_BLOCKS)
+    return sf_layout == AC4K_SF_AC4K ? launch_flat<AC4K_SF_AC4K>(out, sf, in, src, shape, stride, items, true, stream)
+                                     : launch_flat<AC4K_SF_TILE128X4>(out, sf, in, src, shape, stride, items, true, stream);
+  if (!scratch || numel > (1 << 24)) {
+    if (int e = ac4k_global_scale_bf16(in, numel, max_scale, g_out, stream_)) return e;
+    src.g = g_out;
+    // what the reduction read last is still in L2: begin there
+    src.last_first = nbatch == 1;
+    return quantize_impl<false>(out, sf, in, src, shape, stride, swizzle, sf_layout, stream);
+  }
+  // 128 x 256 tiles from one CTA per SM on; below that the flat kernel's 256 blocks per CTA fill the chip better.  Under the
+  // flat one the reduction itself may start under the kernel before it (22.9 -> 21.3 us for quantise + GEMM at
+  // 666 x 4096 x 4096); on larger tensors the three kernels then compete (55.8 -> 57.6 us at 4096^3).  Letting the GEMM start while the
+  // reduction still waits, for the sake of its weight prefetch, costs 2.4 us at 50 x 8192 x 8192 and gains nothing at 1 row.
+  const int64_t tiles = ceil_div(Kp, Kp <= 128 ? 128 : 256) * ceil_div(M, kTileRows) * nbatch;
+  const bool flat = vec && tiles < di.sms;
+  const int64_t blocks = std::min<int64_t>(std::min<int64_t>(ceil_div(ceil_div(numel, 8), 512 * 2), (int64_t)di.sms * 2), AC4K_QUANTIZE_SCRATCH_BYTES / 4);
+  src.partial = static_cast<const uint32_t *>(scratch);
+  src.n_partial = (int)blocks;
+  auto *const launch_amax = flat ? &launch_reduction<true> : &launch_reduction<false>;
+  if (int e = launch_amax((unsigned)blocks, static_cast<const uint16_t *>(in), numel, static_cast<uint32_t *>(scratch), stream)) return e;
+  if (flat)
+    return sf_layout == AC4K_SF_AC4K ? launch_flat<AC4K_SF_AC4K>(out, sf, in, src, shape, stride, items, false, stream)
+                                     : launch_flat<AC4K_SF_TILE128X4>(out, sf, in, src, shape, stride, items, false, stream);
+  return quantize_impl<true>(out, sf, in, src, shape, stride, swizzle, sf_layout, stream);
 }

@@ -42,22 +42,28 @@ __device__ __forceinline__ uint8_t convert1(uint32_t bits16, float r) {
   return (uint8_t)f32_to_s8_rni_sat(f);
 }
 
-__device__ __forceinline__ float load_scale_max(const void *p, int is_int) {
-  return is_int ? (float)__ldg(static_cast<const int32_t *>(p)) : __ldg(static_cast<const float *>(p));
+// The largest code: a scalar on the device (fp32 or int32), or - p NULL - a value of the launch.
+struct ScaleMax {
+  const void *p;
+  int is_int;
+  float v;
+};
+__device__ __forceinline__ float load_scale_max(const ScaleMax &m) {
+  if (m.p == nullptr) return m.v;
+  return m.is_int ? (float)__ldg(static_cast<const int32_t *>(m.p)) : __ldg(static_cast<const float *>(m.p));
 }
 
 // ----------------------------------------------------------------------------------------
 // Contiguous rows.  A group of G threads (32 = one warp, or 256 = the CTA) owns one row and
 // caches up to CACHE 16-byte chunks per thread; longer rows are re-read for the second pass.
 // ----------------------------------------------------------------------------------------
-template <int FMT, int G, int CACHE>
-__global__ void __launch_bounds__(256)
+template <int FMT, int G, int CACHE, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 rowwise_quantize_kernel(uint8_t *__restrict__ out, float *__restrict__ sf,
-                        const uint16_t *__restrict__ in, const void *__restrict__ scale_max_p,
-                        int scale_max_is_int, int64_t M, int64_t K, int64_t d1, int64_t stride0,
+                        const uint16_t *__restrict__ in, const ScaleMax scale_max, int64_t M, int64_t K, int64_t d1, int64_t stride0,
                         int64_t stride1, int64_t row_stride) {
-  constexpr int ROWS = 256 / G;
-  __shared__ uint32_t s_m[8];
+  constexpr int ROWS = THREADS / G;
+  __shared__ uint32_t s_m[THREADS / 32];
   const int64_t Kp = align_up(K, 16);
   const int64_t M16 = align_up(M, 16);
   const int64_t batch = blockIdx.y;
@@ -70,6 +76,8 @@ rowwise_quantize_kernel(uint8_t *__restrict__ out, float *__restrict__ sf,
 
   uint4 v[CACHE];
   uint32_t m2 = 0;
+  grid_dependency_wait();
+  grid_launch_dependents();
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {
     const int64_t ch = (int64_t)c * G + t;
@@ -89,15 +97,16 @@ rowwise_quantize_kernel(uint8_t *__restrict__ out, float *__restrict__ sf,
   uint32_t m = max(m2 & 0xFFFFu, m2 >> 16);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-  if (G == 256) {
+  if (G > 32) {
+    static_assert(G == 32 || G == THREADS, "a row per warp or per CTA");
     if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
     __syncthreads();
     m = s_m[0];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) m = max(m, s_m[i]);
+    for (int i = 1; i < THREADS / 32; ++i) m = max(m, s_m[i]);
   }
   const float amax = bf16_bits_to_f32(m);
-  const float smax = load_scale_max(scale_max_p, scale_max_is_int);
+  const float smax = load_scale_max(scale_max);
   if (t == 0 && row < M16) sf[batch * M16 + row] = live ? __fdiv_rn(amax, smax) : 0.0f;
   if (!live) return;
   const float r = __fdiv_rn(smax, amax);
@@ -122,8 +131,7 @@ rowwise_quantize_kernel(uint8_t *__restrict__ out, float *__restrict__ sf,
 template <int FMT, bool PERMUTE>
 __global__ void __launch_bounds__(256)
 rowwise_quantize_strided_kernel(uint8_t *__restrict__ out, float *__restrict__ sf,
-                                const uint16_t *__restrict__ in, const void *__restrict__ scale_max_p,
-                                int scale_max_is_int, int64_t M, int64_t K, int64_t d1,
+                                const uint16_t *__restrict__ in, const ScaleMax scale_max, int64_t M, int64_t K, int64_t d1,
                                 int64_t stride0, int64_t stride1, int64_t stride_m, int64_t stride_k) {
   const int64_t Kp = align_up(K, 16);
   const int64_t M16 = align_up(M, 16);
@@ -142,7 +150,7 @@ rowwise_quantize_strided_kernel(uint8_t *__restrict__ out, float *__restrict__ s
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
   const float amax = bf16_bits_to_f32(m);
-  const float smax = load_scale_max(scale_max_p, scale_max_is_int);
+  const float smax = load_scale_max(scale_max);
   if (lane == 0) sf[batch * M16 + row] = live ? __fdiv_rn(amax, smax) : 0.0f;
   if (!live) return;
   const float r = __fdiv_rn(smax, amax);
@@ -202,7 +210,7 @@ colmax_kernel(float *__restrict__ sf, const uint16_t *__restrict__ in, int64_t M
 template <int FMT, bool PERMUTE>
 __global__ void __launch_bounds__(256)
 transpose_quantize_kernel(uint8_t *__restrict__ out, const float *__restrict__ amax_bits, const uint16_t *__restrict__ in,
-                          const void *__restrict__ scale_max_p, int scale_max_is_int, int64_t M, int64_t K, int64_t M16, int64_t d1,
+                          const ScaleMax scale_max, int64_t M, int64_t K, int64_t M16, int64_t d1,
                           int64_t stride0, int64_t stride1, int64_t stride_k) {
   __shared__ uint32_t tile[kTrCols][kTrRows / 4 + 1];       // [column][4 reduce-rows per word], padded
   __shared__ float rs[kTrCols];
@@ -210,7 +218,7 @@ transpose_quantize_kernel(uint8_t *__restrict__ out, const float *__restrict__ a
   const int64_t Kp = align_up(K, 16);
   const int64_t c0 = (int64_t)blockIdx.y * kTrCols, k0 = (int64_t)blockIdx.x * kTrRows;
   const uint16_t *base = in + (batch / d1) * stride0 + (batch % d1) * stride1;
-  const float smax = load_scale_max(scale_max_p, scale_max_is_int);
+  const float smax = load_scale_max(scale_max);
   if (threadIdx.x < kTrCols) {
     const int64_t c = c0 + threadIdx.x;
     rs[threadIdx.x] = c < M ? __fdiv_rn(smax, __ldg(amax_bits + batch * M16 + c)) : 0.0f;
@@ -261,22 +269,85 @@ transpose_quantize_kernel(uint8_t *__restrict__ out, const float *__restrict__ a
   }
 }
 
-__global__ void colmax_to_scale_kernel(float *__restrict__ sf, const void *__restrict__ scale_max_p, int scale_max_is_int, int64_t M,
+__global__ void colmax_to_scale_kernel(float *__restrict__ sf, const ScaleMax scale_max, int64_t M,
                                        int64_t M16, int64_t total) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
-  const float smax = load_scale_max(scale_max_p, scale_max_is_int);
+  const float smax = load_scale_max(scale_max);
   sf[i] = (i % M16) < M ? __fdiv_rn(sf[i], smax) : 0.0f;
 }
 
+// ----------------------------------------------------------------------------------------
+// The same case (columns contiguous) over a short reduce dimension, in one launch instead of four: a CTA takes 64 columns
+// of one batch entry, walks the reduce dimension twice (the second time from L1 / L2), and transposes 64 x 64 pieces
+// through shared memory.  Single 2-byte loads, so odd row lengths and any alignment are taken too.
+// ----------------------------------------------------------------------------------------
+static constexpr int kShortCols = 64, kShortThreads = 512, kShortGroups = kShortThreads / kShortCols;
+static constexpr int kShortMaxK = 512;
+
+template <int FMT, bool PERMUTE>
+__global__ void __launch_bounds__(kShortThreads)
+column_quantize_short_kernel(uint8_t *__restrict__ out, float *__restrict__ sf, const uint16_t *__restrict__ in, const ScaleMax scale_max,
+                             int64_t M, int K, int64_t M16, int64_t d1, int64_t stride0, int64_t stride1, int64_t stride_k) {
+  __shared__ uint32_t red[kShortGroups][kShortCols];
+  __shared__ uint32_t tile[kShortCols][kShortCols / 4 + 1];       // [column][4 reduce-rows per word], padded
+  const int64_t batch = blockIdx.y;
+  const int cx = threadIdx.x & (kShortCols - 1), ry = threadIdx.x / kShortCols;
+  const int64_t col = (int64_t)blockIdx.x * kShortCols + cx;
+  const uint16_t *base = in + (batch / d1) * stride0 + (batch % d1) * stride1 + col;
+  const bool live = col < M;
+  const int Kp = (K + 15) / 16 * 16;
+  uint32_t m = 0;
+  grid_dependency_wait();
+  grid_launch_dependents();
+  if (live) {
+#pragma unroll 8
+    for (int k = ry; k < K; k += kShortGroups) m = max(m, (uint32_t)__ldg(base + (int64_t)k * stride_k) & 0x7FFFu);
+  }
+  red[ry][cx] = m;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kShortGroups; ++i) m = max(m, red[i][cx]);
+  const float amax = bf16_bits_to_f32(m), smax = load_scale_max(scale_max);
+  if (ry == 0 && col < M16) sf[batch * M16 + col] = live ? __fdiv_rn(amax, smax) : 0.0f;
+  const float r = live ? __fdiv_rn(smax, amax) : 0.0f;
+  for (int k0 = 0; k0 < Kp; k0 += kShortCols) {
+    __syncthreads();                                              // the piece before this one has been written out
+#pragma unroll
+    for (int i = 0; i < kShortCols / 4 / kShortGroups; ++i) {
+      const int kq = ry + kShortGroups * i;
+      float a[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int k = k0 + 4 * kq + j;
+        const uint32_t e = live && k < K ? (uint32_t)__ldg(base + (int64_t)k * stride_k) : 0u;
+        a[j] = __fmul_rn(bf16_bits_to_f32(e), r);                 // (padding: 0 * r, NaN for a column of zeros like the rest)
+      }
+      tile[cx][kq] = FMT == kFmtE4M3 ? f32x4_to_e4m3x4(a[0], a[1], a[2], a[3]) : f32x4_to_s8x4(a[0], a[1], a[2], a[3]);
+    }
+    __syncthreads();
+    if (threadIdx.x < kShortCols * 4) {
+      const int c = threadIdx.x >> 2, g = threadIdx.x & 3;
+      const int64_t oc = (int64_t)blockIdx.x * kShortCols + c;
+      const int k = k0 + 16 * g;
+      if (oc < M && k < Kp) {
+        const uint32_t n0 = tile[c][4 * g], n1 = tile[c][4 * g + 1], n2 = tile[c][4 * g + 2], n3 = tile[c][4 * g + 3];
+        uint4 o = make_uint4(n0, n1, n2, n3);
+        if (PERMUTE) o = make_uint4(__byte_perm(n0, n2, 0x5410), __byte_perm(n0, n2, 0x7632), __byte_perm(n1, n3, 0x5410), __byte_perm(n1, n3, 0x7632));
+        *reinterpret_cast<uint4 *>(out + (batch * M + oc) * Kp + k) = o;
+      }
+    }
+  }
+}
+
 template <int FMT>
-static int launch_rowwise(void *out, float *sf, const void *in, const void *scale_max, int is_int,
+static int launch_rowwise(void *out, float *sf, const void *in, const ScaleMax &scale_max,
                           const int64_t shape[4], const int64_t stride[4], int swizzle,
                           cudaStream_t stream) {
   if (!shape || !stride) return fail(AC4K_ERR_NULL, "shape/stride is NULL");
   for (int i = 0; i < 4; ++i)
     if (shape[i] < 0) return fail(AC4K_ERR_SHAPE, "shape[%d] is negative", i);
-  if (!out || !sf || !scale_max) return fail(AC4K_ERR_NULL, "out/sf/scale_max is NULL");
+  if (!out || !sf) return fail(AC4K_ERR_NULL, "out/sf is NULL");
   const int64_t d1 = shape[1], M = shape[2], K = shape[3];
   const int64_t nbatch = shape[0] * shape[1];
   if (nbatch == 0 || M == 0) return 0;
@@ -291,19 +362,24 @@ static int launch_rowwise(void *out, float *sf, const void *in, const void *scal
                       ((reinterpret_cast<uintptr_t>(in) & 15) == 0) &&
                       ((reinterpret_cast<uintptr_t>(out) & 7) == 0);
   if (vec_ok) {
-    if (K <= 32 * 8 * 4) {   // short rows: one warp per row, 8 rows per CTA
-      dim3 grid((unsigned)ceil_div(M16, 8), (unsigned)nbatch);
-      rowwise_quantize_kernel<FMT, 32, 4><<<grid, 256, 0, stream>>>(outp, sf, inp, scale_max, is_int, M, K,
-                                                                   d1, stride[0], stride[1], stride[2]);
-    } else {                 // long rows: one CTA per row, 8192 elements cached in registers
-      dim3 grid((unsigned)M16, (unsigned)nbatch);
-      rowwise_quantize_kernel<FMT, 256, 4><<<grid, 256, 0, stream>>>(outp, sf, inp, scale_max, is_int, M, K,
-                                                                    d1, stride[0], stride[1], stride[2]);
-    }
-    AC4K_LAUNCH_CHECK("rowwise_quantize_kernel");
-    return 0;
+    // Rows of up to 1024 elements: a warp each.  Longer ones: a CTA each, as small as leaves a thread four or five vectors, so
+    // that a thread has them all in flight and an SM many CTAs.  [4099, 5120] to FP8: 13.4 us with 256 threads (2.5 vectors
+    // each), 10.4 us with 128 (6.0 TB/s); [8000, 2048]: 18.3 and 12.4 (64 threads); equal at 8192 columns.
+#define AC4K_LAUNCH_ROWS(G, C, T) \
+  return launch_kernel<true>(rowwise_quantize_kernel<FMT, G, C, T>, dim3((unsigned)ceil_div(M16, T / G), (unsigned)nbatch), T, 0, stream, outp, sf, \
+                             inp, scale_max, M, K, d1, stride[0], stride[1], stride[2])
+    if (K <= 32 * 8 * 4) AC4K_LAUNCH_ROWS(32, 4, 256);
+    if (K <= 64 * 8 * 4) AC4K_LAUNCH_ROWS(64, 4, 64);
+    if (K <= 128 * 8 * 5) AC4K_LAUNCH_ROWS(128, 5, 128);
+    AC4K_LAUNCH_ROWS(256, 4, 256);
+#undef AC4K_LAUNCH_ROWS
   }
-  // columns contiguous, rows strided: the transposing kernels
+  // columns contiguous, rows strided: one kernel over a short reduce dimension, else the transposing kernels
+  if (stride[2] == 1 && K > 0 && K <= kShortMaxK && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ceil_div(M16, kShortCols) <= 0x7fffffff) {
+    dim3 g((unsigned)ceil_div(M16, kShortCols), (unsigned)nbatch);
+    return launch_kernel<true>(swizzle ? column_quantize_short_kernel<FMT, true> : column_quantize_short_kernel<FMT, false>, g, kShortThreads, 0,
+                               stream, outp, sf, inp, scale_max, M, (int)K, M16, d1, stride[0], stride[1], stride[3]);
+  }
   const bool tr_ok = stride[2] == 1 && K > 0 && M % 2 == 0 && stride[3] % 2 == 0 && stride[0] % 2 == 0 && stride[1] % 2 == 0 &&
                      ((reinterpret_cast<uintptr_t>(in) & 3) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0) &&
                      ceil_div(K, kTrRows) <= 0x7fffffff && ceil_div(M, kTrCols) <= 65535;
@@ -314,24 +390,24 @@ static int launch_rowwise(void *out, float *sf, const void *in, const void *scal
     AC4K_LAUNCH_CHECK("colmax_kernel");
     dim3 g2((unsigned)ceil_div(align_up(K, 16), kTrRows), (unsigned)ceil_div(M, kTrCols), (unsigned)nbatch);
     if (swizzle)
-      transpose_quantize_kernel<FMT, true><<<g2, 256, 0, stream>>>(outp, sf, inp, scale_max, is_int, M, K, M16, d1, stride[0],
+      transpose_quantize_kernel<FMT, true><<<g2, 256, 0, stream>>>(outp, sf, inp, scale_max, M, K, M16, d1, stride[0],
                                                                    stride[1], stride[3]);
     else
-      transpose_quantize_kernel<FMT, false><<<g2, 256, 0, stream>>>(outp, sf, inp, scale_max, is_int, M, K, M16, d1, stride[0],
+      transpose_quantize_kernel<FMT, false><<<g2, 256, 0, stream>>>(outp, sf, inp, scale_max, M, K, M16, d1, stride[0],
                                                                     stride[1], stride[3]);
     AC4K_LAUNCH_CHECK("transpose_quantize_kernel");
     const int64_t total = nbatch * M16;
-    colmax_to_scale_kernel<<<(unsigned)ceil_div(total, 256), 256, 0, stream>>>(sf, scale_max, is_int, M, M16, total);
+    colmax_to_scale_kernel<<<(unsigned)ceil_div(total, 256), 256, 0, stream>>>(sf, scale_max, M, M16, total);
     AC4K_LAUNCH_CHECK("colmax_to_scale_kernel");
     return 0;
   }
   dim3 grid((unsigned)ceil_div(M16, 8), (unsigned)nbatch);
   if (swizzle)
     rowwise_quantize_strided_kernel<FMT, true><<<grid, 256, 0, stream>>>(
-        outp, sf, inp, scale_max, is_int, M, K, d1, stride[0], stride[1], stride[2], stride[3]);
+        outp, sf, inp, scale_max, M, K, d1, stride[0], stride[1], stride[2], stride[3]);
   else
     rowwise_quantize_strided_kernel<FMT, false><<<grid, 256, 0, stream>>>(
-        outp, sf, inp, scale_max, is_int, M, K, d1, stride[0], stride[1], stride[2], stride[3]);
+        outp, sf, inp, scale_max, M, K, d1, stride[0], stride[1], stride[2], stride[3]);
   AC4K_LAUNCH_CHECK("rowwise_quantize_strided_kernel");
   return 0;
 }
@@ -343,13 +419,27 @@ using namespace ac4k;
 extern "C" int ac4k_quantize_fp8(void *out, float *sf, const void *in, const float *scale_max,
                                  const int64_t shape[4], const int64_t stride[4], int swizzle,
                                  ac4k_stream_t stream) {
-  return launch_rowwise<kFmtE4M3>(out, sf, in, scale_max, 0, shape, stride, swizzle,
+  if (shape && stride && !scale_max) return fail(AC4K_ERR_NULL, "scale_max is NULL");
+  return launch_rowwise<kFmtE4M3>(out, sf, in, ScaleMax{scale_max, 0, 0.0f}, shape, stride, swizzle,
                                   static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int ac4k_quantize_int8(void *out, float *sf, const void *in, const int32_t *scale_max,
                                   const int64_t shape[4], const int64_t stride[4],
                                   ac4k_stream_t stream) {
-  return launch_rowwise<kFmtS8>(out, sf, in, scale_max, 1, shape, stride, 0,
+  if (shape && stride && !scale_max) return fail(AC4K_ERR_NULL, "scale_max is NULL");
+  return launch_rowwise<kFmtS8>(out, sf, in, ScaleMax{scale_max, 1, 0.0f}, shape, stride, 0,
+                                static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int ac4k_quantize_fp8_max(void *out, float *sf, const void *in, float scale_max, const int64_t shape[4],
+                                     const int64_t stride[4], int swizzle, ac4k_stream_t stream) {
+  return launch_rowwise<kFmtE4M3>(out, sf, in, ScaleMax{nullptr, 0, scale_max}, shape, stride, swizzle,
+                                  static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int ac4k_quantize_int8_max(void *out, float *sf, const void *in, int32_t scale_max, const int64_t shape[4],
+                                      const int64_t stride[4], ac4k_stream_t stream) {
+  return launch_rowwise<kFmtS8>(out, sf, in, ScaleMax{nullptr, 1, (float)scale_max}, shape, stride, 0,
                                 static_cast<cudaStream_t>(stream));
 }

@@ -81,6 +81,17 @@ int ac4k_quantize_nvfp4(void *out, void *sf, const void *in, const float *global
                         const int64_t shape[4], const int64_t stride[4], int swizzle,
                         int sf_layout, ac4k_stream_t stream);
 
+/* ac4k_global_scale_bf16 of `in` (dense: its elements are the product of `shape`, contiguous in memory from `in` on, in
+ * whatever order of the dimensions) followed by ac4k_quantize_nvfp4 with that scale, in as few launches as the size
+ * allows; g_out receives the scale.  scratch: AC4K_QUANTIZE_SCRATCH_BYTES on the device for this call alone (4-byte
+ * aligned, contents undefined before and after), or NULL, which costs a launch more on mid-size tensors (and nothing up
+ * to AC4K_QUANTIZE_ONE_LAUNCH_BLOCKS blocks of 16 in rows that are contiguous along K, K a multiple of 16). */
+#define AC4K_QUANTIZE_SCRATCH_BYTES 4096
+#define AC4K_QUANTIZE_ONE_LAUNCH_BLOCKS 8192
+int ac4k_quantize_nvfp4_dynamic(void *out, void *sf, float *g_out, void *scratch, const void *in, float max_scale,
+                                const int64_t shape[4], const int64_t stride[4], int swizzle, int sf_layout,
+                                ac4k_stream_t stream);
+
 /* Per-row (whole reduce dim) e4m3 quantiser.  Replaces ac4k::quantize_fp8,
  * include/ac4k_kernel/ops.h:31-33, lib/cuda/sm120/quantize_fp8.cu:192-290.
  *   out: [outer0, outer1, M, align16(K)] e4m3;  sf: [outer0, outer1, align16(M)] fp32. */
@@ -94,6 +105,12 @@ int ac4k_quantize_fp8(void *out, float *sf, const void *in, const float *scale_m
 int ac4k_quantize_int8(void *out, float *sf, const void *in, const int32_t *scale_max,
                        const int64_t shape[4], const int64_t stride[4],
                        ac4k_stream_t stream);
+
+/* The two per-row quantisers with the largest code as a value of the call instead of a scalar on the device. */
+int ac4k_quantize_fp8_max(void *out, float *sf, const void *in, float scale_max, const int64_t shape[4],
+                          const int64_t stride[4], int swizzle, ac4k_stream_t stream);
+int ac4k_quantize_int8_max(void *out, float *sf, const void *in, int32_t scale_max, const int64_t shape[4],
+                           const int64_t stride[4], ac4k_stream_t stream);
 
 /* D[M,N] = cast((A_gs*B_gs) * A_fp4[M,K] * B_fp4[N,K]^T + bias[N]).
  * Replaces ac4k::linear_nvfp4, include/ac4k_kernel/ops.h:43-48,
