@@ -99,15 +99,21 @@ def build(force: bool = False, verbose: bool = False, extra: str | None = None, 
 
 
 def build_pybind(force: bool = False) -> str:
-    """Compile the pybind11 `_cuda_ops` module (host code only) against torch's headers and link it to
-    libac4k_b200.so (found through an $ORIGIN-relative run path).  Returns the path of the module."""
+    """Compile the pybind11 modules (host code only) against torch's headers and link them to libac4k_b200.so
+    (found through an $ORIGIN-relative run path): `_host_calls`, the operators' host side, and `_cuda_ops`, the
+    reference's module.  Returns the path of the latter."""
+    _build_module("_host_calls", "host_calls.cc", force)
+    return _build_module("_cuda_ops", "bindings_pybind.cc", force)
+
+
+def _build_module(name: str, source: str, force: bool) -> str:
     import sysconfig
     import torch
     from torch.utils import cpp_extension
-    src = os.path.join(CSRC, "bindings_pybind.cc")
+    src = os.path.join(CSRC, source)
     out_dir = os.path.join(PKG_DIR, "native")
     os.makedirs(out_dir, exist_ok=True)
-    target = os.path.join(out_dir, "_cuda_ops" + sysconfig.get_config_var("EXT_SUFFIX"))
+    target = os.path.join(out_dir, name + sysconfig.get_config_var("EXT_SUFFIX"))
     deps = [src, os.path.join(ROOT, "include", "ac4k_b200.h"), os.path.abspath(__file__)]
     if not os.path.exists(LIB_PATH):
         build()
@@ -117,7 +123,7 @@ def build_pybind(force: bool = False) -> str:
     cuda_home = os.environ.get("CUDA_HOME") or "/usr/local/cuda"
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-           "-DTORCH_EXTENSION_NAME=_cuda_ops", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-DTORCH_EXTENSION_NAME={name}", "-DTORCH_API_INCLUDE_EXTENSION_H",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     for inc in cpp_extension.include_paths():
         cmd += ["-isystem", inc]

@@ -4,6 +4,12 @@
 same interface; both call the same C ABI."""
 
 
+try:
+    from . import _host_calls as host_calls      # the operators in one native call each (csrc/host_calls.cc)
+except ImportError:                              # not built: the Python wrappers make the same launches, at more host time
+    host_calls = None
+
+
 def load():
     """Import and return the compiled module; raises ImportError with the build command if it is not built."""
     try:

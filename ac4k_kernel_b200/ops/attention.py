@@ -12,6 +12,7 @@ import math
 import torch
 
 from .. import _cuda_ops
+from ..native import host_calls
 from .quant import quantize
 
 mha_nvfp4_fwd = _cuda_ops.mha_nvfp4_fwd
@@ -86,6 +87,10 @@ def _nvfp4_attention(q, k, v, layout, out=None):
 def attention(q, k, v, *, layout="BNHD", precision="int8+fp8e4m3", out=None):
     """q, k: [B, N, H, Dqk] or [B, H, N, Dqk] bf16; v: same with Dv; returns bf16 in q's layout.
     Keyword-only options and defaults of the reference (attention.py:196-204)."""
+    if host_calls is not None:
+        made = host_calls.attention(q, k, v, layout, precision, out)
+        if made is not None:
+            return made
     assert layout in ["BNHD", "BHND"], f"Unsupported layout: {layout}"
     assert precision in ["nvfp4", "int8+fp8e4m3"], f"Unsupported precision: {precision}"
     assert q.ndim == 4 and k.ndim == 4 and v.ndim == 4

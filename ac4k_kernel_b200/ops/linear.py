@@ -7,6 +7,7 @@ long as both operands use the same one.
 import torch
 
 from .. import _cuda_ops
+from ..native import host_calls
 
 linear_nvfp4 = _cuda_ops.linear_nvfp4
 
@@ -33,6 +34,10 @@ def linear(x, x_scale, x_global_scale, weight, weight_scale, weight_global_scale
     """x: packed nvfp4 [M, K/2] u8; weight: packed nvfp4 [N, K/2] u8; *_scale: e4m3 block
     scales; *_global_scale: fp32 0-dim; bias: [N] or [1, N] bf16/fp16/fp32; out: optional
     [M, N] bf16/fp16/fp32 (bf16 when allocated here).  Returns out."""
+    if host_calls is not None:
+        made = host_calls.linear(x, x_scale, x_global_scale, weight, weight_scale, weight_global_scale, bias, out)
+        if made is not None:
+            return made
     return _OP(x, x_scale, x_global_scale, weight, weight_scale, weight_global_scale, bias,
                out=out)
 
@@ -43,6 +48,11 @@ def linear_requant(x, x_scale, x_global_scale, weight, weight_scale, weight_glob
     epilogue rounds the result to bf16 and quantises it to NVFP4 (blocks of 16 along N), so the output
     can feed the next `linear()` directly.  Bit-identical to the two-call sequence; the reference has
     no counterpart.  Returns (packed [M, N/2] u8, block scales in `sf_layout`, out_global_scale)."""
+    if host_calls is not None:
+        made = host_calls.linear_requant(x, x_scale, x_global_scale, weight, weight_scale, weight_global_scale,
+                                         out_global_scale, bias, sf_layout)
+        if made is not None:
+            return made
     from .utils import align_up, ceil_div
     if (bias is not None) and (bias.ndim == 1):
         bias = bias.reshape(1, -1)

@@ -11,6 +11,7 @@ import torch
 
 from .utils import align_up, ceil_div
 from .. import _cuda_ops
+from ..native import host_calls
 
 quantize_nvfp4 = _cuda_ops.quantize_nvfp4
 quantize_fp8 = _cuda_ops.quantize_fp8
@@ -105,5 +106,9 @@ def quantize(input, cross_dim, reduce_dim, max_scale=None, precision="nvfp4", sw
     `max_scale` defaults to 6*448, 448 and 127.  `swizzle` permutes the reduce dim in groups
     of 32 ([4,4,2] -> (1,0,2)) for nvfp4 and of 16 ([2,4,2] -> (1,0,2)) for fp8e4m3.
     """
+    if host_calls is not None and output is None and sf is None:
+        made = host_calls.quantize(input, cross_dim, reduce_dim, max_scale, precision, swizzle, sf_layout)
+        if made is not None:
+            return made
     return _OP(input, cross_dim, reduce_dim, max_scale=max_scale, precision=precision,
                swizzle=swizzle, output=output, sf=sf, sf_layout=sf_layout)

@@ -7,6 +7,7 @@ from typing import Optional
 import torch
 
 from .. import _cuda_ops
+from ..native import host_calls
 
 rope3d_kernel = _cuda_ops.rope3d
 
@@ -27,4 +28,8 @@ def rope3d(x: torch.Tensor, grid_sizes: torch.Tensor, freqs: torch.Tensor,
            output: Optional[torch.Tensor] = None) -> torch.Tensor:
     """x: [B, S, N, D] bf16; grid_sizes: [B, 3] int32 (frames, height, width); freqs: [max_pos, D // 2] complex128;
     output: optional [B, S, N, D] bf16.  Returns output (positions behind a batch entry's grid are copied from x)."""
+    if host_calls is not None:
+        made = host_calls.rope3d(x, grid_sizes, freqs, output)
+        if made is not None:
+            return made
     return _OP(x, grid_sizes, freqs, output=output)
