@@ -26,7 +26,8 @@
 // next.  [1, 16384, 16, 128], kernel alone: 1 688 us with four warps per group, a row per thread, and O rescaled before the
 // exponentials (a wait for the previous P V and a chain of small loads and stores); 1 728 with eight warps per group, 1 654 with
 // the rescale behind the exponentials (a quarter of the exponentials as a polynomial on the FMA pipe); 1 640 with an eighth of
-// them there, 1 579 with none: the polynomial costs thirteen issue slots a pair, and those bound the kernel now.
+// them there, 1 579 with none: the polynomial costs thirteen issue slots a pair, and those bound the kernel now; 1 555 with the
+// two threads that share a block finishing one row's block scales each instead of both rows' twice.
 // Sharing one score buffer keeps the groups a few hundred cycles apart (group B's S is issued when group A has copied its own
 // out), so that one group's waits, maxima and fences run under the other's exponentials.
 // Tensor memory: S 128 + O_A 128 + O_B 128 + scales 40 columns of 512.
@@ -355,6 +356,7 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
     const int q = warp & 3;                   // tensor-memory lane quarter of the warp
     const int half = (warp >> 2) & 1;         // its 16 lanes of the quarter
     const int t4 = lane & 3;
+    const bool odd = t4 & 1;
     const int row_l = q * 32 + half * 16 + (lane >> 2);          // query rows of the thread inside the tile: row_l, row_l + 8
     const uint32_t lane_addr = (uint32_t)(q * 32 + half * 16) << 16;
     const uint32_t t_s = tmem_base + lane_addr + S_COL, t_o = tmem_base + lane_addr + O_COL + 128 * g;
@@ -397,20 +399,26 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       // positions 8 t4 .. 8 t4 + 7, so threads t4 = 0, 1 share the first block and 2, 3 the second.  ex2 is monotonic, so a
       // block's largest probability is ex2 of its largest score: it is known before the block's probabilities are, and
       // their conversion does not have to wait for all of them.
-      float bs[4][2], m_new[2];
+      // Of the two threads that share a block, the even one finishes the first row's maximum and the odd one the second's.
+      float own[4], m_new[2];
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
+      for (int gg = 0; gg < 4; ++gg) {
+        float x[2];
 #pragma unroll
-        for (int gg = 0; gg < 4; ++gg) {
+        for (int r = 0; r < 2; ++r) {
           float v[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(s[16 * gg + 4 * (i >> 1) + 2 * r + (i & 1)]);
-          const float x = max3(max3(v[0], v[1], v[2]), max3(v[3], v[4], v[5]), fmaxf(v[6], v[7]));
-          bs[gg][r] = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
+          x[r] = max3(max3(v[0], v[1], v[2]), max3(v[3], v[4], v[5]), fmaxf(v[6], v[7]));
         }
-        float v = max3(fmaxf(bs[0][r], bs[1][r]), bs[2][r], bs[3][r]);
+        own[gg] = fmaxf(odd ? x[1] : x[0], __shfl_xor_sync(0xffffffffu, odd ? x[0] : x[1], 1));
+      }
+      {
+        float v = max3(fmaxf(own[0], own[1]), own[2], own[3]);
         v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
-        m_new[r] = fmaxf(m[r], v * c1);
+        const float mine = fmaxf(odd ? m[1] : m[0], v * c1), other = __shfl_xor_sync(0xffffffffu, mine, 1);
+        m_new[0] = odd ? other : mine;
+        m_new[1] = odd ? mine : other;
       }
       const bool moved = j > 0 && __any_sync(0xffffffffu, m_new[0] != m[0] || m_new[1] != m[1]);     // warp-uniform
       float a[2] = {1.0f, 1.0f};
@@ -430,18 +438,20 @@ mha_nvfp4_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       // Probabilities, row sum, NVFP4 quantisation of P in blocks of 16 keys.
       const uint32_t p_row = p_row0 + (j & 1) * P_BYTES;
       const float2 c1_2 = make_float2(c1, c1);
+      const float m_own = odd ? m[1] : m[0];
 #pragma unroll
       for (int gg = 0; gg < 4; ++gg) {
-        // block scales of both rows: e4m3 byte (row 0 low) and, from the table, what the probabilities are multiplied with
-        const float b0 = ex2_approx(fmaf(bs[gg][0], c1, -m[0])), b1 = ex2_approx(fmaf(bs[gg][1], c1, -m[1]));
-        uint16_t sb2;
-        asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(sb2) : "f"(__fmul_rn(kPGlobal, __fmul_rn(b1, kOneSixth))),
-            "f"(__fmul_rn(kPGlobal, __fmul_rn(b0, kOneSixth))));
-        float sc[2];
+        // Block scale of the thread's own row: e4m3 byte and, from the table, what the block's probabilities are multiplied
+        // with; the other row's multiplier comes from the neighbour.
+        const float b = ex2_approx(fmaf(own[gg], c1, -m_own));
+        uint16_t sb;
+        asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(sb) : "f"(0.0f), "f"(__fmul_rn(kPGlobal, __fmul_rn(b, kOneSixth))));
+        float sc_own;
         // (the table is written once before the first barrier: these loads may be scheduled freely)
-        asm("ld.shared::cta.f32 %0, [%1];" : "=f"(sc[0]) : "r"(sLUT + ((uint32_t)sb2 & 0xffu) * 4));
-        asm("ld.shared::cta.f32 %0, [%1];" : "=f"(sc[1]) : "r"(sLUT + ((uint32_t)sb2 >> 8) * 4));
-        st_shared_u8(sfp0 + (j & 1) * SF_BYTES + (gg >> 1) * 512 + 2 * (gg & 1), (uint32_t)sb2 >> (8 * (t4 & 1)));
+        asm("ld.shared::cta.f32 %0, [%1];" : "=f"(sc_own) : "r"(sLUT + (uint32_t)sb * 4));
+        const float sc_other = __shfl_xor_sync(0xffffffffu, sc_own, 1);
+        const float sc[2] = {odd ? sc_other : sc_own, odd ? sc_own : sc_other};
+        st_shared_u8(sfp0 + (j & 1) * SF_BYTES + (gg >> 1) * 512 + 2 * (gg & 1), sb);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const float2 negm2 = make_float2(-m[r], -m[r]), sc2 = make_float2(sc[r], sc[r]);
