@@ -388,8 +388,10 @@ nvfp4_quantize_flat_kernel(uint8_t *__restrict__ out, uint32_t *__restrict__ sf,
     if (SF_LAYOUT == AC4K_SF_AC4K) return ((int64_t)b * KT + k64) * rows_sf + row;
     return (((int64_t)b * (rows_sf >> 7) + (row >> 7)) * KT + k64) * 128 + (row & 31) * 4 + ((row & 127) >> 5);
   };
-  grid_launch_dependents();
+  // (the next kernel is let in after the wait: a GEMM that starts to prefetch its weights under the one before it costs 0.4 us
+  // a call at 1 x 8192 x 8192)
   if (CLUSTER) grid_dependency_wait();
+  grid_launch_dependents();
 
   Block16 v;
 #pragma unroll
