@@ -6,8 +6,9 @@ One nvcc invocation per .cu (in parallel), then a link step.  The library links 
 runtime statically and resolves the driver entry point it needs (tensor-map encoding) at
 run time, so it has no link-time dependency on libcuda.
 
-`--pybind` (or build_pybind()) also compiles csrc/bindings_pybind.cc with the host compiler into
-`native/_cuda_ops*.so`: the pybind11 module with the reference's names and signatures, linked
+csrc/host_calls.cc, the operators' host side, is compiled with the host compiler into `native/_host_calls*.so`.
+
+`--pybind` (or build_pybind()) also compiles csrc/bindings_pybind.cc into `native/_cuda_ops*.so`: the pybind11 module with the reference's names and signatures, linked
 against the library above.
 """
 from __future__ import annotations
@@ -140,6 +141,7 @@ def _build_module(name: str, source: str, force: bool) -> str:
 if __name__ == "__main__":
     path = build(force="--force" in sys.argv, verbose="--verbose" in sys.argv)
     print(path)
+    print(_build_module("_host_calls", "host_calls.cc", "--force" in sys.argv))
     if "--hooks" in sys.argv:
         print(build_hooks(force="--force" in sys.argv))
     if "--pybind" in sys.argv:
