@@ -60,9 +60,9 @@ def test_odd_values_in_one_call(rows, fill):
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", ["fp8e4m3", "int8"])
 @pytest.mark.parametrize("b,k,h,d", [(1, 1, 1, 1), (2, 15, 3, 65), (2, 16, 1, 64), (1, 17, 2, 63), (1, 100, 12, 65), (1, 128, 2, 128),
-                                     (1, 511, 1, 100), (1, 512, 2, 17), (1, 513, 2, 65), (1, 513, 2, 66)])
+                                     (1, 512, 2, 64), (1, 1023, 1, 100), (1, 1024, 2, 17), (1, 1025, 2, 65), (1, 1025, 2, 66)])
 def test_columns_contiguous(b, k, h, d, precision):
-    """[B, N, H, D] along N: one launch up to 512 rows, three beyond, the strided kernel where D is odd"""
+    """[B, N, H, D] along N: one launch up to 1024 rows, four beyond, the strided kernel where D is odd"""
     from ac4k_kernel_b200 import ops
     x = (gaussian((b, k, h, d), seed=k + d) * 2).bfloat16().cuda()
     x[:, :, :, d // 2] = 0                                             # a column of zeros: 0 * inf
