@@ -17,8 +17,8 @@
 // quantiser (every 16 keys viewed as [2, 4, 2] and transposed to [4, 2, 2]), i.e. one 32-bit column, and one 16x128b store
 // writes a warp's tile.  Tensor memory: S 128 + O 2 x 128 + P 2 groups x 2 buffers x 32 = 512 columns.
 //
-// What bounds it: issue slots and dependency latencies of the softmax warps (ncu, before P moved to tensor memory and the
-// polynomial exponentials to the ex2 pipe: 63 % of the issue slots, ex2 pipe 46 %, ALU 47 %, tensor memory 48 %, tensor pipe 30 %).
+// What bounds it: the ex2 pipe (16 per clock and SM; 74 % busy) and, where it idles, the phases in which the warps of a scheduler
+// wait for S, for tensor memory or for one another (issue slots 56 %, ALU 48 %, tensor memory 59 %, tensor pipe 36 %).
 // [1, 16384, 16, 128], kernel alone: 1 667 us with four warps per group, a row per thread; 1 566 with eight; 1 475 with O rescaled
 // behind the exponentials instead of in front of them; 1 406 with an eighth of the exponentials as a polynomial on the FMA
 // pipe instead of a quarter; 1 344 with P in tensor memory; 1 332 with every exponential on the ex2 pipe (the polynomial

@@ -22,8 +22,8 @@
 //              global scale 1 / 2688) and written into shared memory in the layouts the tensor core reads
 //              (64-byte-swizzled K-major operand, 32 x 16-byte scale chunks), then O rescaled in tensor memory if a
 //              maximum of the warp moved; at the end O * gV / (2688 * row sum) is stored as bf16.
-// The softmax warps bound this kernel: their issue slots and dependency latencies, with the ex2 pipe (16 per clock and SM)
-// next.  [1, 16384, 16, 128], kernel alone: 1 688 us with four warps per group, a row per thread, and O rescaled before the
+// The softmax warps bound this kernel: the ex2 pipe (16 per clock and SM; 68 % busy), issue slots (59 %) and the waits in which
+// both idle.  [1, 16384, 16, 128], kernel alone: 1 688 us with four warps per group, a row per thread, and O rescaled before the
 // exponentials (a wait for the previous P V and a chain of small loads and stores); 1 728 with eight warps per group, 1 654 with
 // the rescale behind the exponentials (a quarter of the exponentials as a polynomial on the FMA pipe); 1 640 with an eighth of
 // them there, 1 579 with none: the polynomial costs thirteen issue slots a pair, and those bound the kernel now; 1 555 with the
