@@ -6,7 +6,8 @@
 //
 // Each function returns None instead of a result when anything about the call is not what it expects (a wrong shape, a
 // tensor subclass, an option it does not know): the Python wrapper then takes its own path, which computes the same or
-// raises its own error.  So nothing here decides what is accepted and what is refused.
+// raises its own error.  So nothing here decides what is accepted and what is refused.  The interpreter lock is given up for
+// allocations and launches (a launch waits while the driver's queue is full).
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -75,6 +76,13 @@ struct View {
   }
 };
 
+// `work` without the interpreter lock (taken again when it returns or throws)
+template <typename F>
+auto unlocked(F &&work) {
+  py::gil_scoped_release release;
+  return work();
+}
+
 struct Nvfp4 { at::Tensor q, sf, scale; };
 
 Nvfp4 quantize_nvfp4_of(const at::Tensor &x, int64_t cross, int64_t reduce, float max_scale, bool swizzle, bool tiled) {
@@ -132,14 +140,14 @@ py::object quantize(py::handle input, int64_t cross, int64_t reduce, py::handle 
   if (precision == "nvfp4") {
     const auto ms = number_or(max_scale, 6.0 * 448.0, false);
     if (!ms || (sf_layout != "ac4k" && sf_layout != "128x4")) return py::none();
-    Nvfp4 r = quantize_nvfp4_of(*x, cross, reduce, (float)*ms, swizzle, sf_layout == "128x4");
+    const Nvfp4 r = unlocked([&] { return quantize_nvfp4_of(*x, cross, reduce, (float)*ms, swizzle, sf_layout == "128x4"); });
     return py::make_tuple(r.q, r.sf, r.scale);
   }
   const bool fp8 = precision == "fp8e4m3";
   if (!fp8 && precision != "int8") return py::none();
   const auto ms = number_or(max_scale, fp8 ? 448.0 : 127.0, !fp8);
   if (!ms) return py::none();
-  Rowwise r = quantize_rows_of(*x, cross, reduce, fp8, *ms, fp8 && swizzle);
+  const Rowwise r = unlocked([&] { return quantize_rows_of(*x, cross, reduce, fp8, *ms, fp8 && swizzle); });
   return py::make_tuple(r.q, r.sf);
 }
 
@@ -188,10 +196,12 @@ py::object linear(py::handle a, py::handle a_sf, py::handle a_gs, py::handle b, 
     if (!plain(d) || !d.is_contiguous() || dt_code(d.scalar_type()) < 0 || !same_shape(d, {g.M, g.N})) return py::none();
   }
   const c10::cuda::CUDAGuard guard(d.defined() ? d.device() : g.a.device());
-  if (!d.defined()) d = empty({g.M, g.N}, at::kBFloat16, g.a);
-  check(ac4k_linear_nvfp4(d.data_ptr(), dt_code(d.scalar_type()), g.a.data_ptr(), g.a_sf.data_ptr(), g.ags(), g.b.data_ptr(), g.b_sf.data_ptr(),
-                          g.bgs(), g.bias_ptr(), g.bias_dt(), g.M, g.N, g.K, g.layout, stream_of(d)),
-        "linear_nvfp4");
+  unlocked([&] {
+    if (!d.defined()) d = empty({g.M, g.N}, at::kBFloat16, g.a);
+    check(ac4k_linear_nvfp4(d.data_ptr(), dt_code(d.scalar_type()), g.a.data_ptr(), g.a_sf.data_ptr(), g.ags(), g.b.data_ptr(), g.b_sf.data_ptr(),
+                            g.bgs(), g.bias_ptr(), g.bias_dt(), g.M, g.N, g.K, g.layout, stream_of(d)),
+          "linear_nvfp4");
+  });
   return out.is_none() ? py::cast(d) : py::reinterpret_borrow<py::object>(out);
 }
 
@@ -202,13 +212,16 @@ py::object linear_requant(py::handle a, py::handle a_sf, py::handle a_gs, py::ha
   if (!g.ok || !scalar_of(out_gs, &gs) || g.N % 64 || (sf_layout != "ac4k" && sf_layout != "128x4")) return py::none();
   const bool tiled = sf_layout == "128x4";
   const c10::cuda::CUDAGuard guard(g.a.device());
-  at::Tensor o = empty({g.M, g.N / 2}, at::kByte, g.a);
-  at::Tensor sf = tiled ? empty({ceil_div(g.M, 128), g.N / 64, 32, 4, 4}, at::kFloat8_e4m3fn, g.a)
-                        : empty({g.N / 64, align_up(g.M, 16), 4}, at::kFloat8_e4m3fn, g.a);
-  check(ac4k_linear_nvfp4_requant(o.data_ptr(), sf.data_ptr(), static_cast<const float *>(gs.data_ptr()), tiled ? AC4K_SF_TILE128X4 : AC4K_SF_AC4K,
-                                  g.a.data_ptr(), g.a_sf.data_ptr(), g.ags(), g.b.data_ptr(), g.b_sf.data_ptr(), g.bgs(), g.bias_ptr(),
-                                  g.bias_dt(), g.M, g.N, g.K, g.layout, stream_of(o)),
-        "linear_nvfp4_requant");
+  at::Tensor o, sf;
+  unlocked([&] {
+    o = empty({g.M, g.N / 2}, at::kByte, g.a);
+    sf = tiled ? empty({ceil_div(g.M, 128), g.N / 64, 32, 4, 4}, at::kFloat8_e4m3fn, g.a)
+                          : empty({g.N / 64, align_up(g.M, 16), 4}, at::kFloat8_e4m3fn, g.a);
+    check(ac4k_linear_nvfp4_requant(o.data_ptr(), sf.data_ptr(), static_cast<const float *>(gs.data_ptr()), tiled ? AC4K_SF_TILE128X4 : AC4K_SF_AC4K,
+                                    g.a.data_ptr(), g.a_sf.data_ptr(), g.ags(), g.b.data_ptr(), g.b_sf.data_ptr(), g.bgs(), g.bias_ptr(),
+                                    g.bias_dt(), g.M, g.N, g.K, g.layout, stream_of(o)),
+          "linear_nvfp4_requant");
+  });
   return py::make_tuple(o, sf, py::reinterpret_borrow<py::object>(out_gs));
 }
 
@@ -225,9 +238,11 @@ py::object rope3d(py::handle hx, py::handle hgrid, py::handle hfreqs, py::handle
   const c10::cuda::CUDAGuard guard(x->device());
   at::Tensor out = given ? *given : at::empty_like(*x);
   if (!out.is_contiguous()) return py::none();
-  check(ac4k_rope3d(out.data_ptr(), x->data_ptr(), static_cast<const int32_t *>(grid->data_ptr()), freqs->data_ptr(), B, S, N, D, freqs->size(0),
-                    stream_of(*x)),
-        "rope3d");
+  unlocked([&] {
+    check(ac4k_rope3d(out.data_ptr(), x->data_ptr(), static_cast<const int32_t *>(grid->data_ptr()), freqs->data_ptr(), B, S, N, D, freqs->size(0),
+                      stream_of(*x)),
+          "rope3d");
+  });
   return given ? py::reinterpret_borrow<py::object>(hout) : py::cast(out);
 }
 
@@ -258,39 +273,43 @@ py::object attention(py::handle hq, py::handle hk, py::handle hv, const std::str
     s[0] = out.stride(0); s[1] = out.stride(h_dim); s[2] = out.stride(n_dim); s[3] = out.stride(3);
   };
   int64_t os[4];
-  if (nvfp4) {
-    const Nvfp4 qq = quantize_nvfp4_of(q, n_dim, 3, 2688.0f, false, true), kk = quantize_nvfp4_of(k, n_dim, 3, 2688.0f, false, true);
-    const Nvfp4 vv = quantize_nvfp4_of(v, 3, n_dim, 2688.0f, true, true);
-    out_strides(os);
-    auto gs = [](const Nvfp4 &t) { return static_cast<const float *>(t.scale.data_ptr()); };
-    check(ac4k_mha_nvfp4_fwd(out.data_ptr(), os, qq.q.data_ptr(), qq.sf.data_ptr(), gs(qq), kk.q.data_ptr(), kk.sf.data_ptr(), gs(kk),
-                             vv.q.data_ptr(), vv.sf.data_ptr(), gs(vv), B, H, Nq, Nkv, qq.q.size(3) * 2, Dv, sm_scale, AC4K_SF_TILE128X4,
-                             stream_of(q)),
-          "mha_nvfp4_fwd");
-  } else {
-    // k - mean(k): the subtraction happens inside the K quantiser
-    const at::Tensor mean = k.detach().mean(at::IntArrayRef{n_dim}, true);
-    if (mean.stride(3) != 1) return py::none();
-    const int64_t Dp = align_up(D, 16);
-    auto int8_of = [&](const at::Tensor &t, int64_t n, int64_t block, const at::Tensor *sub, at::Tensor *sf) {
-      *sf = empty({B, H, ceil_div(n, block)}, at::kFloat, q);
-      at::Tensor y = empty({B, H, n, Dp}, at::kChar, q);
-      const int64_t shape[4] = {B, H, n, D}, stride[4] = {t.stride(0), t.stride(h_dim), t.stride(n_dim), t.stride(3)};
-      const int64_t ss[2] = {sub ? sub->stride(0) : 0, sub ? sub->stride(h_dim) : 0};
-      check(ac4k_quantize_int8_block(y.data_ptr(), static_cast<float *>(sf->data_ptr()), t.data_ptr(), shape, stride, block,
-                                     sub ? sub->data_ptr() : nullptr, sub ? ss : nullptr, stream_of(q)),
-            "quantize_int8_block");
-      return y;
-    };
-    at::Tensor q_sf, k_sf;
-    const at::Tensor q8 = int8_of(q, Nq, 64, nullptr, &q_sf), k8 = int8_of(k, Nkv, 128, &mean, &k_sf);
-    const Rowwise v8 = quantize_rows_of(v, 3, n_dim, true, 2.25, true);
-    out_strides(os);
-    auto f = [](const at::Tensor &t) { return static_cast<const float *>(t.data_ptr()); };
-    check(ac4k_mha_int8_x_fp8_fwd(out.data_ptr(), os, q8.data_ptr(), f(q_sf), 64, k8.data_ptr(), f(k_sf), 128, v8.q.data_ptr(), f(v8.sf), B, H,
-                                  Nq, Nkv, Dp, Dv, sm_scale, stream_of(q)),
-          "mha_int8_x_fp8_fwd");
-  }
+  const bool done = unlocked([&] {
+    if (nvfp4) {
+      const Nvfp4 qq = quantize_nvfp4_of(q, n_dim, 3, 2688.0f, false, true), kk = quantize_nvfp4_of(k, n_dim, 3, 2688.0f, false, true);
+      const Nvfp4 vv = quantize_nvfp4_of(v, 3, n_dim, 2688.0f, true, true);
+      out_strides(os);
+      auto gs = [](const Nvfp4 &t) { return static_cast<const float *>(t.scale.data_ptr()); };
+      check(ac4k_mha_nvfp4_fwd(out.data_ptr(), os, qq.q.data_ptr(), qq.sf.data_ptr(), gs(qq), kk.q.data_ptr(), kk.sf.data_ptr(), gs(kk),
+                               vv.q.data_ptr(), vv.sf.data_ptr(), gs(vv), B, H, Nq, Nkv, qq.q.size(3) * 2, Dv, sm_scale, AC4K_SF_TILE128X4,
+                               stream_of(q)),
+            "mha_nvfp4_fwd");
+    } else {
+      // k - mean(k): the subtraction happens inside the K quantiser
+      const at::Tensor mean = k.detach().mean(at::IntArrayRef{n_dim}, true);
+      if (mean.stride(3) != 1) return false;
+      const int64_t Dp = align_up(D, 16);
+      auto int8_of = [&](const at::Tensor &t, int64_t n, int64_t block, const at::Tensor *sub, at::Tensor *sf) {
+        *sf = empty({B, H, ceil_div(n, block)}, at::kFloat, q);
+        at::Tensor y = empty({B, H, n, Dp}, at::kChar, q);
+        const int64_t shape[4] = {B, H, n, D}, stride[4] = {t.stride(0), t.stride(h_dim), t.stride(n_dim), t.stride(3)};
+        const int64_t ss[2] = {sub ? sub->stride(0) : 0, sub ? sub->stride(h_dim) : 0};
+        check(ac4k_quantize_int8_block(y.data_ptr(), static_cast<float *>(sf->data_ptr()), t.data_ptr(), shape, stride, block,
+                                       sub ? sub->data_ptr() : nullptr, sub ? ss : nullptr, stream_of(q)),
+              "quantize_int8_block");
+        return y;
+      };
+      at::Tensor q_sf, k_sf;
+      const at::Tensor q8 = int8_of(q, Nq, 64, nullptr, &q_sf), k8 = int8_of(k, Nkv, 128, &mean, &k_sf);
+      const Rowwise v8 = quantize_rows_of(v, 3, n_dim, true, 2.25, true);
+      out_strides(os);
+      auto f = [](const at::Tensor &t) { return static_cast<const float *>(t.data_ptr()); };
+      check(ac4k_mha_int8_x_fp8_fwd(out.data_ptr(), os, q8.data_ptr(), f(q_sf), 64, k8.data_ptr(), f(k_sf), 128, v8.q.data_ptr(), f(v8.sf), B, H,
+                                    Nq, Nkv, Dp, Dv, sm_scale, stream_of(q)),
+            "mha_int8_x_fp8_fwd");
+    }
+    return true;
+  });
+  if (!done) return py::none();
   return hout.is_none() ? py::cast(out) : py::reinterpret_borrow<py::object>(hout);
 }
 

@@ -189,6 +189,25 @@ def test_native_host_side_is_the_python_path():
         ops.linear(*ops.quantize(x, 0, 1), *w)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 50, 300])
+def test_captured(m):
+    """quantise (one cluster, flat, flat with a ragged tile) and GEMM replayed from a graph on new inputs"""
+    from ac4k_kernel_b200 import ops
+    w = ops.quantize((gaussian((512, 1024), seed=1) * 0.05).bfloat16().cuda(), 0, 1)
+    x = gaussian((m, 1024), seed=2).cuda()
+    ops.linear(*ops.quantize(x, 0, 1), *w)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        y = ops.linear(*ops.quantize(x, 0, 1), *w)
+    for seed in (3, 4):
+        x.copy_(gaussian((m, 1024), seed=seed).cuda() * seed)
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, ops.linear(*ops.quantize(x, 0, 1), *w))
+
+
 def test_native_host_side_leaves_other_tensors_to_python():
     from ac4k_kernel_b200.native import host_calls
     if host_calls is None:
