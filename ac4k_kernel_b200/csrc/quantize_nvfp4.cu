@@ -384,6 +384,7 @@ nvfp4_quantize_flat_kernel(uint8_t *__restrict__ out, uint32_t *__restrict__ sf,
   const int items = nbatch * M * nblk;
   const int stride = gridDim.x * blockDim.x;
   const int it = blockIdx.x * blockDim.x + threadIdx.x;         // this thread's block
+  if (CLUSTER && gridDim.x > 1) ptx::cluster_arrive_relaxed();  // (waited for where the first store to a peer is)
   auto sf_word = [&](int b, int row, int k64) -> int64_t {
     if (SF_LAYOUT == AC4K_SF_AC4K) return ((int64_t)b * KT + k64) * rows_sf + row;
     return (((int64_t)b * (rows_sf >> 7) + (row >> 7)) * KT + k64) * 128 + (row & 31) * 4 + ((row & 127) >> 5);
@@ -418,6 +419,7 @@ nvfp4_quantize_flat_kernel(uint8_t *__restrict__ out, uint32_t *__restrict__ sf,
     uint32_t m = cta_max(max(m2 & 0xFFFFu, m2 >> 16), s_m);
     if (gridDim.x > 1) {
       const uint32_t rank = ptx::cluster_ctarank();
+      ptx::cluster_wait();                                        // every CTA of the cluster runs
       if (threadIdx.x < gridDim.x) ptx::st_shared_cluster_u32(ptx::map_to_cta(ptx::smem_u32(s_peer + rank), threadIdx.x), m);
       ptx::cluster_sync();
       m = 0;

@@ -419,6 +419,10 @@ __device__ __forceinline__ void cluster_sync_relaxed() {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
+// The two halves of such a barrier, for the one in front of the first access to a peer's shared memory, which has to be known
+// to run (a cluster is scheduled together, but its CTAs do not begin together): arrive on entry, wait where the access is.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 // arrive on an mbarrier given by a shared::cluster address (own or peer CTA).  Default semantics
 // (release at CTA scope): the cluster-scope release form was measured at ~0.7 us per arrive,
 // and the data handed over here (tensor memory) is ordered by the tcgen05 fences instead.
