@@ -131,7 +131,12 @@ def _build_module(name: str, source: str, force: bool) -> str:
     cmd += ["-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda_home, "include"),
             "-I", os.path.join(ROOT, "include"), src, "-o", target,
             "-L", PKG_DIR, "-l:libac4k_b200.so", "-L", torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
-            "-ltorch_python", "-Wl,-rpath,$ORIGIN/..", f"-Wl,-rpath,{torch_lib}"]
+            "-ltorch_python",
+            # The process's own libstdc++ and not a second, static one, which a compiler that comes without the shared one
+            # links by itself: two of them disagree about the stream facets, and the first number that is formatted (any
+            # TORCH_CHECK message with one) ends the process.
+            "-l:libstdc++.so.6",
+            "-Wl,-rpath,$ORIGIN/..", f"-Wl,-rpath,{torch_lib}"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("building the pybind module failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
