@@ -129,18 +129,40 @@ std::optional<double> number_or(py::handle h, double fallback, bool whole) {
   return v;
 }
 
-py::object quantize(py::handle input, int64_t cross, int64_t reduce, py::handle max_scale, const std::string &precision, bool swizzle,
-                    const std::string &sf_layout) {
+// Options come as they are: pybind's own conversions would raise a TypeError for what a wrapper may accept or refuse otherwise.
+std::optional<std::string> text_of(py::handle h) {
+  if (!PyUnicode_CheckExact(h.ptr())) return std::nullopt;
+  Py_ssize_t n = 0;
+  const char *s = PyUnicode_AsUTF8AndSize(h.ptr(), &n);
+  if (s == nullptr) { PyErr_Clear(); return std::nullopt; }
+  return std::string(s, (size_t)n);
+}
+std::optional<int64_t> index_of(py::handle h) {
+  if (!PyLong_CheckExact(h.ptr())) return std::nullopt;
+  const int64_t v = PyLong_AsLongLong(h.ptr());
+  if (PyErr_Occurred()) { PyErr_Clear(); return std::nullopt; }
+  return v;
+}
+
+// precision, layouts: what the wrapper looks at for this precision, no more
+py::object quantize(py::handle input, py::handle hcross, py::handle hreduce, py::handle max_scale, py::handle hprecision, py::handle hswizzle,
+                    py::handle hlayout) {
   const auto x = tensor_of(input, at::kBFloat16);
-  if (!x || x->dim() < 2 || x->dim() > 4) return py::none();
+  const auto icross = index_of(hcross), ireduce = index_of(hreduce);
+  const auto iprecision = text_of(hprecision);
+  if (!x || x->dim() < 2 || x->dim() > 4 || !icross || !ireduce || !iprecision || !PyBool_Check(hswizzle.ptr())) return py::none();
+  int64_t cross = *icross, reduce = *ireduce;
+  const std::string &precision = *iprecision;
+  const bool swizzle = hswizzle.ptr() == Py_True;
   if (cross < 0) cross += x->dim();
   if (reduce < 0) reduce += x->dim();
   if (cross < 0 || reduce < 0 || cross >= x->dim() || reduce >= x->dim() || cross == reduce) return py::none();
   const c10::cuda::CUDAGuard guard(x->device());
   if (precision == "nvfp4") {
     const auto ms = number_or(max_scale, 6.0 * 448.0, false);
-    if (!ms || (sf_layout != "ac4k" && sf_layout != "128x4")) return py::none();
-    const Nvfp4 r = unlocked([&] { return quantize_nvfp4_of(*x, cross, reduce, (float)*ms, swizzle, sf_layout == "128x4"); });
+    const auto sf_layout = text_of(hlayout);
+    if (!ms || !sf_layout || (*sf_layout != "ac4k" && *sf_layout != "128x4")) return py::none();
+    const Nvfp4 r = unlocked([&] { return quantize_nvfp4_of(*x, cross, reduce, (float)*ms, swizzle, *sf_layout == "128x4"); });
     return py::make_tuple(r.q, r.sf, r.scale);
   }
   const bool fp8 = precision == "fp8e4m3";
@@ -206,11 +228,12 @@ py::object linear(py::handle a, py::handle a_sf, py::handle a_gs, py::handle b, 
 }
 
 py::object linear_requant(py::handle a, py::handle a_sf, py::handle a_gs, py::handle b, py::handle b_sf, py::handle b_gs, py::handle out_gs,
-                          py::handle bias, const std::string &sf_layout) {
+                          py::handle bias, py::handle hlayout) {
   const Gemm g(a, a_sf, a_gs, b, b_sf, b_gs, bias);
   at::Tensor gs;
-  if (!g.ok || !scalar_of(out_gs, &gs) || g.N % 64 || (sf_layout != "ac4k" && sf_layout != "128x4")) return py::none();
-  const bool tiled = sf_layout == "128x4";
+  const auto sf_layout = text_of(hlayout);
+  if (!g.ok || !scalar_of(out_gs, &gs) || g.N % 64 || !sf_layout || (*sf_layout != "ac4k" && *sf_layout != "128x4")) return py::none();
+  const bool tiled = *sf_layout == "128x4";
   const c10::cuda::CUDAGuard guard(g.a.device());
   at::Tensor o, sf;
   unlocked([&] {
@@ -246,9 +269,11 @@ py::object rope3d(py::handle hx, py::handle hgrid, py::handle hfreqs, py::handle
   return given ? py::reinterpret_borrow<py::object>(hout) : py::cast(out);
 }
 
-py::object attention(py::handle hq, py::handle hk, py::handle hv, const std::string &layout, const std::string &precision, py::handle hout) {
-  const bool nvfp4 = precision == "nvfp4", bnhd = layout == "BNHD";
-  if ((!nvfp4 && precision != "int8+fp8e4m3") || (!bnhd && layout != "BHND")) return py::none();
+py::object attention(py::handle hq, py::handle hk, py::handle hv, py::handle hlayout, py::handle hprecision, py::handle hout) {
+  const auto layout = text_of(hlayout), precision = text_of(hprecision);
+  if (!layout || !precision) return py::none();
+  const bool nvfp4 = *precision == "nvfp4", bnhd = *layout == "BNHD";
+  if ((!nvfp4 && *precision != "int8+fp8e4m3") || (!bnhd && *layout != "BHND")) return py::none();
   const auto tq = tensor_of(hq, at::kBFloat16, 4, nvfp4), tk = tensor_of(hk, at::kBFloat16, 4, nvfp4), tv = tensor_of(hv, at::kBFloat16, 4);
   if (!tq || !tk || !tv) return py::none();
   const at::Tensor &q = *tq, &k = *tk, &v = *tv;

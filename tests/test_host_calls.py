@@ -53,3 +53,32 @@ def test_refused_by_the_library(both_paths, kw):
     assert both_paths(lambda: ops.quantize(x, 0, 1, **kw)) == [RuntimeError, RuntimeError]
     with pytest.raises(RuntimeError, match=r"code -2\): max_scale must be positive"):
         ops.quantize(x, 0, 1, **kw)
+
+
+@pytest.mark.gpu
+def test_options_are_left_to_the_wrappers(both_paths):
+    """What the wrappers accept or refuse with an error of their own: options of other types than the usual ones"""
+    from ac4k_kernel_b200 import ops
+    x, q = gaussian((64, 128), seed=1).cuda(), gaussian((1, 20, 2, 64), seed=2).cuda()
+    w = ops.quantize(x, 0, 1)
+
+    def same(fn):
+        native, python = both_paths(fn)
+        assert isinstance(native, tuple) and len(native) == len(python)
+        assert all(torch.equal(a.view(torch.uint8) if a.dtype == torch.float8_e4m3fn else a,
+                               b.view(torch.uint8) if b.dtype == torch.float8_e4m3fn else b) for a, b in zip(native, python))
+    for precision in ("int8", "fp8e4m3"):
+        same(lambda: ops.quantize(x, 0, 1, precision=precision, sf_layout=None))
+    same(lambda: ops.quantize(x, 0, 1, swizzle=1))
+    same(lambda: ops.quantize(x, True, False, precision="int8"))
+    same(lambda: ops.quantize(x, 0, 1, max_scale=torch.tensor(100.0)))
+    for fn, error in ((lambda: ops.quantize(x, 0, 1, precision=None), AssertionError),
+                      (lambda: ops.quantize(x, 0, 1, sf_layout=None), AssertionError),
+                      (lambda: ops.quantize(x, None, 1), TypeError),
+                      (lambda: ops.quantize(x, 2 ** 70, 1), None),
+                      (lambda: ops.quantize(x, 0, 1, precision="fp8e4m3", swizzle=None), TypeError),
+                      (lambda: ops.attention(q, q, q, layout=None), AssertionError),
+                      (lambda: ops.attention(q, q, q, precision=1), AssertionError),
+                      (lambda: ops.linear_requant(*w, *w, w[2], sf_layout=None), ValueError)):
+        native, python = both_paths(fn)
+        assert native is python and issubclass(native, Exception) and error in (None, native)
