@@ -27,7 +27,8 @@ namespace {
 int64_t align_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
 int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-// A dense CUDA tensor whose memory may be handed to a kernel as it is: no subclass or mode tensor, no functorch wrapper.
+// A dense CUDA tensor whose memory may be handed to a kernel as it is: no mode tensor, no functorch wrapper.  (Python
+// subclasses without a dispatch of their own look the same here; tensor_of declines them by their type.)
 bool plain(const at::Tensor &t) {
   if (!t.defined() || !t.is_cuda() || t.layout() != at::kStrided) return false;
   const c10::DispatchKeySet odd({c10::DispatchKey::Python, c10::DispatchKey::PythonTLSSnapshot, c10::DispatchKey::FuncTorchBatched,
@@ -37,7 +38,7 @@ bool plain(const at::Tensor &t) {
 }
 
 std::optional<at::Tensor> tensor_of(py::handle h, at::ScalarType dt, int64_t dim = -1, bool dense = true) {
-  if (!THPVariable_Check(h.ptr())) return std::nullopt;
+  if (!THPVariable_CheckExact(h.ptr())) return std::nullopt;       // (a torch.Tensor or a Parameter, no subclass of them)
   const at::Tensor &t = THPVariable_Unpack(h.ptr());
   if (!plain(t) || t.scalar_type() != dt || (dim >= 0 && t.dim() != dim) || (dense && !t.is_contiguous())) return std::nullopt;
   return t;
@@ -195,7 +196,7 @@ struct Gemm {
       if (!same_shape(a_sf, {ceil_div(M, 128), kt, 32, 4, 4}) || !same_shape(b_sf, {ceil_div(N, 128), kt, 32, 4, 4})) return;
     }
     if (!hbias.is_none()) {
-      if (!THPVariable_Check(hbias.ptr())) return;
+      if (!THPVariable_CheckExact(hbias.ptr())) return;
       bias = THPVariable_Unpack(hbias.ptr());
       if (!plain(bias) || dt_code(bias.scalar_type()) < 0 || !bias.is_contiguous()) return;
       if (!(bias.dim() == 1 && bias.size(0) == N) && !(bias.dim() == 2 && bias.size(0) == 1 && bias.size(1) == N)) return;
@@ -213,7 +214,7 @@ py::object linear(py::handle a, py::handle a_sf, py::handle a_gs, py::handle b, 
   if (!g.ok) return py::none();
   at::Tensor d;
   if (!out.is_none()) {
-    if (!THPVariable_Check(out.ptr())) return py::none();
+    if (!THPVariable_CheckExact(out.ptr())) return py::none();
     d = THPVariable_Unpack(out.ptr());
     if (!plain(d) || !d.is_contiguous() || dt_code(d.scalar_type()) < 0 || !same_shape(d, {g.M, g.N})) return py::none();
   }

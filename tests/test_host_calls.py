@@ -82,3 +82,27 @@ def test_options_are_left_to_the_wrappers(both_paths):
                       (lambda: ops.linear_requant(*w, *w, w[2], sf_layout=None), ValueError)):
         native, python = both_paths(fn)
         assert native is python and issubclass(native, Exception) and error in (None, native)
+
+
+class Sub(torch.Tensor):
+    pass
+
+
+@pytest.mark.gpu
+def test_subclasses_are_left_to_the_wrappers(both_paths):
+    """A subclass without a dispatch of its own: results are of the type that the wrappers make them (empty_like for RoPE)"""
+    from ac4k_kernel_b200 import ops
+    x, q = gaussian((64, 128), seed=1).cuda(), gaussian((1, 24, 2, 64), seed=2).cuda()
+    w, bias = ops.quantize(x, 0, 1), gaussian((64,), seed=3).cuda()
+    grid, freqs = torch.tensor([[2, 3, 4]], dtype=torch.int32, device="cuda"), torch.zeros((8, 32), dtype=torch.complex128, device="cuda")
+
+    def sub(t):
+        return t.as_subclass(Sub)
+    for fn in (lambda: ops.rope3d(sub(q), grid, freqs), lambda: ops.rope3d(q, sub(grid), freqs), lambda: ops.rope3d(q, grid, freqs, sub(q.clone())),
+               lambda: ops.attention(sub(q), q, q), lambda: ops.attention(q, q, sub(q), precision="nvfp4"),
+               lambda: ops.quantize(sub(x), 0, 1)[0], lambda: ops.quantize(sub(x), 0, 1, precision="int8")[0],
+               lambda: ops.linear(*w, *w, bias=sub(bias)), lambda: ops.linear(*w, *w, out=sub(torch.empty((64, 64), device="cuda"))),
+               lambda: ops.linear_requant(*w, *w, sub(w[2]))[2]):
+        native, python = both_paths(fn)
+        assert type(native) is type(python) and torch.equal(native.as_subclass(torch.Tensor), python.as_subclass(torch.Tensor))
+    assert type(ops.quantize(torch.nn.Parameter(x), 0, 1)[0]) is torch.Tensor
