@@ -42,7 +42,8 @@ __device__ __forceinline__ uint32_t rope_pair(uint32_t xy, double2 f) {
 // that, and as rounding to fp32 and then to bf16 is monotonic, it ends on the bf16 value of both ends (themselves rounded
 // to fp32) if they agree.  Where they do not (a few pairs in ten thousand: a rounding boundary lies between them), the vector
 // is computed in fp64.  So it is where e is not between 2^-122 (lost bits of underflowing products stay far below it) and 2^100
-// (nothing overflows), or is NaN.
+// (nothing overflows), or is NaN.  A pair of zeros has e = 0 and is exact in fp32: it is accepted as it is (by way of fp64, behind
+// the fp32 form, a tensor of zeros took 425 us where other values take 250, and 385 in fp64 alone; now 243).
 struct RopeFactor { float x, y, e; };
 __device__ __forceinline__ RopeFactor rope_factor(const double2 &f) {
   const float x = (float)f.x, y = (float)f.y, m = fmaxf(fabsf(x), fabsf(y));
@@ -55,12 +56,14 @@ static constexpr uint32_t kRopeMinE = (127u - 122u) << 23, kRopeRangeE = 222u <<
 __device__ __forceinline__ uint32_t rope_pair_fast(uint32_t xy, const RopeFactor &f, uint32_t &diff, uint32_t &out_of_range) {
   const float xr = __uint_as_float(xy << 16), xi = __uint_as_float(xy & 0xffff0000u);
   const float re = __fmaf_rn(xr, f.x, -__fmul_rn(xi, f.y)), im = __fmaf_rn(xr, f.y, __fmul_rn(xi, f.x));
-  const float e = __fmul_rn(__fadd_rn(fabsf(xr), fabsf(xi)), f.e);
+  const float a = __fadd_rn(fabsf(xr), fabsf(xi)), e = __fmul_rn(a, f.e);
   const __nv_bfloat162 lo = __floats2bfloat162_rn(__fsub_rn(re, e), __fsub_rn(im, e));
   const __nv_bfloat162 hi = __floats2bfloat162_rn(__fadd_rn(re, e), __fadd_rn(im, e));
   const uint32_t l = *reinterpret_cast<const uint32_t *>(&lo);
-  diff |= l ^ *reinterpret_cast<const uint32_t *>(&hi);
-  out_of_range = max(out_of_range, __float_as_uint(e) - kRopeMinE);
+  if (a != 0.0f || e != 0.0f) {          // (a pair of zeros under a good factor is exact, the sign of its zeros included)
+    diff |= l ^ *reinterpret_cast<const uint32_t *>(&hi);
+    out_of_range = max(out_of_range, __float_as_uint(e) - kRopeMinE);
+  }
   return l;
 }
 

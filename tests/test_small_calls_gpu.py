@@ -162,6 +162,54 @@ def test_rope_near_rounding_boundaries(d):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("d", [128, 72, 512, 1032])
+def test_rope_zero_pairs(d):
+    """Pairs of zeros of either sign beside others, under usual, negative, zero, tiny, infinite and NaN factors"""
+    from ac4k_kernel_b200 import ops
+    s, n = 12, 5
+    g = torch.Generator().manual_seed(d)
+    x = torch.randn((1, s, n, d), generator=g).bfloat16()
+    pairs = torch.rand((1, s, n, d // 2, 1), generator=g) < 0.6
+    zero = torch.where(torch.rand(x.shape, generator=g) < 0.5, 0.0, -0.0).bfloat16()
+    x = torch.where(pairs.expand(-1, -1, -1, -1, 2).reshape(x.shape), zero, x)
+    x[0, :, 0], x[0, :, 1, ::2] = zero[0, :, 0], zero[0, :, 1, ::2]      # whole heads; single zeros
+    freqs = E.rope_params_ref(s, d)
+    for row, f in enumerate((-1 + 0j, 0j, complex(-0.0, -0.0), 1e-35 - 1e-42j, complex(float("inf"), 1), complex(float("nan"), 0), -1e-320 + 1j)):
+        freqs[row + 1] = torch.full((d // 2,), f, dtype=torch.complex128)
+    grid = torch.tensor([[s, 1, 1]], dtype=torch.int32)
+    got = ops.rope3d(x.cuda(), grid.cuda(), freqs.cuda()).cpu()
+    want = E.rope3d_ref(x, grid, freqs)
+    nan = torch.isnan(want.float())
+    assert bool(nan.any()) and torch.equal(nan, torch.isnan(got.float()))
+    assert torch.equal(got.view(torch.int16)[~nan], want.view(torch.int16)[~nan])
+
+
+def _milliseconds(fn):
+    """median of nine single calls on the device"""
+    t = []
+    for i in range(12):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        fn()
+        b.record()
+        b.synchronize()
+        if i >= 3:
+            t.append(a.elapsed_time(b))
+    return sorted(t)[4]
+
+
+@pytest.mark.gpu
+def test_rope_zeros_take_no_longer():
+    """Zeros took the fp32 and the fp64 form one after the other: 1.7 times the time of other values, not 1.0"""
+    from ac4k_kernel_b200 import ops
+    grid, freqs = torch.tensor([[21, 30, 40]], dtype=torch.int32, device="cuda"), E.rope_params_ref(64, 128).cuda()
+    x = torch.randn((1, 25200, 40, 128), device="cuda", dtype=torch.bfloat16)
+    usual = _milliseconds(lambda: ops.rope3d(x, grid, freqs))
+    x[..., 4::8], x[..., 5::8] = 0, 0                                    # a pair of every vector of eight
+    assert _milliseconds(lambda: ops.rope3d(x, grid, freqs)) < 1.35 * usual
+
+
+@pytest.mark.gpu
 def test_native_host_side_is_the_python_path():
     """Same results as the wrappers' own path, and the same refusals"""
     from ac4k_kernel_b200 import ops
