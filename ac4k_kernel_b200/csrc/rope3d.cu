@@ -20,8 +20,10 @@
 
 namespace ac4k {
 
-// MODE 0 (see the kernel): a warp per CTA where its lanes hold a head's factors (D <= 256), else four.  [1, 75600, 40, 128], bit-identical: 384 us with 256 threads, one vector in flight and fp64 throughout; 322 with
-// five in flight; 298 with the fp32 form below in its present shape (128 threads); 262 with 64 threads; 253 with 32 (6.1 TB/s).
+// MODE 0 (see the kernel), many positions: a warp per CTA where its lanes hold a head's factors (D <= 256), else four.
+// [1, 75600, 40, 128], bit-identical, calls back to back: 386 us with 256 threads, one vector in flight and fp64 throughout; 322
+// with five in flight; 298 with the fp32 form below in its present shape (128 threads); 262 with 64 threads; 252 with 32 (6.1
+// TB/s; a call on inputs that are not the last call's takes 271, 5.7 TB/s).
 static constexpr int kRopeWarpsPerSm = 24;   // 80 registers per thread
 static constexpr int kRopeThreads = 256, kRopeCtasPerSm = 5;     // MODE 1 and 2
 static constexpr int kRopeBatch = 5;         // vectors a thread has in flight
@@ -95,7 +97,7 @@ __device__ __forceinline__ int rope_row(int c, int c1, int c2, int fi, int hi, i
 //         (or, 32-bit counts exceeded, more than 2^33 elements per position).
 // MODE 2: one pair per access (D % 8 != 0 or tensors not 16-byte aligned), factors in shared memory.
 template <int MODE>
-__global__ void __launch_bounds__(MODE == 0 ? 128 : kRopeThreads, MODE == 0 ? kRopeWarpsPerSm / 4 : kRopeCtasPerSm) rope3d_kernel(const uint16_t *__restrict__ x, const int32_t *__restrict__ grid_sizes,
+__global__ void __launch_bounds__(kRopeThreads, MODE == 0 ? kRopeWarpsPerSm * 32 / kRopeThreads : kRopeCtasPerSm) rope3d_kernel(const uint16_t *__restrict__ x, const int32_t *__restrict__ grid_sizes,
                                                                const double2 *__restrict__ freqs, uint16_t *__restrict__ out,
                                                                int64_t BS, int S, int N, int D, int C, int max_pos, int active) {
   __shared__ double2 sf[MODE == 0 ? 1 : kRopeMaxC];
@@ -203,11 +205,15 @@ extern "C" int ac4k_rope3d(void *out, const void *x, const int32_t *grid_sizes, 
   if (int e = get_device_info(&di)) return e;
   const int64_t BS = B * S;
   const bool vec = (D % 8 == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-  // threads of a multiple of C / 4 vectors (D % 8 == 0), so that their pairs repeat
-  const int64_t round = D / 8;
-  const int threads0 = round <= 32 ? 32 : 128;
+  // Threads of a multiple of C / 4 vectors (D % 8 == 0), so that their pairs repeat.  As few as hold them, one warp or four, where
+  // there are positions enough for every SM's warps; else more, as long as a position has a vector for each.  (One warp a
+  // position alone, of 128 heads x 256: 23.5 us for 100 positions and 39.6 for 1000; 7.8 and 30.2 with 256 threads always; 6.2
+  // and 27.0 by this rule.)
+  const int64_t round = D / 8, nvec = N * D / 8;
+  int threads0 = round <= 32 ? 32 : 128;
+  while (threads0 < kRopeThreads && threads0 < nvec && BS * (threads0 / 32) < (int64_t)di.sms * kRopeWarpsPerSm) threads0 *= 2;
   const int active = vec && round <= threads0 ? (int)(threads0 / round * round) : 0;
-  const int mode = !vec ? 2 : (active && N * D / 8 < (1 << 30) ? 0 : 1);
+  const int mode = !vec ? 2 : (active && nvec < (1 << 30) ? 0 : 1);
   const int threads = mode == 0 ? threads0 : kRopeThreads;
   const unsigned blocks = (unsigned)std::min<int64_t>(BS, (int64_t)di.sms * (mode == 0 ? kRopeWarpsPerSm * 32 / threads0 : kRopeCtasPerSm));
   const uint16_t *xp = static_cast<const uint16_t *>(x);
