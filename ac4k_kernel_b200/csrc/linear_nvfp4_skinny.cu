@@ -81,16 +81,22 @@ __device__ __forceinline__ void store_out(typename OutT<OUT_DT>::type *dst, floa
   else *dst = (typename OutT<OUT_DT>::type)v;
 }
 
-// One K slice: the accumulator is the sum.  alpha, bias, round, store row by row.
+// One K slice: the accumulator is the sum.  alpha, bias, round, store row by row, in groups of eight rows
+// (one row at a time with its own bound cost 10 ns a row: 4.25 against 3.46 us at 64 x 512 x 512, 5.56 against 4.78 at 64 x 20000 x 1024).
 template <int NT, int OUT_DT>
 __device__ __forceinline__ void finish_rows(const uint32_t (&own)[NT], const GemmArgs &p, int n, typename OutT<OUT_DT>::type *dst) {
   const float alpha = __fmul_rn(__ldg(p.a_gs), __ldg(p.b_gs));
   const float b = p.bias != nullptr ? load_bias(p.bias, p.bias_dt, n) : 0.0f;
 #pragma unroll
-  for (int m = 0; m < NT; ++m) {
-    float v = __fmul_rn(__uint_as_float(own[m]), alpha);
-    if (p.bias != nullptr) v = __fadd_rn(v, b);
-    if (m < p.M) store_out<OUT_DT>(dst + (int64_t)m * p.N, v);
+  for (int m0 = 0; m0 < NT; m0 += 8) {
+    if (m0 >= p.M) break;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int m = m0 + i;
+      float v = __fmul_rn(__uint_as_float(own[m]), alpha);
+      if (p.bias != nullptr) v = __fadd_rn(v, b);
+      if (m < p.M) store_out<OUT_DT>(dst + (int64_t)m * p.N, v);
+    }
   }
 }
 
