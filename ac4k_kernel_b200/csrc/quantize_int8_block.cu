@@ -24,7 +24,7 @@ static constexpr int kQ8MaxElemsPerThread = 128;     // 128 tokens x 256 feature
 // between the maximum and the codes (packed bf16: eight rows a warp), further ones are read again from L1 / L2.  The quotient
 // as in quantize8_by_reciprocal below.  [11, 100, 12, 65]: 23 us (k) and 13 us (q) with one element per thread and step, an index
 // division and an fp32 division each; 15 and 15 without the index division and the registers; 8.5 each like this.
-static constexpr int kQ8AnyThreads = 512, kQ8AnyRows = 128 / (kQ8AnyThreads / 32);
+static constexpr int kQ8AnyRows = 8;       // rows of the block that a warp takes at most
 
 // trunc(RN(f / s)), |f / s| <= 127, as a byte; rs = RN(1 / s)
 __device__ __forceinline__ uint32_t quantize_code(float f, float s, float rs) {
@@ -36,10 +36,11 @@ __device__ __forceinline__ uint32_t quantize_code(float f, float s, float rs) {
   return (uint32_t)__float2int_rz(__fdiv_rn(f, s)) & 0xffu;
 }
 
-__global__ void __launch_bounds__(kQ8AnyThreads) quantize_int8_block_kernel(
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) quantize_int8_block_kernel(
     int8_t *__restrict__ y, float *__restrict__ scale, const uint16_t *__restrict__ x, int N, int D, int Dp, int block, int nblk,
     int64_t sb, int64_t sh, int64_t sn, int64_t sd, int H, const uint16_t *__restrict__ sub, int64_t ub, int64_t uh) {
-  constexpr int kWarps = kQ8AnyThreads / 32;
+  constexpr int kWarps = THREADS / 32;
   __shared__ float red[kWarps];
   const int blk = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int n0 = blk * block;
@@ -367,7 +368,17 @@ extern "C" int ac4k_quantize_int8_block(void *out, float *scale, const void *in,
     AC4K_Q8V_LAUNCH(16);
 #undef AC4K_Q8V_LAUNCH
   }
-  return launch_kernel<true>(quantize_int8_block_kernel, grid, kQ8AnyThreads, 0, stream, static_cast<int8_t *>(out), scale,
-                             static_cast<const uint16_t *>(in), (int)N, (int)D, (int)Dp, (int)block, (int)nblk, stride[0], stride[1], stride[2],
-                             stride[3], (int)H, subp, ub, uh);
+#define AC4K_Q8_LAUNCH(T)                                                                                                                  \
+  return launch_kernel<true>(quantize_int8_block_kernel<T>, grid, T, 0, stream, static_cast<int8_t *>(out), scale,                           \
+                             static_cast<const uint16_t *>(in), (int)N, (int)D, (int)Dp, (int)block, (int)nblk, stride[0], stride[1], stride[2], \
+                             stride[3], (int)H, subp, ub, uh)
+  static_assert(kQ8AnyRows * (512 / 32) >= 128 && kQ8AnyRows * (128 / 32) >= 32, "rows of a block");
+  // 16 warps; four where the blocks are short and there are enough of them for the chip, since every warp walks the features,
+  // however few rows it has: [1, 4096, 16, 66] in blocks of 16 took 34.8 us with 16 warps and takes 19.3 with four, in blocks of 32
+  // 23.3 and 17.2; [1, 64, 1, 65] in blocks of 16 2.3 and 3.6.  Blocks of 64 and 128: 16 warps are as fast as eight or faster.
+  DeviceInfo di;
+  if (int e = get_device_info(&di)) return e;
+  if (block <= 32 && nblk * H * B >= 2 * (int64_t)di.sms) AC4K_Q8_LAUNCH(128);
+  AC4K_Q8_LAUNCH(512);
+#undef AC4K_Q8_LAUNCH
 }

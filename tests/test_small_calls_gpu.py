@@ -78,7 +78,8 @@ def test_columns_contiguous(b, k, h, d, precision):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("b,n,h,d,layout,block", [(11, 100, 12, 65, "BNHD", 128), (1, 129, 2, 1, "BHND", 64), (1, 130, 1, 127, "BNHD", 16),
-                                                 (1, 65, 2, 131, "BHND", 128), (2, 40, 1, 66, "BNHD", 32)])
+                                                 (1, 65, 2, 131, "BHND", 128), (2, 40, 1, 66, "BNHD", 32),
+                                                 (1, 1007, 5, 66, "BNHD", 16), (2, 1000, 5, 131, "BHND", 32)])     # four warps a block
 def test_block_quantiser_any_head_dimension(b, n, h, d, layout, block):
     from ac4k_kernel_b200.ops.attention import _int8_quantize
     x = (gaussian((b, n, h, d) if layout == "BNHD" else (b, h, n, d), seed=n + d) * 3).bfloat16().cuda()
@@ -253,6 +254,15 @@ def test_decode_rows_of_one_slice_take_no_longer():
         a = ops.quantize(gaussian((m, 512), seed=m).cuda(), 0, 1, sf_layout="128x4")
         t.append(_graph_microseconds(lambda: ops.linear(*a, *w), calls=100))
     assert t[0] < 1.55 * t[1]
+
+
+@pytest.mark.gpu
+def test_short_token_blocks_take_no_longer():
+    """[1, 4096, 16, 66] in blocks of 16 tokens against blocks of 128: twice the time with sixteen warps a block, 1.1 with four"""
+    from ac4k_kernel_b200.ops.attention import _int8_quantize
+    x = gaussian((1, 4096, 16, 66), seed=1).cuda()
+    t = [_graph_microseconds(lambda: _int8_quantize(x, "BNHD", 1, BLOCK_SIZE=block)) for block in (16, 128)]
+    assert t[0] < 1.5 * t[1]
 
 
 @pytest.mark.gpu
