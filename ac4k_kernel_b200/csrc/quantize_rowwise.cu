@@ -283,8 +283,23 @@ __global__ void colmax_to_scale_kernel(float *__restrict__ sf, const ScaleMax sc
 // through shared memory.  Single 2-byte loads, so odd row lengths and any alignment are taken too.
 // ----------------------------------------------------------------------------------------
 static constexpr int kShortCols = 64, kShortThreads = 512, kShortGroups = kShortThreads / kShortCols;
-static constexpr int kShortMaxK = 1024;    // one launch against four, per call: 7.2 / 18.6 us at 512 x 40 heads x 128 columns, 10.7 / 16.5 at 1024 x 16,
-                                           // 28.1 / 16.5 at 2048 x 16 (a CTA walks the rows alone)
+static constexpr int kShortMaxK = 1024;    // (a CTA walks the rows alone: 28.1 against 16.5 us at 2048 x 16 heads x 128 columns)
+
+// Whether that kernel is the one for [nbatch, K, M].  us in a replayed graph, this kernel / the other route (which costs four
+// launches, 20 us of host time a call, where the transposing kernels are the other one):
+//   transposing kernels   columns of up to 64: this one (300 x 1024 x 64: 25 / 32; 1280 x 77 x 64: 13 / 22; 1024 x 1024 x 8: 48 /
+//                         88).  Wider ones are read twice here too and two CTAs share a tile of theirs: up to 4e5 rows walked by
+//                         all CTAs, 2e5 where one alone walks more than 768, and eight CTAs per SM (640 CTAs x 512 rows: 22 / 26,
+//                         x 1000: 59 / 53; 256 x 1024: 24 / 21; 4800 x 16: 32 / 22)
+//   a warp per row        rows enough for eight warps per SM and half of the 64 columns of a CTA in use, a quarter over up to 128
+//                         rows (40 x 512 x 63: 6.4 / 6.8; 8 x 512 x 63: 6.3 / 4.0; 1 x 1024 x 1: 9.6 / 3.6; 300 x 1024 x 17: 19 /
+//                         14, x 128: 4.6 / 5.3)
+static bool column_short(int64_t nbatch, int64_t K, int64_t M, bool transposing, int sms) {
+  if (K <= 0 || K > kShortMaxK) return false;
+  if (!transposing) return M >= (K <= 128 ? kShortCols / 4 : kShortCols / 2) && nbatch * M > 8 * (int64_t)sms;
+  const int64_t ctas = nbatch * ceil_div(M, kShortCols);
+  return M <= kShortCols || (ctas <= 8 * (int64_t)sms && ctas * K <= (K <= 768 ? 400000 : 200000));
+}
 
 template <int FMT, bool PERMUTE>
 __global__ void __launch_bounds__(kShortThreads)
@@ -376,14 +391,18 @@ static int launch_rowwise(void *out, float *sf, const void *in, const ScaleMax &
 #undef AC4K_LAUNCH_ROWS
   }
   // columns contiguous, rows strided: one kernel over a short reduce dimension, else the transposing kernels
-  if (stride[2] == 1 && K > 0 && K <= kShortMaxK && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ceil_div(M16, kShortCols) <= 0x7fffffff) {
-    dim3 g((unsigned)ceil_div(M16, kShortCols), (unsigned)nbatch);
-    return launch_kernel<true>(swizzle ? column_quantize_short_kernel<FMT, true> : column_quantize_short_kernel<FMT, false>, g, kShortThreads, 0,
-                               stream, outp, sf, inp, scale_max, M, (int)K, M16, d1, stride[0], stride[1], stride[3]);
-  }
   const bool tr_ok = stride[2] == 1 && K > 0 && M % 2 == 0 && stride[3] % 2 == 0 && stride[0] % 2 == 0 && stride[1] % 2 == 0 &&
                      ((reinterpret_cast<uintptr_t>(in) & 3) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0) &&
                      ceil_div(K, kTrRows) <= 0x7fffffff && ceil_div(M, kTrCols) <= 65535;
+  if (stride[2] == 1 && K > 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ceil_div(M16, kShortCols) <= 0x7fffffff) {
+    DeviceInfo di;
+    if (int e = get_device_info(&di)) return e;
+    if (column_short(nbatch, K, M, tr_ok, di.sms)) {
+      dim3 g((unsigned)ceil_div(M16, kShortCols), (unsigned)nbatch);
+      return launch_kernel<true>(swizzle ? column_quantize_short_kernel<FMT, true> : column_quantize_short_kernel<FMT, false>, g, kShortThreads, 0,
+                                 stream, outp, sf, inp, scale_max, M, (int)K, M16, d1, stride[0], stride[1], stride[3]);
+    }
+  }
   if (tr_ok) {
     AC4K_CUDA_TRY(cudaMemsetAsync(sf, 0, (size_t)(nbatch * M16) * sizeof(float), stream));
     dim3 g1((unsigned)ceil_div(K, kTrChunk), (unsigned)ceil_div(M, kTrCols), (unsigned)nbatch);

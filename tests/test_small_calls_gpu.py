@@ -60,9 +60,12 @@ def test_odd_values_in_one_call(rows, fill):
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", ["fp8e4m3", "int8"])
 @pytest.mark.parametrize("b,k,h,d", [(1, 1, 1, 1), (2, 15, 3, 65), (2, 16, 1, 64), (1, 17, 2, 63), (1, 100, 12, 65), (1, 128, 2, 128),
-                                     (1, 512, 2, 64), (1, 1023, 1, 100), (1, 1024, 2, 17), (1, 1025, 2, 65), (1, 1025, 2, 66)])
+                                     (1, 512, 2, 64), (1, 1023, 1, 100), (1, 1024, 2, 17), (1, 1025, 2, 65), (1, 1025, 2, 66),
+                                     (300, 20, 1, 17), (300, 130, 1, 17), (40, 64, 1, 63), (8, 64, 1, 63),       # one launch; a warp a row; one; a warp a row
+                                     (150, 16, 4, 640), (3, 770, 1, 5000), (1, 1024, 1, 13000)])                 # four launches, one, four
 def test_columns_contiguous(b, k, h, d, precision):
-    """[B, N, H, D] along N: one launch up to 1024 rows, four beyond, the strided kernel where D is odd"""
+    """[B, N, H, D] along N: one launch over a short N where there are columns for its CTAs and not too many, else four launches,
+    or, where D is odd, a warp for each row"""
     from ac4k_kernel_b200 import ops
     x = (gaussian((b, k, h, d), seed=k + d) * 2).bfloat16().cuda()
     x[:, :, :, d // 2] = 0                                             # a column of zeros: 0 * inf
@@ -263,6 +266,17 @@ def test_short_token_blocks_take_no_longer():
     x = gaussian((1, 4096, 16, 66), seed=1).cuda()
     t = [_graph_microseconds(lambda: _int8_quantize(x, "BNHD", 1, BLOCK_SIZE=block)) for block in (16, 128)]
     assert t[0] < 1.5 * t[1]
+
+
+@pytest.mark.gpu
+def test_one_column_takes_no_cta_of_64():
+    """A column of 1024 values by itself: as long as 64 of them when a CTA walked it alone, a third of that with a warp"""
+    from ac4k_kernel_b200 import ops
+    t = []
+    for m in (1, 64):
+        x = gaussian((1024, m), seed=m).cuda()
+        t.append(_graph_microseconds(lambda: ops.quantize(x, 1, 0, precision="fp8e4m3")))
+    assert t[0] < 0.6 * t[1]
 
 
 @pytest.mark.gpu
