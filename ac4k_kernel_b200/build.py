@@ -6,10 +6,11 @@ One nvcc invocation per .cu (in parallel), then a link step.  The library links 
 runtime statically and resolves the driver entry point it needs (tensor-map encoding) at
 run time, so it has no link-time dependency on libcuda.
 
-csrc/host_calls.cc, the operators' host side, is compiled with the host compiler into `native/_host_calls*.so`.
+csrc/host_calls.cc, the operators' host side, is compiled with the host compiler into `native/_host_calls*.so` where torch is
+installed (the library alone needs neither torch nor Python).
 
-`--pybind` (or build_pybind()) also compiles csrc/bindings_pybind.cc into `native/_cuda_ops*.so`: the pybind11 module with the reference's names and signatures, linked
-against the library above.
+`--pybind` (or build_pybind()) also compiles csrc/bindings_pybind.cc into `native/_cuda_ops*.so`: the pybind11 module with
+the reference's names and signatures, linked against the library above.
 """
 from __future__ import annotations
 
@@ -143,11 +144,20 @@ def _build_module(name: str, source: str, force: bool) -> str:
     return target
 
 
+def main(args: list[str]) -> None:
+    force = "--force" in args
+    print(build(force=force, verbose="--verbose" in args))
+    try:
+        import torch  # noqa: F401
+    except ImportError:
+        print("torch is not installed: the library is built, native/_host_calls is not", file=sys.stderr)
+    else:
+        print(_build_module("_host_calls", "host_calls.cc", force))
+    if "--hooks" in args:
+        print(build_hooks(force=force))
+    if "--pybind" in args:
+        print(build_pybind(force=force))
+
+
 if __name__ == "__main__":
-    path = build(force="--force" in sys.argv, verbose="--verbose" in sys.argv)
-    print(path)
-    print(_build_module("_host_calls", "host_calls.cc", "--force" in sys.argv))
-    if "--hooks" in sys.argv:
-        print(build_hooks(force="--force" in sys.argv))
-    if "--pybind" in sys.argv:
-        print(build_pybind(force="--force" in sys.argv))
+    main(sys.argv[1:])

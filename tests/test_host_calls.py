@@ -1,5 +1,6 @@
 """The operators' native host side (csrc/host_calls.cc) against the Python wrappers' own path: what it refuses."""
 import glob
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -43,6 +44,17 @@ def test_modules_use_the_shared_libstdcxx(path):
         pytest.skip("no readelf")
     needed = subprocess.run(["readelf", "-d", path], capture_output=True, text=True, check=True).stdout
     assert "libstdc++.so.6" in needed
+
+
+def test_the_library_builds_without_torch(monkeypatch, capsys):
+    spec = importlib.util.spec_from_file_location("build_without_torch", os.path.join(PKG, "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    monkeypatch.setattr(build, "build", lambda **_: "the library")
+    monkeypatch.setitem(sys.modules, "torch", None)
+    build.main([])
+    printed = capsys.readouterr()
+    assert printed.out == "the library\n" and "torch is not installed" in printed.err
 
 
 @pytest.mark.gpu
