@@ -57,6 +57,25 @@ def test_the_library_builds_without_torch(monkeypatch, capsys):
     assert printed.out == "the library\n" and "torch is not installed" in printed.err
 
 
+@pytest.mark.parametrize("error,said", [(ModuleNotFoundError("none"), "is not built"), (ImportError("undefined symbol: x"), "does not load")])
+def test_a_missing_module_is_said(monkeypatch, error, said):
+    """Everything works without it, at several times the host time: not silently"""
+    import ac4k_kernel_b200.native as native
+
+    class Finder:
+        @staticmethod
+        def find_spec(name, path=None, target=None):
+            if name.endswith("_host_calls"):
+                raise error
+    spec = importlib.util.spec_from_file_location("without_host_calls", native.__file__, submodule_search_locations=[])
+    module = importlib.util.module_from_spec(spec)
+    monkeypatch.setitem(sys.modules, "without_host_calls", module)
+    monkeypatch.setattr(sys, "meta_path", [Finder, *sys.meta_path])
+    with pytest.warns(RuntimeWarning, match=said):
+        spec.loader.exec_module(module)
+    assert module.host_calls is None
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("kw", [dict(max_scale=-1.0), dict(max_scale=0), dict(max_scale=-5)])
 def test_refused_by_the_library(both_paths, kw):
