@@ -1,10 +1,12 @@
-"""The operators' native host side (csrc/host_calls.cc) against the Python wrappers' own path: what it refuses."""
+"""The operators' native host side (csrc/host_calls.cc) against the Python wrappers' own path: the same bits, the same refusals,
+on any stream and from several threads."""
 import glob
 import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import threading
 
 import pytest
 import torch
@@ -113,6 +115,207 @@ def test_options_are_left_to_the_wrappers(both_paths):
                       (lambda: ops.linear_requant(*w, *w, w[2], sf_layout=None), ValueError)):
         native, python = both_paths(fn)
         assert native is python and issubclass(native, Exception) and error in (None, native)
+
+
+def _bytes(v):
+    """results as a list of byte tensors"""
+    out = []
+    for t in v if isinstance(v, tuple) else (v,):
+        assert isinstance(t, torch.Tensor), t
+        out.append((t.shape, t.stride(), t.dtype, t.contiguous().reshape(-1).view(torch.uint8)))
+    return out
+
+
+def _same(a, b):
+    a, b = _bytes(a), _bytes(b)
+    return len(a) == len(b) and all(x[:3] == y[:3] and torch.equal(x[3], y[3]) for x, y in zip(a, b))
+
+
+def _offset(t):
+    """the same values one element behind a 256-byte boundary"""
+    buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    buf[1:] = t.reshape(-1)
+    return buf[1:].view(t.shape)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,cross,reduce", [((20, 256), 0, 1), ((300, 4104), 0, 1), ((3, 70, 1000), 1, 2), ((2, 130, 3, 80), 3, 1), ((2, 33, 3, 65), -1, -3),
+                                                ((2, 2, 50, 64), -2, -1), ((64, 96), 1, 0), ((1, 1024, 1, 130), 3, 1)])
+def test_quantize_same_bits(both_paths, shape, cross, reduce):
+    """every precision and option; also on a tensor that is not 16-byte aligned"""
+    from ac4k_kernel_b200 import ops
+    x = gaussian(shape, seed=sum(shape)).cuda()
+    for kw in (dict(), dict(sf_layout="128x4"), dict(swizzle=True), dict(max_scale=1000), dict(max_scale=0.1), dict(precision="fp8e4m3"),
+               dict(precision="fp8e4m3", swizzle=True, max_scale=2.25), dict(precision="fp8e4m3", max_scale=100), dict(precision="int8"),
+               dict(precision="int8", max_scale=100), dict(precision="int8", max_scale=-5), dict(precision="int8", max_scale=12.0)):
+        native, python = both_paths(lambda: ops.quantize(x, cross, reduce, **kw))
+        assert _same(native, python), kw
+        assert all(_same(v, python) for v in both_paths(lambda: ops.quantize(_offset(x), cross, reduce, **kw))), kw
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", ["ac4k", "128x4"])
+@pytest.mark.parametrize("m", [1, 37, 100, 300])
+def test_linear_same_bits(both_paths, m, layout):
+    from ac4k_kernel_b200 import ops
+    n, k = 192, 528
+    a, w = ops.quantize(gaussian((m, k), seed=m).cuda(), 0, 1, sf_layout=layout), ops.quantize(gaussian((n, k), seed=1).cuda(), 0, 1, sf_layout=layout)
+    gs = torch.tensor(0.01, device="cuda")
+    for dtype in (torch.bfloat16, torch.float16, torch.float32):
+        bias = gaussian((n,), seed=2).to(dtype).cuda()
+        for b in (None, bias, bias.view(1, n)):
+            assert _same(*both_paths(lambda: ops.linear(*a, *w, bias=b)))
+            out = torch.empty((m, n), dtype=dtype, device="cuda")
+
+            def given():
+                out.fill_(float("nan"))
+                assert ops.linear(*a, *w, b, out) is out
+                return out.clone()
+            assert _same(*both_paths(given))
+            for out_layout in ("ac4k", "128x4"):
+                assert _same(*both_paths(lambda: ops.linear_requant(*a, *w, gs, bias=b, sf_layout=out_layout)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,d", [(3, 128), (2, 20), (1, 1032)])
+def test_rope_same_bits(both_paths, n, d):
+    from ac4k_kernel_b200 import ops
+    from oracle import emulation as E
+    x, freqs = gaussian((2, 24, n, d), seed=d).cuda(), E.rope_params_ref(8, d).cuda()
+    grid = torch.tensor([[2, 3, 4], [1, 2, 3]], dtype=torch.int32, device="cuda")
+    out = torch.empty_like(x)
+
+    def given():
+        out.zero_()
+        assert ops.rope3d(x, grid, freqs, out) is out
+        return out.clone()
+    results = [*both_paths(lambda: ops.rope3d(x, grid, freqs)), *both_paths(given), *both_paths(lambda: ops.rope3d(_offset(x), grid, freqs))]
+    assert all(_same(results[0], r) for r in results)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["nvfp4", "int8+fp8e4m3"])
+@pytest.mark.parametrize("nq,nkv,d,dv", [(70, 70, 80, 80), (1, 200, 128, 64), (130, 515, 65, 33)])
+def test_attention_same_bits(both_paths, nq, nkv, d, dv, precision):
+    """head dimensions that differ, rows that are not 16-byte aligned; the INT8 path also takes q and k that are not contiguous"""
+    from ac4k_kernel_b200 import ops
+    q, k, v = gaussian((2, nq, 3, d), seed=1).cuda(), gaussian((2, nkv, 3, d), seed=2).cuda(), gaussian((2, nkv, 3, dv), seed=3).cuda()
+    native, python = both_paths(lambda: ops.attention(q, k, v, precision=precision))
+    assert _same(native, python) and not bool(torch.isnan(native.float()).any())
+    assert all(_same(r, python) for r in both_paths(lambda: ops.attention(_offset(q), _offset(k), _offset(v), precision=precision)))
+    t = [x.transpose(1, 2).contiguous() for x in (q, k, v)]
+    buf = torch.empty((2, 3, nq + 1, dv + 3), dtype=torch.bfloat16, device="cuda")[:, :, 1:, 3:]      # rows at odd offsets
+
+    def given():
+        buf.zero_()
+        assert ops.attention(*t, layout="BHND", precision=precision, out=buf) is buf
+        return buf.clone()
+    for r in (*both_paths(lambda: ops.attention(*t, layout="BHND", precision=precision)), *both_paths(given)):
+        assert torch.equal(r, python.transpose(1, 2))
+    strided = [x.transpose(1, 2) for x in t[:2]]
+    results = both_paths(lambda: ops.attention(*strided, v, precision=precision))
+    assert results == [RuntimeError, RuntimeError] if precision == "nvfp4" else all(torch.equal(r, python) for r in results)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,cross,reduce,swizzle", [((50, 8192), 0, 1, False), ((666, 4096), 0, 1, False), ((2049, 4096), 0, 1, False), ((16, 8192), 0, 1, False),
+                                                        ((2, 100, 3, 128), 3, 1, True), ((2, 33, 3, 65), 3, 1, True), ((4100, 4096), 0, 1, False)])
+def test_dynamic_entry_with_and_without_scratch(shape, cross, reduce, swizzle):
+    """ac4k_quantize_nvfp4_dynamic called as from C: scratch may be NULL at any size"""
+    from ac4k_kernel_b200 import _cuda_ops as ct
+    from ac4k_kernel_b200 import ops
+    x = gaussian(shape, seed=4).cuda()
+    want = ops.quant.Ac4kQuantizeOp()(x, cross, reduce, swizzle=swizzle)
+    size, stride, _ = ct._view4(x, cross, reduce)
+    scratch = torch.full((1024,), -1, dtype=torch.int32, device="cuda")
+    for s in (None, scratch.data_ptr()):
+        q, sf, g = torch.empty_like(want[0]), torch.empty_like(want[1]), torch.empty((), device="cuda")
+        rc = ct.LIB.ac4k_quantize_nvfp4_dynamic(q.data_ptr(), sf.data_ptr(), g.data_ptr(), s, x.data_ptr(), 2688.0, ct._I64x4(*size),
+                                                ct._I64x4(*stride), int(swizzle), 0, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0 and _same((q, sf, g), want)
+
+
+def _work(i):
+    """a call of every operator on inputs of its own; returns the results in one tuple"""
+    from ac4k_kernel_b200 import ops
+    from oracle import emulation as E
+    x, w = gaussian((50 + 300 * (i % 2), 1024), seed=i).cuda(), gaussian((512, 1024), seed=i + 50).cuda()
+    q, k, v = (gaussian((1, 200 + 30 * i, 2, 64), seed=i + j).cuda() for j in (100, 200, 300))
+    grid, freqs = torch.tensor([[q.shape[1], 1, 1]], dtype=torch.int32, device="cuda"), E.rope_params_ref(512, 64).cuda()
+    torch.cuda.synchronize()
+
+    def run():
+        a, b = ops.quantize(x * 1.5, 0, 1), ops.quantize(w, 0, 1)          # (the inputs are made on the stream as well)
+        y = ops.linear(*a, *b)
+        turned = ops.rope3d(q + k, grid, freqs)
+        return (*a, *b, y, *ops.quantize(y, 0, 1, precision="int8"), *ops.quantize(y, 0, 1, precision="fp8e4m3"), turned,
+                ops.attention(turned, k, v), ops.attention(turned, k, v, precision="nvfp4"))
+    return run
+
+
+@pytest.mark.gpu
+def test_side_streams():
+    """Operators on two streams at once, behind work of those streams: as on the default stream"""
+    from ac4k_kernel_b200 import _lib
+    runs = [_work(i) for i in range(4)]
+    want = [r() for r in runs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    got = {}
+    busy = torch.randn((4096, 4096), device="cuda")
+    for _ in range(5):
+        for i, r in enumerate(runs):
+            with torch.cuda.stream(streams[i % 2]):
+                torch.mm(busy, busy)                                     # the host is ahead of the stream
+                got[i] = r()
+        torch.cuda.synchronize()
+        assert all(_same(got[i], want[i]) for i in range(4))
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("i", [0, 1])
+def test_captured_operators(i):
+    """every operator in one graph, replayed over results of its own that are cleared in between"""
+    run = _work(i)
+    want = run()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        got = run()
+    for _ in range(3):
+        for r in got:
+            r.view(torch.uint8).fill_(0x55) if r.dim() else r.fill_(7.0)
+        g.replay()
+        torch.cuda.synchronize()
+        assert _same(got, want)
+
+
+@pytest.mark.gpu
+def test_several_threads():
+    """Three host threads, each with a stream of its own (the native calls run without the interpreter lock)"""
+    from ac4k_kernel_b200 import _lib
+    runs = [_work(i) for i in range(3)]
+    want = [r() for r in runs]
+    torch.cuda.synchronize()
+    failed = []
+
+    def thread(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(30):
+                    got = runs[i]()
+                    torch.cuda.current_stream().synchronize()
+                    assert _same(got, want[i])
+        except BaseException as e:
+            failed.append((i, repr(e)))
+    threads = [threading.Thread(target=thread, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(timeout=120)
+    assert not failed and not any(t.is_alive() for t in threads), failed
+    assert _lib.device_status() == 0
 
 
 class Sub(torch.Tensor):
