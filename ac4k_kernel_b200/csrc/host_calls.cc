@@ -284,7 +284,6 @@ py::object attention(py::handle hq, py::handle hk, py::handle hv, py::handle hla
     if (t->size(0) != B || t->size(h_dim) != H || t->size(n_dim) != Nkv) return py::none();
   if (k.size(3) != D || D < 1 || D > 128 || Dv < 1 || Dv > 128 || B < 1 || H < 1 || Nq < 1 || Nkv < 1) return py::none();
   if (k.device() != q.device() || v.device() != q.device()) return py::none();
-  if (nvfp4 && align_up(D, 64) > 128) return py::none();
   at::Tensor out;
   if (!hout.is_none()) {
     const auto t = tensor_of(hout, at::kBFloat16, 4, false);

@@ -13,11 +13,6 @@ __device__ __forceinline__ float ex2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float rcp_approx(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 // max of three (one FMNMX3), and two fp32 operations in one instruction on an aligned register pair
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;

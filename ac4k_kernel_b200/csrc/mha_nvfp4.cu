@@ -26,7 +26,7 @@
 // both idle.  [1, 16384, 16, 128], kernel alone: 1 688 us with four warps per group, a row per thread, and O rescaled before the
 // exponentials (a wait for the previous P V and a chain of small loads and stores); 1 728 with eight warps per group, 1 654 with
 // the rescale behind the exponentials (a quarter of the exponentials as a polynomial on the FMA pipe); 1 640 with an eighth of
-// them there, 1 579 with none: the polynomial costs thirteen issue slots a pair, and those bound the kernel now; 1 555 with the
+// them there, 1 579 with none: the polynomial costs thirteen issue slots a pair, more than it relieves the ex2 pipe of; 1 555 with the
 // two threads that share a block finishing one row's block scales each instead of both rows' twice.
 // Sharing one score buffer keeps the groups a few hundred cycles apart (group B's S is issued when group A has copied its own
 // out), so that one group's waits, maxima and fences run under the other's exponentials.
@@ -96,26 +96,8 @@ struct MhaArgs {
 #define AC4K_TRM(region, it, ev) do { } while (0)
 #endif
 
-// two non-negative fp32 -> two e4m3 bytes (a in the low byte) and their values back as fp32
-__device__ __forceinline__ uint32_t e4m3x2_round_trip(float a, float b, float &fa, float &fb) {
-  uint16_t pk;
-  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(pk) : "f"(b), "f"(a));
-  uint32_t h2;
-  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"(pk));
-  const __half2 hh = *reinterpret_cast<const __half2 *>(&h2);
-  fa = __low2float(hh);
-  fb = __high2float(hh);
-  return pk;
-}
-__device__ __forceinline__ void tmem_st_32x32b_x32_f(uint32_t taddr, const float (&v)[32]) {
-  uint32_t u[32];
-#pragma unroll
-  for (int i = 0; i < 32; ++i) u[i] = __float_as_uint(v[i]);
-  tmem_st_32x32b_x32(taddr, u);
-}
-
 // SF_TILED: block scales arrive as 512-byte chunks that tensor memory takes as they are (bulk copies).  Otherwise they
-// are in the reference's layout, one 32-bit word per row and K = 64 step, rows contiguous: warp 10 transposes each
+// are in the reference's layout, one 32-bit word per row and K = 64 step, rows contiguous: warp 2 transposes each
 // chunk (128 words -> 32 rows of 4 words) into shared memory with plain loads.
 template <bool SF_TILED>
 __global__ void __launch_bounds__(mha::kThreads, 1)

@@ -5,9 +5,9 @@
 // approximate reciprocals replaced by correctly rounded fp32 operations:
 //     alpha = 1 / g ;  sf = e4m3(alpha * (amax16 * fp32(1/6))) ;
 //     r = sf ? alpha * (1 / float(sf)) : 0 ;  code = e2m1(float(x) * r)
-// Three kernels: a tiled one for rows that are contiguous along K (the linear path), a transposing one
-// for rows that are contiguous along the cross dimension (attention's V), and a strided one (any
-// cross/reduce strides, optional K permutation) for everything else.
+// Four kernels: a tiled one for rows that are contiguous along K (the linear path) and a flat one for those tensors that are too
+// small for its tiles, a transposing one for rows that are contiguous along the cross dimension (attention's V), and a strided one
+// (any cross/reduce strides, optional K permutation) for everything else.
 #include <algorithm>
 
 #include "common.cuh"

@@ -106,7 +106,6 @@ __global__ void __launch_bounds__(kRopeThreads, MODE == 0 ? kRopeWarpsPerSm * 32
   const int64_t row_elems = (int64_t)N * D;
   const int c0 = (int)((threadIdx.x * 4) % C);                  // MODE 0: this thread's four pairs
   if (MODE == 0 && (int)threadIdx.x >= active) return;          // (no barrier in this mode)
-  grid_dependency_wait();
   // position ps = (b, pos), carried along without dividing again
   int b = (int)(blockIdx.x / (uint32_t)S), pos = (int)(blockIdx.x % (uint32_t)S);
   const int step_b = (int)(gridDim.x / (uint32_t)S), step_pos = (int)(gridDim.x % (uint32_t)S);

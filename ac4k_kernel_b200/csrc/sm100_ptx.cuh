@@ -44,17 +44,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 // Bounded wait: false if the phase did not complete within `limit_ns` (the kernels pass the limit they were
 // launched with: kWaitTimeoutNs unless a test build shortened it).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned long long limit_ns = kWaitTimeoutNs) {
@@ -74,37 +63,11 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 }
 
 // ---- TMA --------------------------------------------------------------------------------
-// x is the innermost (byte) coordinate and must be a multiple of 16 bytes.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *tmap, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
+// x is the innermost coordinate, in elements of the map; x times the element size is a multiple of 16 bytes
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void *tmap, int x, int y, int z, int w, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
       ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
-      : "memory");
-}
-// linear copy: src/dst 16-byte aligned, bytes a multiple of 16
-__device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-      : "memory");
-}
-// same, with the destination and the barrier named as shared::cta addresses (own CTA only)
-__device__ __forceinline__ void bulk_load_1d_local(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_2d_local(uint32_t dst, const void *tmap, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
 // Hint: bring the box into L2.  Returns no data, so it may be issued before griddepcontrol.wait: lines
@@ -168,25 +131,6 @@ __host__ __device__ constexpr uint32_t make_idesc_mxf4nvf4(int m, int n) {
   return (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// ---- tcgen05 ----------------------------------------------------------------------------
-// D[tmem] (+)= A[smem] * B[smem]^T with per-16-element block scales taken from tensor memory.
-__device__ __forceinline__ void mma_mxf4nvf4(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %6, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(sfa_tmem), "r"(sfb_tmem), "r"(accumulate)
-      : "memory");
-}
-// 32 rows x 16 bytes of shared memory -> 4 columns of tensor memory, replicated to the four
-// 32-lane quarters.
-__device__ __forceinline__ void tmem_cp_32x128b_warpx4(uint32_t taddr, uint64_t sdesc) {
-  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
-}
-// arrive on an mbarrier once all tcgen05 operations issued so far by this thread are done
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
 // each lane reads 32 consecutive 32-bit columns of its own tensor-memory lane
 __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
@@ -198,33 +142,6 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)
         "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
         "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
       : "r"(taddr)
-      : "memory");
-}
-// each lane writes N consecutive 32-bit columns of its own tensor-memory lane
-__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
-        "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
-        "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_32x32b_x64(uint32_t taddr, const uint32_t (&v)[64]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x64.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63, %64};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]), "r"(v[32]), "r"(v[33]), "r"(v[34]), "r"(v[35]), "r"(v[36]), "r"(v[37]), "r"(v[38]), "r"(v[39]), "r"(v[40]), "r"(v[41]), "r"(v[42]), "r"(v[43]), "r"(v[44]), "r"(v[45]), "r"(v[46]), "r"(v[47]), "r"(v[48]), "r"(v[49]), "r"(v[50]), "r"(v[51]), "r"(v[52]), "r"(v[53]), "r"(v[54]), "r"(v[55]), "r"(v[56]), "r"(v[57]), "r"(v[58]), "r"(v[59]), "r"(v[60]), "r"(v[61]), "r"(v[62]), "r"(v[63])
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -240,8 +157,6 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32_sync(uint32_t taddr, uint32_t
 #pragma unroll
   for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(v[i]) : : "memory");
 }
-
-
 __device__ __forceinline__ void tmem_ld_32x32b_x64_sync(uint32_t taddr, uint32_t (&v)[64]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x64.b32 "
@@ -313,11 +228,6 @@ __device__ __forceinline__ void tmem_pin(uint32_t (&v)[N]) {
   for (int i = 0; i < N; ++i) asm volatile("" : "+r"(v[i]) : : "memory");
 }
 
-__device__ __forceinline__ uint32_t ld_shared_volatile(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-  return v;
-}
 __device__ __forceinline__ void st_shared_v4f(uint32_t addr, float a, float b, float c, float d) {
   asm volatile("st.shared::cta.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
@@ -330,9 +240,6 @@ __device__ __forceinline__ float2 ld_shared_v2f(uint32_t addr) {
   float2 v;
   asm volatile("ld.shared::cta.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
   return v;
-}
-__device__ __forceinline__ void st_shared_release(uint32_t addr, uint32_t v) {
-  asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
 // (a0 * s, a1 * s) in fp32, round to nearest, packed to two bf16 / fp16 (element 0 in the low half)
@@ -372,25 +279,6 @@ __device__ __forceinline__ uint32_t scale_pack_f16x2(uint32_t a0, uint32_t a1, f
   return out;
 }
 
-// 32-byte global store (one full sector per lane)
-__device__ __forceinline__ void st_global_v8(void *p, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e,
-                                             uint32_t f, uint32_t g, uint32_t h) {
-  asm volatile("st.global.L1::no_allocate.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-               ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d), "r"(e), "r"(f), "r"(g), "r"(h)
-               : "memory");
-}
-
-// 16-byte global load served by L2 (never by this SM's L1, which may hold a stale line)
-__device__ __forceinline__ uint4 ld_global_cg_v4(const void *p) {
-  uint4 v;
-  asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
-}
-// 16-byte global store without L1 allocation (used for peer memory)
-__device__ __forceinline__ void st_global_v4(void *p, uint4 v) {
-  asm volatile("st.global.L1::no_allocate.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
-
 // ---- CTA pairs (cta_group::2) and clusters ----------------------------------------------
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -402,10 +290,6 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
-}
-// 16-byte store into the shared memory of a CTA of this cluster (address from map_to_cta)
-__device__ __forceinline__ void st_shared_cluster_v4(uint32_t addr, float a, float b, float c, float d) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 __device__ __forceinline__ void st_shared_cluster_u32(uint32_t addr, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
@@ -429,17 +313,6 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
-__device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-// TMA load whose completion is signalled on an mbarrier that may live in the peer CTA of the pair
-// (shared::cluster addresses for both the destination and the barrier)
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void *tmap, int x, int y, uint32_t bar_cluster_addr) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar_cluster_addr)
-      : "memory");
-}
 // TMA store shared -> global (tiled, clipped at the tensor bounds); x in elements of the map
 __device__ __forceinline__ void tma_store_2d(const void *tmap, int x, int y, uint32_t src) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
@@ -451,27 +324,8 @@ __device__ __forceinline__ void tma_store_3d(const void *tmap, int x, int y, int
                ::"l"(tmap), "r"(x), "r"(y), "r"(z), "r"(src)
                : "memory");
 }
-// same, with an L2 cache policy for the written lines (from make_policy_evict_first / _last)
-__device__ __forceinline__ void tma_store_2d_hint(const void *tmap, int x, int y, uint32_t src, uint64_t policy) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group.L2::cache_hint [%0, {%1, %2}], [%3], %4;"
-               ::"l"(tmap), "r"(x), "r"(y), "r"(src), "l"(policy)
-               : "memory");
-}
-__device__ __forceinline__ uint64_t make_policy_evict_first() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-__device__ __forceinline__ uint64_t make_policy_evict_last() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_group_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void bulk_wait_group_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void bulk_wait_group0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols)
@@ -482,29 +336,6 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 }
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// one MMA over both CTAs of the pair: M = 256 (128 rows per CTA), B halves read from both CTAs
-__device__ __forceinline__ void mma_mxf4nvf4_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                                  uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %6, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(sfa_tmem), "r"(sfb_tmem), "r"(accumulate)
-      : "memory");
-}
-// completion of this thread's earlier tcgen05 work -> one arrival on the mbarrier at this
-// shared-memory offset in every CTA of `cta_mask` (both CTAs of the pair: 3).  This is the
-// commit's own arrival fan-out, not a multicast load.
-__device__ __forceinline__ void tc_commit_pair_both(uint32_t bar, uint16_t cta_mask) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"(cta_mask)
-               : "memory");
-}
-// completion of this thread's earlier tcgen05 work -> one arrival on an mbarrier given by a
-// shared::cluster address (own or peer CTA)
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr)
-               : "memory");
 }
 
 // ---- warp-wide issue ----------------------------------------------------------------------
@@ -530,10 +361,6 @@ __device__ __forceinline__ void mbar_arrive_expect_tx_if(uint32_t pred, uint32_t
   asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %2, 0;\n@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}"
                ::"r"(bar), "r"(bytes), "r"(pred) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_cluster_if(uint32_t pred, uint32_t bar_cluster_addr) {
-  asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %1, 0;\n@q mbarrier.arrive.shared::cluster.b64 _, [%0];\n}"
-               ::"r"(bar_cluster_addr), "r"(pred) : "memory");
-}
 __device__ __forceinline__ void tma_load_2d_if(uint32_t pred, uint32_t dst, const void *tmap, int x, int y, uint32_t bar) {
   asm volatile(
       "{\n.reg .pred q;\nsetp.ne.b32 q, %5, 0;\n"
@@ -541,6 +368,7 @@ __device__ __forceinline__ void tma_load_2d_if(uint32_t pred, uint32_t dst, cons
       ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar), "r"(pred)
       : "memory");
 }
+// load whose completion is signalled on an mbarrier that may be the peer CTA's of the pair (shared::cluster addresses)
 __device__ __forceinline__ void tma_load_2d_pair_if(uint32_t pred, uint32_t dst, const void *tmap, int x, int y,
                                                     uint32_t bar_cluster_addr) {
   asm volatile(
@@ -557,6 +385,7 @@ __device__ __forceinline__ void tma_load_3d_pair_if(uint32_t pred, uint32_t dst,
       ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar_cluster_addr), "r"(pred)
       : "memory");
 }
+// linear copy: source and destination 16-byte aligned, bytes a multiple of 16
 __device__ __forceinline__ void bulk_load_1d_if(uint32_t pred, uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
   asm volatile(
       "{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\n"
@@ -564,6 +393,7 @@ __device__ __forceinline__ void bulk_load_1d_if(uint32_t pred, uint32_t dst, con
       ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "r"(pred)
       : "memory");
 }
+// D[tmem] (+)= A[smem] * B[smem]^T with per-16-element block scales taken from tensor memory
 __device__ __forceinline__ void mma_mxf4nvf4_if(uint32_t pred, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                                 uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
   asm volatile(
@@ -572,6 +402,7 @@ __device__ __forceinline__ void mma_mxf4nvf4_if(uint32_t pred, uint32_t d_tmem, 
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(sfa_tmem), "r"(sfb_tmem), "r"(accumulate), "r"(pred)
       : "memory");
 }
+// the same over both CTAs of the pair: M = 256 (128 rows per CTA), B halves read from both
 __device__ __forceinline__ void mma_mxf4nvf4_pair_if(uint32_t pred, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                                      uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
   asm volatile(
@@ -592,11 +423,14 @@ __device__ __forceinline__ void tmem_cp_32x128b_warpx4_pair_if(uint32_t pred, ui
   asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %2, 0;\n@q tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;\n}"
                ::"r"(taddr), "l"(sdesc), "r"(pred) : "memory");
 }
+// arrive on an mbarrier once all tcgen05 operations issued so far by this thread are done
 __device__ __forceinline__ void tc_commit_if(uint32_t pred, uint32_t bar) {
   asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %1, 0;\n"
                "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}"
                ::"r"(bar), "r"(pred) : "memory");
 }
+// the same: one arrival on the mbarrier at this shared-memory offset in every CTA of `cta_mask` (both of the pair: 3); the
+// commit's own arrival fan-out, not a multicast load
 __device__ __forceinline__ void tc_commit_pair_both_if(uint32_t pred, uint32_t bar, uint16_t cta_mask) {
   asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %2, 0;\n"
                "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}"
