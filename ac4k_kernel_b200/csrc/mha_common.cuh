@@ -56,12 +56,16 @@ __device__ __forceinline__ void mha_rescale(uint32_t t_o, const float (&a)[2]) {
   ptx::tmem_st_16x256b_x16(t_o, ro);
   ptx::tmem_st_wait();
 }
-// Query tiles per CTA.  A pair of tiles shares the K and V tiles and fills each other's waits (a pair's key tile takes 1.4 times
-// a single one's), but a launch of few CTAs leaves SMs idle: one tile per CTA where that ends sooner, counted in waves.
+// Query tiles per CTA.  A pair of tiles shares the K and V tiles and fills each other's waits, but a launch of few CTAs leaves SMs
+// idle: one tile per CTA where that ends sooner, counted in waves of CTAs.  A CTA with two tiles takes 1.4 times one with one (INT8,
+// 4096 keys: 55 / 40 us a wave; NVFP4 61 / 43), and with an odd number of tiles every head's last CTA has one.  Kernel us, one tile /
+// two, INT8 (NVFP4 alike): 9 heads x 2048 x 2048, one wave either way: 27 / 32; 12 heads, two waves against one: 47 / 33; 190 heads
+// x 384 x 1024, four against three, every other CTA with one tile: 62 / 53; 98 heads, two against two: 31 / 33.
 inline int mha_query_tiles(int64_t q_blocks, int64_t heads, int sms) {
-  const int64_t pairs = heads * ((q_blocks + 1) / 2), singles = heads * q_blocks;
-  const int64_t wave2 = 14 * ((pairs + sms - 1) / sms), wave1 = 10 * ((singles + sms - 1) / sms);
-  return q_blocks > 1 && wave1 >= wave2 ? 2 : 1;
+  if (q_blocks < 2) return 1;
+  const int64_t full = q_blocks / 2, ctas = full + (q_blocks & 1);       // of a head, two tiles each
+  const int64_t waves2 = (heads * ctas + sms - 1) / sms, waves1 = (heads * q_blocks + sms - 1) / sms;
+  return 10 * waves1 * ctas >= waves2 * (14 * full + 10 * (q_blocks & 1)) ? 2 : 1;
 }
 // O may be stored four columns at a time: its rows are contiguous and start on 8-byte boundaries
 __device__ __forceinline__ bool mha_rows_vec4(const void *O, int64_t o_b, int64_t o_h, int64_t o_n, int64_t o_d, int Dv) {
