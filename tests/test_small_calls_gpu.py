@@ -256,7 +256,7 @@ def test_decode_rows_of_one_slice_take_no_longer():
     for m in (64, 1):
         a = ops.quantize(gaussian((m, 512), seed=m).cuda(), 0, 1, sf_layout="128x4")
         t.append(_graph_microseconds(lambda: ops.linear(*a, *w), calls=100))
-    assert t[0] < 1.55 * t[1]
+    assert t[0] < 1.58 * t[1]
 
 
 @pytest.mark.gpu
@@ -292,6 +292,19 @@ def test_query_tiles_by_the_time_they_take():
         o = torch.empty((1, 190, nq, 128), dtype=torch.bfloat16, device="cuda")
         t.append(_graph_microseconds(lambda: _cuda_ops.mha_int8_x_fp8_fwd(o, *args, 128 ** -0.5), calls=5))
     assert t[0] < 0.95 * t[1]
+
+
+@pytest.mark.gpu
+def test_narrow_rows_fill_the_chip():
+    """q of attention, rows of 128 features, against as many bytes in long rows: 1.16 - 1.19 of the time with four CTAs of the
+    narrow tiles on an SM, 1.09 - 1.10 with five"""
+    from ac4k_kernel_b200 import _cuda_ops, ops
+    t = []
+    for shape, cross, reduce in (((1, 75600, 40, 128), 1, 3), ((75600, 5120), 0, 1)):
+        x = torch.randn(shape, device="cuda", dtype=torch.bfloat16)
+        q, sf, g = ops.quantize(x, cross, reduce, sf_layout="128x4")
+        t.append(min(_graph_microseconds(lambda: _cuda_ops.quantize_nvfp4(q, sf, x, g, cross, reduce, False), calls=5) for _ in range(3)))
+    assert t[0] < 1.14 * t[1]
 
 
 @pytest.mark.gpu
