@@ -62,18 +62,23 @@ __device__ __forceinline__ uint32_t rope_pair_fast(uint32_t xy, const RopeFactor
   const __nv_bfloat162 lo = __floats2bfloat162_rn(__fsub_rn(re, e), __fsub_rn(im, e));
   const __nv_bfloat162 hi = __floats2bfloat162_rn(__fadd_rn(re, e), __fadd_rn(im, e));
   const uint32_t l = *reinterpret_cast<const uint32_t *>(&lo);
-  if (a != 0.0f || e != 0.0f) {          // (a pair of zeros under a good factor is exact, the sign of its zeros included)
+  if (a != 0.0f) {          // (a pair of zeros under a good factor is exact, the sign of its zeros included)
     diff |= l ^ *reinterpret_cast<const uint32_t *>(&hi);
     out_of_range = max(out_of_range, __float_as_uint(e) - kRopeMinE);
   }
   return l;
 }
 
+// not 0 if one of four factors is for fp64 alone
+__device__ __forceinline__ uint32_t rope_unusable(const RopeFactor *ff) {
+  const float s = (ff[0].e + ff[1].e) + (ff[2].e + ff[3].e);         // (positive or NaN)
+  return s == s ? 0u : 0xffffffffu;
+}
 // eight elements (four pairs) of a vector; f(i): factor i in fp64
 template <typename Exact>
-__device__ __forceinline__ uint4 rope_vec(const uint4 &q, const RopeFactor *ff, Exact &&f) {
+__device__ __forceinline__ uint4 rope_vec(const uint4 &q, const RopeFactor *ff, uint32_t unusable, Exact &&f) {
   uint4 o;
-  uint32_t diff = 0, range = 0;
+  uint32_t diff = 0, range = unusable;
   o.x = rope_pair_fast(q.x, ff[0], diff, range);
   o.y = rope_pair_fast(q.y, ff[1], diff, range);
   o.z = rope_pair_fast(q.z, ff[2], diff, range);
@@ -134,17 +139,19 @@ __global__ void __launch_bounds__(kRopeThreads, MODE == 0 ? kRopeWarpsPerSm * 32
       };
       load_batch(threadIdx.x);
       RopeFactor ff[4];
+      uint32_t unusable = 0;
       auto exact = [&](int i) { return __ldg(freqs + (int64_t)rope_row(c0 + i, c1, c2, fi, hi, wi) * C + c0 + i); };
       if (inside) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) ff[i] = rope_factor(exact(i));
+        unusable = rope_unusable(ff);
       }
       for (int v0 = threadIdx.x; v0 < nvec; v0 += kRopeBatch * active) {
         if (v0 != (int)threadIdx.x) load_batch(v0);
 #pragma unroll
         for (int u = 0; u < kRopeBatch; ++u) {
           const int v = v0 + u * active;
-          if (v < nvec) __stcs(d4 + v, inside ? rope_vec(q[u], ff, exact) : q[u]);
+          if (v < nvec) __stcs(d4 + v, inside ? rope_vec(q[u], ff, unusable, exact) : q[u]);
         }
       }
       continue;
@@ -166,7 +173,7 @@ __global__ void __launch_bounds__(kRopeThreads, MODE == 0 ? kRopeWarpsPerSm * 32
         uint4 q = __ldcs(s4 + v);
         if (inside) {
           const int cv = (int)((v * 4) % C);                      // first of this vector's four pairs
-          q = rope_vec(q, sff + cv, [&](int i) { return sf[cv + i]; });
+          q = rope_vec(q, sff + cv, rope_unusable(sff + cv), [&](int i) { return sf[cv + i]; });
         }
         __stcs(d4 + v, q);
       }
