@@ -309,7 +309,8 @@ def test_narrow_rows_fill_the_chip():
 
 @pytest.mark.gpu
 def test_native_host_side_is_the_python_path():
-    """Same results as the wrappers' own path, and the same refusals"""
+    """Attention's results are the wrappers' own, given an output or not, and so are some refusals (all operators and options:
+    test_host_calls.py)"""
     from ac4k_kernel_b200 import ops
     from ac4k_kernel_b200.native import host_calls
     import sys
