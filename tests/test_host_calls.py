@@ -215,6 +215,10 @@ def test_attention_same_bits(both_paths, nq, nkv, d, dv, precision):
     strided = [x.transpose(1, 2) for x in t[:2]]
     results = both_paths(lambda: ops.attention(*strided, v, precision=precision))
     assert results == [RuntimeError, RuntimeError] if precision == "nvfp4" else all(torch.equal(r, python) for r in results)
+    if precision != "nvfp4":
+        shared = k[:, :, :1].expand(-1, -1, 3, -1)                       # one key head for three query heads: a stride of 0
+        native, python = both_paths(lambda: ops.attention(q, shared, v, precision=precision))
+        assert _same(native, python) and _same(native, ops.attention(q, shared.contiguous(), v, precision=precision))
 
 
 @pytest.mark.gpu
