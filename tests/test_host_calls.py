@@ -239,7 +239,7 @@ def test_dynamic_entry_with_and_without_scratch(shape, cross, reduce, swizzle):
         assert rc == 0 and _same((q, sf, g), want)
 
 
-def _work(i):
+def _every_operator(i):
     """a call of every operator on inputs of its own; returns the results in one tuple"""
     from ac4k_kernel_b200 import ops
     from oracle import emulation as E
@@ -261,7 +261,7 @@ def _work(i):
 def test_side_streams():
     """Operators on two streams at once, behind work of those streams: as on the default stream"""
     from ac4k_kernel_b200 import _lib
-    runs = [_work(i) for i in range(4)]
+    runs = [_every_operator(i) for i in range(4)]
     want = [r() for r in runs]
     torch.cuda.synchronize()
     streams = [torch.cuda.Stream() for _ in range(2)]
@@ -281,7 +281,7 @@ def test_side_streams():
 @pytest.mark.parametrize("i", [0, 1])
 def test_captured_operators(i):
     """every operator in one graph, replayed over results of its own that are cleared in between"""
-    run = _work(i)
+    run = _every_operator(i)
     want = run()
     torch.cuda.synchronize()
     g = torch.cuda.CUDAGraph()
@@ -299,7 +299,7 @@ def test_captured_operators(i):
 def test_several_threads():
     """Three host threads, each with a stream of its own (the native calls run without the interpreter lock)"""
     from ac4k_kernel_b200 import _lib
-    runs = [_work(i) for i in range(3)]
+    runs = [_every_operator(i) for i in range(3)]
     want = [r() for r in runs]
     torch.cuda.synchronize()
     failed = []
