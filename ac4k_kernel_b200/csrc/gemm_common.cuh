@@ -51,8 +51,10 @@ enum { EPI_PLAIN = 0, EPI_GATHER = 1, EPI_REQUANT = 2 };   // epilogue variants 
 static constexpr int kMaxDst = 8;     // output destinations of one launch (this GPU + up to 7 peers)
 
 // Tensor maps of the output destinations of the pair kernel's TMA-store epilogue: [0] this GPU's buffer,
-// [1 .. n_dst) the further destinations of the fused all-gather.
+// [1 .. n_dst) the further destinations of the fused all-gather.  A launch with one destination, permuted rows and an M that is no
+// multiple of 4 has the second maps of its output and of A (get_tmap_rows4) in two of the places behind it.
 struct DstMaps { CUtensorMap m[kMaxDst]; };
+static constexpr int kDstHiOut = 1, kDstHiA = 2;
 
 struct GemmArgs {
   const uint8_t *sfa;
@@ -78,6 +80,7 @@ struct GemmArgs {
   int KT;               // K / 64
   int rows_sfa, rows_sfb;   // padded row counts of the scale tensors (16- or 128-aligned)
   int tiles_m, tiles_n;
+  int row_classes;      // pair kernel, permuted rows: classes row % 4 of A and the output in the first of their two maps (4: one map)
   int splits;           // split-K factor (1-CTA kernel only); > 1 writes fp32 partials to `ws`
   int kt_per_split;     // K stages (of 256 elements) per split
   float *ws;            // [splits, M, N] fp32 partial sums when splits > 1
@@ -148,8 +151,9 @@ __device__ __forceinline__ void store_row32(void *D, int64_t off, const float (&
 // 2-D byte tensor map [rows, row_bytes] with a (128 B x box_rows) box and 128-byte swizzle
 int get_tmap(const void *ptr, int64_t rows, int64_t row_bytes, int box_rows, CUtensorMap *out);
 // same bytes with the rows as (row / 4, row % 4): a box of 128 B x 32 x 4 brings rows 4 l + q of a 128-row block to
-// shared-memory row q * 32 + l; rows must be a multiple of 4
-int get_tmap_rows4(const void *ptr, int64_t rows, int64_t row_bytes, CUtensorMap *out);
+// shared-memory row q * 32 + l.  rows no multiple of 4: `lo` has the classes row % 4 < rows % 4 (boxes 128 B x 32 x rows % 4), `hi`
+// the others; else `hi` is left alone
+int get_tmap_rows4(const void *ptr, int64_t rows, int64_t row_bytes, CUtensorMap *lo, CUtensorMap *hi);
 // tiled scales [row blocks][K/64][512 B] as a matrix of 512-byte rows, boxes of box_ksteps rows
 int get_tmap_sf_tiled(const void *ptr, int64_t row_blocks, int64_t kt, int box_ksteps, CUtensorMap *out);
 // scales in the row layout [K/64][rows] words: boxes of 128 words (the rows of a 128-row block) x 4 K steps
@@ -161,8 +165,8 @@ unsigned long long *debug_trace_ptr();
 int get_tmap_bf16_4d(const void *ptr, const int64_t shape[4], const int64_t stride[4], int box_rows, CUtensorMap *out);
 // 16-bit output [rows, cols] with a row pitch of ld elements: boxes of 64 columns x 32 rows, 128-byte swizzle
 int get_tmap_out16(const void *ptr, int64_t rows, int64_t cols, int64_t ld, CUtensorMap *out);
-// the same output with the rows as (row / 4, row % 4): boxes of 64 columns x 32 x 1; rows must be a multiple of 4
-int get_tmap_out16_rows4(const void *ptr, int64_t rows, int64_t cols, int64_t ld, CUtensorMap *out);
+// the same output with the rows as (row / 4, row % 4): boxes of 64 columns x 32 x 1, and two maps as above
+int get_tmap_out16_rows4(const void *ptr, int64_t rows, int64_t cols, int64_t ld, CUtensorMap *lo, CUtensorMap *hi);
 // 2-CTA kernel launcher (linear_nvfp4_2cta.cu); D must be bf16/fp16 with N % 8 == 0.  sf_mode 0: scales in the row
 // layout read with plain loads (ta, tb, dm from get_tmap / get_tmap_out16); 1: tiled scales (tsa, tsb from
 // get_tmap_sf_tiled); 2: scales in the row layout by TMA (tsa, tsb from get_tmap_sf_rows; ta, tb from get_tmap_rows4,

@@ -418,11 +418,11 @@ struct TmapKey {
   const void *ptr;
   int64_t d0, d1, pitch;   // extents: innermost (elements), outer; row pitch in elements
   int box0, box1, kind, dev;
-  bool rows4;              // rank 3: the d1 rows as (row / 4, row % 4), box {box0, box1, box2}
+  int classes;             // > 0: rank 3, the rows as (row / 4, row % 4 < classes), box {box0, box1, box2}
   int box2;
   bool operator==(const TmapKey &o) const {
     return ptr == o.ptr && d0 == o.d0 && d1 == o.d1 && pitch == o.pitch && box0 == o.box0 && box1 == o.box1 &&
-           kind == o.kind && dev == o.dev && rows4 == o.rows4 && box2 == o.box2;
+           kind == o.kind && dev == o.dev && classes == o.classes && box2 == o.box2;
   }
 };
 struct TmapEntry { TmapKey key; CUtensorMap map; };
@@ -430,15 +430,15 @@ enum { kTmapOperand = 0, kTmapWords = 1, kTmapOut16 = 2, kTmapOperand64 = 3 };
 
 // kind kTmapOperand / kTmapOperand64: bytes, 128- / 64-byte swizzle; kTmapWords: 32-bit words, not swizzled;
 // kTmapOut16: 16-bit elements, 128-byte swizzle.
-// rows4: a rank-3 map {d0, d1 / 4, 4} with strides {4 * pitch, pitch}: coordinate (x, i, q) is row 4 i + q, and a box
-// {box0, box1, box2} lands in shared memory with q outermost.
+// classes > 0: a rank-3 map {d0, ceil(d1 / 4), classes} with strides {4 * pitch, pitch}: coordinate (x, i, q) is row 4 i + q, and a
+// box {box0, box1, box2} lands in shared memory with q outermost.
 static int encode_cached(int kind, const void *ptr, int64_t d0, int64_t d1, int64_t pitch, int box0, int box1,
-                         CUtensorMap *out, bool rows4 = false, int box2 = 1) {
+                         CUtensorMap *out, int classes = 0, int box2 = 1) {
   static std::mutex mu;
   static std::vector<TmapEntry> cache;
   int dev = 0;
   cudaGetDevice(&dev);
-  TmapKey key{ptr, d0, d1, pitch, box0, box1, kind, dev, rows4, box2};
+  TmapKey key{ptr, d0, d1, pitch, box0, box1, kind, dev, classes, box2};
   {
     std::lock_guard<std::mutex> lk(mu);
     for (auto &e : cache)
@@ -456,14 +456,14 @@ static int encode_cached(int kind, const void *ptr, int64_t d0, int64_t d1, int6
   cuuint64_t gstride[2] = {(cuuint64_t)pitch * esize, 0};
   cuuint32_t box[3] = {(cuuint32_t)box0, (cuuint32_t)box1, (cuuint32_t)box2};
   cuuint32_t estr[3] = {1, 1, 1};
-  if (rows4) {
-    gdim[1] = (cuuint64_t)(d1 / 4);
-    gdim[2] = 4;
+  if (classes > 0) {
+    gdim[1] = (cuuint64_t)ceil_div(d1, 4);
+    gdim[2] = (cuuint64_t)classes;
     gstride[0] = (cuuint64_t)pitch * esize * 4;
     gstride[1] = (cuuint64_t)pitch * esize;
   }
   CUtensorMap m;
-  CUresult r = enc(&m, dt, rows4 ? 3 : 2,
+  CUresult r = enc(&m, dt, classes > 0 ? 3 : 2,
                    const_cast<void *>(ptr), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    swz,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -493,12 +493,22 @@ int get_tmap_out16(const void *ptr, int64_t rows, int64_t cols, int64_t ld, CUte
   return encode_cached(kTmapOut16, ptr, cols, rows, ld, 64, 32, out);
 }
 
-int get_tmap_rows4(const void *ptr, int64_t rows, int64_t row_bytes, CUtensorMap *out) {
-  return encode_cached(kTmapOperand, ptr, row_bytes, rows, row_bytes, BKB, 32, out, true, 4);
+// The maps of the row classes q = row % 4 must not reach past the last row: classes below rows % 4 have one row more than the others,
+// so a row count that is no multiple of 4 takes two maps, `lo` for the classes [0, rows % 4) and `hi` for the rest.
+int get_tmap_rows4(const void *ptr, int64_t rows, int64_t row_bytes, CUtensorMap *lo, CUtensorMap *hi) {
+  const int r = rows % 4 ? (int)(rows % 4) : 4;
+  if (int e = encode_cached(kTmapOperand, ptr, row_bytes, rows, row_bytes, BKB, 32, lo, r, r)) return e;
+  if (r == 4) return 0;
+  // (rows < 4: no row in those classes; the kernel loads the box all the same, here the first row in place of rows that nothing uses)
+  if (rows < 4) return encode_cached(kTmapOperand, ptr, row_bytes, 1, row_bytes, BKB, 32, hi, 1, 4 - r);
+  return encode_cached(kTmapOperand, static_cast<const uint8_t *>(ptr) + r * row_bytes, row_bytes, rows - r, row_bytes, BKB, 32, hi, 4 - r, 4 - r);
 }
 
-int get_tmap_out16_rows4(const void *ptr, int64_t rows, int64_t cols, int64_t ld, CUtensorMap *out) {
-  return encode_cached(kTmapOut16, ptr, cols, rows, ld, 64, 32, out, true, 1);
+int get_tmap_out16_rows4(const void *ptr, int64_t rows, int64_t cols, int64_t ld, CUtensorMap *lo, CUtensorMap *hi) {
+  const int r = rows % 4 ? (int)(rows % 4) : 4;
+  if (int e = encode_cached(kTmapOut16, ptr, cols, rows, ld, 64, 32, lo, r, 1)) return e;
+  if (r == 4 || rows < 4) return 0;
+  return encode_cached(kTmapOut16, static_cast<const uint16_t *>(ptr) + r * ld, cols, rows - r, ld, 64, 32, hi, 4 - r, 1);
 }
 
 // Scale factors in the row layout [K/64][rows][4 bytes] seen as a [K/64, rows] matrix of words: the 128 words of a
@@ -800,19 +810,18 @@ static int linear_impl(void *D, int d_dtype, const void *A, const void *A_sf, co
                 pl.ws_bytes, ws_capacity);
   const bool tiled = sf_layout == AC4K_SF_TILE128X4;
   if (use_pair) {
-    // Scales in the reference's row layout: with M and N multiples of 4 the operands are loaded with their rows
-    // permuted inside each 128-row block, so that the scales can be used as they lie in memory (rank-3 maps; a
-    // row count that is no multiple of 4 would let such a map reach up to 3 rows past the tensor); otherwise
-    // warps of the kernel re-order the scales.  g_dbg bit 0x200 keeps the re-ordering warps (measurement).
-    const bool perm = !tiled && M % 4 == 0 && N % 4 == 0 && !(g_dbg & 0x200);
+    // Scales in the reference's row layout: the operands are loaded with their rows permuted inside each 128-row block, so
+    // that the scales can be used as they lie in memory (rank-3 maps, two of them where M is no multiple of 4; N is, 16-bit rows
+    // being whole 16-byte pieces).  Only the gathered output, with its one map per destination, has warps re-order the scales
+    // for such an M.  g_dbg bit 0x200 does so for all of its launches (measurement).
+    const bool perm = !tiled && !(out && out->n_more > 0 && (M % 4 != 0 || (g_dbg & 0x200)));
     const int sf_mode = tiled ? 1 : (perm ? 2 : 0);
     CUtensorMap tsa = ta, tsb = tb;      // placeholders when the scales are read with plain loads
     if (tiled) {
       if (int e = get_tmap_sf_tiled(A_sf, a.rows_sfa / 128, a.KT, 4, &tsa)) return e;
       if (int e = get_tmap_sf_tiled(B_sf, a.rows_sfb / 128, a.KT, 4, &tsb)) return e;
     } else if (perm) {
-      if (int e = get_tmap_rows4(A, M, K / 2, &ta)) return e;
-      if (int e = get_tmap_rows4(B, N, K / 2, &tb)) return e;
+      if (int e = get_tmap_rows4(B, N, K / 2, &tb, nullptr)) return e;
       if (int e = get_tmap_sf_rows(A_sf, a.rows_sfa, a.KT, &tsa)) return e;
       if (int e = get_tmap_sf_rows(B_sf, a.rows_sfb, a.KT, &tsb)) return e;
     }
@@ -820,11 +829,16 @@ static int linear_impl(void *D, int d_dtype, const void *A, const void *A_sf, co
     // stores are clipped at this launch's last column
     DstMaps dm;
     for (int i = 0; i < kMaxDst; ++i) dm.m[i] = ta;
+    a.row_classes = perm && M % 4 ? (int)(M % 4) : 4;
+    if (perm)
+      if (int e = get_tmap_rows4(A, M, K / 2, &ta, &dm.m[kDstHiA])) return e;
     if (!requant) {
-      auto out_map = perm ? get_tmap_out16_rows4 : get_tmap_out16;
-      if (int e = out_map(D, M, a.col_off + N, a.ldd, &dm.m[0])) return e;
-      for (int i = 1; i < a.n_dst; ++i)
-        if (int e = out_map(a.D_more[i - 1], M, a.col_off + N, a.ldd, &dm.m[i])) return e;
+      for (int i = 0; i < a.n_dst; ++i) {
+        const void *dst = i == 0 ? D : a.D_more[i - 1];
+        if (int e = perm ? get_tmap_out16_rows4(dst, M, a.col_off + N, a.ldd, &dm.m[i], &dm.m[kDstHiOut])
+                         : get_tmap_out16(dst, M, a.col_off + N, a.ldd, &dm.m[i]))
+          return e;
+      }
     }
     return launch_linear_2cta(d_dtype, sf_mode, ta, tb, tsa, tsb, dm, a, stream);
   }

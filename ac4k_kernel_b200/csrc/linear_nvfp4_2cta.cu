@@ -19,19 +19,21 @@
 //   warp 0      TMA producer: A, B and - for tiled scales - three scale boxes per stage, all
 //               completing on the leader CTA's barrier of the stage
 //   warp 1      MMA issuer (leader CTA only): per stage 12 scale copies, 4 MMAs, 1 commit
-//   warps 2-5   only for scales in the row layout [K/64][rows][4] when M or N is not a multiple of 4:
+//   warps 2-5   only for scales in the row layout [K/64][rows][4], a gathered output and an M that is not a multiple of 4:
 //               each warp takes every fourth stage, reads the stage's scale words from global
 //               memory and writes them to shared memory in the 32 x 16-byte order tcgen05.cp wants
 //   warps 6-13  epilogue: tcgen05.ld of 128 accumulator columns per warp into registers
 //               (* alpha, + bias, packed to 16 bit), hand the accumulator back, then store
-// Scales in the row layout, M and N multiples of 4 (SF_MODE == kSfPerm): tcgen05.cp puts word w of a 512-byte
+// Scales in the row layout (SF_MODE == kSfPerm, kSfPermRagged): tcgen05.cp puts word w of a 512-byte
 // chunk on lane w / 4, column w % 4, and the MMA takes the scales of its row q * 32 + l from lane l, column q.
 // So the 512 bytes that hold the scale words of 128 consecutive rows in row order are the chunk of those rows in
 // the order (4 l + q -> q * 32 + l): the operand boxes are loaded with their rows in that order (rank-3 tensor
 // maps: bytes, row / 4, row % 4), the scales arrive by TMA as they lie in memory, and nothing is re-ordered by
 // threads (the generic-proxy stores of the scale warps slow the tensor pipe down by 12 - 30 % per stage).  The
 // accumulator's rows and columns come out in the same order; the epilogue maps its lane to row 4 l + q, pairs
-// the columns back in registers and stores through a rank-3 map of the output.
+// the columns back in registers and stores through a rank-3 map of the output.  An M that is no multiple of 4 takes two maps of A and of
+// the output, and two loads a stage (with re-ordering warps, as before / now, us: 666 x 4096 x 4096 12.7 / 11.8, 1001 x 8192 x 4096
+// 21.1 / 19.2, 4095 x 4096 x 4096 34.9 / 32.3).
 // Barriers that gate the MMA live in the leader CTA and are signalled by both CTAs; barriers that
 // release stages / publish the accumulator exist in both CTAs and are signalled by one
 // tcgen05.commit whose arrival fans out to both.
@@ -179,8 +181,9 @@ __device__ __forceinline__ void drain_permuted(uint32_t (&w)[64], uint32_t t_row
 }
 
 // where the block scales come from: kSfWarps - row layout, re-ordered by warps 2-5; kSfTiled - 128x4 tiles by TMA;
-// kSfPerm - row layout by TMA, operand rows permuted instead
-enum { kSfWarps = 0, kSfTiled = 1, kSfPerm = 2 };
+// kSfPerm - row layout by TMA, operand rows permuted instead; kSfPermRagged - the same for an M that is no multiple of 4, whose
+// rows take two maps (a variant of its own: as a condition in kSfPerm it cost that one 0.5 us of 11 at 668 x 4096 x 4096)
+enum { kSfWarps = 0, kSfTiled = 1, kSfPerm = 2, kSfPermRagged = 3 };
 
 template <int SF_MODE, int OUT_DT, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreadsPair, 1)
@@ -189,7 +192,7 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
                          const __grid_constant__ DstMaps dmaps, const GemmArgs p) {
   using namespace pair;
   constexpr bool SF_TILED = SF_MODE != kSfWarps;      // the scales arrive by TMA, laid out for tcgen05.cp
-  constexpr bool PERM = SF_MODE == kSfPerm;
+  constexpr bool RAGGED = SF_MODE == kSfPermRagged, PERM = SF_MODE == kSfPerm || RAGGED;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t smem_base = smem_u32(smem_raw);
   if (smem_base & 1023u) {      // the swizzled boxes need 1024-byte alignment; never seen, but not promised either
@@ -268,6 +271,7 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
     for (int kt = 0; kt < npre; ++kt) {
       if (PERM) {
         tma_prefetch_3d_if(el, &tma_a, kt * BKB, m0 >> 2, 0);
+        if (RAGGED) tma_prefetch_3d_if(el, &dmaps.m[kDstHiA], kt * BKB, m0 >> 2, 0);
         tma_prefetch_3d_if(el, &tma_b, kt * BKB, nb0 >> 2, 0);
       } else {
         tma_prefetch_2d_if(el, &tma_a, kt * BKB, m0);
@@ -311,6 +315,7 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
           // rows 4 l + q of the 128-row block land on shared-memory row q * 32 + l; the scale words of K step k lie
           // in row order at word k * rows + row: one box of 128 words x 4 K steps per 128-row block
           tma_load_3d_pair_if(el, sA + s * A_BYTES, &tma_a, kt * BKB, m0 >> 2, 0, lf);
+          if (RAGGED) tma_load_3d_pair_if(el, sA + s * A_BYTES + p.row_classes * (32 * BKB), &dmaps.m[kDstHiA], kt * BKB, m0 >> 2, 0, lf);
           tma_load_3d_pair_if(el, sB + s * B_BYTES, &tma_b, kt * BKB, nb0 >> 2, 0, lf);
           tma_load_2d_pair_if(el, sSFA + s * SFA_BYTES, &tma_sfa, m0, kt * KS, lf);
           tma_load_2d_pair_if(el, sSFB + s * SFB_BYTES, &tma_sfb, tn * BN, kt * KS, lf);
@@ -626,7 +631,7 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
 #pragma unroll
         for (int h2 = 0; h2 < 2; ++h2) {
           const int x0 = (int)col_base + 64 * h2;
-          if (col0 + 64 * h2 >= p.N || y0 >= p.M) break;     // warp-uniform: nothing of this box is inside the output
+          if (col0 + 64 * h2 >= p.N || y0 + (RAGGED ? q : 0) >= p.M) break;     // warp-uniform: nothing of this box is inside the output
           if (lane == 0) bulk_wait_group_read0();            // the previous store has read the buffer
           __syncwarp();
 #pragma unroll
@@ -636,7 +641,8 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            if (PERM) tma_store_3d(&dmaps.m[0], x0, y0 >> 2, q, stage_buf);
+            if (RAGGED && q >= p.row_classes) tma_store_3d(&dmaps.m[kDstHiOut], x0, y0 >> 2, q - p.row_classes, stage_buf);
+            else if (PERM) tma_store_3d(&dmaps.m[0], x0, y0 >> 2, q, stage_buf);
             else tma_store_2d(&dmaps.m[0], x0, y0, stage_buf);
             if (EPI == EPI_GATHER) {
               // peers in turn, starting behind this rank, so that the ranks do not all write to the same GPU at once
@@ -722,8 +728,12 @@ template <int OUT_DT, int EPI>
 static int launch_pair_mode(int sf_mode, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tsa, const CUtensorMap &tsb,
                             const DstMaps &dm, const GemmArgs &args, int sms, cudaStream_t stream) {
   if (sf_mode == kSfTiled) return launch_pair<kSfTiled, OUT_DT, EPI>(ta, tb, tsa, tsb, dm, args, sms, stream);
-  if (sf_mode == kSfPerm) return launch_pair<kSfPerm, OUT_DT, EPI>(ta, tb, tsa, tsb, dm, args, sms, stream);
-  return launch_pair<kSfWarps, OUT_DT, EPI>(ta, tb, tsa, tsb, dm, args, sms, stream);
+  if constexpr (EPI == EPI_GATHER) {
+    if (sf_mode == kSfWarps) return launch_pair<kSfWarps, OUT_DT, EPI>(ta, tb, tsa, tsb, dm, args, sms, stream);
+  } else {
+    if (args.row_classes < 4) return launch_pair<kSfPermRagged, OUT_DT, EPI>(ta, tb, tsa, tsb, dm, args, sms, stream);
+  }
+  return launch_pair<kSfPerm, OUT_DT, EPI>(ta, tb, tsa, tsb, dm, args, sms, stream);
 }
 
 // sf_mode: 0 - scales in the row layout, re-ordered by warps (operand and output maps of rank 2); 1 - scales in 128x4

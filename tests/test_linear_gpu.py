@@ -145,6 +145,24 @@ def test_row_layout_scale_paths(ops, m, n, k, bdt):
     run_case(ops, m, n, k, seed=31, layout="ac4k", bias_dtype=bdt, out_dtype=torch.bfloat16)
 
 
+@pytest.mark.parametrize("m", [129, 130, 131, 255, 257, 258, 387])
+@pytest.mark.parametrize("n,k,odt,bdt", [(136, 64, torch.bfloat16, None), (264, 1088, torch.float16, torch.bfloat16)])
+def test_row_layout_ragged_rows(ops, m, n, k, odt, bdt):
+    """M of every remainder by 4: two maps of A and of the output"""
+    run_case(ops, m, n, k, seed=m, layout="ac4k", bias_dtype=bdt, out_dtype=odt)
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 6, 127, 129, 130, 259])
+def test_requantised_ragged_rows(ops, m):
+    """the same in front of the re-quantising epilogue, which this kernel also has for the fewest rows: bit for bit what linear and
+    quantize of its bf16 output give"""
+    a, b = gaussian((m, 512), seed=m).cuda(), gaussian((192, 512), seed=5).cuda()
+    qa, qb = ops.quantize(a, 0, 1), ops.quantize(b, 0, 1)
+    want = ops.quantize(ops.linear(*qa, *qb), 0, 1)
+    got = ops.linear_requant(*qa, *qb, want[2], sf_layout="ac4k")
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1].view(torch.uint8), want[1].view(torch.uint8))
+
+
 def test_random_shapes(ops):
     """test/test_linear_bench.py:156-161: 20 random M, N, K in [2, 555]."""
     rng = random.Random(9567)
