@@ -26,7 +26,7 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libac4k_b200.so")
 
-SOURCES = ["cabi.cu", "quantize_nvfp4.cu", "quantize_rowwise.cu", "linear_nvfp4.cu",
+SOURCES = ["cabi.cu", "quantize_nvfp4.cu", "quantize_nvfp4_resident.cu", "quantize_rowwise.cu", "linear_nvfp4.cu",
            "linear_nvfp4_2cta.cu", "linear_nvfp4_skinny.cu", "mha_nvfp4.cu", "rope3d.cu", "mha_int8_fp8.cu", "quantize_int8_block.cu"]
 
 NVCC_FLAGS = [

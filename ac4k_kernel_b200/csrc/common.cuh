@@ -84,6 +84,12 @@ int launch_kernel(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, c
   return 0;
 }
 
+// The one-launch NVFP4 quantiser (quantize_nvfp4_resident.cu); arguments as ac4k_quantize_nvfp4_dynamic, which see.  Returns
+// kResidentDeclined, with nothing launched, for a tensor that it does not take.
+static constexpr int kResidentDeclined = -1000;
+int launch_quantize_resident(void *out, void *sf, float *g_out, void *scratch, const void *in, float max_scale, const int64_t shape[4],
+                             const int64_t stride[4], int swizzle, int sf_layout, cudaStream_t stream);
+
 // ---- small integer helpers --------------------------------------------------------------
 __host__ __device__ constexpr int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 __host__ __device__ constexpr int64_t align_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }
@@ -187,10 +193,12 @@ __device__ __forceinline__ BlockScale block_scale(float amax, float alpha) {
   return o;
 }
 
-__device__ __forceinline__ float load_alpha(const float *gscale) {
-  float g = __ldg(gscale);
-  return g == 0.0f ? 0.0f : __frcp_rn(g);
+// max|x| (bf16 bits) -> global scale; 0 for a tensor of zeros
+__device__ __forceinline__ float global_scale_of(uint32_t amax_bits, float max_scale) {
+  return amax_bits ? __fdiv_rn(bf16_bits_to_f32(amax_bits), max_scale) : 0.0f;
 }
+__device__ __forceinline__ float alpha_of(float g) { return g == 0.0f ? 0.0f : __frcp_rn(g); }
+__device__ __forceinline__ float load_alpha(const float *gscale) { return alpha_of(__ldg(gscale)); }
 
 // four packed bf16 pairs -> 8 e2m1 codes (one word); products in fp32, round to nearest
 __device__ __forceinline__ uint32_t quantize8_x2(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, float r) {

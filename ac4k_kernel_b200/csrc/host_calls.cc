@@ -300,10 +300,24 @@ py::object attention(py::handle hq, py::handle hk, py::handle hv, py::handle hla
   int64_t os[4];
   const bool done = unlocked([&] {
     if (nvfp4) {
-      const Nvfp4 qq = quantize_nvfp4_of(q, n_dim, 3, 2688.0f, false, true), kk = quantize_nvfp4_of(k, n_dim, 3, 2688.0f, false, true);
-      const Nvfp4 vv = quantize_nvfp4_of(v, 3, n_dim, 2688.0f, true, true);
+      const int64_t Dp = align_up(D, 64), Kp = align_up(Nkv, 64);
+      auto operand = [&](int64_t m, int64_t kp) {
+        return Nvfp4{empty({B, H, m, kp / 2}, at::kByte, q), empty({B, H, ceil_div(m, 128), kp / 64, 32, 4, 4}, at::kFloat8_e4m3fn, q), scalar_like(q)};
+      };
+      const Nvfp4 qq = operand(Nq, Dp), kk = operand(Nkv, Dp), vv = operand(Dv, Kp);
+      const at::Tensor scratch = empty({AC4K_QUANTIZE_SCRATCH_BYTES / 4}, at::kInt, q);
       out_strides(os);
-      auto gs = [](const Nvfp4 &t) { return static_cast<const float *>(t.scale.data_ptr()); };
+      void *const codes[3] = {qq.q.data_ptr(), kk.q.data_ptr(), vv.q.data_ptr()}, *const sfs[3] = {qq.sf.data_ptr(), kk.sf.data_ptr(), vv.sf.data_ptr()};
+      auto gs = [](const Nvfp4 &t) { return static_cast<float *>(t.scale.data_ptr()); };
+      float *const scales[3] = {gs(qq), gs(kk), gs(vv)};
+      const void *const ins[3] = {q.data_ptr(), k.data_ptr(), v.data_ptr()};
+      int64_t strides[3][4];
+      for (int i = 0; i < 3; ++i) {
+        const at::Tensor &t = i == 0 ? q : (i == 1 ? k : v);
+        strides[i][0] = t.stride(0); strides[i][1] = t.stride(h_dim); strides[i][2] = t.stride(n_dim); strides[i][3] = t.stride(3);
+      }
+      check(ac4k_attention_quantize_nvfp4(codes, sfs, scales, scratch.data_ptr(), ins, strides, B, H, Nq, Nkv, D, Dv, stream_of(q)),
+            "attention_quantize_nvfp4");
       check(ac4k_mha_nvfp4_fwd(out.data_ptr(), os, qq.q.data_ptr(), qq.sf.data_ptr(), gs(qq), kk.q.data_ptr(), kk.sf.data_ptr(), gs(kk),
                                vv.q.data_ptr(), vv.sf.data_ptr(), gs(vv), B, H, Nq, Nkv, qq.q.size(3) * 2, Dv, sm_scale, AC4K_SF_TILE128X4,
                                stream_of(q)),

@@ -40,12 +40,6 @@ struct ScaleSource {
   bool last_first;      // tiled kernel: take the row tiles from the last to the first
 };
 
-// max|x| (bf16 bits) -> global scale; 0 for a tensor of zeros
-__device__ __forceinline__ float global_scale_of(uint32_t amax_bits, float max_scale) {
-  return amax_bits ? __fdiv_rn(bf16_bits_to_f32(amax_bits), max_scale) : 0.0f;
-}
-__device__ __forceinline__ float alpha_of(float g) { return g == 0.0f ? 0.0f : __frcp_rn(g); }
-
 // maximum of one value per thread over the CTA, in every thread (s_m: one word per warp; ends with all threads past a barrier)
 __device__ __forceinline__ uint32_t cta_max(uint32_t m, uint32_t *s_m) {
   m = __reduce_max_sync(0xFFFFFFFFu, m);
@@ -730,6 +724,10 @@ extern "C" int ac4k_quantize_nvfp4_dynamic(void *out, void *sf, float *g_out, vo
   if (int e = get_device_info(&di)) return e;
   // Routes by size (measured on a B200; microseconds of the whole call on resident inputs stand beside the kernels):
   //   whole tensor in the registers of one cluster            one launch
+  //   columns contiguous (attention's V), or four to seven     the one-launch kernel of quantize_nvfp4_resident.cu.  One launch / two, us:
+  //   of its tiles an SM                                       V of [1, 16384, 16, 128] 30 / 50, [1, 1000, 16, 128] 7.1 / 13.2, [2, 104, 8,
+  //                                                            128] 5.0 / 7.1; rows of 1000 x 5120 8.4 / 9.9, 2048 x 4096 9.7 / 11.3, but
+  //                                                            666 x 4096 7.3 / 5.3 (its grid barrier) and 3000 x 4096 18 / 13
   //   up to 2^24 elements                                      maxima per CTA, then a quantiser that reduces them: two launches,
   //                                                            the second one set up under the first
   //   larger                                                   zeroed accumulator + atomic maximum + quantiser: a few hundred
@@ -740,6 +738,11 @@ extern "C" int ac4k_quantize_nvfp4_dynamic(void *out, void *sf, float *g_out, vo
   if (vec && items <= AC4K_QUANTIZE_ONE_LAUNCH_BLOCKS)
     return sf_layout == AC4K_SF_AC4K ? launch_flat<AC4K_SF_AC4K>(out, sf, in, src, shape, stride, items, true, stream)
                                      : launch_flat<AC4K_SF_TILE128X4>(out, sf, in, src, shape, stride, items, true, stream);
+  const int64_t resident_tiles = nbatch * ceil_div(M, 128) * (Kp / 64);
+  if (scratch && (swizzle || stride[3] != 1 || (resident_tiles >= 4 * (int64_t)di.sms && resident_tiles <= 7 * (int64_t)di.sms))) {
+    const int e = launch_quantize_resident(out, sf, g_out, scratch, in, max_scale, shape, stride, swizzle, sf_layout, stream);
+    if (e != kResidentDeclined) return e;
+  }
   if (!scratch || numel > (1 << 24)) {
     if (int e = ac4k_global_scale_bf16(in, numel, max_scale, g_out, stream_)) return e;
     src.g = g_out;

@@ -92,6 +92,13 @@ int ac4k_quantize_nvfp4_dynamic(void *out, void *sf, float *g_out, void *scratch
                                 const int64_t shape[4], const int64_t stride[4], int swizzle, int sf_layout,
                                 ac4k_stream_t stream);
 
+/* The three NVFP4 quantisers in front of ac4k_mha_nvfp4_fwd (128x4 scales, v permuted along the keys), in one launch where their
+ * strides allow it: out, sf, g_out, in and stride of q [B, H, Nq, D], k [B, H, Nkv, D] and v [B, H, Nkv, Dv], strides in elements and in
+ * that order.  Same bytes as three calls of ac4k_quantize_nvfp4_dynamic; scratch as there, for the three. */
+int ac4k_attention_quantize_nvfp4(void *const out[3], void *const sf[3], float *const g_out[3], void *scratch, const void *const in[3],
+                                  const int64_t stride[3][4], int64_t B, int64_t H, int64_t Nq, int64_t Nkv, int64_t D, int64_t Dv,
+                                  ac4k_stream_t stream);
+
 /* Per-row (whole reduce dim) e4m3 quantiser.  Replaces ac4k::quantize_fp8,
  * include/ac4k_kernel/ops.h:31-33, lib/cuda/sm120/quantize_fp8.cu:192-290.
  *   out: [outer0, outer1, M, align16(K)] e4m3;  sf: [outer0, outer1, align16(M)] fp32. */

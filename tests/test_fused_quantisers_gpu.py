@@ -1,0 +1,115 @@
+"""The quantisers that do more than one thing in a launch, against the calls that they stand for: the one-launch NVFP4 quantiser and
+the three operands of an attention layer (bit for bit), at the sizes where tiles, slots and shares of the grid change; K less its mean
+in one launch."""
+import ctypes
+
+import pytest
+import torch
+
+from tests.helpers import gaussian
+
+pytestmark = pytest.mark.gpu
+
+
+def _u8(t):
+    return t.view(torch.uint8)
+
+
+def _reference(x, cross, reduce, swizzle, layout):
+    """global scale and quantiser as two calls of the direct interface"""
+    from ac4k_kernel_b200.ops.quant import Ac4kQuantizeOp
+    return Ac4kQuantizeOp()(x, cross, reduce, swizzle=swizzle, sf_layout=layout)
+
+
+def _same(got, want):
+    return torch.equal(got[0], want[0]) and torch.equal(_u8(got[1]), _u8(want[1])) and torch.equal(got[2].view(torch.int32), want[2].view(torch.int32))
+
+
+@pytest.mark.parametrize("layout", ["ac4k", "128x4"])
+@pytest.mark.parametrize("m,k", [
+    (148, 8192), (257, 8192), (2048, 4160), (4096, 4096), (4097, 4112),      # up to a tile per CTA; a ragged tile; what fits on chip and just more
+    (1000, 16384), (12345, 2064), (33000, 1024), (40000, 128), (8192, 8192),   # each slot used again once, and many times
+])
+def test_one_launch_rows(m, k, layout):
+    from ac4k_kernel_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    x = torch.randn((m, k), generator=g, device="cuda", dtype=torch.bfloat16)
+    x[m // 2, k // 3] = -77.0                                      # the maximum, once
+    assert _same(ops.quantize(x, 0, 1, sf_layout=layout), _reference(x, 0, 1, False, layout))
+
+
+@pytest.mark.parametrize("layout", ["ac4k", "128x4"])
+@pytest.mark.parametrize("swizzle", [False, True])
+@pytest.mark.parametrize("shape", [(1, 700, 3, 128), (2, 1031, 5, 64), (1, 5000, 16, 72), (1, 9000, 16, 128), (3, 130, 1, 8)])
+def test_one_launch_columns(shape, swizzle, layout):
+    from ac4k_kernel_b200 import ops
+    x = (gaussian(shape, seed=shape[1]) * 2).bfloat16().cuda()
+    x[0, shape[1] - 1, 0, 1] = 50.0
+    assert _same(ops.quantize(x, 3, 1, swizzle=swizzle, sf_layout=layout), _reference(x, 3, 1, swizzle, layout))
+
+
+@pytest.mark.parametrize("fill", [0.0, float("nan"), float("inf"), 1e-38])
+def test_one_launch_odd_values(fill):
+    from ac4k_kernel_b200 import ops
+    x = torch.full((4100, 2048), fill, device="cuda", dtype=torch.bfloat16)
+    assert _same(ops.quantize(x, 0, 1), _reference(x, 0, 1, False, "ac4k"))
+    x[1000:, 512:] = gaussian((3100, 1536), seed=2).bfloat16().cuda()
+    assert _same(ops.quantize(x, 0, 1), _reference(x, 0, 1, False, "ac4k"))
+
+
+def test_one_launch_replayed_and_on_two_streams():
+    from ac4k_kernel_b200 import ops
+    xs = [torch.randn((3000, 4096), device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    want = [_reference(x, 0, 1, False, "ac4k") for x in xs]
+    streams = [torch.cuda.Stream() for _ in xs]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(20):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(ops.quantize(xs[i], 0, 1))
+    torch.cuda.synchronize()
+    assert all(_same(t, want[i]) for i in range(2) for t in got[i])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = ops.quantize(xs[0], 0, 1)
+    for scale in (1.0, -3.0, 0.5):
+        xs[0].copy_(xs[1] * scale)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert _same(out, _reference(xs[0], 0, 1, False, "ac4k"))
+
+
+def _attention_operands(q, k, v, h_dim, n_dim):
+    from ac4k_kernel_b200._lib import LIB
+    b, h, d, dv = q.shape[0], q.shape[h_dim], q.shape[3], v.shape[3]
+    nq, nkv = q.shape[n_dim], k.shape[n_dim]
+    dev = {"device": "cuda"}
+    made, kp = [], (nkv + 63) // 64 * 64
+    for m, c in ((nq, (d + 63) // 64 * 64), (nkv, (d + 63) // 64 * 64), (dv, kp)):
+        made.append((torch.empty((b, h, m, c // 2), dtype=torch.uint8, **dev),
+                     torch.empty((b, h, (m + 127) // 128, c // 64, 32, 4, 4), dtype=torch.float8_e4m3fn, **dev),
+                     torch.empty((), dtype=torch.float32, **dev)))
+    scratch = torch.empty(1024, dtype=torch.int32, **dev)
+    pointers = lambda ts: (ctypes.c_void_p * 3)(*[t.data_ptr() for t in ts])
+    strides = (ctypes.c_int64 * 12)(*[t.stride(i) for t in (q, k, v) for i in (0, h_dim, n_dim, 3)])
+    rc = LIB.ac4k_attention_quantize_nvfp4(pointers([m[0] for m in made]), pointers([m[1] for m in made]), pointers([m[2] for m in made]),
+                                           scratch.data_ptr(), pointers([q, k, v]), strides, b, h, nq, nkv, d, dv,
+                                           torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    return made
+
+
+@pytest.mark.parametrize("layout", ["BNHD", "BHND"])
+@pytest.mark.parametrize("b,h,nq,nkv,d,dv", [
+    (1, 1, 1, 1, 64, 64), (2, 8, 104, 104, 128, 128), (1, 3, 1000, 77, 96, 128), (1, 16, 3000, 4000, 128, 128),
+    (1, 1, 130, 129, 80, 72), (3, 5, 65, 257, 40, 128),
+    (2, 3, 100, 100, 100, 65),                                      # no tensor map for these strides: a call each
+])
+def test_attention_operands(layout, b, h, nq, nkv, d, dv):
+    n_dim, h_dim = (1, 2) if layout == "BNHD" else (2, 1)
+    shape = lambda n, c: (b, n, h, c) if layout == "BNHD" else (b, h, n, c)
+    q, k, v = ((gaussian(shape(n, c), seed=n + c + i) * (1 + i)).bfloat16().cuda() for i, (n, c) in enumerate(((nq, d), (nkv, d), (nkv, dv))))
+    got = _attention_operands(q, k, v, h_dim, n_dim)
+    for t, (x, cross, reduce, swizzle) in zip(got, ((q, n_dim, 3, False), (k, n_dim, 3, False), (v, 3, n_dim, True))):
+        assert _same(t, _reference(x, cross, reduce, swizzle, "128x4"))
