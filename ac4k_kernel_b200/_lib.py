@@ -48,6 +48,7 @@ SIGNATURES = {
                                           ctypes.c_int64, ctypes.c_int64, ctypes.c_float, ctypes.c_int, _vp]),
     "ac4k_attention_quantize_nvfp4": (ctypes.c_int, [_vp] * 6 + [ctypes.c_int64] * 6 + [_vp]),
     "ac4k_quantize_int8_block": (ctypes.c_int, [_vp, _vp, _vp, _c_i64p, _c_i64p, ctypes.c_int64, _vp, _c_i64p, _vp]),
+    "ac4k_attention_quantize_int8": (ctypes.c_int, [_vp] * 7 + [_c_i64p, _vp, _c_i64p, _vp, _c_i64p, _vp, _c_i64p] + [ctypes.c_int64] * 6 + [_vp]),
     "ac4k_mha_int8_x_fp8_fwd": (ctypes.c_int, [_vp, _c_i64p, _vp, _vp, ctypes.c_int64, _vp, _vp, ctypes.c_int64, _vp, _vp,
                                                ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64,
                                                ctypes.c_int64, ctypes.c_int64, ctypes.c_float, _vp]),

@@ -90,6 +90,10 @@ static constexpr int kResidentDeclined = -1000;
 int launch_quantize_resident(void *out, void *sf, float *g_out, void *scratch, const void *in, float max_scale, const int64_t shape[4],
                              const int64_t stride[4], int swizzle, int sf_layout, cudaStream_t stream);
 
+// V of the attention operator to e4m3 along its keys (ac4k_quantize_fp8_max, permuted), beside the quantiser in front of it where one
+// kernel does it (quantize_rowwise.cu)
+int launch_fp8_beside(void *out, float *sf, const void *in, float scale_max, const int64_t shape[4], const int64_t stride[4], cudaStream_t stream);
+
 // ---- small integer helpers --------------------------------------------------------------
 __host__ __device__ constexpr int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 __host__ __device__ constexpr int64_t align_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }

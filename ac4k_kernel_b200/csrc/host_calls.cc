@@ -14,6 +14,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <array>
 #include <cmath>
 #include <optional>
 #include <string>
@@ -323,26 +324,26 @@ py::object attention(py::handle hq, py::handle hk, py::handle hv, py::handle hla
                                stream_of(q)),
             "mha_nvfp4_fwd");
     } else {
-      // k - mean(k): the subtraction happens inside the K quantiser
-      const at::Tensor mean = k.detach().mean(at::IntArrayRef{n_dim}, true);
-      if (mean.stride(3) != 1) return false;
+      // k - mean(k): the subtraction happens inside the K quantiser, the mean too where it takes that many keys
+      at::Tensor mean;
+      int64_t ms[2] = {0, 0};
+      if (Nkv > AC4K_ATTENTION_MEAN_TOKENS) {
+        mean = k.detach().mean(at::IntArrayRef{n_dim}, true);
+        if (mean.stride(3) != 1) return false;
+        ms[0] = mean.stride(0); ms[1] = mean.stride(h_dim);
+      }
       const int64_t Dp = align_up(D, 16);
-      auto int8_of = [&](const at::Tensor &t, int64_t n, int64_t block, const at::Tensor *sub, at::Tensor *sf) {
-        *sf = empty({B, H, ceil_div(n, block)}, at::kFloat, q);
-        at::Tensor y = empty({B, H, n, Dp}, at::kChar, q);
-        const int64_t shape[4] = {B, H, n, D}, stride[4] = {t.stride(0), t.stride(h_dim), t.stride(n_dim), t.stride(3)};
-        const int64_t ss[2] = {sub ? sub->stride(0) : 0, sub ? sub->stride(h_dim) : 0};
-        check(ac4k_quantize_int8_block(y.data_ptr(), static_cast<float *>(sf->data_ptr()), t.data_ptr(), shape, stride, block,
-                                       sub ? sub->data_ptr() : nullptr, sub ? ss : nullptr, stream_of(q)),
-              "quantize_int8_block");
-        return y;
-      };
-      at::Tensor q_sf, k_sf;
-      const at::Tensor q8 = int8_of(q, Nq, 64, nullptr, &q_sf), k8 = int8_of(k, Nkv, 128, &mean, &k_sf);
-      const Rowwise v8 = quantize_rows_of(v, 3, n_dim, true, 2.25, true);
-      out_strides(os);
-      auto f = [](const at::Tensor &t) { return static_cast<const float *>(t.data_ptr()); };
-      check(ac4k_mha_int8_x_fp8_fwd(out.data_ptr(), os, q8.data_ptr(), f(q_sf), 64, k8.data_ptr(), f(k_sf), 128, v8.q.data_ptr(), f(v8.sf), B, H,
+      const at::Tensor q8 = empty({B, H, Nq, Dp}, at::kChar, q), k8 = empty({B, H, Nkv, Dp}, at::kChar, q);
+      const at::Tensor q_sf = empty({B, H, ceil_div(Nq, 64)}, at::kFloat, q), k_sf = empty({B, H, ceil_div(Nkv, 128)}, at::kFloat, q);
+      const at::Tensor v8 = empty({B, H, Dv, align_up(Nkv, 16)}, at::kFloat8_e4m3fn, q), v_sf = empty({B, H, align_up(Dv, 16)}, at::kFloat, q);
+      auto f = [](const at::Tensor &t) { return static_cast<float *>(t.data_ptr()); };
+      auto order = [&](const at::Tensor &t) { return std::array<int64_t, 4>{t.stride(0), t.stride(h_dim), t.stride(n_dim), t.stride(3)}; };
+      out_strides(os);          // (everything is allocated in front of the first launch: the quantisers run side by side)
+      check(ac4k_attention_quantize_int8(q8.data_ptr(), f(q_sf), k8.data_ptr(), f(k_sf), v8.data_ptr(), f(v_sf), q.data_ptr(), order(q).data(),
+                                         k.data_ptr(), order(k).data(), v.data_ptr(), order(v).data(), mean.defined() ? mean.data_ptr() : nullptr,
+                                         ms, B, H, Nq, Nkv, D, Dv, stream_of(q)),
+            "attention_quantize_int8");
+      check(ac4k_mha_int8_x_fp8_fwd(out.data_ptr(), os, q8.data_ptr(), f(q_sf), 64, k8.data_ptr(), f(k_sf), 128, v8.data_ptr(), f(v_sf), B, H,
                                     Nq, Nkv, Dp, Dv, sm_scale, stream_of(q)),
             "mha_int8_x_fp8_fwd");
     }

@@ -304,7 +304,7 @@ static bool column_short(int64_t nbatch, int64_t K, int64_t M, bool transposing,
 template <int FMT, bool PERMUTE>
 __global__ void __launch_bounds__(kShortThreads)
 column_quantize_short_kernel(uint8_t *__restrict__ out, float *__restrict__ sf, const uint16_t *__restrict__ in, const ScaleMax scale_max,
-                             int64_t M, int K, int64_t M16, int64_t d1, int64_t stride0, int64_t stride1, int64_t stride_k) {
+                             int64_t M, int K, int64_t M16, int64_t d1, int64_t stride0, int64_t stride1, int64_t stride_k, bool beside) {
   __shared__ uint32_t red[kShortGroups][kShortCols];
   __shared__ uint32_t tile[kShortCols][kShortCols / 4 + 1];       // [column][4 reduce-rows per word], padded
   const int64_t batch = blockIdx.y;
@@ -314,7 +314,7 @@ column_quantize_short_kernel(uint8_t *__restrict__ out, float *__restrict__ sf, 
   const bool live = col < M;
   const int Kp = (K + 15) / 16 * 16;
   uint32_t m = 0;
-  grid_dependency_wait();
+  if (!beside) grid_dependency_wait();
   grid_launch_dependents();
   if (live) {
 #pragma unroll 8
@@ -354,12 +354,13 @@ column_quantize_short_kernel(uint8_t *__restrict__ out, float *__restrict__ sf, 
       }
     }
   }
+  if (beside) grid_dependency_wait();      // (beside: see quantize_int8_block.cu)
 }
 
 template <int FMT>
 static int launch_rowwise(void *out, float *sf, const void *in, const ScaleMax &scale_max,
                           const int64_t shape[4], const int64_t stride[4], int swizzle,
-                          cudaStream_t stream) {
+                          cudaStream_t stream, bool beside = false) {
   if (!shape || !stride) return fail(AC4K_ERR_NULL, "shape/stride is NULL");
   for (int i = 0; i < 4; ++i)
     if (shape[i] < 0) return fail(AC4K_ERR_SHAPE, "shape[%d] is negative", i);
@@ -400,7 +401,7 @@ static int launch_rowwise(void *out, float *sf, const void *in, const ScaleMax &
     if (column_short(nbatch, K, M, tr_ok, di.sms)) {
       dim3 g((unsigned)ceil_div(M16, kShortCols), (unsigned)nbatch);
       return launch_kernel<true>(swizzle ? column_quantize_short_kernel<FMT, true> : column_quantize_short_kernel<FMT, false>, g, kShortThreads, 0,
-                                 stream, outp, sf, inp, scale_max, M, (int)K, M16, d1, stride[0], stride[1], stride[3]);
+                                 stream, outp, sf, inp, scale_max, M, (int)K, M16, d1, stride[0], stride[1], stride[3], beside);
     }
   }
   if (tr_ok) {
@@ -430,6 +431,10 @@ static int launch_rowwise(void *out, float *sf, const void *in, const ScaleMax &
         outp, sf, inp, scale_max, M, K, d1, stride[0], stride[1], stride[2], stride[3]);
   AC4K_LAUNCH_CHECK("rowwise_quantize_strided_kernel");
   return 0;
+}
+
+int launch_fp8_beside(void *out, float *sf, const void *in, float scale_max, const int64_t shape[4], const int64_t stride[4], cudaStream_t stream) {
+  return launch_rowwise<kFmtE4M3>(out, sf, in, ScaleMax{nullptr, 0, scale_max}, shape, stride, 1, stream, true);
 }
 
 }  // namespace ac4k

@@ -213,6 +213,19 @@ int ac4k_mha_nvfp4_fwd(void *O, const int64_t o_stride[4], const void *Q, const 
 int ac4k_quantize_int8_block(void *out, float *scale, const void *in, const int64_t shape[4], const int64_t stride[4],
                              int64_t block, const void *sub, const int64_t sub_stride[2], ac4k_stream_t stream);
 
+/* The three quantisers in front of ac4k_mha_int8_x_fp8_fwd as the attention operator calls it, side by side on the stream:
+ *   q  [B, H, Nq, D]    -> q8, q_sf    blocks of 64 tokens           (ac4k_quantize_int8_block)
+ *   k  [B, H, Nkv, D]   -> k8, k_sf    blocks of 128 tokens, less the mean over the tokens
+ *   v  [B, H, Nkv, Dv]  -> v8, v_sf    per channel along the keys    (ac4k_quantize_fp8_max, permuted, maximum 2.25)
+ * Strides in elements, ordered [B, H, N, D].  D at most 128.  k_mean: bf16 [B, H, D] by mean_stride[0], mean_stride[1] and 1, or NULL
+ * for up to AC4K_ATTENTION_MEAN_TOKENS keys: computed here.  The six outputs must have been allocated before the call, in memory
+ * that nothing enqueued on the stream after their allocation uses. */
+#define AC4K_ATTENTION_MEAN_TOKENS 1024
+int ac4k_attention_quantize_int8(void *q8, float *q_sf, void *k8, float *k_sf, void *v8, float *v_sf, const void *q,
+                                 const int64_t q_stride[4], const void *k, const int64_t k_stride[4], const void *v,
+                                 const int64_t v_stride[4], const void *k_mean, const int64_t mean_stride[2], int64_t B, int64_t H,
+                                 int64_t Nq, int64_t Nkv, int64_t D, int64_t Dv, ac4k_stream_t stream);
+
 /* O = softmax(sm_scale * Q K^T) V with Q, K in INT8 (scales per block of tokens), P and V in FP8 e4m3 (V with one scale
  * per channel), bf16 output.  Replaces ac4k::mha_int8_x_fp8_fwd, include/ac4k_kernel/ops.h:19-25,
  * lib/cuda_bindings.cc:57-58, lib/cuda/sm120/mha_int8_x_fp8.cu:979-1137 (checks) and :403-975 (kernel).

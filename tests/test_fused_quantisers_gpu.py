@@ -113,3 +113,44 @@ def test_attention_operands(layout, b, h, nq, nkv, d, dv):
     got = _attention_operands(q, k, v, h_dim, n_dim)
     for t, (x, cross, reduce, swizzle) in zip(got, ((q, n_dim, 3, False), (k, n_dim, 3, False), (v, 3, n_dim, True))):
         assert _same(t, _reference(x, cross, reduce, swizzle, "128x4"))
+
+
+@pytest.mark.parametrize("layout", ["BNHD", "BHND"])
+@pytest.mark.parametrize("b,h,n,d", [(1, 1, 1, 1), (2, 3, 100, 65), (1, 2, 127, 128), (3, 2, 128, 128), (1, 2, 129, 66), (1, 4, 640, 100),
+                                     (2, 1, 1000, 96), (1, 3, 1024, 128)])
+def test_keys_less_their_mean(layout, b, h, n, d):
+    """against the quantiser with a given mean.  With means that are exact, bit for bit.  Else the two means are fp32 sums in different
+    orders, so that a mean (of 2 to 4) may differ by an ulp of bf16, 2^-6, and a difference (below 16) that it is taken off by one of
+    2^-4 more: `moved`, the bound of what an element of either changes by, and a block's maximum with it"""
+    from ac4k_kernel_b200._lib import LIB
+    n_dim, h_dim = (1, 2) if layout == "BNHD" else (2, 1)
+    shape = (b, n, h, d) if layout == "BNHD" else (b, h, n, d)
+    for exact in (True, False):
+        k = gaussian(shape, seed=n + d).cuda()
+        k = ((k * 8).round() if exact else k * 2 + 3).bfloat16()      # (sums of whole numbers are exact in any order)
+        q, v = k.clone(), k.clone()
+        mean = k.double().mean(dim=n_dim, keepdim=True).float().bfloat16() if exact else k.mean(dim=n_dim, keepdim=True)
+        made = []
+        for given in (mean, None):
+            outs = []
+            for m, block in ((n, 64), (n, 128)):
+                outs += [torch.empty((b, h, m, (d + 15) // 16 * 16), dtype=torch.int8, device="cuda"),
+                         torch.empty((b, h, (m + block - 1) // block), device="cuda")]
+            outs += [torch.empty((b, h, d, (n + 15) // 16 * 16), dtype=torch.uint8, device="cuda"), torch.zeros((b, h, (d + 15) // 16 * 16), device="cuda")]
+            st = lambda t: (ctypes.c_int64 * 4)(*[t.stride(i) for i in (0, h_dim, n_dim, 3)])
+            ms = (ctypes.c_int64 * 2)(mean.stride(0), mean.stride(h_dim))
+            rc = LIB.ac4k_attention_quantize_int8(*[t.data_ptr() for t in outs], q.data_ptr(), st(q), k.data_ptr(), st(k), v.data_ptr(), st(v),
+                                                  given.data_ptr() if given is not None else None, ms, b, h, n, n, d, d,
+                                                  torch.cuda.current_stream().cuda_stream)
+            assert rc == 0
+            made.append(outs)
+        torch.cuda.synchronize()
+        for i in (0, 1, 4, 5):                                       # q and v: the same calls
+            assert torch.equal(made[0][i], made[1][i])
+        if exact:
+            assert torch.equal(made[0][2], made[1][2]) and torch.equal(made[0][3], made[1][3])
+        else:
+            moved = 2.0 ** -6 + 2.0 ** -4
+            assert ((made[0][3] - made[1][3]).abs() <= moved / 127).all()
+            rows = made[0][3].repeat_interleave(128, dim=2)[:, :, :n, None]
+            assert ((made[0][2].int() - made[1][2].int()).abs() <= 1 + 2 * moved / rows.clamp(min=1e-30)).all()
