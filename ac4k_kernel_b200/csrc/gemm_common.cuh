@@ -80,6 +80,7 @@ struct GemmArgs {
   int KT;               // K / 64
   int rows_sfa, rows_sfb;   // padded row counts of the scale tensors (16- or 128-aligned)
   int tiles_m, tiles_n;
+  int pair_bn;          // pair kernel: output columns of a tile, 256 or (128x4 scales, one destination) 192
   int row_classes;      // pair kernel, permuted rows: classes row % 4 of A and the output in the first of their two maps (4: one map)
   int splits;           // split-K factor (1-CTA kernel only); > 1 writes fp32 partials to `ws`
   int kt_per_split;     // K stages (of 256 elements) per split

@@ -682,6 +682,15 @@ static SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int bn, int sms) {
   return pl;
 }
 
+// Columns of the pair kernel's tiles: 192 where that costs no further round of tiles.  A 192-column tile takes 0.91 of a 256-column
+// one's time, not 0.75: its stages bring 89 bytes per clock into an SM instead of 73.  256 / 192 columns, us, 128x4 scales, as many rounds
+// of either: 129 x 1024 x 512 5.2 / 4.7, 300 x 3072 x 3072 8.9 / 8.4, 666 x 4096 x 4096 11.1 / 10.6 (one round each), 512 x 12288 x
+// 4096 18.4 / 17.2 (two); a fifth round for four: 4096^3 31.4 / 35.3, 2048 x 8192 x 4096 32.3 / 35.2.
+static int pair_tile_columns(int64_t M, int64_t N, int sms) {
+  const int64_t tiles_m = ceil_div(M, 256), clusters = sms / 2;
+  return ceil_div(tiles_m * ceil_div(N, 192), clusters) == ceil_div(tiles_m * ceil_div(N, 256), clusters) ? 192 : 256;
+}
+
 // ws_mode: 0 = workspace from the stream-ordered allocator (cudaMallocAsync / cudaFreeAsync),
 //          1 = fixed workspace of ws_capacity bytes, its address obtained from ws_fixed() only when a
 //              call really needs scratch (no allocation in this call)
@@ -774,7 +783,8 @@ static int linear_impl(void *D, int d_dtype, const void *A, const void *A_sf, co
   }
   CUtensorMap ta, tb;
   if (int e = get_tmap(A, M, K / 2, BM, &ta)) return e;
-  if (int e = get_tmap(B, N, K / 2, use_pair ? 128 : bn, &tb)) return e;
+  const int pair_bn = sf_layout == AC4K_SF_TILE128X4 && !(out && out->n_more > 0) ? pair_tile_columns(M, N, di.sms) : 256;
+  if (int e = get_tmap(B, N, K / 2, use_pair ? pair_bn / 2 : bn, &tb)) return e;
 
   GemmArgs a = {};
   a.sfa = static_cast<const uint8_t *>(A_sf);
@@ -810,6 +820,7 @@ static int linear_impl(void *D, int d_dtype, const void *A, const void *A_sf, co
   a.dbg = g_dbg;
   a.trace = g_trace;
   a.wait_ns = g_wait_ns ? g_wait_ns : kWaitTimeoutNs;
+  a.pair_bn = pair_bn;
   a.splits = pl.splits;
   a.kt_per_split = pl.kt_per_split;
   a.ws = nullptr;

@@ -67,32 +67,37 @@ using namespace ptx;
 #endif
 
 namespace pair {
-static constexpr int BN = 256;                      // output columns of the pair tile
 static constexpr int BMP = 256;                     // output rows of the pair tile
 static constexpr int KS = 4;                        // K = 64 steps per stage
 static constexpr int A_BYTES = 128 * BKB;           // this CTA's 128 rows of A, K = 256
-static constexpr int B_BYTES = 128 * BKB;           // this CTA's 128 rows of B, K = 256
 static constexpr int SFA_BYTES = KS * 512;          // [K step][32 x 16 B]
 static constexpr int SFB_BYTES = 2 * KS * 512;      // [128-row block of B][K step][32 x 16 B]
-static constexpr int STAGE_TX = A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES;    // bytes one CTA's TMA loads of a stage bring
 static constexpr int STAGES = 5;
-// Tensor memory (512 columns): two accumulators of 256 columns that share 48 columns, and the scales
-// of one stage.  Tiles alternate between the accumulators; the shared columns are the last 48 of the
-// first accumulator's tile and the first 48 of the second one's, so between two tiles only those 48
-// columns have to be read out before the next tile's first MMA may write them - the other 208 are
-// drained while the next tile's MMAs already run.
-static constexpr int ACC1_COL = 208;                // accumulator 0: columns 0 - 255, accumulator 1: 208 - 463
-static constexpr int SHARED_COLS = BN - ACC1_COL;   // 48
-static constexpr int SF_COL = ACC1_COL + BN;        // 464: per K step 4 columns for A, then 8 per K step for B
-static constexpr int SF_COLS = KS * 12;
 static constexpr int BIAS_BYTES = 8 * 128 * 4;      // one tile's bias as fp32, 128 columns per epilogue warp
 static constexpr int OUT_STAGE_BYTES = 32 * 128;    // per epilogue warp: 32 rows x 64 columns of 16-bit outputs
 static constexpr int BAR_BYTES = 256;
-// no slack for aligning the base: the kernel declares the array 1024-byte aligned and checks it
-static constexpr int SMEM_BYTES = STAGES * STAGE_TX + 8 * OUT_STAGE_BYTES + BIAS_BYTES + BAR_BYTES;
-static_assert(SF_COL + SF_COLS <= kTmemCols, "tensor memory overflow");
-static_assert(SMEM_BYTES <= 227 * 1024, "shared memory overflow");
-static constexpr int kThreadsPair = 448;           // 14 warps: 144 registers per thread for the epilogue
+static constexpr int kThreadsPair = 448;            // 14 warps: 144 registers per thread for the epilogue
+// BN_: output columns of the pair tile, 256 or 192
+template <int BN_>
+struct Tile {
+  static constexpr int BN = BN_;
+  static constexpr int B_ROWS = BN / 2;             // this CTA's rows of B
+  static constexpr int B_BYTES = B_ROWS * BKB;      // K = 256
+  static constexpr int STAGE_TX = A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES;    // bytes one CTA's TMA loads of a stage bring
+  // Tensor memory (512 columns): two accumulators that the tiles use in turn, and the scales of one stage.  Two of 256 columns share
+  // 48: the last 48 of the first accumulator's tile and the first 48 of the second one's, so between two tiles only those 48
+  // columns have to be read out before the next tile's first MMA may write them - the other 208 are drained while the next
+  // tile's MMAs already run.  Two of 192 share none.
+  static constexpr int ACC1_COL = BN == 256 ? 208 : BN;      // accumulator 0: columns [0, BN), accumulator 1: from here
+  static constexpr int SHARED_COLS = BN - ACC1_COL;          // 48, 0
+  static constexpr int SF_COL = ACC1_COL + BN;      // per K step 4 columns for A, then 8 per K step for B
+  static constexpr int SF_COLS = KS * 12;
+  // no slack for aligning the base: the kernel declares the array 1024-byte aligned and checks it
+  static constexpr int SMEM_BYTES = STAGES * STAGE_TX + 8 * OUT_STAGE_BYTES + BIAS_BYTES + BAR_BYTES;
+  static_assert(SF_COL + SF_COLS <= kTmemCols, "tensor memory overflow");
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory overflow");
+  static_assert(B_BYTES % 1024 == 0, "a stage's B starts on a swizzle atom");
+};
 }  // namespace pair
 
 // N accumulator columns starting at COL0 of this thread's 128-column segment: * alpha (+ bias from shared
@@ -185,12 +190,15 @@ __device__ __forceinline__ void drain_permuted(uint32_t (&w)[64], uint32_t t_row
 // rows take two maps (a variant of its own: as a condition in kSfPerm it cost that one 0.5 us of 11 at 668 x 4096 x 4096)
 enum { kSfWarps = 0, kSfTiled = 1, kSfPerm = 2, kSfPermRagged = 3 };
 
-template <int SF_MODE, int OUT_DT, int EPI>
+template <int SF_MODE, int OUT_DT, int EPI, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreadsPair, 1)
 linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                          const __grid_constant__ CUtensorMap tma_sfa, const __grid_constant__ CUtensorMap tma_sfb,
                          const __grid_constant__ DstMaps dmaps, const GemmArgs p) {
   using namespace pair;
+  using T2 = Tile<BN>;
+  constexpr int B_ROWS = T2::B_ROWS, B_BYTES = T2::B_BYTES, STAGE_TX = T2::STAGE_TX, ACC1_COL = T2::ACC1_COL, SF_COL = T2::SF_COL;
+  static_assert(BN == 256 || (SF_MODE == kSfTiled && EPI != EPI_GATHER), "192-column tiles: scales in 128x4 tiles, one destination");
   constexpr bool SF_TILED = SF_MODE != kSfWarps;      // the scales arrive by TMA, laid out for tcgen05.cp
   constexpr bool RAGGED = SF_MODE == kSfPermRagged, PERM = SF_MODE == kSfPerm || RAGGED;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -266,7 +274,7 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
     const uint32_t el = elect_one();
     int tm, tn;
     tile_coords(cluster_id, p.tiles_m, p.tiles_n, tm, tn);
-    const int m0 = tm * BMP + (int)rank * 128, nb0 = tn * BN + (int)rank * 128;
+    const int m0 = tm * BMP + (int)rank * 128, nb0 = tn * BN + (int)rank * B_ROWS;
     const int npre = k_tiles < STAGES ? k_tiles : STAGES;
     for (int kt = 0; kt < npre; ++kt) {
       if (PERM) {
@@ -294,9 +302,9 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
       int tm, tn;
       tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
       const int m0 = tm * BMP + (int)rank * 128;        // this CTA's rows of A
-      const int nb0 = tn * BN + (int)rank * 128;        // this CTA's rows of B
+      const int nb0 = tn * BN + (int)rank * B_ROWS;     // this CTA's rows of B
       const int sfa_row0 = (m0 / 128) * p.KT;           // tiled scales: row of [row block][K step] x 512 B
-      const int sfb_row0 = (tn * (BN / 128)) * p.KT;
+      const int sfb_row0 = (tn * BN / 128) * p.KT;      // (the tile's columns lie in this 128-row block of B's scales and the next)
       bool ok = true;
       for (int kt = 0; kt < k_tiles; ++kt) {
         ok = warp_all(mbar_wait(empty_bar + 8 * s, ph ^ 1, p.wait_ns));
@@ -353,10 +361,19 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
         ok = warp_all(mbar_wait(tempty_bar + 8 * acc, ((acc_phs >> acc) & 1) ^ 1, p.wait_ns));
         if (!ok) break;
         acc_phs ^= 1u << acc;
-        ok = warp_all(mbar_wait(shared_free_bar, shared_ph ^ 1, p.wait_ns));
-        if (!ok) break;
-        shared_ph ^= 1;
+        if (T2::SHARED_COLS > 0) {
+          ok = warp_all(mbar_wait(shared_free_bar, shared_ph ^ 1, p.wait_ns));
+          if (!ok) break;
+          shared_ph ^= 1;
+        }
         tc_fence_after();
+        // scale columns of B: every other 192-column tile begins in the middle of a 128-row block, two columns further on
+        uint32_t sfb_off = 0;
+        if (BN == 192) {
+          int tm, tn;
+          tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
+          sfb_off = (tn & 1) * 2;
+        }
         const uint32_t d_tmem = tmem_base + acc * ACC1_COL;
         for (int kt = 0; kt < k_tiles; ++kt) {
           if (el) AC4K_TR(0, it, 0);
@@ -364,7 +381,7 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
           if (!ok) break;
           tc_fence_after();
           if (el) AC4K_TR(0, it, 1);
-          const uint32_t t_sf = tmem_base + SF_COL;
+          const uint32_t t_sf = tmem_base + SF_COL, t_sfb = t_sf + KS * 4 + sfb_off;
           const uint64_t adesc = adesc0 + (uint64_t)(s * (A_BYTES >> 4));
           const uint64_t bdesc = bdesc0 + (uint64_t)(s * (B_BYTES >> 4));
           const uint64_t sfadesc = sfadesc0 + (uint64_t)(s * (SFA_BYTES >> 4));
@@ -379,7 +396,7 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
             }
 #pragma unroll
             for (int j = 0; j < KS; ++j)    // K step j: 32 bytes further inside the 128-byte swizzle atom
-              mma_mxf4nvf4_pair_if(el, d_tmem, adesc + 2 * j, bdesc + 2 * j, idesc, t_sf + j * 4, t_sf + KS * 4 + j * 8,
+              mma_mxf4nvf4_pair_if(el, d_tmem, adesc + 2 * j, bdesc + 2 * j, idesc, t_sf + j * 4, t_sfb + j * 8,
                                    (kt > 0 || j > 0) ? 1u : 0u);
           } else {
             for (int j = 0; j < nk; ++j) {
@@ -388,7 +405,7 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
               tmem_cp_32x128b_warpx4_pair_if(el, t_sf + KS * 4 + j * 8 + 4, sfbdesc + (KS + j) * 32);
             }
             for (int j = 0; j < nk; ++j)
-              mma_mxf4nvf4_pair_if(el, d_tmem, adesc + 2 * j, bdesc + 2 * j, idesc, t_sf + j * 4, t_sf + KS * 4 + j * 8,
+              mma_mxf4nvf4_pair_if(el, d_tmem, adesc + 2 * j, bdesc + 2 * j, idesc, t_sf + j * 4, t_sfb + j * 8,
                                    (kt > 0 || j > 0) ? 1u : 0u);
           }
           tc_commit_pair_both_if(el, empty_bar + 8 * s, 3);                 // stage free in both CTAs
@@ -507,15 +524,22 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
           if (has_bias) drain_permuted<OUT_DT, true, 0, 1, 2, 3>(w, t_row, shared, alpha, bias_s, lane, leader_shared_free);
           else drain_permuted<OUT_DT, false, 0, 1, 2, 3>(w, t_row, shared, alpha, bias_s, lane, leader_shared_free);
         }
-      } else if (half == (int)acc) {
-        // none of the shared columns: columns 0 - 127 of accumulator 0 or 128 - 255 of accumulator 1
+      } else if (BN == 192 || half == (int)acc) {
+        // none of the shared columns: columns 0 - 127 of accumulator 0 or 128 - 255 of accumulator 1, or 192-column accumulators, of
+        // which the second half's warps have the last 64 columns
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
+          if (BN == 192 && c == 1 && half == 1) {
+#pragma unroll
+            for (int i = 32; i < 64; ++i) w[i] = 0u;
+            break;
+          }
           uint32_t r[64];
           tmem_ld_32x32b_x64_sync(t_row + c * 64, r);
           if (c == 0) pack_cols<OUT_DT, 0, 64>(r, w, alpha, has_bias, bias_s);
           else pack_cols<OUT_DT, 64, 64>(r, w, alpha, has_bias, bias_s);
         }
+      } else if constexpr (BN == 192) {
       } else if (half == 0) {
         // accumulator 1, tile columns 0 - 127: the shared ones are this warp's first 48
         {
@@ -601,7 +625,7 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
 #pragma unroll
           for (int h2 = 0; h2 < 2; ++h2) {
             const int c64 = col0 + 64 * h2;
-            if (c64 >= p.N) break;
+            if (c64 >= p.N || 128 * half + 64 * h2 >= BN) break;
             if (row < p.M) {
               uint4 *dst = reinterpret_cast<uint4 *>(p.q_out + (int64_t)row * (p.N / 2) + c64 / 2);
               __stcs(dst, make_uint4(codes[8 * h2], codes[8 * h2 + 1], codes[8 * h2 + 2], codes[8 * h2 + 3]));
@@ -631,7 +655,7 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
 #pragma unroll
         for (int h2 = 0; h2 < 2; ++h2) {
           const int x0 = (int)col_base + 64 * h2;
-          if (col0 + 64 * h2 >= p.N || y0 + (RAGGED ? q : 0) >= p.M) break;     // warp-uniform: nothing of this box is inside the output
+          if (col0 + 64 * h2 >= p.N || 128 * half + 64 * h2 >= BN || y0 + (RAGGED ? q : 0) >= p.M) break;     // warp-uniform: nothing of this box is inside the output
           if (lane == 0) bulk_wait_group_read0();            // the previous store has read the buffer
           __syncwarp();
 #pragma unroll
@@ -677,21 +701,21 @@ linear_nvfp4_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   AC4K_TR_LAUNCH(false);
 }
 
-template <int SF_MODE, int OUT_DT, int EPI>
+template <int SF_MODE, int OUT_DT, int EPI, int BN = 256>
 static int launch_pair(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tsa, const CUtensorMap &tsb,
                        const DstMaps &dm, const GemmArgs &args, int sms, cudaStream_t stream) {
-  auto kern = linear_nvfp4_2cta_kernel<SF_MODE, OUT_DT, EPI>;
+  auto kern = linear_nvfp4_2cta_kernel<SF_MODE, OUT_DT, EPI, BN>;
   // Once per device: the shared-memory attribute, and how many CTA pairs can be resident at once (not every
   // SM can be paired on every part); the kernel is persistent, so launching more clusters than that would
   // serialise whole waves.
   static PerDevice<int> max_clusters;
   int clusters = 0;
   if (int e = max_clusters.get(&clusters, [&](int &v) {
-        AC4K_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::SMEM_BYTES));
+        AC4K_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::Tile<BN>::SMEM_BYTES));
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(sms & ~1);
         cfg.blockDim = dim3(pair::kThreadsPair);
-        cfg.dynamicSmemBytes = pair::SMEM_BYTES;
+        cfg.dynamicSmemBytes = pair::Tile<BN>::SMEM_BYTES;
         cudaLaunchAttribute attr;
         attr.id = cudaLaunchAttributeClusterDimension;
         attr.val.clusterDim.x = 2;
@@ -713,7 +737,7 @@ static int launch_pair(const CUtensorMap &ta, const CUtensorMap &tb, const CUten
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * clusters);
   cfg.blockDim = dim3(pair::kThreadsPair);
-  cfg.dynamicSmemBytes = pair::SMEM_BYTES;
+  cfg.dynamicSmemBytes = pair::Tile<BN>::SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -727,6 +751,8 @@ static int launch_pair(const CUtensorMap &ta, const CUtensorMap &tb, const CUten
 template <int OUT_DT, int EPI>
 static int launch_pair_mode(int sf_mode, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tsa, const CUtensorMap &tsb,
                             const DstMaps &dm, const GemmArgs &args, int sms, cudaStream_t stream) {
+  if constexpr (EPI != EPI_GATHER)
+    if (args.pair_bn == 192) return launch_pair<kSfTiled, OUT_DT, EPI, 192>(ta, tb, tsa, tsb, dm, args, sms, stream);
   if (sf_mode == kSfTiled) return launch_pair<kSfTiled, OUT_DT, EPI>(ta, tb, tsa, tsb, dm, args, sms, stream);
   if constexpr (EPI == EPI_GATHER) {
     if (sf_mode == kSfWarps) return launch_pair<kSfWarps, OUT_DT, EPI>(ta, tb, tsa, tsb, dm, args, sms, stream);
@@ -743,7 +769,7 @@ int launch_linear_2cta(int d_dtype, int sf_mode, const CUtensorMap &ta, const CU
   DeviceInfo di;
   if (int e = get_device_info(&di)) return e;
   args.tiles_m = (int)ceil_div(args.M, pair::BMP);
-  args.tiles_n = (int)ceil_div(args.N, pair::BN);
+  args.tiles_n = (int)ceil_div(args.N, args.pair_bn);
   // the instantiations that forward tiles to further destinations or re-quantise the output are
   // separate: their extra registers and code would otherwise slow the plain GEMM down
   if (args.q_out != nullptr) {

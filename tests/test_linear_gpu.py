@@ -162,6 +162,15 @@ def test_requantised_ragged_rows(ops, m):
     assert torch.equal(got[0], want[0]) and torch.equal(got[1].view(torch.uint8), want[1].view(torch.uint8))
 
 
+@pytest.mark.parametrize("m", [129, 256, 387])
+@pytest.mark.parametrize("n,k,odt,bdt", [(136, 64, torch.bfloat16, None), (192, 320, torch.float16, None), (200, 1088, torch.bfloat16, torch.float32),
+                                         (384, 256, torch.bfloat16, torch.bfloat16), (584, 512, torch.float16, torch.bfloat16), (4096, 128, torch.bfloat16, None)])
+def test_tiles_of_192_columns(ops, m, n, k, odt, bdt):
+    """128x4 scales, as many rounds of 192-column tiles as of 256-column ones: tiles that begin in the middle of a 128-row block of B's
+    scales, and an N that ends in either half"""
+    run_case(ops, m, n, k, seed=m + n, layout="128x4", bias_dtype=bdt, out_dtype=odt)
+
+
 def test_random_shapes(ops):
     """test/test_linear_bench.py:156-161: 20 random M, N, K in [2, 555]."""
     rng = random.Random(9567)
