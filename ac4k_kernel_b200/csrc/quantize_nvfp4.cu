@@ -725,9 +725,10 @@ extern "C" int ac4k_quantize_nvfp4_dynamic(void *out, void *sf, float *g_out, vo
   // Routes by size (measured on a B200; microseconds of the whole call on resident inputs stand beside the kernels):
   //   whole tensor in the registers of one cluster            one launch
   //   columns contiguous (attention's V), or four to seven     the one-launch kernel of quantize_nvfp4_resident.cu.  One launch / two, us:
-  //   of its tiles an SM                                       V of [1, 16384, 16, 128] 30 / 50, [1, 1000, 16, 128] 7.1 / 13.2, [2, 104, 8,
-  //                                                            128] 5.0 / 7.1; rows of 1000 x 5120 8.4 / 9.9, 2048 x 4096 9.7 / 11.3, but
-  //                                                            666 x 4096 7.3 / 5.3 (its grid barrier) and 3000 x 4096 18 / 13
+  //   of its tiles an SM, or 2^24 to 2^25 elements             V of [1, 16384, 16, 128] 30 / 50, [1, 1000, 16, 128] 7.1 / 13.2, [2, 104, 8,
+  //                                                            128] 5.0 / 7.1; rows of 1000 x 5120 8.6 / 9.8, 2048 x 4096 10.3 / 11.0, 4100 x
+  //                                                            4096 18.0 / 21.9, 8192 x 4096 31.0 / 33.5, but 666 x 4096 7.3 / 5.4 (its grid
+  //                                                            barrier), 4096 x 4096 17.5 / 16.4, 8192 x 8192 58.1 / 57.7
   //   up to 2^24 elements                                      maxima per CTA, then a quantiser that reduces them: two launches,
   //                                                            the second one set up under the first
   //   larger                                                   zeroed accumulator + atomic maximum + quantiser: a few hundred
@@ -739,7 +740,8 @@ extern "C" int ac4k_quantize_nvfp4_dynamic(void *out, void *sf, float *g_out, vo
     return sf_layout == AC4K_SF_AC4K ? launch_flat<AC4K_SF_AC4K>(out, sf, in, src, shape, stride, items, true, stream)
                                      : launch_flat<AC4K_SF_TILE128X4>(out, sf, in, src, shape, stride, items, true, stream);
   const int64_t resident_tiles = nbatch * ceil_div(M, 128) * (Kp / 64);
-  if (scratch && (swizzle || stride[3] != 1 || (resident_tiles >= 4 * (int64_t)di.sms && resident_tiles <= 7 * (int64_t)di.sms))) {
+  if (scratch && (swizzle || stride[3] != 1 || (resident_tiles >= 4 * (int64_t)di.sms && resident_tiles <= 7 * (int64_t)di.sms) ||
+                  (numel > (1 << 24) && numel <= (1 << 25)))) {
     const int e = launch_quantize_resident(out, sf, g_out, scratch, in, max_scale, shape, stride, swizzle, sf_layout, stream);
     if (e != kResidentDeclined) return e;
   }

@@ -13,7 +13,6 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
-#include <type_traits>
 
 #include "gemm_common.cuh"
 
@@ -25,7 +24,6 @@ enum { kRows = 0, kTransposed = 1, kTransposedPermuted = 2 };
 static constexpr int kTileBytes = 128 * 128;
 static constexpr int kWarps = 16, kThreads = 32 * (kWarps + 1);      // consumers and one producer warp
 static constexpr int kMaxSlots = 14;
-static constexpr int kBatch = 2;                  // tiles that a thread of kRows quantises side by side
 // beside the slots: reciprocal table, one word per warp, barriers, scale words of the transposed form (two buffers a team)
 static constexpr int kMiscBytes = 128 * 4 + 32 * 4 + 2 * kMaxSlots * 8, kScaleBytes = 4 * 2 * 128 * 4;
 constexpr int teams(int mode) { return mode == kRows ? 1 : 4; }
@@ -207,70 +205,31 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
     const int j = lane >> 2, blk = lane & 3;
     const int row_l = SF_LAYOUT == AC4K_SF_AC4K ? warp * 8 + j : (j >> 1) * 32 + 2 * warp + (j & 1);
     const uint32_t at0 = tiles_s + row_l * 128 + (((2 * blk) ^ (row_l & 7)) << 4), at1 = tiles_s + row_l * 128 + (((2 * blk + 1) ^ (row_l & 7)) << 4);
+    // (several tiles side by side in one thread, to fill the chain from a block's words to its codes, gained nothing where the tiles
+    // are there already and took twice as long where they are loaded again: 8192 x 8192 86 us against 57)
     Tile t(first + n - 1, p);
-    int s = s_last, u = u_last;
-    // where this thread's codes and its row's scale word of tile t go (counted on from tile to tile, like the coordinates)
-    uint8_t *out_t;
-    uint32_t *sf_t;
-    bool row_ok, word_ok;
-    auto aim = [&]() {
+    for (int q = 0, s = s_last, u = u_last; q < n; ++q) {
+      ok = warp_all(mbar_wait(full + 8 * s, u & 1));
+      if (!ok) break;
+      const uint4 v0 = ld_shared_v4u(at0 + s * kTileBytes), v1 = ld_shared_v4u(at1 + s * kTileBytes);
+      if (n > S) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty + 8 * s);
+      }
       const int row = t.mid * 128 + row_l;
-      out_t = p.out + ((int64_t)t.b * p.M + row) * (Kp / 2) + t.fast * 32 + blk * 8;
-      sf_t = sf_w + sf_word(t.b, row, t.fast);
-      row_ok = row < p.M;
-      word_ok = blk == 0 && row < rows_sf;
-    };
-    aim();
-    // N tiles at a time: the chain of one block, from its words to its codes, is several times as long as the sixteen warps' issue
-    // of one tile
-    auto quantise = [&](auto count) {
-      constexpr int N = decltype(count)::value;
-      uint4 v0[N], v1[N];
-      uint8_t *out_at[N];
-      uint32_t *sf_at[N];
-      bool live[N], store[N];
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        if (ok) ok = warp_all(mbar_wait(full + 8 * s, u & 1));
-        v0[i] = ld_shared_v4u(at0 + s * kTileBytes);
-        v1[i] = ld_shared_v4u(at1 + s * kTileBytes);
-        if (n > S) {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(empty + 8 * s);
-        }
-        out_at[i] = out_t;
-        sf_at[i] = sf_t;
-        live[i] = row_ok;
-        store[i] = word_ok;
-        const bool same_rows = t.fast > 0;
-        t.back(p);
-        out_t -= 32;
-        sf_t -= SF_LAYOUT == AC4K_SF_AC4K ? rows_sf : 128;
-        if (!same_rows) aim();
-        if (--s < 0) { s = S - 1; --u; }
-        if (s == s_last) u += 2;
-      }
-      float r[N];
-      uint32_t word[N];
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        const uint32_t sb = block_scale_of(hmax_bf16x2_to_f32(amax_bf16x2(v0[i], v1[i])), alpha, s_rcp, r[i]);
-        word[i] = live[i] ? sb << (8 * blk) : 0u;
-      }
-#pragma unroll
-      for (int i = 0; i < N; ++i) word[i] |= __shfl_xor_sync(0xFFFFFFFFu, word[i], 1);
-#pragma unroll
-      for (int i = 0; i < N; ++i) word[i] |= __shfl_xor_sync(0xFFFFFFFFu, word[i], 2);
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        const uint2 codes = make_uint2(quantize8_x2(v0[i].x, v0[i].y, v0[i].z, v0[i].w, r[i]), quantize8_x2(v1[i].x, v1[i].y, v1[i].z, v1[i].w, r[i]));
-        if (live[i]) __stcs(reinterpret_cast<uint2 *>(out_at[i]), codes);
-        if (store[i]) *sf_at[i] = word[i];
-      }
-    };
-    int q = 0;
-    for (; q + kBatch <= n; q += kBatch) quantise(std::integral_constant<int, kBatch>());
-    for (; q < n; ++q) quantise(std::integral_constant<int, 1>());
+      float r;
+      const uint32_t sb = block_scale_of(hmax_bf16x2_to_f32(amax_bf16x2(v0, v1)), alpha, s_rcp, r);
+      uint32_t word = row < p.M ? sb << (8 * blk) : 0u;
+      word |= __shfl_xor_sync(0xFFFFFFFFu, word, 1);
+      word |= __shfl_xor_sync(0xFFFFFFFFu, word, 2);
+      if (row < p.M)
+        __stcs(reinterpret_cast<uint2 *>(p.out + ((int64_t)t.b * p.M + row) * (Kp / 2) + t.fast * 32 + blk * 8),
+               make_uint2(quantize8_x2(v0.x, v0.y, v0.z, v0.w, r), quantize8_x2(v1.x, v1.y, v1.z, v1.w, r)));
+      if (blk == 0 && row < rows_sf) sf_w[sf_word(t.b, row, t.fast)] = word;
+      t.back(p);
+      if (--s < 0) { s = S - 1; --u; }
+      if (s == s_last) u += 2;
+    }
   } else {
     const int g32 = tt >> 5;                               // 32 K-elements of the tile; the lane: rows 2 lane, 2 lane + 1
     uint32_t buf = 0;
@@ -457,9 +416,6 @@ static int launch_attention(void *const out[3], void *const sf[3], float *const 
     if (mode != (i == 2 ? kTransposedPermuted : kRows)) return kResidentDeclined;
     total += a[i].tiles;
   }
-  // (three launches for larger ones: q and k by the two-launch kernels, whose stores are whole lines.  One launch / three, us of the
-  // attention call: [1, 16384, 16, 128] 1634 / 1677, [2, 1444 / 794, 18, 128] 51 / 71, [2, 105 / 447, 7, 64] 15 / 22)
-  if (total > 16384) return kResidentDeclined;
   int ctas[3], used = 0, smem = 0;
   for (int i = 0; i < 3; ++i) {
     // (rounded down, so that the three fit; at least one)
