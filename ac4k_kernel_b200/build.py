@@ -131,7 +131,7 @@ def _build_module(name: str, source: str, force: bool) -> str:
         cmd += ["-isystem", inc]
     cmd += ["-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda_home, "include"),
             "-I", os.path.join(ROOT, "include"), src, "-o", target,
-            "-L", PKG_DIR, "-l:libac4k_b200.so", "-L", torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
+            "-L", PKG_DIR, "-l:libac4k_b200.so", "-L", torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch",
             "-ltorch_python",
             # The process's own libstdc++ and not a second, static one, which a compiler that comes without the shared one
             # links by itself: two of them disagree about the stream facets, and the first number that is formatted (any

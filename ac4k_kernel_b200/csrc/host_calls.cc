@@ -9,7 +9,12 @@
 // raises its own error.  So nothing here decides what is accepted and what is refused.  The interpreter lock is given up for
 // allocations and launches (a launch waits while the driver's queue is full).
 #include <ATen/ATen.h>
+#include <ATen/Context.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/record_function.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
@@ -52,8 +57,16 @@ bool scalar_of(py::handle h, at::Tensor *out) {
 }
 bool same_shape(const at::Tensor &t, std::initializer_list<int64_t> want) { return t.sizes() == at::IntArrayRef(want.begin(), want.size()); }
 
+// An uninitialised tensor.  Straight from the allocator's factory where nothing listens to operator calls (no dispatch mode, tracer
+// or function transform, no deterministic filling, no profiler): through the dispatcher a tensor costs 0.2 us more, 0.6 us of the 6.3
+// of a small quantize(), 0.9 us of the 17 of a small attention().
 at::Tensor empty(at::IntArrayRef sizes, at::ScalarType dt, const at::Tensor &like) {
-  return at::empty(sizes, at::TensorOptions().dtype(dt).device(like.device()));
+  const c10::DispatchKeySet listeners({c10::DispatchKey::Tracer, c10::DispatchKey::FuncTorchDynamicLayerFrontMode, c10::DispatchKey::Functionalize,
+                                       c10::DispatchKey::PythonDispatcher});
+  if (c10::impl::dispatch_mode_enabled() || c10::impl::tls_local_dispatch_key_set().included_.has_any(listeners) ||
+      at::globalContext().deterministicAlgorithms() || at::hasCallbacks())
+    return at::empty(sizes, at::TensorOptions().dtype(dt).device(like.device()));
+  return at::Tensor(at::detail::empty_cuda(sizes, dt, like.device(), std::nullopt));
 }
 at::Tensor scalar_like(const at::Tensor &like) { return empty({}, at::kFloat, like); }
 
