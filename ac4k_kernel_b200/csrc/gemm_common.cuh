@@ -28,7 +28,7 @@ static constexpr int kTmemCols = 512;
 static constexpr int kGroupM = 8;     // tile rasterisation: walk 8 M-tiles per N-tile
 
 enum : unsigned { kStatusTimeoutProducer = 0xA1, kStatusTimeoutMma = 0xA2, kStatusTimeoutSf = 0xA3,
-                  kStatusTimeoutEpilogue = 0xA4, kStatusSmemAlign = 0xB1 };
+                  kStatusTimeoutEpilogue = 0xA4, kStatusTimeoutGrid = 0xA5, kStatusSmemAlign = 0xB1 };
 
 template <int BN>
 struct Cfg {
@@ -162,6 +162,9 @@ int get_tmap_sf_rows(const void *ptr, int64_t rows, int64_t kt, CUtensorMap *out
 // 2-D byte tensor map with a (64 B x box_rows) box and 64-byte swizzle
 int get_tmap64(const void *ptr, int64_t rows, int64_t row_bytes, int box_rows, CUtensorMap *out);
 unsigned long long *debug_trace_ptr();
+// experiment switches and wait limit of debug-hook builds (0 otherwise)
+int debug_flags();
+unsigned long long debug_wait_ns();
 // bf16 [B, H, N, D] by element strides (D contiguous, the others multiples of 8): boxes of D x box_rows x 1 x 1
 int get_tmap_bf16_4d(const void *ptr, const int64_t shape[4], const int64_t stride[4], int box_rows, CUtensorMap *out);
 // the same tensor in boxes of 64 x 128 x 1 x 1 with the 128-byte swizzle

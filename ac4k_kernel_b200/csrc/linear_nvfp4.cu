@@ -635,7 +635,10 @@ using namespace ac4k;
 //                               dependency wait (pair kernel)
 //                               256 the pair kernel's producer leaves out the loads of its very first stage, so that
 //                               the waits for it expire (the wait-expiry test)
+//                               0x400 the last CTA of a tensor in the one-launch quantiser does not write its word, so that the
+//                               others' meeting expires
 //   ac4k_debug_set_wait_ns(ns)  limit of the device-side waits of later launches (0 = the default 2 s)
+//   ac4k_debug_one_launches()   launches of the one-launch NVFP4 quantiser so far (quantize_nvfp4_resident.cu)
 //   ac4k_debug_set_trace(ptr)   device buffer for the clock stamps of builds with -DAC4K_TRACE_ENABLED
 #ifdef AC4K_DEBUG_HOOKS
 static int g_force_bn = 0;
@@ -655,6 +658,8 @@ static constexpr unsigned long long g_wait_ns = 0;
 #endif
 // the clock-stamp buffer of trace builds for the other kernels of the library (NULL otherwise)
 unsigned long long *ac4k::debug_trace_ptr() { return g_trace; }
+int ac4k::debug_flags() { return g_dbg; }
+unsigned long long ac4k::debug_wait_ns() { return g_wait_ns; }
 
 // Split-K plan of the single-CTA kernel for shapes with too few output tiles to occupy the GPU (65 <= M <= 128,
 // or any M with an output the other kernels do not store): how many K slices, and the fp32 workspace

@@ -1,8 +1,8 @@
 // BF16 -> NVFP4 with the tensor's own global scale in ONE launch: a cooperative grid of one CTA per SM reduces the tensor to its
-// maximum, meets at a grid barrier, and quantises.  The tiles that a CTA read last are still in its shared memory then (up to 224 KB
+// maximum, meets (see below), and quantises.  The tiles that a CTA read last are still in its shared memory then (up to 224 KB
 // an SM, 33 MB of the chip), so a tensor of at most that size is read from memory once; of a larger one the rest is read again from
 // the end backwards, while the L2 still has what was read last.  Same bits as the two-launch route of quantize_nvfp4.cu (same arithmetic).
-// What bounds it: the read of the tensor (5.6 TB/s), 1.5 us of grid barrier, and behind it the issue of some hundred instructions a
+// What bounds it: the read of the tensor (5.6 TB/s), the meeting, and behind it the issue of some hundred instructions a
 // block by 16 warps; which sizes take it stands at ac4k_quantize_nvfp4_dynamic, with the times of both routes.
 //
 // A tile is 16 KB, one TMA box with the 128-byte swizzle: 128 rows x 64 K-elements of a tensor whose rows are contiguous along K
@@ -10,9 +10,19 @@
 // 16 consumer warps in teams; a team takes every n-th tile of the CTA's contiguous share.  kRows: one team, a thread has one
 // 16-element block of the tile, four lanes a row, and conflict-free 16-byte reads.  Transposed: teams of four warps, a thread has two
 // rows x 32 K-elements (a warp reads 32 words of one 128-byte line at a time), and the scale bytes meet in shared memory.
-#include <cooperative_groups.h>
-
+//
+// The meeting.  Every CTA of a tensor leaves its maximum in a word of its own, {48-bit tag of the launch, maximum}; CTA 0 waits for all
+// of them and answers each CTA in a second word of that CTA, with the maximum of all or, where one did not come within the
+// launch's limit, with kNoMaximum; the others wait for that answer, for twice as long.  The words are in the call's scratch, whose contents
+// are undefined: a tag is not repeated in a process and starts at a random number, so that a word that has not been written yet does not
+// have it (2^-48).  A captured launch is replayed with the same tag, so no word may keep it: each has one reader, which clears it, and
+// a CTA without an answer clears what it left itself.  (All CTAs polling all words: 2 - 3 us longer, 148 readers on the same ten lines.)
+// That all CTAs of the grid are on the chip together is what a cooperative launch promises (it fails otherwise).  Programmatic
+// serialisation does not take that away: it lets the grid begin when every CTA of the kernel in front has begun, and those wait for
+// nothing of this one.
 #include <algorithm>
+#include <atomic>
+#include <random>
 
 #include "gemm_common.cuh"
 
@@ -24,26 +34,33 @@ enum { kRows = 0, kTransposed = 1, kTransposedPermuted = 2 };
 static constexpr int kTileBytes = 128 * 128;
 static constexpr int kWarps = 16, kThreads = 32 * (kWarps + 1);      // consumers and one producer warp
 static constexpr int kMaxSlots = 14;
-// beside the slots: reciprocal table, one word per warp, barriers, scale words of the transposed form (two buffers a team)
-static constexpr int kMiscBytes = 128 * 4 + 32 * 4 + 2 * kMaxSlots * 8, kScaleBytes = 4 * 2 * 128 * 4;
+// beside the slots: reciprocal table, two words per warp, barriers, scale words of the transposed form (two buffers a team)
+static constexpr int kMiscBytes = 128 * 4 + 2 * 32 * 4 + 2 * kMaxSlots * 8, kScaleBytes = 4 * 2 * 128 * 4;
+static constexpr uint32_t kNoMaximum = 0xFFFF;        // |x| of bf16 has 15 bits
+// a meeting's place in scratch: a maximum and an answer per CTA
+constexpr int64_t meeting_words(int64_t ctas) { return 2 * ctas; }
 constexpr int teams(int mode) { return mode == kRows ? 1 : 4; }
 // a slot that is used again belongs to one team (its barriers' parities would be ambiguous to a team that skips a use)
 constexpr int max_slots(int mode) { return mode == kRows ? kMaxSlots : 12; }
 constexpr int smem_bytes(int mode, int slots) { return 1024 + slots * kTileBytes + kMiscBytes + (mode == kRows ? 0 : kScaleBytes); }
 static_assert(smem_bytes(kRows, max_slots(kRows)) <= 227 * 1024 && smem_bytes(kTransposed, max_slots(kTransposed)) <= 227 * 1024, "shared memory overflow");
+static_assert(kWarps < 32, "a lane per warp's maximum");
 static_assert(max_slots(kTransposed) % teams(kTransposed) == 0, "a slot belongs to one team");
 }  // namespace resident
 
 struct ResidentArgs {
   uint8_t *out;
   uint8_t *sf;
-  uint32_t *partial;       // one word per CTA
+  unsigned long long *maxima, *answers;  // the meeting: one word of each per CTA
+  unsigned long long tag;                // 48 bits, not 0
   float *g_out;
   float max_scale;
   int M, K, d1;
   int n_fast, n_mid;       // tiles along the tile order's first and second dimension
   int tiles, slots;
   unsigned int *status;
+  unsigned long long wait_ns;            // limit of a wait for a load; CTA 0 waits twice as long for the others' maxima, they four times for its answer
+  int dbg;                               // experiment switches (builds with -DAC4K_DEBUG_HOOKS), else 0
 };
 
 __device__ __forceinline__ uint4 ld_shared_v4u(uint32_t addr) {
@@ -76,6 +93,20 @@ __device__ __forceinline__ uint32_t block_scale_of(float amax, float alpha, cons
   return sb;
 }
 
+// Waits for a word with `tag`, clears it, and gives its low 16 bits; false, and `value` left alone, where it did not come within the limit
+__device__ __forceinline__ bool wait_tagged(unsigned long long *word, unsigned long long tag, unsigned long long limit_ns, uint32_t &value) {
+  unsigned long long w, t0 = 0;
+  for (int k = 0; (w = ld_relaxed_gpu_u64(word)) >> 16 != tag; ++k) {
+    if (k & 63) continue;
+    const unsigned long long now = globaltimer();
+    if (k == 0) t0 = now;
+    else if (now - t0 > limit_ns) return false;
+  }
+  st_relaxed_gpu_u64(word, 0);
+  value = (uint32_t)w & 0xFFFFu;
+  return true;
+}
+
 // One tensor by `ctas` CTAs of the grid, of which this is number `cta`.
 template <int SF_LAYOUT, int MODE>
 __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const ResidentArgs &p, int cta, int ctas) {
@@ -85,8 +116,8 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
   const uint32_t tiles_s = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *misc = smem_raw + (tiles_s - smem_u32(smem_raw)) + p.slots * kTileBytes;
   float *s_rcp = reinterpret_cast<float *>(misc);
-  uint32_t *s_m = reinterpret_cast<uint32_t *>(misc + 512);
-  const uint32_t full = smem_u32(misc + 640), empty = full + 8 * kMaxSlots;
+  uint32_t *s_m = reinterpret_cast<uint32_t *>(misc + 512), *s_all = s_m + 32;
+  const uint32_t full = smem_u32(misc + 768), empty = full + 8 * kMaxSlots;
   uint32_t *s_sf = reinterpret_cast<uint32_t *>(misc + kMiscBytes);       // transposed: [team][buffer][K = 64 step][64 rows]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = p.slots;
@@ -136,7 +167,7 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
     const uint32_t el = elect_one();
     Tile t(first, p);
     for (int i = 0, s = 0, u = 0; i < n && ok; ++i) {
-      if (u > 0) ok = warp_all(mbar_wait(empty + 8 * s, (u - 1) & 1));
+      if (u > 0) ok = warp_all(mbar_wait(empty + 8 * s, (u - 1) & 1, p.wait_ns));
       if (ok) issue(el, t, s);
       t.next(p);
       if (++s == S) { s = 0; ++u; }
@@ -144,7 +175,7 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
   } else {
     for (int i = team, s = team, u = 0; i < n; i += TEAMS) {
       if (s >= S) { s -= S; ++u; }
-      ok = warp_all(mbar_wait(full + 8 * s, u & 1));
+      ok = warp_all(mbar_wait(full + 8 * s, u & 1, p.wait_ns));
       if (!ok) break;
 #pragma unroll
       for (int c = 0; c < TEAMS; ++c) {
@@ -158,23 +189,50 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
       s += TEAMS;
     }
   }
-  // the maximum over the CTA, then over the grid
+  // the maximum over the CTA, then over the CTAs of the tensor
   {
     uint32_t m = __reduce_max_sync(0xFFFFFFFFu, max(m2 & 0xFFFFu, m2 >> 16));
     if (lane == 0) s_m[warp] = m;
     __syncthreads();
     if (warp == 0) {
       m = __reduce_max_sync(0xFFFFFFFFu, lane <= kWarps ? s_m[lane] : 0u);
-      if (lane == 0) __stcg(p.partial + cta, m);
+      if (lane == 0) s_all[kWarps] = m;
+      if (lane == 0 && cta != 0 && !(AC4K_DBG(p, 0x400) && cta == ctas - 1)) st_relaxed_gpu_u64(p.maxima + cta, p.tag << 16 | m);
     }
+    __syncwarp();
   }
-  cooperative_groups::this_grid().sync();
+  uint32_t m = kNoMaximum;
+  if (cta == 0) {
+    bool all = true;
+    uint32_t mine = 0;
+    if (warp < kWarps)
+      for (int i = 1 + threadIdx.x; i < ctas; i += 32 * kWarps) {
+        uint32_t other;
+        if (wait_tagged(p.maxima + i, p.tag, 2 * p.wait_ns, other)) mine = max(mine, other);
+        else all = false;
+      }
+    mine = __reduce_max_sync(0xFFFFFFFFu, mine);
+    if (lane == 0 && warp < kWarps) s_all[warp] = mine;
+    if (!all) atomicExch(p.status, kStatusTimeoutGrid);
+    all = !__syncthreads_or(!all);
+    if (all) m = __reduce_max_sync(0xFFFFFFFFu, lane <= kWarps ? s_all[lane] : 0u);
+    for (int i = 1 + threadIdx.x; i < ctas; i += kThreads) st_relaxed_gpu_u64(p.answers + i, p.tag << 16 | m);
+  } else {
+    if (threadIdx.x == 0) {
+      if (!wait_tagged(p.answers + cta, p.tag, 4 * p.wait_ns, m)) atomicExch(p.status, kStatusTimeoutGrid);
+      if (m == kNoMaximum) st_relaxed_gpu_u64(p.maxima + cta, 0);
+      s_all[0] = m;
+    }
+    __syncthreads();
+    m = s_all[0];
+  }
+  if (m == kNoMaximum) return;
   if (warp == kWarps) {
     const uint32_t el = elect_one();
     if (n > S) {
       Tile t(first + n - 1 - S, p);
       for (int q = S, s = s_last, u = u_last; q < n && ok; ++q) {      // the load behind use u of slot s
-        ok = warp_all(mbar_wait(empty + 8 * s, u & 1));
+        ok = warp_all(mbar_wait(empty + 8 * s, u & 1, p.wait_ns));
         if (ok) issue(el, t, s);
         t.back(p);
         // from the last tile's slot on, each slot's use is one less below the wrap, and one more a round later
@@ -185,9 +243,6 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
     if (!ok && lane == 0) atomicExch(p.status, kStatusTimeoutProducer);
     return;
   }
-  uint32_t m = 0;
-  for (int i = lane; i < ctas; i += 32) m = max(m, __ldcg(p.partial + i));
-  m = __reduce_max_sync(0xFFFFFFFFu, m);
   const float g = global_scale_of(m, p.max_scale), alpha = alpha_of(g);
   if ((cta | threadIdx.x) == 0) *p.g_out = g;
 
@@ -209,7 +264,7 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
     // are there already and took twice as long where they are loaded again: 8192 x 8192 86 us against 57)
     Tile t(first + n - 1, p);
     for (int q = 0, s = s_last, u = u_last; q < n; ++q) {
-      ok = warp_all(mbar_wait(full + 8 * s, u & 1));
+      ok = warp_all(mbar_wait(full + 8 * s, u & 1, p.wait_ns));
       if (!ok) break;
       const uint4 v0 = ld_shared_v4u(at0 + s * kTileBytes), v1 = ld_shared_v4u(at1 + s * kTileBytes);
       if (n > S) {
@@ -237,7 +292,7 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
     for (int q = 0, s = s_last, u = u_last; q < n; ++q, t.back(p), s == 0 ? (s = S - 1, --u) : --s, u += s == s_last ? 2 : 0) {
       if ((n - 1 - q) % TEAMS != team) continue;
       // (a warp whose wait ran out goes on, so that its team does not hang at the barrier below)
-      if (ok) ok = warp_all(mbar_wait(full + 8 * s, u & 1));
+      if (ok) ok = warp_all(mbar_wait(full + 8 * s, u & 1, p.wait_ns));
       uint32_t w[32];                                      // element j of row 2 lane (low half) and of row 2 lane + 1 (high half)
 #pragma unroll
       for (int j = 0; j < 32; ++j)
@@ -285,7 +340,7 @@ __global__ void __launch_bounds__(resident::kThreads, 1)
 nvfp4_quantize_resident_kernel(const __grid_constant__ CUtensorMap tma, const ResidentArgs p) {
   resident_quantize<SF_LAYOUT, MODE>(tma, p, blockIdx.x, gridDim.x);
 }
-// q, k and v of the attention operator, each with a share of the grid: one launch and one grid barrier for the three.
+// q, k and v of the attention operator, each with a share of the grid and a meeting of its own, in one launch.
 template <int SF_LAYOUT>
 __global__ void __launch_bounds__(resident::kThreads, 1)
 nvfp4_quantize_attention_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
@@ -296,6 +351,36 @@ nvfp4_quantize_attention_kernel(const __grid_constant__ CUtensorMap tma_q, const
   else if (cta < ctas_q + ctas_k) resident_quantize<SF_LAYOUT, resident::kRows>(tma_k, k, cta - ctas_q, ctas_k);
   else resident_quantize<SF_LAYOUT, resident::kTransposedPermuted>(tma_v, v, cta - ctas_q - ctas_k, (int)gridDim.x - ctas_q - ctas_k);
 }
+
+// 48 bits, not 0, not repeated within 2^48 launches of the process
+static unsigned long long next_tag() {
+  static std::atomic<unsigned long long> next = [] {
+    try {
+      std::random_device rd;
+      return (unsigned long long)rd() << 32 | rd();
+    } catch (...) {      // (no source of random numbers)
+      return (unsigned long long)reinterpret_cast<uintptr_t>(&next_tag) * 0x9E3779B97F4A7C15ull;
+    }
+  }();
+  for (;;)
+    if (const unsigned long long t = next.fetch_add(1, std::memory_order_relaxed) & 0xFFFFFFFFFFFFull) return t;
+}
+
+// The place of the next `ctas` CTAs' meeting behind `at`
+static void set_meeting(ResidentArgs *a, unsigned long long *&at, int64_t ctas) {
+  a->maxima = at;
+  a->answers = at + ctas;
+  a->tag = next_tag();
+  at += resident::meeting_words(ctas);
+}
+static unsigned long long *first_word(void *scratch) { return reinterpret_cast<unsigned long long *>((reinterpret_cast<uintptr_t>(scratch) + 7) & ~(uintptr_t)7); }
+// at most one CTA per SM, behind up to 4 bytes in front of the first word
+static bool meetings_fit(int sms) { return 8 * resident::meeting_words(sms) + 4 <= AC4K_QUANTIZE_SCRATCH_BYTES; }
+
+#ifdef AC4K_DEBUG_HOOKS
+static std::atomic<int> g_one_launches{0};      // what launch_cooperative launched so far, so that a test can say which route a call took
+extern "C" __attribute__((visibility("default"))) int ac4k_debug_one_launches() { return g_one_launches.load(); }
+#endif
 
 // Cooperative, and beside the tail of the kernel in front of it; kResidentDeclined where the grid does not fit at once (a context with
 // fewer SMs than the device).
@@ -319,11 +404,14 @@ static int launch_cooperative(void (*kern)(KArgs...), int grid, size_t smem, cud
     return kResidentDeclined;
   }
   AC4K_CUDA_TRY(e);
+#ifdef AC4K_DEBUG_HOOKS
+  ++g_one_launches;
+#endif
   return 0;
 }
 
 template <int SF_LAYOUT, int MODE>
-static int launch_resident(const CUtensorMap &tm, ResidentArgs a, int sms, cudaStream_t stream) {
+static int launch_resident(const CUtensorMap &tm, ResidentArgs a, void *scratch, int sms, cudaStream_t stream) {
   using namespace resident;
   auto kern = nvfp4_quantize_resident_kernel<SF_LAYOUT, MODE>;
   static PerDevice<int> attr_set;
@@ -335,12 +423,14 @@ static int launch_resident(const CUtensorMap &tm, ResidentArgs a, int sms, cudaS
       }))
     return e;
   const int grid = std::min(a.tiles, sms);
+  unsigned long long *at = first_word(scratch);
+  set_meeting(&a, at, grid);
   a.slots = std::min((int)ceil_div(a.tiles, grid), max_slots(MODE));
   return launch_cooperative(kern, grid, smem_bytes(MODE, a.slots), stream, tm, a);
 }
 
 // Tensor map and arguments for one tensor; kResidentDeclined where no map can have its strides.
-static int resident_plan(void *out, void *sf, float *g_out, void *partial, const void *in, float max_scale, const int64_t shape[4],
+static int resident_plan(void *out, void *sf, float *g_out, const void *in, float max_scale, const int64_t shape[4],
                          const int64_t stride[4], int swizzle, int sf_layout, int *mode, CUtensorMap *tm, ResidentArgs *a) {
   using namespace resident;
   const int64_t nbatch = shape[0] * shape[1], M = shape[2], K = shape[3], Kp = align_up(K, 64);
@@ -372,9 +462,10 @@ static int resident_plan(void *out, void *sf, float *g_out, void *partial, const
   if (!a->status || get_tmap_bf16_tiles(in, dims, strides, tm)) return kResidentDeclined;
   a->out = static_cast<uint8_t *>(out);
   a->sf = static_cast<uint8_t *>(sf);
-  a->partial = static_cast<uint32_t *>(partial);
   a->g_out = g_out;
   a->max_scale = max_scale;
+  a->wait_ns = debug_wait_ns() ? debug_wait_ns() : kWaitTimeoutNs;
+  a->dbg = debug_flags();
   a->M = (int)M; a->K = (int)K; a->d1 = (int)shape[1];
   a->n_fast = (int)n_fast; a->n_mid = (int)n_mid; a->tiles = (int)(nbatch * n_fast * n_mid);
   return 0;
@@ -385,19 +476,19 @@ int launch_quantize_resident(void *out, void *sf, float *g_out, void *scratch, c
   using namespace resident;
   DeviceInfo di;
   if (int e = get_device_info(&di)) return e;
-  if (di.cc_major != 10 || di.sms * 4 > AC4K_QUANTIZE_SCRATCH_BYTES) return kResidentDeclined;
+  if (di.cc_major != 10 || !meetings_fit(di.sms)) return kResidentDeclined;
   int mode;
   CUtensorMap tm;
   ResidentArgs a;
-  if (int e = resident_plan(out, sf, g_out, scratch, in, max_scale, shape, stride, swizzle, sf_layout, &mode, &tm, &a)) return e;
+  if (int e = resident_plan(out, sf, g_out, in, max_scale, shape, stride, swizzle, sf_layout, &mode, &tm, &a)) return e;
   if (sf_layout == AC4K_SF_AC4K) {
-    if (mode == kRows) return launch_resident<AC4K_SF_AC4K, kRows>(tm, a, di.sms, stream);
-    if (mode == kTransposed) return launch_resident<AC4K_SF_AC4K, kTransposed>(tm, a, di.sms, stream);
-    return launch_resident<AC4K_SF_AC4K, kTransposedPermuted>(tm, a, di.sms, stream);
+    if (mode == kRows) return launch_resident<AC4K_SF_AC4K, kRows>(tm, a, scratch, di.sms, stream);
+    if (mode == kTransposed) return launch_resident<AC4K_SF_AC4K, kTransposed>(tm, a, scratch, di.sms, stream);
+    return launch_resident<AC4K_SF_AC4K, kTransposedPermuted>(tm, a, scratch, di.sms, stream);
   }
-  if (mode == kRows) return launch_resident<AC4K_SF_TILE128X4, kRows>(tm, a, di.sms, stream);
-  if (mode == kTransposed) return launch_resident<AC4K_SF_TILE128X4, kTransposed>(tm, a, di.sms, stream);
-  return launch_resident<AC4K_SF_TILE128X4, kTransposedPermuted>(tm, a, di.sms, stream);
+  if (mode == kRows) return launch_resident<AC4K_SF_TILE128X4, kRows>(tm, a, scratch, di.sms, stream);
+  if (mode == kTransposed) return launch_resident<AC4K_SF_TILE128X4, kTransposed>(tm, a, scratch, di.sms, stream);
+  return launch_resident<AC4K_SF_TILE128X4, kTransposedPermuted>(tm, a, scratch, di.sms, stream);
 }
 
 // The CTAs are shared out by the tensors' tiles.
@@ -406,21 +497,22 @@ static int launch_attention(void *const out[3], void *const sf[3], float *const 
   using namespace resident;
   DeviceInfo di;
   if (int e = get_device_info(&di)) return e;
-  if (di.cc_major != 10 || di.sms < 3 || di.sms * 4 > AC4K_QUANTIZE_SCRATCH_BYTES) return kResidentDeclined;
+  if (di.cc_major != 10 || di.sms < 3 || !meetings_fit(di.sms)) return kResidentDeclined;
   CUtensorMap tm[3];
   ResidentArgs a[3];
   int64_t total = 0;
   for (int i = 0; i < 3; ++i) {
     int mode;
-    if (int e = resident_plan(out[i], sf[i], g_out[i], nullptr, in[i], max_scale, shape[i], stride[i], i == 2, AC4K_SF_TILE128X4, &mode, &tm[i], &a[i])) return e;
+    if (int e = resident_plan(out[i], sf[i], g_out[i], in[i], max_scale, shape[i], stride[i], i == 2, AC4K_SF_TILE128X4, &mode, &tm[i], &a[i])) return e;
     if (mode != (i == 2 ? kTransposedPermuted : kRows)) return kResidentDeclined;
     total += a[i].tiles;
   }
   int ctas[3], used = 0, smem = 0;
+  unsigned long long *at = first_word(scratch);
   for (int i = 0; i < 3; ++i) {
     // (rounded down, so that the three fit; at least one)
     ctas[i] = std::min(a[i].tiles, std::max(1, (int)(total <= di.sms ? a[i].tiles : a[i].tiles * (int64_t)(di.sms - 2) / total)));
-    a[i].partial = static_cast<uint32_t *>(scratch) + used;
+    set_meeting(&a[i], at, ctas[i]);
     used += ctas[i];
     const int m = i == 2 ? kTransposedPermuted : kRows;
     a[i].slots = std::min((int)ceil_div(a[i].tiles, ctas[i]), max_slots(m));

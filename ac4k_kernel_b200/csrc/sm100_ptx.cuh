@@ -1,6 +1,6 @@
 // Thin inline-PTX wrappers for the sm_100a features the GEMM uses: mbarrier, TMA (tiled and
 // linear bulk copies), tensor memory allocation, tcgen05.mma / cp / ld / commit / fences.
-// Every wait is bounded: it gives up after kWaitTimeoutNs and reports through its return value.
+// Every wait is bounded: it gives up after the limit it is given (kWaitTimeoutNs) and reports through its return value.
 #pragma once
 
 #include <stdint.h>
@@ -55,6 +55,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
       if (mbar_try_wait(bar, parity)) return true;
     if (globaltimer() - t0 > limit_ns) return false;
   }
+}
+
+// words in global memory that CTAs of one grid write for each other
+__device__ __forceinline__ void st_relaxed_gpu_u64(unsigned long long *p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_relaxed_gpu_u64(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
 }
 
 // generic-proxy writes to shared memory -> visible to the async proxy (TMA, tcgen05.cp/mma)

@@ -59,11 +59,12 @@ const char *ac4k_version(void);          /* "0.1.0" */
 const char *ac4k_last_error(void);
 
 /* Device-side status word of the current device: 0, or the code left by a kernel whose
- * bounded wait expired (0xA1 TMA producer, 0xA2 MMA issuer, 0xA3 scale warps, 0xA4 epilogue).
+ * bounded wait expired (0xA1 TMA producer, 0xA2 MMA issuer, 0xA3 scale warps, 0xA4 epilogue, 0xA5 meeting of a
+ * grid's CTAs).
  * Synchronises the device.  `clear` != 0 resets the word.  Returns AC4K_ERR_TIMEOUT when such a code is
  * found, 0 when the word is 0.  Launches are asynchronous, so an entry point that enqueued the kernel has
  * long returned 0 by then: this call is the only place where an expired wait is reported, and the outputs of
- * the launch that left the code are undefined.  Every device-side wait (mbarrier, flag) is bounded (2 s) and
+ * the launch that left the code are undefined.  Every device-side wait (mbarrier, flag) is bounded (2 s, 8 s for 0xA5) and
  * the kernel leaves through its normal exit, releasing tensor memory, so the context stays usable. */
 int ac4k_device_status(uint32_t *status_out, int clear);
 

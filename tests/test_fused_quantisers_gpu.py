@@ -6,7 +6,7 @@ import ctypes
 import pytest
 import torch
 
-from tests.helpers import gaussian
+from tests.helpers import dynamic_nvfp4, gaussian, hooks_library
 
 pytestmark = pytest.mark.gpu
 
@@ -78,6 +78,48 @@ def test_one_launch_replayed_and_on_two_streams():
         graph.replay()
         torch.cuda.synchronize()
         assert _same(out, _reference(xs[0], 0, 1, False, "ac4k"))
+
+
+@pytest.mark.parametrize("shape,cross,reduce,swizzle", [((3000, 2048), 0, 1, False), ((4100, 4096), 0, 1, False), ((1, 9000, 16, 128), 3, 1, True)])
+def test_one_launch_meets_over_any_scratch(shape, cross, reduce, swizzle):
+    """The CTAs' words lie in scratch that holds anything, also what a call before left there, and may begin on any multiple of 4; on
+    two streams at once; and in a graph, which is replayed with the words' tag of its capture."""
+    hooks = hooks_library()
+    xs = [(gaussian(shape, seed=i) * (1 + 3 * i)).cuda() for i in range(2)]
+    want = [_reference(x, cross, reduce, swizzle, "ac4k") for x in xs]
+    launches, calls = hooks.ac4k_debug_one_launches(), 0
+    g = torch.Generator().manual_seed(1)
+    for fill in (torch.zeros(1024, dtype=torch.int32), torch.full((1024,), -1, dtype=torch.int32),
+                 torch.randint(-2 ** 31, 2 ** 31 - 1, (1024,), generator=g, dtype=torch.int32)):
+        for offset in (0, 1):
+            scratch = torch.zeros(1026, dtype=torch.int32, device="cuda")
+            scratch[offset:offset + 1024] = fill.cuda()
+            for i in (0, 1, 0):
+                assert _same(dynamic_nvfp4(hooks, xs[i], cross, reduce, swizzle, scratch=scratch[offset:].data_ptr()), want[i])
+                calls += 1
+            assert scratch[offset + 1024:].sum() == 0 and (offset == 0 or scratch[0] == 0)
+    streams = [torch.cuda.Stream() for _ in xs]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(20):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(dynamic_nvfp4(hooks, xs[i], cross, reduce, swizzle))
+                calls += 1
+    torch.cuda.synchronize()
+    assert all(_same(t, want[i]) for i in range(2) for t in got[i])
+    x = xs[0].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs = [dynamic_nvfp4(hooks, x, cross, reduce, swizzle) for _ in range(3)]
+    calls += 3
+    for i in (0, 1, 1, 0):
+        x.copy_(xs[i])
+        for _ in range(10):
+            graph.replay()
+        torch.cuda.synchronize()
+        assert all(_same(t, want[i]) for t in outs)
+    assert hooks.ac4k_debug_one_launches() == launches + calls        # none took another route
 
 
 def _attention_operands(q, k, v, h_dim, n_dim):

@@ -16,6 +16,8 @@ import os
 import pytest
 import torch
 
+from tests.helpers import dynamic_nvfp4, gaussian, hooks_library
+
 pytestmark = pytest.mark.gpu
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -69,4 +71,34 @@ def test_expired_wait_reports_status_and_context_survives():
     assert torch.equal(out2, want)
     # ... and so does the shipped library, which shares the context
     assert torch.equal(ops.linear(a4, asf, ag, b4, bsf, bg), want)
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("shape,cross,reduce,swizzle", [((4100, 4096), 0, 1, False), ((1, 700, 3, 128), 3, 1, True), ((1, 9000, 16, 128), 3, 1, False)])
+def test_expired_meeting_of_the_one_launch_quantiser(shape, cross, reduce, swizzle):
+    """The CTAs of the one-launch quantiser wait for one another's maxima: one that does not come ends the wait of all the others at their
+    limit, a code is left, and the next call, on the same scratch, is right."""
+    from ac4k_kernel_b200 import _lib, ops
+    hooks = hooks_library()
+    x = gaussian(shape, seed=3).cuda()
+    want = ops.quant.Ac4kQuantizeOp()(x, cross, reduce, swizzle=swizzle)
+    scratch = torch.full((1024,), -1, dtype=torch.int32, device="cuda")
+    status = ctypes.c_uint32(0)
+    assert hooks.ac4k_device_status(ctypes.byref(status), 1) == 0 and status.value == 0
+    launches = hooks.ac4k_debug_one_launches()
+    try:
+        hooks.ac4k_debug_set_wait_ns(3_000_000)
+        hooks.ac4k_debug_set_flags(0x400)                # the last CTA writes no maximum
+        dynamic_nvfp4(hooks, x, cross, reduce, swizzle, scratch=scratch.data_ptr())
+        rc = hooks.ac4k_device_status(ctypes.byref(status), 1)
+    finally:
+        hooks.ac4k_debug_set_flags(0)
+        hooks.ac4k_debug_set_wait_ns(0)
+    assert rc == -7 and status.value == 0xA5, (rc, hex(status.value))
+    assert b"meeting of a grid" in hooks.ac4k_last_error()
+    got = dynamic_nvfp4(hooks, x, cross, reduce, swizzle, scratch=scratch.data_ptr())
+    assert hooks.ac4k_debug_one_launches() == launches + 2
+    assert hooks.ac4k_device_status(ctypes.byref(status), 1) == 0 and status.value == 0
+    for a, b in zip(got, want):
+        assert torch.equal(a.reshape(-1).view(torch.uint8), b.reshape(-1).view(torch.uint8))
     assert _lib.device_status() == 0
