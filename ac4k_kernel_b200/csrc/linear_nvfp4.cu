@@ -637,6 +637,8 @@ using namespace ac4k;
 //                               the waits for it expire (the wait-expiry test)
 //                               0x400 the last CTA of a tensor in the one-launch quantiser does not write its word, so that the
 //                               others' meeting expires
+//                               0x800 the last CTA of a tensor there begins to load one and a half limits late, when the waits for
+//                               its first tile have expired
 //   ac4k_debug_set_wait_ns(ns)  limit of the device-side waits of later launches (0 = the default 2 s)
 //   ac4k_debug_one_launches()   launches of the one-launch NVFP4 quantiser so far (quantize_nvfp4_resident.cu)
 //   ac4k_debug_set_trace(ptr)   device buffer for the clock stamps of builds with -DAC4K_TRACE_ENABLED

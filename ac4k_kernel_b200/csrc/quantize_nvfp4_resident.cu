@@ -13,7 +13,7 @@
 //
 // The meeting.  Every CTA of a tensor leaves its maximum in a word of its own, {48-bit tag of the launch, maximum}; CTA 0 waits for all
 // of them and answers each CTA in a second word of that CTA, with the maximum of all or, where one did not come within the
-// launch's limit, with kNoMaximum; the others wait for that answer, for twice as long.  The words are in the call's scratch, whose contents
+// launch's limit or gave up on a load, with kNoMaximum; the others wait for that answer, for twice as long.  The words are in the call's scratch, whose contents
 // are undefined: a tag is not repeated in a process and starts at a random number, so that a word that has not been written yet does not
 // have it (2^-48).  A captured launch is replayed with the same tag, so no word may keep it: each has one reader, which clears it, and
 // a CTA without an answer clears what it left itself.  (All CTAs polling all words: 2 - 3 us longer, 148 readers on the same ten lines.)
@@ -107,9 +107,15 @@ __device__ __forceinline__ bool wait_tagged(unsigned long long *word, unsigned l
   return true;
 }
 
-// One tensor by `ctas` CTAs of the grid, of which this is number `cta`.
+// The way out of a wait that expired: the CTA's copies in flight get another limit to land in, before its shared memory is given back.
+// (Waiting for each of them on its barrier, by any count of what was issued, cost 2 - 4 % of every call: 4100 x 4096 15.9 -> 16.6 us.)
+__device__ __forceinline__ void land_copies(unsigned long long limit_ns) {
+  for (const unsigned long long t0 = globaltimer(); globaltimer() - t0 < limit_ns;) {}
+}
+
+// One tensor by `ctas` CTAs of the grid, of which this is number `cta`; false where a wait expired.
 template <int SF_LAYOUT, int MODE>
-__device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const ResidentArgs &p, int cta, int ctas) {
+__device__ __forceinline__ bool resident_quantize(const CUtensorMap &tma, const ResidentArgs &p, int cta, int ctas) {
   using namespace resident;
   constexpr int TEAMS = teams(MODE), TEAM_WARPS = kWarps / TEAMS;
   extern __shared__ uint8_t smem_raw[];
@@ -166,6 +172,8 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
   if (warp == kWarps) {
     const uint32_t el = elect_one();
     Tile t(first, p);
+    if (AC4K_DBG(p, 0x800) && cta == ctas - 1)
+      for (const unsigned long long t0 = globaltimer(); globaltimer() - t0 < p.wait_ns + p.wait_ns / 2;) {}
     for (int i = 0, s = 0, u = 0; i < n && ok; ++i) {
       if (u > 0) ok = warp_all(mbar_wait(empty + 8 * s, (u - 1) & 1, p.wait_ns));
       if (ok) issue(el, t, s);
@@ -192,7 +200,9 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
   // the maximum over the CTA, then over the CTAs of the tensor
   {
     uint32_t m = __reduce_max_sync(0xFFFFFFFFu, max(m2 & 0xFFFFu, m2 >> 16));
-    if (lane == 0) s_m[warp] = m;
+    // (a warp that gave up has not seen every tile: what the CTA leaves is not a maximum then, and no CTA goes on)
+    if (!ok && lane == 0) atomicExch(p.status, warp == kWarps ? kStatusTimeoutProducer : kStatusTimeoutEpilogue);
+    if (lane == 0) s_m[warp] = ok ? m : kNoMaximum;
     __syncthreads();
     if (warp == 0) {
       m = __reduce_max_sync(0xFFFFFFFFu, lane <= kWarps ? s_m[lane] : 0u);
@@ -226,7 +236,7 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
     __syncthreads();
     m = s_all[0];
   }
-  if (m == kNoMaximum) return;
+  if (m == kNoMaximum) return false;
   if (warp == kWarps) {
     const uint32_t el = elect_one();
     if (n > S) {
@@ -241,7 +251,7 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
       }
     }
     if (!ok && lane == 0) atomicExch(p.status, kStatusTimeoutProducer);
-    return;
+    return ok;
   }
   const float g = global_scale_of(m, p.max_scale), alpha = alpha_of(g);
   if ((cta | threadIdx.x) == 0) *p.g_out = g;
@@ -333,12 +343,13 @@ __device__ __forceinline__ void resident_quantize(const CUtensorMap &tma, const 
     }
   }
   if (!ok && lane == 0) atomicExch(p.status, kStatusTimeoutEpilogue);
+  return ok;
 }
 
 template <int SF_LAYOUT, int MODE>
 __global__ void __launch_bounds__(resident::kThreads, 1)
 nvfp4_quantize_resident_kernel(const __grid_constant__ CUtensorMap tma, const ResidentArgs p) {
-  resident_quantize<SF_LAYOUT, MODE>(tma, p, blockIdx.x, gridDim.x);
+  if (!resident_quantize<SF_LAYOUT, MODE>(tma, p, blockIdx.x, gridDim.x)) land_copies(p.wait_ns);
 }
 // q, k and v of the attention operator, each with a share of the grid and a meeting of its own, in one launch.
 template <int SF_LAYOUT>
@@ -347,9 +358,11 @@ nvfp4_quantize_attention_kernel(const __grid_constant__ CUtensorMap tma_q, const
                                 const __grid_constant__ CUtensorMap tma_v, const ResidentArgs q, const ResidentArgs k, const ResidentArgs v,
                                 int ctas_q, int ctas_k) {
   const int cta = blockIdx.x;
-  if (cta < ctas_q) resident_quantize<SF_LAYOUT, resident::kRows>(tma_q, q, cta, ctas_q);
-  else if (cta < ctas_q + ctas_k) resident_quantize<SF_LAYOUT, resident::kRows>(tma_k, k, cta - ctas_q, ctas_k);
-  else resident_quantize<SF_LAYOUT, resident::kTransposedPermuted>(tma_v, v, cta - ctas_q - ctas_k, (int)gridDim.x - ctas_q - ctas_k);
+  bool ok;
+  if (cta < ctas_q) ok = resident_quantize<SF_LAYOUT, resident::kRows>(tma_q, q, cta, ctas_q);
+  else if (cta < ctas_q + ctas_k) ok = resident_quantize<SF_LAYOUT, resident::kRows>(tma_k, k, cta - ctas_q, ctas_k);
+  else ok = resident_quantize<SF_LAYOUT, resident::kTransposedPermuted>(tma_v, v, cta - ctas_q - ctas_k, (int)gridDim.x - ctas_q - ctas_k);
+  if (!ok) land_copies(q.wait_ns);
 }
 
 // 48 bits, not 0, not repeated within 2^48 launches of the process
