@@ -547,6 +547,19 @@ static int launch_attention(void *const out[3], void *const sf[3], float *const 
 
 using namespace ac4k;
 
+// The elements lie side by side in some order of the dimensions: ac4k_quantize_nvfp4_dynamic takes the maximum of as many from `in` on
+static bool is_dense(const int64_t shape[4], const int64_t stride[4]) {
+  int order[4] = {0, 1, 2, 3};
+  std::sort(order, order + 4, [&](int a, int b) { return stride[a] < stride[b]; });
+  int64_t next = 1;
+  for (int i : order) {
+    if (shape[i] == 1) continue;
+    if (stride[i] != next) return false;
+    next *= shape[i];
+  }
+  return true;
+}
+
 extern "C" int ac4k_attention_quantize_nvfp4(void *const out[3], void *const sf[3], float *const g_out[3], void *scratch, const void *const in[3],
                                              const int64_t stride[3][4], int64_t B, int64_t H, int64_t Nq, int64_t Nkv, int64_t D, int64_t Dv,
                                              ac4k_stream_t stream) {
@@ -567,6 +580,8 @@ extern "C" int ac4k_attention_quantize_nvfp4(void *const out[3], void *const sf[
       return fail(AC4K_ERR_ALIGN, "out must be 8-byte, sf 4-byte and in 2-byte aligned");
   const int e = launch_attention(out, sf, g_out, scratch, in, shape, st, kMaxScale, static_cast<cudaStream_t>(stream));
   if (e != kResidentDeclined) return e;
+  for (int i = 0; i < 3; ++i)
+    if (!is_dense(shape[i], st[i])) return fail(AC4K_ERR_SHAPE, "operand %d is not dense, and the one launch does not take its address or strides", i);
   for (int i = 0; i < 3; ++i)
     if (int rc = ac4k_quantize_nvfp4_dynamic(out[i], sf[i], g_out[i], scratch, in[i], kMaxScale, shape[i], st[i], i == 2, AC4K_SF_TILE128X4, stream)) return rc;
   return 0;

@@ -95,7 +95,9 @@ int ac4k_quantize_nvfp4_dynamic(void *out, void *sf, float *g_out, void *scratch
 
 /* The three NVFP4 quantisers in front of ac4k_mha_nvfp4_fwd (128x4 scales, v permuted along the keys), in one launch where their
  * strides allow it: out, sf, g_out, in and stride of q [B, H, Nq, D], k [B, H, Nkv, D] and v [B, H, Nkv, Dv], strides in elements and in
- * that order.  Same bytes as three calls of ac4k_quantize_nvfp4_dynamic; scratch as there, for the three. */
+ * that order.  Same bytes as three calls of ac4k_quantize_nvfp4_dynamic; scratch as there, for the three.
+ * An operand is dense (see ac4k_quantize_nvfp4_dynamic), or a view that the one launch takes: 16-byte aligned, D and Dv contiguous, the
+ * other strides positive multiples of 8 elements.  A call with any other view returns AC4K_ERR_SHAPE and launches nothing. */
 int ac4k_attention_quantize_nvfp4(void *const out[3], void *const sf[3], float *const g_out[3], void *scratch, const void *const in[3],
                                   const int64_t stride[3][4], int64_t B, int64_t H, int64_t Nq, int64_t Nkv, int64_t D, int64_t Dv,
                                   ac4k_stream_t stream);

@@ -123,7 +123,7 @@ def test_one_launch_meets_over_any_scratch(shape, cross, reduce, swizzle):
 
 
 def _attention_operands(q, k, v, h_dim, n_dim):
-    from ac4k_kernel_b200._lib import LIB
+    from ac4k_kernel_b200._lib import LIB, last_error
     b, h, d, dv = q.shape[0], q.shape[h_dim], q.shape[3], v.shape[3]
     nq, nkv = q.shape[n_dim], k.shape[n_dim]
     dev = {"device": "cuda"}
@@ -138,7 +138,7 @@ def _attention_operands(q, k, v, h_dim, n_dim):
     rc = LIB.ac4k_attention_quantize_nvfp4(pointers([m[0] for m in made]), pointers([m[1] for m in made]), pointers([m[2] for m in made]),
                                            scratch.data_ptr(), pointers([q, k, v]), strides, b, h, nq, nkv, d, dv,
                                            torch.cuda.current_stream().cuda_stream)
-    assert rc == 0
+    assert rc == 0, last_error()
     return made
 
 
@@ -155,6 +155,36 @@ def test_attention_operands(layout, b, h, nq, nkv, d, dv):
     got = _attention_operands(q, k, v, h_dim, n_dim)
     for t, (x, cross, reduce, swizzle) in zip(got, ((q, n_dim, 3, False), (k, n_dim, 3, False), (v, 3, n_dim, True))):
         assert _same(t, _reference(x, cross, reduce, swizzle, "128x4"))
+
+
+@pytest.mark.parametrize("d,taken", [(128, True), (100, False), (65, False)])
+def test_attention_operands_of_a_fused_projection(d, taken):
+    """q, k and v as views into one tensor: right where one launch takes them, refused where the calls it stands for would have taken
+    the maximum of other elements"""
+    qkv = (gaussian((2, 130, 3, 5, d), seed=d) * torch.tensor([1.0, 4.0, 9.0]).view(1, 1, 3, 1, 1)).bfloat16().cuda()
+    views = [qkv[:, :, i] for i in range(3)]
+    if not taken:
+        with pytest.raises(AssertionError, match="is not dense"):
+            _attention_operands(*views, 2, 1)
+        return
+    for t, want in zip(_attention_operands(*views, 2, 1), _attention_operands(*[v.contiguous() for v in views], 2, 1)):
+        assert _same(t, want)
+
+
+@pytest.mark.parametrize("view", ["one past the start", "every other row", "a head for all", "turned"])
+def test_attention_operands_that_are_no_dense_tensors(view):
+    """the check for a dense operand, against views of every kind with strides that no tensor map takes"""
+    x = gaussian((2, 66, 6, 70), seed=1).cuda()
+    dense = gaussian((2, 33, 3, 36), seed=2).cuda()
+    v = {"one past the start": x.flatten()[1:1 + dense.numel()].view(dense.shape), "every other row": x[:, ::2, :3, :36],
+         "a head for all": dense[:, :, :1].expand(-1, -1, 3, -1), "turned": dense.transpose(1, 2).contiguous().transpose(1, 2)}[view]
+    if view in ("one past the start", "turned"):
+        got = _attention_operands(v, v, v, 2, 1)
+        want = _attention_operands(*[v.clone(memory_format=torch.contiguous_format)] * 3, 2, 1)
+        assert all(_same(a, b) for a, b in zip(got, want))
+    else:
+        with pytest.raises(AssertionError, match="is not dense"):
+            _attention_operands(v, v, v, 2, 1)
 
 
 @pytest.mark.parametrize("layout", ["BNHD", "BHND"])
