@@ -431,3 +431,28 @@ def quantize_int8_block(out, scale, input, layout, block_size, sub=None):
         check(LIB.ac4k_quantize_int8_block(out.data_ptr(), scale.data_ptr(), x.data_ptr(), _I64x4(B, H, N, D),
                                            _I64x4(*x.stride()), int(block_size), sub_ptr, sub_strides, _stream(input)),
               "quantize_int8_block")
+
+
+ATTENTION_MEAN_TOKENS = 1024
+
+
+def attention_quantize_int8(q8, q_sf, k8, k_sf, v8, v_sf, q, k, v, layout):
+    """The quantisers of `attention(precision="int8+fp8e4m3")` for up to ATTENTION_MEAN_TOKENS keys, in one call: q in blocks of 64
+    tokens, k less its mean over the tokens in blocks of 128, v per channel along the keys (permuted, maximum 2.25).  q, k, v: bf16 in
+    `layout`, any strides; outputs as of `quantize_int8_block` and `quantize_fp8`, all allocated before the call."""
+    _require(layout in ("BNHD", "BHND"), f"Unsupported layout: {layout}")
+    x = [t.permute(0, 2, 1, 3) if layout == "BNHD" else t for t in (q, k, v)]
+    for t, nm in zip(x, ("q", "k", "v")):
+        _require(t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 4, f"{nm} must be a 4D bfloat16 CUDA tensor")
+    (B, H, Nq, D), Nkv, Dv = x[0].shape, x[1].size(2), x[2].size(3)
+    _require(list(x[1].shape) == [B, H, Nkv, D] and list(x[2].shape) == [B, H, Nkv, Dv], "q / k / v shapes do not match")
+    for t, dt, want, nm in ((q8, torch.int8, [B, H, Nq, _align_up(D, 16)], "q8"), (q_sf, torch.float32, [B, H, _ceil_div(Nq, 64)], "q_sf"),
+                            (k8, torch.int8, [B, H, Nkv, _align_up(D, 16)], "k8"), (k_sf, torch.float32, [B, H, _ceil_div(Nkv, 128)], "k_sf"),
+                            (v8, torch.float8_e4m3fn, [B, H, Dv, _align_up(Nkv, 16)], "v8"), (v_sf, torch.float32, [B, H, _align_up(Dv, 16)], "v_sf")):
+        _check_tensor(t, dt, nm)
+        _require(list(t.shape) == want, f"{nm} has an invalid shape")
+    with torch.cuda.device(q.device):
+        check(LIB.ac4k_attention_quantize_int8(q8.data_ptr(), q_sf.data_ptr(), k8.data_ptr(), k_sf.data_ptr(), v8.data_ptr(), v_sf.data_ptr(),
+                                               x[0].data_ptr(), _I64x4(*x[0].stride()), x[1].data_ptr(), _I64x4(*x[1].stride()),
+                                               x[2].data_ptr(), _I64x4(*x[2].stride()), None, None, B, H, Nq, Nkv, D, Dv, _stream(q)),
+              "attention_quantize_int8")

@@ -14,6 +14,7 @@ import torch
 from .. import _cuda_ops
 from ..native import host_calls
 from .quant import quantize
+from .utils import align_up, ceil_div
 
 mha_nvfp4_fwd = _cuda_ops.mha_nvfp4_fwd
 mha_int8_x_fp8_fwd = _cuda_ops.mha_int8_x_fp8_fwd
@@ -39,6 +40,18 @@ def _int8_quantize(x, layout, dim, type="token", BLOCK_SIZE=64, HDIM_ALIGN=16, s
     return y, scale
 
 
+def _one_mean_kernel(q, k, v, n_dim, blocks):
+    """What the native host side hands to one call of the library (csrc/host_calls.cc), which also takes the mean of the keys: the sums
+    in another order than torch's may differ by a bit of bf16, so both paths take the same one."""
+    h_dim = 3 - n_dim
+    if blocks != (64, 128) or any(t.dtype != torch.bfloat16 or not t.is_cuda or t.device != q.device for t in (q, k, v)):
+        return False
+    if any(t.shape[i] != q.shape[i] for t in (k, v) for i in (0, h_dim)) or v.shape[n_dim] != k.shape[n_dim] or k.shape[3] != q.shape[3]:
+        return False
+    return (min(q.numel(), k.numel(), v.numel()) > 0 and k.shape[n_dim] <= _cuda_ops.ATTENTION_MEAN_TOKENS and max(q.shape[3], v.shape[3]) <= 128
+            and v.is_contiguous())
+
+
 def _int8_x_fp8_attention(q, k, v, layout, Q_QUANTIZE_BLOCK_SIZE=64, K_QUANTIZE_BLOCK_SIZE=128, out=None):
     assert layout in ["BNHD", "BHND"], f"Unsupported layout: {layout}"
     B, Dqk = q.shape[0], q.shape[-1]
@@ -50,10 +63,18 @@ def _int8_x_fp8_attention(q, k, v, layout, Q_QUANTIZE_BLOCK_SIZE=64, K_QUANTIZE_
     n_dim = 1 if layout == "BNHD" else 2
     # k - mean(k): softmax is invariant to it and it shrinks the range INT8 has to cover (attention.py:157); the
     # subtraction happens inside the K quantiser
-    k_mean = k.mean(dim=n_dim, keepdim=True)
-    q_int8, q_sf = _int8_quantize(q, layout, n_dim, BLOCK_SIZE=Q_QUANTIZE_BLOCK_SIZE)
-    k_int8, k_sf = _int8_quantize(k, layout, n_dim, BLOCK_SIZE=K_QUANTIZE_BLOCK_SIZE, sub=k_mean)
-    v_fp8, v_sf = quantize(v, 3, n_dim, swizzle=True, max_scale=2.25, precision="fp8e4m3")
+    if _one_mean_kernel(q, k, v, n_dim, (Q_QUANTIZE_BLOCK_SIZE, K_QUANTIZE_BLOCK_SIZE)):
+        Nkv, D16 = k.shape[n_dim], align_up(Dqk, 16)
+        q_int8, k_int8 = (torch.empty((B, H, n, D16), dtype=torch.int8, device=q.device) for n in (Nq, Nkv))
+        q_sf, k_sf = (torch.empty((B, H, ceil_div(n, b)), dtype=torch.float32, device=q.device) for n, b in ((Nq, 64), (Nkv, 128)))
+        v_fp8 = torch.empty((B, H, Dv, align_up(Nkv, 16)), dtype=torch.float8_e4m3fn, device=q.device)
+        v_sf = torch.empty((B, H, align_up(Dv, 16)), dtype=torch.float32, device=q.device)
+        _cuda_ops.attention_quantize_int8(q_int8, q_sf, k_int8, k_sf, v_fp8, v_sf, q, k, v, layout)
+    else:
+        k_mean = k.mean(dim=n_dim, keepdim=True)
+        q_int8, q_sf = _int8_quantize(q, layout, n_dim, BLOCK_SIZE=Q_QUANTIZE_BLOCK_SIZE)
+        k_int8, k_sf = _int8_quantize(k, layout, n_dim, BLOCK_SIZE=K_QUANTIZE_BLOCK_SIZE, sub=k_mean)
+        v_fp8, v_sf = quantize(v, 3, n_dim, swizzle=True, max_scale=2.25, precision="fp8e4m3")
     if out is None:
         out_shape = (B, Nq, H, Dv) if layout == "BNHD" else (B, H, Nq, Dv)
         out = torch.empty(out_shape, dtype=torch.bfloat16, device=q.device)

@@ -37,6 +37,12 @@ def test_no_measurement_switches_in_the_default_build():
     assert "ac4k_debug" not in exported
 
 
+def test_constants_are_those_of_the_header():
+    from ac4k_kernel_b200 import _cuda_ops
+    text = open(os.path.join(ROOT, "include", "ac4k_b200.h")).read()
+    assert f"#define AC4K_ATTENTION_MEAN_TOKENS {_cuda_ops.ATTENTION_MEAN_TOKENS}\n" in text
+
+
 def test_module_mirrors_reference_names():
     import ac4k_kernel_b200 as pkg
     from ac4k_kernel_b200 import _cuda_ops

@@ -222,6 +222,20 @@ def test_attention_same_bits(both_paths, nq, nkv, d, dv, precision):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,d", [(1024, 128), (1000, 65), (515, 96), (100, 128)])
+def test_attention_takes_one_mean(both_paths, n, d):
+    """The keys' mean is a sum in fp32 that is rounded to bf16: of this many means, sums in two orders round some differently"""
+    from ac4k_kernel_b200 import ops
+    for seed in range(4):
+        k = (gaussian((4, n, 40, d), seed=seed).float() * 2 + 3).bfloat16().cuda()
+        q, v = gaussian((4, 64, 40, d), seed=seed + 10).cuda(), gaussian((4, n, 40, d), seed=seed + 20).cuda()
+        assert _same(*both_paths(lambda: ops.attention(q, k, v)))
+        turned = [t.transpose(1, 2).contiguous() for t in (q, k, v)]
+        assert _same(*both_paths(lambda: ops.attention(*turned, layout="BHND")))
+        assert _same(*both_paths(lambda: ops.attention(q[:, :, :1].expand(-1, -1, 40, -1), k[..., :1].expand(-1, -1, -1, d), v)))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("shape,cross,reduce,swizzle", [((50, 8192), 0, 1, False), ((666, 4096), 0, 1, False), ((2049, 4096), 0, 1, False), ((16, 8192), 0, 1, False),
                                                         ((2, 100, 3, 128), 3, 1, True), ((2, 33, 3, 65), 3, 1, True), ((4100, 4096), 0, 1, False)])
 def test_dynamic_entry_with_and_without_scratch(shape, cross, reduce, swizzle):
