@@ -641,6 +641,7 @@ using namespace ac4k;
 //                               its first tile have expired
 //   ac4k_debug_set_wait_ns(ns)  limit of the device-side waits of later launches (0 = the default 2 s)
 //   ac4k_debug_one_launches()   launches of the one-launch NVFP4 quantiser so far (quantize_nvfp4_resident.cu)
+//   ac4k_debug_takes_one_launch(...)  the rule that sends a call there (quantize_nvfp4.cu)
 //   ac4k_debug_set_trace(ptr)   device buffer for the clock stamps of builds with -DAC4K_TRACE_ENABLED
 #ifdef AC4K_DEBUG_HOOKS
 static int g_force_bn = 0;

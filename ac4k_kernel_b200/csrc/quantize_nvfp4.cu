@@ -709,6 +709,33 @@ static int launch_reduction(unsigned blocks, const uint16_t *x, int64_t n, uint3
   return launch_kernel<OVERLAP>(amax_partial_kernel, dim3(blocks), 512, 0, stream, x, n, partial);
 }
 
+// Whether the one-launch kernel of quantize_nvfp4_resident.cu is asked (it may still decline).  One launch / two, us, calls in a graph:
+//   columns contiguous (attention's V): always.  V of [1, 16384, 16, 128] 26.7 / 50.6, [1, 75600, 40, 128] 297 / 450, [1, 1000, 16, 128]
+//     5.1 / 12.7, [1, 104, 8, 128] 4.1 / 6.2; 16 keys, an eighth of a tile, [1, 16, 400, 128] 7.7 / 8.7; eight channels, [1, 1000, 16, 8] 4.9 / 6.9
+//   rows, four to seven of its tiles an SM, or 2^24 to 2^25 elements.  1000 x 5120 7.2 / 9.4, 2048 x 4096 8.6 / 11.0, 4100 x 4096
+//     15.9 / 22.6, 8192 x 4096 28.2 / 32.7.  Below, 666 x 4096 has the flat kernel (5.2; 800 x 4096 6.6 / 5.3).  Between and
+//     above, one launch is the faster one too since its CTAs meet without a grid barrier (3000 x 4096 12.6 / 13.3, 4096 x 4096 15.1 / 16.2, 12000 x
+//     4096 42.1 / 45.1): the lines are where they were drawn before that
+//   and of these not where most of a tile would be padding: a tile has 128 rows of one matrix.  With a third of them used they are even
+//     (64 matrices of 1024 columns, 48 rows 8.0 / 8.3, 32 rows 8.1 / 7.5, 16 rows 7.8 / 6.8; four rows of 4096 x 2048 553 / 215; one row of 2^25
+//     2200 / 791), and from 36 tiles an SM on with three quarters (2048 columns, 65 rows: 28 tiles an SM 23.6 / 25.9, 43 33.3 / 32.9, 54 41.5 /
+//     38.4; 1024 columns, 100 rows, 32 tiles 29.4 / 31.8).  Rows that the vectorised kernels do not take go through the strided one, which is
+//     so much slower that only the first of the two lines counts (64 rows of 1032 columns, 29 tiles 23.5 / 41; 32 rows of 2056 39.3 / 37.3)
+static bool takes_one_launch(const int64_t shape[4], const int64_t stride[4], int swizzle, bool vec, int sms) {
+  if (swizzle || stride[3] != 1) return true;
+  const int64_t M = shape[2], rows = align_up(M, 128), nbatch = shape[0] * shape[1], numel = nbatch * M * shape[3];
+  const int64_t tiles = nbatch * (rows / 128) * ceil_div(shape[3], 64);
+  if (rows > 3 * M) return false;
+  if (tiles >= 4 * (int64_t)sms && tiles <= 7 * (int64_t)sms) return true;
+  return numel > (1 << 24) && numel <= (1 << 25) && (!vec || 3 * rows <= 4 * M || tiles <= 36 * (int64_t)sms);
+}
+#ifdef AC4K_DEBUG_HOOKS
+// the same for a 16-byte aligned tensor
+extern "C" __attribute__((visibility("default"))) int ac4k_debug_takes_one_launch(const int64_t shape[4], const int64_t stride[4], int swizzle, int sms) {
+  return takes_one_launch(shape, stride, swizzle, rows_vectorised(nullptr, shape, stride, swizzle), sms);
+}
+#endif
+
 extern "C" int ac4k_quantize_nvfp4_dynamic(void *out, void *sf, float *g_out, void *scratch, const void *in, float max_scale,
                                            const int64_t shape[4], const int64_t stride[4], int swizzle, int sf_layout,
                                            ac4k_stream_t stream_) {
@@ -724,11 +751,7 @@ extern "C" int ac4k_quantize_nvfp4_dynamic(void *out, void *sf, float *g_out, vo
   if (int e = get_device_info(&di)) return e;
   // Routes by size (measured on a B200; microseconds of the whole call on resident inputs stand beside the kernels):
   //   whole tensor in the registers of one cluster            one launch
-  //   columns contiguous (attention's V), or four to seven     the one-launch kernel of quantize_nvfp4_resident.cu.  One launch / two, us:
-  //   of its tiles an SM, or 2^24 to 2^25 elements             V of [1, 16384, 16, 128] 30 / 50, [1, 1000, 16, 128] 7.1 / 13.2, [2, 104, 8,
-  //                                                            128] 5.0 / 7.1; rows of 1000 x 5120 8.6 / 9.8, 2048 x 4096 10.3 / 11.0, 4100 x
-  //                                                            4096 18.0 / 21.9, 8192 x 4096 31.0 / 33.5, but 666 x 4096 7.3 / 5.4 (its grid
-  //                                                            barrier), 4096 x 4096 17.5 / 16.4, 8192 x 8192 58.1 / 57.7
+  //   takes_one_launch(), which see                            the one-launch kernel of quantize_nvfp4_resident.cu
   //   up to 2^24 elements                                      maxima per CTA, then a quantiser that reduces them: two launches,
   //                                                            the second one set up under the first
   //   larger                                                   zeroed accumulator + atomic maximum + quantiser: a few hundred
@@ -739,9 +762,7 @@ extern "C" int ac4k_quantize_nvfp4_dynamic(void *out, void *sf, float *g_out, vo
   if (vec && items <= AC4K_QUANTIZE_ONE_LAUNCH_BLOCKS)
     return sf_layout == AC4K_SF_AC4K ? launch_flat<AC4K_SF_AC4K>(out, sf, in, src, shape, stride, items, true, stream)
                                      : launch_flat<AC4K_SF_TILE128X4>(out, sf, in, src, shape, stride, items, true, stream);
-  const int64_t resident_tiles = nbatch * ceil_div(M, 128) * (Kp / 64);
-  if (scratch && (swizzle || stride[3] != 1 || (resident_tiles >= 4 * (int64_t)di.sms && resident_tiles <= 7 * (int64_t)di.sms) ||
-                  (numel > (1 << 24) && numel <= (1 << 25)))) {
+  if (scratch && takes_one_launch(shape, stride, swizzle, vec, di.sms)) {
     const int e = launch_quantize_resident(out, sf, g_out, scratch, in, max_scale, shape, stride, swizzle, sf_layout, stream);
     if (e != kResidentDeclined) return e;
   }
