@@ -1,7 +1,9 @@
 // BF16 -> NVFP4 with the tensor's own global scale in ONE launch: a cooperative grid of one CTA per SM reduces the tensor to its
 // maximum, meets (see below), and quantises.  The tiles that a CTA read last are still in its shared memory then (up to 224 KB
 // an SM, 33 MB of the chip), so a tensor of at most that size is read from memory once; of a larger one the rest is read again from
-// the end backwards, while the L2 still has what was read last.  Same bits as the two-launch route of quantize_nvfp4.cu (same arithmetic).
+// the end backwards, while the L2 still has what was read last.  Same bits as the two-launch route of quantize_nvfp4.cu (same
+// arithmetic; also of a block with a NaN, which is left out of the block's maximum by the kernels for rows of whole blocks, and wins it in the
+// others: kRowsAnyK, for a K that is no multiple of 16, and the transposed forms).
 // What bounds it: the read of the tensor (5.6 TB/s), the meeting, and behind it the issue of some hundred instructions a
 // block by 16 warps; which sizes take it stands at ac4k_quantize_nvfp4_dynamic, with the times of both routes.
 //
@@ -30,7 +32,8 @@ namespace ac4k {
 using namespace ptx;
 
 namespace resident {
-enum { kRows = 0, kTransposed = 1, kTransposedPermuted = 2 };
+enum { kRows = 0, kTransposed = 1, kTransposedPermuted = 2, kRowsAnyK = 3 };
+constexpr bool is_rows(int mode) { return mode == kRows || mode == kRowsAnyK; }
 static constexpr int kTileBytes = 128 * 128;
 static constexpr int kWarps = 16, kThreads = 32 * (kWarps + 1);      // consumers and one producer warp
 static constexpr int kMaxSlots = 14;
@@ -39,10 +42,10 @@ static constexpr int kMiscBytes = 128 * 4 + 2 * 32 * 4 + 2 * kMaxSlots * 8, kSca
 static constexpr uint32_t kNoMaximum = 0xFFFF;        // |x| of bf16 has 15 bits
 // a meeting's place in scratch: a maximum and an answer per CTA
 constexpr int64_t meeting_words(int64_t ctas) { return 2 * ctas; }
-constexpr int teams(int mode) { return mode == kRows ? 1 : 4; }
+constexpr int teams(int mode) { return is_rows(mode) ? 1 : 4; }
 // a slot that is used again belongs to one team (its barriers' parities would be ambiguous to a team that skips a use)
-constexpr int max_slots(int mode) { return mode == kRows ? kMaxSlots : 12; }
-constexpr int smem_bytes(int mode, int slots) { return 1024 + slots * kTileBytes + kMiscBytes + (mode == kRows ? 0 : kScaleBytes); }
+constexpr int max_slots(int mode) { return is_rows(mode) ? kMaxSlots : 12; }
+constexpr int smem_bytes(int mode, int slots) { return 1024 + slots * kTileBytes + kMiscBytes + (is_rows(mode) ? 0 : kScaleBytes); }
 static_assert(smem_bytes(kRows, max_slots(kRows)) <= 227 * 1024 && smem_bytes(kTransposed, max_slots(kTransposed)) <= 227 * 1024, "shared memory overflow");
 static_assert(kWarps < 32, "a lane per warp's maximum");
 static_assert(max_slots(kTransposed) % teams(kTransposed) == 0, "a slot belongs to one team");
@@ -82,6 +85,16 @@ __device__ __forceinline__ uint32_t maxabs_bf16x2(uint32_t a, uint32_t b) {
 __device__ __forceinline__ uint32_t amax_bf16x2(const uint4 &a, const uint4 &b) {
   return abs_bf16x2(maxabs_bf16x2(maxabs_bf16x2(maxabs_bf16x2(a.x, a.y), maxabs_bf16x2(a.z, a.w)),
                                   maxabs_bf16x2(maxabs_bf16x2(b.x, b.y), maxabs_bf16x2(b.z, b.w))));
+}
+// the same with a NaN above every number: the maximum of the bits
+__device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
+  uint32_t m;
+  asm("max.u16x2 %0, %1, %2;" : "=r"(m) : "r"(a), "r"(b));
+  return m;
+}
+__device__ __forceinline__ uint32_t amax_bits(const uint4 &a, const uint4 &b) {
+  return max_u16x2(max_u16x2(max_u16x2(abs_bf16x2(a.x), abs_bf16x2(a.y)), max_u16x2(abs_bf16x2(a.z), abs_bf16x2(a.w))),
+                   max_u16x2(max_u16x2(abs_bf16x2(b.x), abs_bf16x2(b.y)), max_u16x2(abs_bf16x2(b.z), abs_bf16x2(b.w))));
 }
 // e4m3 scale byte of a block, and the multiplier of its elements
 __device__ __forceinline__ uint32_t block_scale_of(float amax, float alpha, const float *s_rcp, float &r) {
@@ -263,7 +276,7 @@ __device__ __forceinline__ bool resident_quantize(const CUtensorMap &tma, const 
     return (((int64_t)b * (rows_sf >> 7) + (row >> 7)) * KT + k64) * 128 + (row & 31) * 4 + ((row & 127) >> 5);
   };
   uint32_t *sf_w = reinterpret_cast<uint32_t *>(p.sf);
-  if (MODE == kRows) {
+  if (is_rows(MODE)) {
     // Four lanes have the blocks of one row and K = 64 step.  A warp's eight rows are those whose scale words are neighbours in
     // the layout (a whole 32-byte sector); rows of neighbouring lanes differ in their swizzle, so that eight lanes read eight
     // different 16-byte columns of shared memory.
@@ -283,7 +296,7 @@ __device__ __forceinline__ bool resident_quantize(const CUtensorMap &tma, const 
       }
       const int row = t.mid * 128 + row_l;
       float r;
-      const uint32_t sb = block_scale_of(hmax_bf16x2_to_f32(amax_bf16x2(v0, v1)), alpha, s_rcp, r);
+      const uint32_t sb = block_scale_of(hmax_bf16x2_to_f32(MODE == kRows ? amax_bf16x2(v0, v1) : amax_bits(v0, v1)), alpha, s_rcp, r);
       uint32_t word = row < p.M ? sb << (8 * blk) : 0u;
       word |= __shfl_xor_sync(0xFFFFFFFFu, word, 1);
       word |= __shfl_xor_sync(0xFFFFFFFFu, word, 2);
@@ -327,7 +340,7 @@ __device__ __forceinline__ bool resident_quantize(const CUtensorMap &tma, const 
         for (int blk = 0; blk < 2; ++blk) {
           const uint32_t *v = pr + 8 * blk;
           float r;
-          bytes |= block_scale_of(amax16_bf16(v), alpha, s_rcp, r) << (8 * blk);
+          bytes |= block_scale_of(hmax_bf16x2_to_f32(amax_bits(make_uint4(v[0], v[1], v[2], v[3]), make_uint4(v[4], v[5], v[6], v[7]))), alpha, s_rcp, r) << (8 * blk);
           cw[2 * blk] = quantize8_x2(v[0], v[1], v[2], v[3], r);
           cw[2 * blk + 1] = quantize8_x2(v[4], v[5], v[6], v[7], r);
         }
@@ -352,15 +365,15 @@ nvfp4_quantize_resident_kernel(const __grid_constant__ CUtensorMap tma, const Re
   if (!resident_quantize<SF_LAYOUT, MODE>(tma, p, blockIdx.x, gridDim.x)) land_copies(p.wait_ns);
 }
 // q, k and v of the attention operator, each with a share of the grid and a meeting of its own, in one launch.
-template <int SF_LAYOUT>
+template <int SF_LAYOUT, int ROWS>
 __global__ void __launch_bounds__(resident::kThreads, 1)
 nvfp4_quantize_attention_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                                 const __grid_constant__ CUtensorMap tma_v, const ResidentArgs q, const ResidentArgs k, const ResidentArgs v,
                                 int ctas_q, int ctas_k) {
   const int cta = blockIdx.x;
   bool ok;
-  if (cta < ctas_q) ok = resident_quantize<SF_LAYOUT, resident::kRows>(tma_q, q, cta, ctas_q);
-  else if (cta < ctas_q + ctas_k) ok = resident_quantize<SF_LAYOUT, resident::kRows>(tma_k, k, cta - ctas_q, ctas_k);
+  if (cta < ctas_q) ok = resident_quantize<SF_LAYOUT, ROWS>(tma_q, q, cta, ctas_q);
+  else if (cta < ctas_q + ctas_k) ok = resident_quantize<SF_LAYOUT, ROWS>(tma_k, k, cta - ctas_q, ctas_k);
   else ok = resident_quantize<SF_LAYOUT, resident::kTransposedPermuted>(tma_v, v, cta - ctas_q - ctas_k, (int)gridDim.x - ctas_q - ctas_k);
   if (!ok) land_copies(q.wait_ns);
 }
@@ -450,7 +463,7 @@ static int resident_plan(void *out, void *sf, float *g_out, const void *in, floa
   int64_t dims[4] = {shape[0], shape[1], M, K}, strides[4] = {stride[0], stride[1], stride[2], stride[3]};
   int64_t n_fast, n_mid;
   if (!swizzle && stride[3] == 1) {
-    *mode = kRows;
+    *mode = K % 16 ? kRowsAnyK : kRows;
     n_fast = Kp / 64;
     n_mid = ceil_div(M, 128);
   } else if (stride[2] == 1) {
@@ -496,15 +509,18 @@ int launch_quantize_resident(void *out, void *sf, float *g_out, void *scratch, c
   if (int e = resident_plan(out, sf, g_out, in, max_scale, shape, stride, swizzle, sf_layout, &mode, &tm, &a)) return e;
   if (sf_layout == AC4K_SF_AC4K) {
     if (mode == kRows) return launch_resident<AC4K_SF_AC4K, kRows>(tm, a, scratch, di.sms, stream);
+    if (mode == kRowsAnyK) return launch_resident<AC4K_SF_AC4K, kRowsAnyK>(tm, a, scratch, di.sms, stream);
     if (mode == kTransposed) return launch_resident<AC4K_SF_AC4K, kTransposed>(tm, a, scratch, di.sms, stream);
     return launch_resident<AC4K_SF_AC4K, kTransposedPermuted>(tm, a, scratch, di.sms, stream);
   }
   if (mode == kRows) return launch_resident<AC4K_SF_TILE128X4, kRows>(tm, a, scratch, di.sms, stream);
+  if (mode == kRowsAnyK) return launch_resident<AC4K_SF_TILE128X4, kRowsAnyK>(tm, a, scratch, di.sms, stream);
   if (mode == kTransposed) return launch_resident<AC4K_SF_TILE128X4, kTransposed>(tm, a, scratch, di.sms, stream);
   return launch_resident<AC4K_SF_TILE128X4, kTransposedPermuted>(tm, a, scratch, di.sms, stream);
 }
 
-// The CTAs are shared out by the tensors' tiles.
+// The CTAs are shared out by the tensors' tiles.  ROWS: the form of q and k.
+template <int ROWS>
 static int launch_attention(void *const out[3], void *const sf[3], float *const g_out[3], void *scratch, const void *const in[3],
                             const int64_t shape[3][4], const int64_t stride[3][4], float max_scale, cudaStream_t stream) {
   using namespace resident;
@@ -517,7 +533,7 @@ static int launch_attention(void *const out[3], void *const sf[3], float *const 
   for (int i = 0; i < 3; ++i) {
     int mode;
     if (int e = resident_plan(out[i], sf[i], g_out[i], in[i], max_scale, shape[i], stride[i], i == 2, AC4K_SF_TILE128X4, &mode, &tm[i], &a[i])) return e;
-    if (mode != (i == 2 ? kTransposedPermuted : kRows)) return kResidentDeclined;
+    if (mode != (i == 2 ? kTransposedPermuted : ROWS)) return kResidentDeclined;
     total += a[i].tiles;
   }
   int ctas[3], used = 0, smem = 0;
@@ -527,11 +543,11 @@ static int launch_attention(void *const out[3], void *const sf[3], float *const 
     ctas[i] = std::min(a[i].tiles, std::max(1, (int)(total <= di.sms ? a[i].tiles : a[i].tiles * (int64_t)(di.sms - 2) / total)));
     set_meeting(&a[i], at, ctas[i]);
     used += ctas[i];
-    const int m = i == 2 ? kTransposedPermuted : kRows;
+    const int m = i == 2 ? kTransposedPermuted : ROWS;
     a[i].slots = std::min((int)ceil_div(a[i].tiles, ctas[i]), max_slots(m));
     smem = std::max(smem, smem_bytes(m, a[i].slots));
   }
-  auto kern = nvfp4_quantize_attention_kernel<AC4K_SF_TILE128X4>;
+  auto kern = nvfp4_quantize_attention_kernel<AC4K_SF_TILE128X4, ROWS>;
   static PerDevice<int> attr_set;
   int unused = 0;
   if (int e = attr_set.get(&unused, [&](int &v) {
@@ -578,7 +594,8 @@ extern "C" int ac4k_attention_quantize_nvfp4(void *const out[3], void *const sf[
   for (int i = 0; i < 3; ++i)
     if ((reinterpret_cast<uintptr_t>(out[i]) & 7) || (reinterpret_cast<uintptr_t>(sf[i]) & 3) || (reinterpret_cast<uintptr_t>(in[i]) & 1))
       return fail(AC4K_ERR_ALIGN, "out must be 8-byte, sf 4-byte and in 2-byte aligned");
-  const int e = launch_attention(out, sf, g_out, scratch, in, shape, st, kMaxScale, static_cast<cudaStream_t>(stream));
+  const auto launch = D % 16 ? &launch_attention<resident::kRowsAnyK> : &launch_attention<resident::kRows>;
+  const int e = launch(out, sf, g_out, scratch, in, shape, st, kMaxScale, static_cast<cudaStream_t>(stream));
   if (e != kResidentDeclined) return e;
   for (int i = 0; i < 3; ++i)
     if (!is_dense(shape[i], st[i])) return fail(AC4K_ERR_SHAPE, "operand %d is not dense, and the one launch does not take its address or strides", i);

@@ -48,13 +48,17 @@ def test_one_launch_columns(shape, swizzle, layout):
     assert _same(ops.quantize(x, 3, 1, swizzle=swizzle, sf_layout=layout), _reference(x, 3, 1, swizzle, layout))
 
 
-@pytest.mark.parametrize("fill", [0.0, float("nan"), float("inf"), 1e-38])
-def test_one_launch_odd_values(fill):
+@pytest.mark.parametrize("fill", [0.0, float("nan"), float("inf"), float("-inf"), 1e-38, -0.0])
+@pytest.mark.parametrize("shape,cross,reduce,swizzle", [((2048, 4096), 0, 1, False), ((4100, 4096), 0, 1, False), ((20000, 1032), 0, 1, False),
+                                                        ((1000, 4808), 0, 1, False), ((1, 700, 3, 128), 3, 1, True), ((1, 5000, 16, 72), 3, 1, False)])
+def test_one_launch_odd_values(shape, cross, reduce, swizzle, fill):
     from ac4k_kernel_b200 import ops
-    x = torch.full((4100, 2048), fill, device="cuda", dtype=torch.bfloat16)
-    assert _same(ops.quantize(x, 0, 1), _reference(x, 0, 1, False, "ac4k"))
-    x[1000:, 512:] = gaussian((3100, 1536), seed=2).bfloat16().cuda()
-    assert _same(ops.quantize(x, 0, 1), _reference(x, 0, 1, False, "ac4k"))
+    x = torch.full(shape, fill, device="cuda", dtype=torch.bfloat16)
+    assert _same(ops.quantize(x, cross, reduce, swizzle=swizzle), _reference(x, cross, reduce, swizzle, "ac4k"))
+    part = tuple(slice(n // 3, None) for n in shape[:-1])
+    x[part] = gaussian(tuple(x[part].shape), seed=2).bfloat16().cuda()
+    x.view(-1)[5::1001] = fill                                     # blocks with one such value
+    assert _same(ops.quantize(x, cross, reduce, swizzle=swizzle), _reference(x, cross, reduce, swizzle, "ac4k"))
 
 
 def test_one_launch_replayed_and_on_two_streams():
@@ -122,8 +126,9 @@ def test_one_launch_meets_over_any_scratch(shape, cross, reduce, swizzle):
     assert hooks.ac4k_debug_one_launches() == launches + calls        # none took another route
 
 
-def _attention_operands(q, k, v, h_dim, n_dim):
+def _attention_operands(q, k, v, h_dim, n_dim, lib=None):
     from ac4k_kernel_b200._lib import LIB, last_error
+    lib = lib or LIB
     b, h, d, dv = q.shape[0], q.shape[h_dim], q.shape[3], v.shape[3]
     nq, nkv = q.shape[n_dim], k.shape[n_dim]
     dev = {"device": "cuda"}
@@ -135,7 +140,7 @@ def _attention_operands(q, k, v, h_dim, n_dim):
     scratch = torch.empty(1024, dtype=torch.int32, **dev)
     pointers = lambda ts: (ctypes.c_void_p * 3)(*[t.data_ptr() for t in ts])
     strides = (ctypes.c_int64 * 12)(*[t.stride(i) for t in (q, k, v) for i in (0, h_dim, n_dim, 3)])
-    rc = LIB.ac4k_attention_quantize_nvfp4(pointers([m[0] for m in made]), pointers([m[1] for m in made]), pointers([m[2] for m in made]),
+    rc = lib.ac4k_attention_quantize_nvfp4(pointers([m[0] for m in made]), pointers([m[1] for m in made]), pointers([m[2] for m in made]),
                                            scratch.data_ptr(), pointers([q, k, v]), strides, b, h, nq, nkv, d, dv,
                                            torch.cuda.current_stream().cuda_stream)
     assert rc == 0, last_error()
@@ -155,6 +160,30 @@ def test_attention_operands(layout, b, h, nq, nkv, d, dv):
     got = _attention_operands(q, k, v, h_dim, n_dim)
     for t, (x, cross, reduce, swizzle) in zip(got, ((q, n_dim, 3, False), (k, n_dim, 3, False), (v, 3, n_dim, True))):
         assert _same(t, _reference(x, cross, reduce, swizzle, "128x4"))
+
+
+@pytest.mark.parametrize("fill", [0.0, float("nan"), float("inf"), float("-inf"), 1e-38])
+@pytest.mark.parametrize("n,nkv,d", [(130, 200, 128), (6000, 5000, 128), (1000, 900, 40)])
+def test_attention_operands_odd_values_on_two_streams(n, nkv, d, fill):
+    """one launch for the three, asserted; n = 6000 uses slots again"""
+    hooks = hooks_library()
+    q, k, v = gaussian((1, n, 16, d), seed=1).cuda(), gaussian((1, nkv, 16, d), seed=2).cuda(), gaussian((1, nkv, 16, d), seed=3).cuda()
+    k[:, nkv // 2:] = fill
+    v[:, :nkv // 3] = fill
+    q.view(-1)[5::1001], k.view(-1)[3::1001], v.view(-1)[7::1001] = fill, fill, fill
+    sets = [(q, k, v), (v.clone(), q[:, :nkv].contiguous() if n >= nkv else k, k.clone())]
+    want = [[_reference(x, *dims, "128x4") for x, dims in zip(s, ((1, 3, False), (1, 3, False), (3, 1, True)))] for s in sets]
+    streams = [torch.cuda.Stream() for _ in sets]
+    launches = hooks.ac4k_debug_one_launches()
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(10):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(_attention_operands(*sets[i], 2, 1, hooks))
+    torch.cuda.synchronize()
+    assert hooks.ac4k_debug_one_launches() == launches + 20
+    assert all(_same(t, w) for i in range(2) for made in got[i] for t, w in zip(made, want[i]))
 
 
 @pytest.mark.parametrize("d,taken", [(128, True), (100, False), (65, False)])
@@ -226,3 +255,21 @@ def test_keys_less_their_mean(layout, b, h, n, d):
             assert ((made[0][3] - made[1][3]).abs() <= moved / 127).all()
             rows = made[0][3].repeat_interleave(128, dim=2)[:, :, :n, None]
             assert ((made[0][2].int() - made[1][2].int()).abs() <= 1 + 2 * moved / rows.clamp(min=1e-30)).all()
+
+
+@pytest.mark.parametrize("fill", [float("nan"), float("inf"), float("-inf"), 3.3895e38, -3.3895e38, 1e-38])
+@pytest.mark.parametrize("n,d", [(100, 65), (640, 128)])
+def test_keys_less_their_mean_odd_values(n, d, fill):
+    """the mean and the codes of a channel with such values, against torch's mean and the quantiser that is given it, bit for bit (the other
+    means are exact)"""
+    from ac4k_kernel_b200 import _cuda_ops
+    from ac4k_kernel_b200.ops.attention import _int8_quantize
+    k = (gaussian((2, n, 3, d), seed=n) * 8).round().bfloat16().cuda()
+    k[0, n // 3, 1, 5], k[0, n - 1, 1, 5], k[1, 0, 2, d - 1], k[1, n // 2] = fill, fill, fill, fill
+    made = []
+    for m, block in ((n, 64), (n, 128)):
+        made += [torch.empty((2, 3, m, (d + 15) // 16 * 16), dtype=torch.int8, device="cuda"), torch.empty((2, 3, (m + block - 1) // block), device="cuda")]
+    made += [torch.empty((2, 3, d, (n + 15) // 16 * 16), dtype=torch.float8_e4m3fn, device="cuda"), torch.empty((2, 3, (d + 15) // 16 * 16), device="cuda")]
+    _cuda_ops.attention_quantize_int8(*made, k, k, k, "BNHD")
+    codes, scales = _int8_quantize(k, "BNHD", 1, BLOCK_SIZE=128, sub=k.mean(dim=1, keepdim=True))
+    assert torch.equal(made[2], codes) and torch.equal(made[3].view(torch.int32), scales.view(torch.int32))
