@@ -23,6 +23,17 @@ def hooks_library():
     return lib
 
 
+def takes_one_launch(shape, cross, reduce, swizzle=False, sms=148):
+    """The library's own rule, for a contiguous 16-byte aligned tensor: whether the call is sent to the one-launch kernel (no GPU needed)"""
+    lib = hooks_library()
+    stride, n = [0] * len(shape), 1
+    for i in reversed(range(len(shape))):
+        stride[i], n = n, n * shape[i]
+    order = [i for i in range(len(shape)) if i not in (cross, reduce)] + [cross, reduce]
+    pad, c = 4 - len(shape), ctypes.c_int64 * 4
+    return bool(lib.ac4k_debug_takes_one_launch(c(*[1] * pad, *[shape[i] for i in order]), c(*[0] * pad, *[stride[i] for i in order]), int(swizzle), sms))
+
+
 def dynamic_nvfp4(lib, x, cross, reduce, swizzle=False, layout="ac4k", scratch=None):
     """ac4k_quantize_nvfp4_dynamic of `lib` on the current stream; scratch: None for one of its own, or a device address"""
     from ac4k_kernel_b200 import _cuda_ops as ct

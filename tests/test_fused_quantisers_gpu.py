@@ -1,12 +1,12 @@
 """The quantisers that do more than one thing in a launch, against the calls that they stand for: the one-launch NVFP4 quantiser and
 the three operands of an attention layer (bit for bit), at the sizes where tiles, slots and shares of the grid change; K less its mean
-in one launch."""
+in one launch.  That a call takes the one launch is asserted, by the debug-hook build's count of them or by the library's rule."""
 import ctypes
 
 import pytest
 import torch
 
-from tests.helpers import dynamic_nvfp4, gaussian, hooks_library
+from tests.helpers import dynamic_nvfp4, gaussian, hooks_library, takes_one_launch
 
 pytestmark = pytest.mark.gpu
 
@@ -26,11 +26,10 @@ def _same(got, want):
 
 
 @pytest.mark.parametrize("layout", ["ac4k", "128x4"])
-@pytest.mark.parametrize("m,k", [
-    (148, 8192), (257, 8192), (2048, 4160), (4096, 4096), (4097, 4112),      # up to a tile per CTA; a ragged tile; what fits on chip and just more
-    (1000, 16384), (12345, 2064), (33000, 1024), (40000, 128), (8192, 8192),   # each slot used again once, and many times
-])
-def test_one_launch_rows(m, k, layout):
+@pytest.mark.parametrize("m,k", [(148, 8192), (257, 8192), (2048, 4160), (4096, 4096), (4097, 4112), (1000, 16384), (12345, 2064), (33000, 1024), (40000, 128),
+                                 (8192, 8192)])
+def test_rows_of_every_route(m, k, layout):
+    """two launches up to 2^24 elements and beyond 2^25, one launch"""
     from ac4k_kernel_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(m + k)
     x = torch.randn((m, k), generator=g, device="cuda", dtype=torch.bfloat16)
@@ -39,12 +38,34 @@ def test_one_launch_rows(m, k, layout):
 
 
 @pytest.mark.parametrize("layout", ["ac4k", "128x4"])
+@pytest.mark.parametrize("shape", [
+    (520, 8192), (1030, 4800), (1900, 4112), (2048, 4096), (64, 48, 1024), (3, 5, 130, 1280),      # four to seven tiles an SM, ragged along either dimension
+    (4097, 4096), (4097, 4112), (5003, 4096), (12345, 2064),      # 14 tiles fit: a few more, each slot used again once
+    (8192, 4096), (32000, 1032), (300001, 64), (1100000, 16),     # and up to four times; rows shorter than a tile
+])
+def test_one_launch_rows(shape, layout):
+    hooks = hooks_library()
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    x = torch.randn(shape, generator=g, device="cuda", dtype=torch.bfloat16)
+    x[..., shape[-2] // 2, shape[-1] // 3].flatten()[-1] = -77.0      # the maximum, once
+    cross, reduce = len(shape) - 2, len(shape) - 1
+    launches = hooks.ac4k_debug_one_launches()
+    got = dynamic_nvfp4(hooks, x, cross, reduce, False, layout)
+    assert hooks.ac4k_debug_one_launches() == launches + 1
+    assert _same(got, _reference(x, cross, reduce, False, layout))
+
+
+@pytest.mark.parametrize("layout", ["ac4k", "128x4"])
 @pytest.mark.parametrize("swizzle", [False, True])
 @pytest.mark.parametrize("shape", [(1, 700, 3, 128), (2, 1031, 5, 64), (1, 5000, 16, 72), (1, 9000, 16, 128), (3, 130, 1, 8)])
 def test_one_launch_columns(shape, swizzle, layout):
     from ac4k_kernel_b200 import ops
+    hooks = hooks_library()
     x = (gaussian(shape, seed=shape[1]) * 2).bfloat16().cuda()
     x[0, shape[1] - 1, 0, 1] = 50.0
+    launches = hooks.ac4k_debug_one_launches()
+    assert _same(dynamic_nvfp4(hooks, x, 3, 1, swizzle, layout), _reference(x, 3, 1, swizzle, layout))
+    assert hooks.ac4k_debug_one_launches() == launches + 1
     assert _same(ops.quantize(x, 3, 1, swizzle=swizzle, sf_layout=layout), _reference(x, 3, 1, swizzle, layout))
 
 
@@ -53,6 +74,7 @@ def test_one_launch_columns(shape, swizzle, layout):
                                                         ((1000, 4808), 0, 1, False), ((1, 700, 3, 128), 3, 1, True), ((1, 5000, 16, 72), 3, 1, False)])
 def test_one_launch_odd_values(shape, cross, reduce, swizzle, fill):
     from ac4k_kernel_b200 import ops
+    assert takes_one_launch(shape, cross, reduce, swizzle, torch.cuda.get_device_properties(0).multi_processor_count)
     x = torch.full(shape, fill, device="cuda", dtype=torch.bfloat16)
     assert _same(ops.quantize(x, cross, reduce, swizzle=swizzle), _reference(x, cross, reduce, swizzle, "ac4k"))
     part = tuple(slice(n // 3, None) for n in shape[:-1])
@@ -61,27 +83,31 @@ def test_one_launch_odd_values(shape, cross, reduce, swizzle, fill):
     assert _same(ops.quantize(x, cross, reduce, swizzle=swizzle), _reference(x, cross, reduce, swizzle, "ac4k"))
 
 
-def test_one_launch_replayed_and_on_two_streams():
-    from ac4k_kernel_b200 import ops
-    xs = [torch.randn((3000, 4096), device="cuda", dtype=torch.bfloat16) for _ in range(2)]
-    want = [_reference(x, 0, 1, False, "ac4k") for x in xs]
+@pytest.mark.parametrize("shape,cross,reduce,swizzle", [((2000, 4096), 0, 1, False), ((4100, 4096), 0, 1, False), ((1, 9000, 16, 128), 3, 1, True)])
+def test_one_launch_replayed_and_on_two_streams(shape, cross, reduce, swizzle):
+    """through the operator: scratch is the allocator's"""
+    from ac4k_kernel_b200 import _lib, ops
+    assert takes_one_launch(shape, cross, reduce, swizzle, torch.cuda.get_device_properties(0).multi_processor_count)
+    xs = [torch.randn(shape, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    want = [_reference(x, cross, reduce, swizzle, "ac4k") for x in xs]
     streams = [torch.cuda.Stream() for _ in xs]
     torch.cuda.synchronize()
     got = [[], []]
     for _ in range(20):
         for i, s in enumerate(streams):
             with torch.cuda.stream(s):
-                got[i].append(ops.quantize(xs[i], 0, 1))
+                got[i].append(ops.quantize(xs[i], cross, reduce, swizzle=swizzle))
     torch.cuda.synchronize()
     assert all(_same(t, want[i]) for i in range(2) for t in got[i])
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
-        out = ops.quantize(xs[0], 0, 1)
+        out = ops.quantize(xs[0], cross, reduce, swizzle=swizzle)
     for scale in (1.0, -3.0, 0.5):
         xs[0].copy_(xs[1] * scale)
         graph.replay()
         torch.cuda.synchronize()
-        assert _same(out, _reference(xs[0], 0, 1, False, "ac4k"))
+        assert _same(out, _reference(xs[0], cross, reduce, swizzle, "ac4k"))
+    assert _lib.device_status() == 0
 
 
 @pytest.mark.parametrize("shape,cross,reduce,swizzle", [((3000, 2048), 0, 1, False), ((4100, 4096), 0, 1, False), ((1, 9000, 16, 128), 3, 1, True)])

@@ -358,3 +358,76 @@ def test_subclasses_are_left_to_the_wrappers(both_paths):
         native, python = both_paths(fn)
         assert type(native) is type(python) and torch.equal(native.as_subclass(torch.Tensor), python.as_subclass(torch.Tensor))
     assert type(ops.quantize(torch.nn.Parameter(x), 0, 1)[0]) is torch.Tensor
+
+
+def _empties(fn, listener):
+    """how many uninitialised tensors the listener saw fn() make"""
+    if listener == "dispatch mode":
+        from torch.utils._python_dispatch import TorchDispatchMode
+        seen = []
+
+        class Mode(TorchDispatchMode):
+            def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+                seen.append(str(func))
+                return func(*args, **(kwargs or {}))
+        with Mode():
+            fn()
+        return sum(name.startswith("aten.empty") for name in seen)
+    if listener == "profiler":
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as p:
+            fn()
+        return sum(e.count for e in p.key_averages() if e.key == "aten::empty")
+    x = torch.zeros(4, device="cuda")
+    if listener == "tracer":
+        graph = torch.jit.trace(lambda t: (fn()[0], t), x, check_trace=False).graph
+        return str(graph).count("aten::empty")
+    from torch.fx.experimental.proxy_tensor import make_fx
+    return make_fx(lambda t: (fn()[0], t))(x).code.count("aten.empty")
+
+
+@pytest.mark.gpu
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("listener,least", [("dispatch mode", 3), ("profiler", 3), ("tracer", 1), ("make_fx", 1)])
+def test_outputs_are_made_where_listeners_see_them(listener, least):
+    """The native host side takes its outputs straight from the allocator's factory only where nothing listens to operator calls"""
+    from ac4k_kernel_b200 import ops
+    from ac4k_kernel_b200.native import host_calls
+    assert host_calls is not None
+    x = gaussian((20, 256), seed=1).cuda()
+    assert _empties(lambda: ops.quantize(x, 0, 1), listener) >= least
+
+
+@pytest.mark.gpu
+@pytest.mark.filterwarnings("ignore")
+def test_under_modes_and_transforms_as_the_wrappers(both_paths):
+    """the same results, the same kind of tensor, or an error on both paths"""
+    from ac4k_kernel_b200 import ops
+    x = gaussian((20, 256), seed=1).cuda()
+    q = gaussian((1, 70, 2, 64), seed=2).cuda()
+    ones = torch.ones(3, device="cuda")
+
+    def all_ops():
+        return (*ops.quantize(x, 0, 1), *ops.quantize(x, 0, 1, precision="int8"), ops.attention(q, q, q), ops.attention(q, q, q, precision="nvfp4"))
+    want = all_ops()
+
+    def inference():
+        with torch.inference_mode():
+            return all_ops()
+    native, python = both_paths(inference)
+    assert _same(native, want) and _same(python, want) and all(a.is_inference() and b.is_inference() for a, b in zip(native, python))
+
+    def deterministic():
+        before = torch.are_deterministic_algorithms_enabled()
+        torch.use_deterministic_algorithms(True, warn_only=True)
+        try:
+            return all_ops()
+        finally:
+            torch.use_deterministic_algorithms(before)
+    assert all(_same(r, want) for r in both_paths(deterministic))
+    for transform in (lambda: torch.func.vmap(lambda y: ops.quantize(x, 0, 1)[2] * y)(ones),
+                      lambda: torch.func.functionalize(lambda y: ops.quantize(x, 0, 1)[2] * y)(ones),
+                      lambda: torch.func.jvp(lambda y: ops.quantize(x, 0, 1)[2] * y, (ones,), (ones,))[0],
+                      lambda: torch.func.grad(lambda y: (ops.quantize(x, 0, 1)[2] * y).sum())(ones),
+                      lambda: torch.func.vmap(lambda y: ops.quantize(y, 0, 1)[2])(torch.stack([x, x]))):
+        native, python = both_paths(transform)
+        assert (isinstance(native, type) and isinstance(python, type)) or torch.equal(native, python), (native, python)

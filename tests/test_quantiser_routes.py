@@ -1,23 +1,10 @@
 """Which calls of the dynamic NVFP4 quantiser are sent to the one-launch kernel: the rule of csrc/quantize_nvfp4.cu itself, on a device of
 148 SMs, through the debug-hook build (no GPU needed)."""
-import ctypes
-
 import pytest
 
-from tests.helpers import hooks_library
+from tests.helpers import takes_one_launch
 
-N24, N25 = 2 ** 24, 2 ** 25
-
-
-def _asked(shape, cross, reduce, swizzle=False, sms=148):
-    hooks = hooks_library()
-    stride, n = [0] * len(shape), 1
-    for i in reversed(range(len(shape))):
-        stride[i], n = n, n * shape[i]
-    order = [i for i in range(len(shape)) if i not in (cross, reduce)] + [cross, reduce]
-    pad = 4 - len(shape)
-    c = ctypes.c_int64 * 4
-    return bool(hooks.ac4k_debug_takes_one_launch(c(*[1] * pad, *[shape[i] for i in order]), c(*[0] * pad, *[stride[i] for i in order]), int(swizzle), sms))
+N25 = 2 ** 25
 
 
 @pytest.mark.parametrize("shape,asked", [
@@ -26,7 +13,7 @@ def _asked(shape, cross, reduce, swizzle=False, sms=148):
     ((1, 4096, 40, 128), False), ((1100000, 16), True), ((40000, 128), True), ((100000, 8), True), ((33000, 1000), True), ((1000000, 24), True),
 ])
 def test_rows_by_their_tiles(shape, asked):
-    assert _asked(shape, len(shape) - 2, len(shape) - 1) == asked
+    assert takes_one_launch(shape, len(shape) - 2, len(shape) - 1) == asked
 
 
 @pytest.mark.parametrize("shape,asked", [
@@ -37,10 +24,10 @@ def test_rows_by_their_tiles(shape, asked):
 ])
 def test_rows_that_leave_most_of_a_tile_empty(shape, asked):
     """two launches where the tiles would be padding: 16 rows a matrix took 7.8 us for 6.8, four 553 for 215, one 2200 for 791"""
-    assert _asked(shape, len(shape) - 2, len(shape) - 1) == asked
+    assert takes_one_launch(shape, len(shape) - 2, len(shape) - 1) == asked
 
 
 @pytest.mark.parametrize("shape,cross,reduce", [((1, 16, 400, 128), 3, 1), ((1, 75600, 40, 128), 3, 1), ((8, 4000), 1, 0), ((4000, 8), 1, 0)])
 @pytest.mark.parametrize("swizzle", [False, True])
 def test_columns(shape, cross, reduce, swizzle):
-    assert _asked(shape, cross, reduce, swizzle)
+    assert takes_one_launch(shape, cross, reduce, swizzle)
