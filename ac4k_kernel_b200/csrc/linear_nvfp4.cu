@@ -694,6 +694,8 @@ static SplitPlan plan_split(int64_t M, int64_t N, int64_t K, int bn, int sms) {
 // one's time, not 0.75: its stages bring 89 bytes per clock into an SM instead of 73.  256 / 192 columns, us, 128x4 scales, as many rounds
 // of either: 129 x 1024 x 512 5.2 / 4.7, 300 x 3072 x 3072 8.9 / 8.4, 666 x 4096 x 4096 11.1 / 10.6 (one round each), 512 x 12288 x
 // 4096 18.4 / 17.2 (two); a fifth round for four: 4096^3 31.4 / 35.3, 2048 x 8192 x 4096 32.3 / 35.2.
+// (Rounds of sms / 2 clusters: as many as the occupancy query admits where every SM has its pair, 74 here; on a part where that is not
+// so a launch may have a round more than this choice counts with.)
 static int pair_tile_columns(int64_t M, int64_t N, int sms) {
   const int64_t tiles_m = ceil_div(M, 256), clusters = sms / 2;
   return ceil_div(tiles_m * ceil_div(N, 192), clusters) == ceil_div(tiles_m * ceil_div(N, 256), clusters) ? 192 : 256;

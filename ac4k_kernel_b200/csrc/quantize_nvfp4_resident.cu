@@ -4,8 +4,9 @@
 // the end backwards, while the L2 still has what was read last.  Same bits as the two-launch route of quantize_nvfp4.cu (same
 // arithmetic; also of a block with a NaN, which is left out of the block's maximum by the kernels for rows of whole blocks, and wins it in the
 // others: kRowsAnyK, for a K that is no multiple of 16, and the transposed forms).
-// What bounds it: the read of the tensor (5.6 TB/s), the meeting, and behind it the issue of some hundred instructions a
-// block by 16 warps; which sizes take it stands at ac4k_quantize_nvfp4_dynamic, with the times of both routes.
+// What bounds it: latency.  16 warps an SM (shared memory leaves room for no more) issue 200 thread-instructions per block of 16 in the rows
+// form, 172 in the transposed ones, 44 % and 39 % of the issue slots, at 2.3 TB/s; the rest is waits for loads, for the meeting and in the
+// chain from a block's words to its codes.  Which sizes take it stands at takes_one_launch() in quantize_nvfp4.cu, with the times of both routes.
 //
 // A tile is 16 KB, one TMA box with the 128-byte swizzle: 128 rows x 64 K-elements of a tensor whose rows are contiguous along K
 // (kRows), or 128 K-elements x 64 rows of one that is contiguous along the rows (kTransposed, kTransposedPermuted: attention's V).
@@ -14,11 +15,12 @@
 // rows x 32 K-elements (a warp reads 32 words of one 128-byte line at a time), and the scale bytes meet in shared memory.
 //
 // The meeting.  Every CTA of a tensor leaves its maximum in a word of its own, {48-bit tag of the launch, maximum}; CTA 0 waits for all
-// of them and answers each CTA in a second word of that CTA, with the maximum of all or, where one did not come within the
-// launch's limit or gave up on a load, with kNoMaximum; the others wait for that answer, for twice as long.  The words are in the call's scratch, whose contents
-// are undefined: a tag is not repeated in a process and starts at a random number, so that a word that has not been written yet does not
-// have it (2^-48).  A captured launch is replayed with the same tag, so no word may keep it: each has one reader, which clears it, and
-// a CTA without an answer clears what it left itself.  (All CTAs polling all words: 2 - 3 us longer, 148 readers on the same ten lines.)
+// of them and answers each CTA in a second word of that CTA, with the maximum of all or, where one did not come within the launch's
+// limit or gave up on a load, with kNoMaximum; the others wait for that answer, for twice as long.  The words are in the call's scratch,
+// whose contents are undefined: a tag is not repeated in a process and starts at a random number, so that a word that has not been written
+// yet does not have it (2^-48).  A captured launch is replayed with the same tag, so no word may keep it: each has one reader, which clears
+// it, and a CTA without an answer clears what it left itself.  (All CTAs polling all words took 2 - 3 us longer, 148 readers on the same
+// ten lines: V of [1, 1000, 16, 128] 9.8 us for 5.1.)
 // That all CTAs of the grid are on the chip together is what a cooperative launch promises (it fails otherwise).  Programmatic
 // serialisation does not take that away: it lets the grid begin when every CTA of the kernel in front has begun, and those wait for
 // nothing of this one.
@@ -284,7 +286,7 @@ __device__ __forceinline__ bool resident_quantize(const CUtensorMap &tma, const 
     const int row_l = SF_LAYOUT == AC4K_SF_AC4K ? warp * 8 + j : (j >> 1) * 32 + 2 * warp + (j & 1);
     const uint32_t at0 = tiles_s + row_l * 128 + (((2 * blk) ^ (row_l & 7)) << 4), at1 = tiles_s + row_l * 128 + (((2 * blk + 1) ^ (row_l & 7)) << 4);
     // (several tiles side by side in one thread, to fill the chain from a block's words to its codes, gained nothing where the tiles
-    // are there already and took twice as long where they are loaded again: 8192 x 8192 86 us against 57)
+    // are there already and took half as long again where they are loaded again: 8192 x 8192 86 us against 57)
     Tile t(first + n - 1, p);
     for (int q = 0, s = s_last, u = u_last; q < n; ++q) {
       ok = warp_all(mbar_wait(full + 8 * s, u & 1, p.wait_ns));
